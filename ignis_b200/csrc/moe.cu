@@ -502,236 +502,7 @@ __global__ void __launch_bounds__(kThreads, NT <= 2 ? 3 : 2) moe_experts_kernel(
   }
 }
 
-// ---- router ----------------------------------------------------------------------------------
-// One CTA per token: the token's activations in shared memory, each warp takes experts
-// warp, warp + 8, ...; fp32 accumulation in a fixed order (lane-strided, then a butterfly).
-__global__ void __launch_bounds__(256) moe_router_logits_kernel(const uint16_t *x, const uint16_t *w, uint32_t hidden,
-                                                                uint32_t experts, float *logits) {
-  extern __shared__ float xs[];
-  griddep_launch_dependents();
-  griddep_wait();
-  const uint32_t t = blockIdx.x;
-  for (uint32_t k = threadIdx.x; k < hidden; k += blockDim.x) xs[k] = bf16_bits_to_f32(x[static_cast<size_t>(t) * hidden + k]);
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (uint32_t e = warp; e < experts; e += 8) {
-    const uint16_t *row = w + static_cast<size_t>(e) * hidden;
-    float acc = 0.0f;
-    for (uint32_t k = lane * 2; k < hidden; k += 64) {
-      const uint32_t pair = *reinterpret_cast<const uint32_t *>(row + k);
-      acc = fmaf(bf16_bits_to_f32(pair & 0xFFFFu), xs[k], acc);
-      acc = fmaf(__uint_as_float(pair & 0xFFFF0000u), xs[k + 1], acc);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
-    if (lane == 0) logits[static_cast<size_t>(t) * experts + e] = acc;
-  }
-}
-
-// One warp per token: the top_k largest BF16-rounded logits, ties to the lower id, then the
-// softmax over the selected ones in fp32, rounded to BF16 and stored as fp32.
-__global__ void __launch_bounds__(256) moe_router_select_kernel(const float *logits, uint32_t tokens, uint32_t experts,
-                                                                uint32_t top_k, int32_t *ids, float *weights) {
-  griddep_launch_dependents();
-  griddep_wait();
-  const uint32_t t = blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (t >= tokens) return;
-  const float *row = logits + static_cast<size_t>(t) * experts;
-  float sel[32];
-  float prev_v = INFINITY;
-  int prev_id = -1;
-  for (uint32_t r = 0; r < top_k; ++r) {
-    // the largest (value, then lowest id) strictly after the previous pick in that order
-    float best_v = -INFINITY;
-    int best_id = 0x7FFFFFFF;
-    for (uint32_t e = lane; e < experts; e += 32) {
-      const float v = __bfloat162float(__float2bfloat16_rn(row[e]));
-      const bool after_prev = v < prev_v || (v == prev_v && static_cast<int>(e) > prev_id);
-      const bool better = v > best_v || (v == best_v && static_cast<int>(e) < best_id);
-      if (after_prev && better) {
-        best_v = v;
-        best_id = static_cast<int>(e);
-      }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xFFFFFFFFu, best_v, o);
-      const int oi = __shfl_xor_sync(0xFFFFFFFFu, best_id, o);
-      if (ov > best_v || (ov == best_v && oi < best_id)) {
-        best_v = ov;
-        best_id = oi;
-      }
-    }
-    prev_v = best_v;
-    prev_id = best_id;
-    sel[r] = best_v;
-    if (lane == 0) ids[static_cast<size_t>(t) * top_k + r] = best_id;
-  }
-  if (lane == 0) {
-    const float mx = sel[0];
-    float sum = 0.0f;
-    for (uint32_t r = 0; r < top_k; ++r) {
-      sel[r] = expf(sel[r] - mx);
-      sum += sel[r];
-    }
-    for (uint32_t r = 0; r < top_k; ++r) {
-      weights[static_cast<size_t>(t) * top_k + r] = __bfloat162float(__float2bfloat16_rn(sel[r] / sum));
-    }
-  }
-}
-
-// ---- shared expert (FP8 row-scale) and combine ---------------------------------------------------
-// y[t][r] = scale[r] * sum_c e4m3(code[r][c]) * x[t][c]: one warp per output row, up to 8 tokens a
-// pass. MODE 0: two weights, BF16 SwiGLU output; MODE 1: one weight, fp32 output from BF16 input.
-template <int MODE>
-__global__ void __launch_bounds__(256) moe_fp8_rows_kernel(const uint8_t *w0, const uint8_t *w1, uint32_t rows, uint32_t cols,
-                                                           const uint16_t *x, uint32_t tokens, void *y) {
-  griddep_launch_dependents();
-  griddep_wait();
-  const uint32_t row = blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= rows) return;
-  const uint64_t scale_off = (static_cast<uint64_t>(rows) * cols + 255u) & ~static_cast<uint64_t>(255u);
-  const uint8_t *weights[2] = {w0, w1};
-  for (uint32_t t0 = 0; t0 < tokens; t0 += 8) {
-    float acc[2][8];
-#pragma unroll
-    for (int s = 0; s < 2; ++s)
-#pragma unroll
-      for (int t = 0; t < 8; ++t) acc[s][t] = 0.0f;
-    for (uint32_t c = lane * 4; c < cols; c += 128) {
-      float wv[2][4];
-#pragma unroll
-      for (int s = 0; s < (MODE == 0 ? 2 : 1); ++s) {
-        const uint32_t codes = *reinterpret_cast<const uint32_t *>(weights[s] + static_cast<uint64_t>(row) * cols + c);
-        const uint32_t lo = e4m3x2_to_half2(codes & 0xFFFFu), hi = e4m3x2_to_half2(codes >> 16);
-        const __half2 l2 = *reinterpret_cast<const __half2 *>(&lo), h2 = *reinterpret_cast<const __half2 *>(&hi);
-        wv[s][0] = __low2float(l2);
-        wv[s][1] = __high2float(l2);
-        wv[s][2] = __low2float(h2);
-        wv[s][3] = __high2float(h2);
-      }
-#pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        if (t0 + t >= tokens) break;
-        const uint2 xb = *reinterpret_cast<const uint2 *>(x + static_cast<uint64_t>(t0 + t) * cols + c);
-        const float xv[4] = {bf16_bits_to_f32(xb.x & 0xFFFFu), __uint_as_float(xb.x & 0xFFFF0000u),
-                             bf16_bits_to_f32(xb.y & 0xFFFFu), __uint_as_float(xb.y & 0xFFFF0000u)};
-#pragma unroll
-        for (int s = 0; s < (MODE == 0 ? 2 : 1); ++s)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) acc[s][t] = fmaf(wv[s][i], xv[i], acc[s][t]);
-      }
-    }
-#pragma unroll
-    for (int s = 0; s < (MODE == 0 ? 2 : 1); ++s)
-#pragma unroll
-      for (int t = 0; t < 8; ++t)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[s][t] += __shfl_xor_sync(0xFFFFFFFFu, acc[s][t], o);
-    if (lane == 0) {
-      const float s0 = bf16_bits_to_f32(reinterpret_cast<const uint16_t *>(w0 + scale_off)[row]);
-      const float s1 = MODE == 0 ? bf16_bits_to_f32(reinterpret_cast<const uint16_t *>(w1 + scale_off)[row]) : 0.0f;
-      for (int t = 0; t < 8 && t0 + t < tokens; ++t) {
-        if (MODE == 0) {
-          const float g = acc[0][t] * s0, u = acc[1][t] * s1;
-          static_cast<__nv_bfloat16 *>(y)[static_cast<uint64_t>(t0 + t) * rows + row] = __float2bfloat16_rn(g / (1.0f + __expf(-g)) * u);
-        } else {
-          static_cast<float *>(y)[static_cast<uint64_t>(t0 + t) * rows + row] = acc[0][t] * s0;
-        }
-      }
-    }
-  }
-}
-
-// Two E4M3 codes (the low 16 bits of `pair`) as BF16 x 2, exactly: every E4M3 value has a BF16.
-__device__ __forceinline__ uint32_t e4m3x2_to_bf16x2(uint32_t pair) {
-  const uint32_t h = e4m3x2_to_half2(pair);
-  const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&h));
-  const __nv_bfloat162 b = __floats2bfloat162_rn(f.x, f.y);
-  return *reinterpret_cast<const uint32_t *>(&b);
-}
-
-// The same products for many tokens, on the tensor cores: a warp owns 16 weight rows (of both
-// weights in MODE 0) and 64 tokens, a CTA 128 rows. Weights are widened E4M3 -> BF16 (exact) into A
-// fragments, the activations are the B fragments as they lie in memory: inside a chunk of 64
-// columns the MMA's k slots are dealt so that a lane needs 16 contiguous codes of its two rows
-// and 16 contiguous activations of its token. FP32 accumulation, the row scale applied at the end.
-template <int MODE>
-__global__ void __launch_bounds__(256) moe_fp8_gemm_kernel(const uint8_t *w0, const uint8_t *w1, uint32_t rows, uint32_t cols,
-                                                           const uint16_t *x, uint32_t tokens, void *y) {
-  griddep_launch_dependents();
-  griddep_wait();
-  constexpr int S = MODE == 0 ? 2 : 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const uint32_t row0 = (blockIdx.x * 8u + static_cast<uint32_t>(warp)) * 16u;
-  const uint32_t tok0 = blockIdx.y * 64u;
-  if (row0 >= rows) return;
-  const uint8_t *weights[2] = {w0, w1};
-  float acc[S][8][4];
-#pragma unroll
-  for (int s = 0; s < S; ++s)
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[s][nt][e] = 0.0f;
-  for (uint32_t kb = 0; kb < cols; kb += 64) {
-    uint32_t a[S][4][4];  // [weight][MMA j][a0..a3]
-#pragma unroll
-    for (int s = 0; s < S; ++s) {
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const uint4 cw = *reinterpret_cast<const uint4 *>(weights[s] + static_cast<uint64_t>(row0 + g + 8 * half) * cols + kb + 16 * t);
-        const uint32_t w[4] = {cw.x, cw.y, cw.z, cw.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          a[s][j][half] = e4m3x2_to_bf16x2(w[j] & 0xFFFFu);      // k slots 2t, 2t + 1
-          a[s][j][2 + half] = e4m3x2_to_bf16x2(w[j] >> 16);       // k slots 2t + 8, 2t + 9
-        }
-      }
-    }
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-      const uint32_t token = tok0 + nt * 8 + g;
-      uint4 x0 = make_uint4(0u, 0u, 0u, 0u), x1 = x0;
-      if (token < tokens) {
-        const uint4 *src = reinterpret_cast<const uint4 *>(x + static_cast<uint64_t>(token) * cols + kb + 16 * t);
-        x0 = ldg128_coherent(src);
-        x1 = ldg128_coherent(src + 1);
-      }
-      const uint32_t b[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int s = 0; s < S; ++s) mma_bf16_f32(acc[s][nt], a[s][j][0], a[s][j][1], a[s][j][2], a[s][j][3], b[2 * j], b[2 * j + 1]);
-    }
-  }
-  const uint64_t scale_off = (static_cast<uint64_t>(rows) * cols + 255u) & ~static_cast<uint64_t>(255u);
-  float sc[S][2];
-#pragma unroll
-  for (int s = 0; s < S; ++s)
-#pragma unroll
-    for (int half = 0; half < 2; ++half)
-      sc[s][half] = bf16_bits_to_f32(reinterpret_cast<const uint16_t *>(weights[s] + scale_off)[row0 + g + 8 * half]);
-#pragma unroll
-  for (int nt = 0; nt < 8; ++nt) {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const uint32_t token = tok0 + nt * 8 + 2 * t + (e & 1);
-      const int half = e >> 1;
-      if (token >= tokens) continue;
-      const uint64_t at = static_cast<uint64_t>(token) * rows + row0 + g + 8 * half;
-      if (MODE == 0) {
-        const float gv = acc[0][nt][e] * sc[0][half], uv = acc[S - 1][nt][e] * sc[S - 1][half];
-        static_cast<__nv_bfloat16 *>(y)[at] = __float2bfloat16_rn(gv / (1.0f + __expf(-gv)) * uv);
-      } else {
-        static_cast<float *>(y)[at] = acc[0][nt][e] * sc[0][half];
-      }
-    }
-  }
-}
-
+// ---- combine ----------------------------------------------------------------------------------
 // One CTA per token: out = BF16(acc * 2^-32 + sigmoid(x . w_gate) * shared), acc zeroed behind it.
 __global__ void __launch_bounds__(256) moe_combine_kernel(long long *acc, const float *shared, const uint16_t *x,
                                                           const uint16_t *w_gate, uint32_t hidden, uint16_t *out) {
@@ -861,8 +632,7 @@ int32_t run_experts(const Geometry &g, const void *x, uint32_t tokens, const int
 }  // namespace
 
 int32_t prepare_moe_kernels(ErrorSlot &slot) {
-  const cudaError_t err = cudaFuncSetAttribute(moe_router_logits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-  if (err != cudaSuccess) return fail(slot, "ignis_moe_prepare: %s", cudaGetErrorString(err));
+  if (moe_rows_prepare(slot) != 0) return -1;
   if (moe_tc_prepare(slot) != 0) return -1;
   return moe_fp8_tc_prepare(slot);
 }
@@ -949,9 +719,8 @@ int32_t b200q_moe_router_logits(const b200q_moe_geometry *geometry, const void *
   if (!aligned(x, 16) || !aligned(w_router, 16)) return fail(slot, "ignis_moe_router_logits: x and w_router must be 16-byte aligned");
   const DeviceState *dev = prepared(slot, "ignis_moe_router_logits");
   if (dev == nullptr) return -1;
-  const cudaError_t err = launch(moe_router_logits_kernel, dim3(tokens), dim3(256), g_geo.hidden * sizeof(float),
-                                 static_cast<cudaStream_t>(stream), dev->pdl != 0, static_cast<const uint16_t *>(x),
-                                 static_cast<const uint16_t *>(w_router), g_geo.hidden, g_geo.experts, logits);
+  const cudaError_t err = moe_router_logits_launch(*dev, static_cast<const uint16_t *>(x), static_cast<const uint16_t *>(w_router), tokens,
+                                                   g_geo.hidden, g_geo.experts, logits, static_cast<cudaStream_t>(stream));
   if (err != cudaSuccess) return fail(slot, "ignis_moe_router_logits: launch failed: %s", cudaGetErrorString(err));
   return 0;
 }
@@ -964,8 +733,7 @@ int32_t b200q_moe_router(const b200q_moe_geometry *geometry, const void *x, uint
   const Geometry &g_geo = *geometry;
   const DeviceState *dev = prepared(slot, "ignis_moe_router");
   if (dev == nullptr) return -1;
-  const cudaError_t err = launch(moe_router_select_kernel, dim3((tokens + 7u) / 8u), dim3(256), 0, static_cast<cudaStream_t>(stream),
-                                 dev->pdl != 0, static_cast<const float *>(logits), tokens, g_geo.experts, g_geo.top_k, ids, weights);
+  const cudaError_t err = moe_router_select_launch(*dev, logits, tokens, g_geo.experts, g_geo.top_k, ids, weights, static_cast<cudaStream_t>(stream));
   if (err != cudaSuccess) return fail(slot, "ignis_moe_router: launch failed: %s", cudaGetErrorString(err));
   return 0;
 }
@@ -1013,25 +781,9 @@ int32_t b200q_moe_shared_expert(const b200q_moe_geometry *geometry, const void *
     err = moe_fp8_tc_shared_expert(*dev, static_cast<const uint8_t *>(gate), static_cast<const uint8_t *>(up),
                                    static_cast<const uint8_t *>(down), static_cast<const uint16_t *>(x), tokens, g_geo.hidden, g_geo.inter, h,
                                    shared, s);
-  } else if (tokens > 8u) {  // some tokens: warp-level MMAs, 64 tokens a CTA
-    const uint32_t token_blocks = (tokens + 63u) / 64u;
-    err = launch(moe_fp8_gemm_kernel<0>, dim3((g_geo.inter + 127u) / 128u, token_blocks), dim3(256), 0, s, dev->pdl != 0,
-                 static_cast<const uint8_t *>(gate), static_cast<const uint8_t *>(up), g_geo.inter, g_geo.hidden,
-                 static_cast<const uint16_t *>(x), tokens, h);
-    if (err == cudaSuccess) {
-      err = launch(moe_fp8_gemm_kernel<1>, dim3((g_geo.hidden + 127u) / 128u, token_blocks), dim3(256), 0, s, dev->pdl != 0,
-                   static_cast<const uint8_t *>(down), static_cast<const uint8_t *>(down), g_geo.hidden, g_geo.inter,
-                   static_cast<const uint16_t *>(h), tokens, static_cast<void *>(shared));
-    }
   } else {
-    err = launch(moe_fp8_rows_kernel<0>, dim3((g_geo.inter + 7u) / 8u), dim3(256), 0, s, dev->pdl != 0,
-                 static_cast<const uint8_t *>(gate), static_cast<const uint8_t *>(up), g_geo.inter, g_geo.hidden,
-                 static_cast<const uint16_t *>(x), tokens, h);
-    if (err == cudaSuccess) {
-      err = launch(moe_fp8_rows_kernel<1>, dim3((g_geo.hidden + 7u) / 8u), dim3(256), 0, s, dev->pdl != 0,
-                   static_cast<const uint8_t *>(down), static_cast<const uint8_t *>(down), g_geo.hidden, g_geo.inter,
-                   static_cast<const uint16_t *>(h), tokens, static_cast<void *>(shared));
-    }
+    err = moe_rows_shared_expert(*dev, static_cast<const uint8_t *>(gate), static_cast<const uint8_t *>(up), static_cast<const uint8_t *>(down),
+                                 static_cast<const uint16_t *>(x), tokens, g_geo.hidden, g_geo.inter, h, shared, s);
   }
   if (err != cudaSuccess) return fail(slot, "ignis_moe_shared_expert: launch failed: %s", cudaGetErrorString(err));
   return 0;

@@ -61,6 +61,17 @@ cudaError_t moe_fp8_tc_shared_expert(const DeviceState &dev, const uint8_t *gate
                                      uint32_t tokens, uint32_t hidden, uint32_t inter, void *h, float *shared, cudaStream_t stream);
 cudaError_t moe_fp8_tc_status(uint32_t *status, cudaStream_t stream);   // non-zero: one of its bounded waits ran out
 
+// The narrow dense products of the block (moe_rows.cu): the router's logits and selection, and the
+// shared expert of calls the tensor-core kernels do not take.
+constexpr uint32_t kRouterTileMinTokens = 1536;
+int32_t moe_rows_prepare(ErrorSlot &slot);
+cudaError_t moe_router_logits_launch(const DeviceState &dev, const uint16_t *x, const uint16_t *w, uint32_t tokens, uint32_t hidden,
+                                     uint32_t experts, float *logits, cudaStream_t stream);
+cudaError_t moe_router_select_launch(const DeviceState &dev, const float *logits, uint32_t tokens, uint32_t experts, uint32_t top_k,
+                                     int32_t *ids, float *weights, cudaStream_t stream);
+cudaError_t moe_rows_shared_expert(const DeviceState &dev, const uint8_t *gate, const uint8_t *up, const uint8_t *down, const uint16_t *x,
+                                   uint32_t tokens, uint32_t hidden, uint32_t inter, void *h, float *shared, cudaStream_t stream);
+
 }  // namespace b200q
 
 #endif

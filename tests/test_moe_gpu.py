@@ -294,6 +294,30 @@ def test_router_matches_a_torch_model(mo):
     del order
 
 
+@pytest.mark.parametrize("tokens,experts,hidden", [(1, 8, 128), (9, 100, 384), (65, 512, 2048), (1540, 200, 256), (1700, 512, 384), (40, 1100, 128), (3, 4096, 128)])
+def test_router_shapes_and_token_counts(mo, tokens, experts, hidden):
+    """Ragged expert counts and every form of the logits kernel (rows of 16 experts up to 1536 tokens,
+    tiles of 128 x 128 beyond): fp32 logits, the selection they imply, and the same bits for a token
+    whichever form its call took."""
+    top_k = min(10, experts)
+    mo.set_geometry(hidden, 128, experts, top_k)
+    gen = torch.Generator(device="cuda").manual_seed(tokens + experts)
+    x = torch.randn(tokens, hidden, device="cuda", generator=gen).to(torch.bfloat16)
+    wr = (torch.randn(experts, hidden, device="cuda", generator=gen) * 0.1).to(torch.bfloat16)
+    ids, weights, logits = mo.router(x, wr)
+    sum_abs = x.double().abs() @ wr.double().abs().T
+    assert bool(((logits.double() - x.double() @ wr.double().T).abs() <= 2e-6 * sum_abs + 1e-7).all())
+    rounded = logits.to(torch.bfloat16).float()
+    order = torch.sort(rounded, dim=1, descending=True, stable=True).indices[:, :top_k]
+    assert torch.equal(ids.long(), order)
+    top = torch.gather(rounded, 1, order).double()
+    soft = torch.softmax(top, dim=1)
+    assert bool(((weights.double() - soft).abs() <= 2.0 ** -8 * soft + 1e-7).all())
+    last = x[-5:].contiguous()
+    part_ids, part_weights, part_logits = mo.router(last, wr)
+    assert torch.equal(part_logits, logits[-5:]) and torch.equal(part_ids, ids[-5:]) and torch.equal(part_weights, weights[-5:])
+
+
 def test_router_against_the_recorded_checkpoint_router(mo, golden):
     """The reference's own router test at 512 experts x 2560, top-10, on its 192 recorded tokens
     (kernel/tests/test_moe_router.cu:100-165; fixture kernel/tests/fixtures/flash_next/router_ref.bin
@@ -418,7 +442,7 @@ def test_shared_expert_wide_at_config4_widths(mo):
     assert torch.allclose(shared.cpu(), other["shared"], rtol=2 ** -7, atol=2e-3 * float(s_ref.abs().max()))
 
 
-@pytest.mark.parametrize("tokens", [5, 11, 130, 300])   # up to 8: one warp per row; to 64: warp-level MMAs; above: tcgen05, ragged token tiles
+@pytest.mark.parametrize("tokens", [5, 11, 17, 64, 130, 300])   # up to 64: warp-level MMAs, one to eight token tiles a CTA; above: tcgen05, ragged token tiles
 def test_shared_expert_and_combine(mo, tokens):
     mo.set_geometry(256, 128, 8, 2)
     gen = torch.Generator().manual_seed(4)
