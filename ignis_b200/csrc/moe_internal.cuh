@@ -64,6 +64,7 @@ cudaError_t moe_fp8_tc_status(uint32_t *status, cudaStream_t stream);   // non-z
 // The narrow dense products of the block (moe_rows.cu): the router's logits and selection, and the
 // shared expert of calls the tensor-core kernels do not take.
 constexpr uint32_t kRouterTileMinTokens = 1536;
+constexpr uint32_t kFp8TcMinTokens = 256;
 int32_t moe_rows_prepare(ErrorSlot &slot);
 cudaError_t moe_router_logits_launch(const DeviceState &dev, const uint16_t *x, const uint16_t *w, uint32_t tokens, uint32_t hidden,
                                      uint32_t experts, float *logits, cudaStream_t stream);

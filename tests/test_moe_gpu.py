@@ -442,7 +442,24 @@ def test_shared_expert_wide_at_config4_widths(mo):
     assert torch.allclose(shared.cpu(), other["shared"], rtol=2 ** -7, atol=2e-3 * float(s_ref.abs().max()))
 
 
-@pytest.mark.parametrize("tokens", [5, 11, 17, 64, 130, 300])   # up to 64: warp-level MMAs, one to eight token tiles a CTA; above: tcgen05, ragged token tiles
+@pytest.mark.parametrize("tokens", [257, 900, 1601, 3203])   # token tiles of 64, 128 and 256 in each of the two products, the last ragged
+def test_shared_expert_token_tiles(mo, tokens):
+    mo.set_geometry(2048, 768, 512, 10)
+    gen = torch.Generator().manual_seed(tokens)
+    shapes = [(768, 2048), (768, 2048), (2048, 768)]
+    payloads = [torch.from_numpy(mo.fp8_row_scale_payload(torch.randn(r, c, generator=gen) * 0.03)).cuda() for r, c in shapes]
+    x = (torch.randn(tokens, 2048, generator=gen) * 0.5).to(torch.bfloat16).cuda()
+    wide = [(p[: r * c].view(torch.float8_e4m3fn).double().reshape(r, c) * p[r * c:].view(torch.bfloat16).double().unsqueeze(1))
+            for p, (r, c) in zip(payloads, shapes)]     # the code planes are whole multiples of 256 bytes
+    shared, h = mo.shared_expert(*payloads, x)
+    g, u = x.double() @ wide[0].T, x.double() @ wide[1].T
+    want = g / (1 + torch.exp(-g)) * u
+    assert torch.allclose(h.double(), want, rtol=2 ** -7, atol=1e-4 * float(want.abs().max()))
+    down = h.double() @ wide[2].T
+    assert torch.allclose(shared.double(), down, rtol=1e-4, atol=1e-5 * float(down.abs().max()))
+
+
+@pytest.mark.parametrize("tokens", [5, 11, 17, 64, 130, 300])   # up to 256: warp-level MMAs, one to eight token tiles a CTA; above: tcgen05, ragged token tiles
 def test_shared_expert_and_combine(mo, tokens):
     mo.set_geometry(256, 128, 8, 2)
     gen = torch.Generator().manual_seed(4)
