@@ -503,30 +503,82 @@ __global__ void __launch_bounds__(kThreads, NT <= 2 ? 3 : 2) moe_experts_kernel(
 }
 
 // ---- combine ----------------------------------------------------------------------------------
-// One CTA per token: out = BF16(acc * 2^-32 + sigmoid(x . w_gate) * shared), acc zeroed behind it.
+// One CTA per token: out = BF16(acc * 2^-32 + sigmoid(x . w_gate) * shared), acc zeroed behind it. Bound by
+// memory at many tokens (22 bytes per value, most of it the accumulator read and cleared) and by
+// latency at few: a thread takes eight neighbouring columns per trip in 16-byte pieces and asks for its
+// first trip's accumulators and shared values before the gate's sum is known. VEC: every pointer is
+// 16-byte aligned (the accumulator promises 8, the rest less).
+struct CombineLoad {
+  long long a[8];
+  float s[8];
+};
+template <bool VEC>
+__device__ __forceinline__ void combine_load(CombineLoad &v, const long long *acc, const float *shared) {
+  if (VEC) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint4 q = ldg128_coherent(acc + 2 * i);
+      v.a[2 * i] = static_cast<long long>((static_cast<unsigned long long>(q.y) << 32) | q.x);
+      v.a[2 * i + 1] = static_cast<long long>((static_cast<unsigned long long>(q.w) << 32) | q.z);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint4 q = ldg128_coherent(shared + 4 * i);
+      v.s[4 * i] = __uint_as_float(q.x), v.s[4 * i + 1] = __uint_as_float(q.y), v.s[4 * i + 2] = __uint_as_float(q.z), v.s[4 * i + 3] = __uint_as_float(q.w);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v.a[i] = acc[i], v.s[i] = shared[i];
+  }
+}
+
+template <bool VEC>
 __global__ void __launch_bounds__(256) moe_combine_kernel(long long *acc, const float *shared, const uint16_t *x,
                                                           const uint16_t *w_gate, uint32_t hidden, uint16_t *out) {
   griddep_launch_dependents();
   griddep_wait();
   __shared__ float partial[8];
-  const uint32_t t = blockIdx.x;
+  const size_t row = static_cast<size_t>(blockIdx.x) * hidden;
+  CombineLoad v;
+  const uint32_t k_first = threadIdx.x * 8u;
+  if (k_first < hidden) combine_load<VEC>(v, acc + row + k_first, shared + row + k_first);
   float dot = 0.0f;
-  for (uint32_t k = threadIdx.x; k < hidden; k += blockDim.x) {
-    dot = fmaf(bf16_bits_to_f32(x[static_cast<size_t>(t) * hidden + k]), bf16_bits_to_f32(w_gate[k]), dot);
+  for (uint32_t k = k_first; k < hidden; k += 2048u) {   // hidden is a multiple of 128
+    alignas(16) uint16_t xv[8], wv[8];
+    if (VEC) {
+      *reinterpret_cast<uint4 *>(xv) = ldg128_coherent(x + row + k);
+      *reinterpret_cast<uint4 *>(wv) = __ldg(reinterpret_cast<const uint4 *>(w_gate + k));
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) xv[i] = x[row + k + i], wv[i] = w_gate[k + i];
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) dot = fmaf(bf16_bits_to_f32(xv[i]), bf16_bits_to_f32(wv[i]), dot);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xFFFFFFFFu, dot, o);
   if ((threadIdx.x & 31) == 0) partial[threadIdx.x >> 5] = dot;
   __syncthreads();
   float total = 0.0f;
+#pragma unroll
   for (int i = 0; i < 8; ++i) total += partial[i];
   const float gate = 1.0f / (1.0f + __expf(-total));
-  for (uint32_t k = threadIdx.x; k < hidden; k += blockDim.x) {
-    const size_t at = static_cast<size_t>(t) * hidden + k;
-    const float routed = static_cast<float>(static_cast<double>(acc[at]) * (1.0 / 4294967296.0));
-    const __nv_bfloat16 o = __float2bfloat16_rn(routed + gate * shared[at]);
-    out[at] = *reinterpret_cast<const uint16_t *>(&o);
-    acc[at] = 0;
+  for (uint32_t k = k_first; k < hidden; k += 2048u) {
+    if (k != k_first) combine_load<VEC>(v, acc + row + k, shared + row + k);
+    alignas(16) uint16_t o[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float routed = static_cast<float>(static_cast<double>(v.a[i]) * (1.0 / 4294967296.0));
+      o[i] = __bfloat16_as_ushort(__float2bfloat16_rn(routed + gate * v.s[i]));
+    }
+    if (VEC) {
+      *reinterpret_cast<uint4 *>(out + row + k) = *reinterpret_cast<const uint4 *>(o);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4 *>(acc + row + k + 2 * i) = make_uint4(0u, 0u, 0u, 0u);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) out[row + k + i] = o[i], acc[row + k + i] = 0;
+    }
   }
 }
 
@@ -800,8 +852,9 @@ int32_t b200q_moe_combine(const b200q_moe_geometry *geometry, int64_t *acc, cons
   if (tokens == 0) return fail(slot, "ignis_moe_combine: tokens must be positive");
   const DeviceState *dev = prepared(slot, "ignis_moe_combine");
   if (dev == nullptr) return -1;
-  const cudaError_t err = launch(moe_combine_kernel, dim3(tokens), dim3(256), 0, static_cast<cudaStream_t>(stream), dev->pdl != 0,
-                                 reinterpret_cast<long long *>(acc), shared, static_cast<const uint16_t *>(x),
+  const bool vec = aligned(acc, 16) && aligned(shared, 16) && aligned(x, 16) && aligned(w_gate, 16) && aligned(out, 16);
+  const cudaError_t err = launch(vec ? moe_combine_kernel<true> : moe_combine_kernel<false>, dim3(tokens), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                                 dev->pdl != 0, reinterpret_cast<long long *>(acc), shared, static_cast<const uint16_t *>(x),
                                  static_cast<const uint16_t *>(w_gate), g_geo.hidden, static_cast<uint16_t *>(out));
   if (err != cudaSuccess) return fail(slot, "ignis_moe_combine: launch failed: %s", cudaGetErrorString(err));
   return 0;
