@@ -47,7 +47,6 @@ struct DeviceState {
   int a4_decode_kc = 0;      // B200Q_A4_DECODE_KC: cluster size of that kernel (0: planned)
   int a4_decode_groups = 0;  // B200Q_A4_DECODE_GROUPS: quantizer groups per CTA of that kernel (0: chosen by the token count)
   int a4_decode_ctas = 2;  // B200Q_A4_DECODE_CTAS: CTAs of that kernel per SM (1: one CTA with a ring twice as deep)
-  int a16_mma_wide = 1;  // B200Q_A16_MMA_WIDE: beyond 256 tokens the A16 tensor-core kernel takes token tiles of 512 (two accumulators per decoded stage)
   int w4a4_pair = 1;     // B200Q_W4A4_PAIR: the prefill GEMM on CTA pairs (cta_group::2, 256 x 256 tiles); 0: one CTA per 128 x 256 tile
   int gemv_xu = 8;       // B200Q_GEMV_XU: words per row of 8 decoded by the hardware E2M1 conversion
   int sm_cap = 0;        // IGNIS_TRELLIS_SM_CAP
@@ -109,6 +108,13 @@ __device__ __forceinline__ uint64_t l2_evict_first_policy() {
 // 32 bytes of a read-only stream that is touched once: no L1 allocation, evict-first in L2.
 __device__ __forceinline__ void ldg256_stream(const void *p, uint32_t (&r)[8], uint64_t policy) {
   asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8], %9;"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "l"(p), "l"(policy));
+}
+// The same for a stream of which every reader takes one 32-byte sector at a time: the L2 fetches the
+// line's four sectors with the first of them.
+__device__ __forceinline__ void ldg256_stream_line(const void *p, uint32_t (&r)[8], uint64_t policy) {
+  asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.L2::128B.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8], %9;"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                : "l"(p), "l"(policy));
 }

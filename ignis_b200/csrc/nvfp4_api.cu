@@ -61,28 +61,21 @@ int32_t decode_route(ErrorSlot &slot, const DeviceState &dev, const b200q_nvfp4_
   const size_t out_elem = (epilogue & kEpilogueF32) ? 4u : 2u;
   uint32_t groups = 0;
   for (uint32_t i = 0; i < count; ++i) groups += w[i]->n / 32u;
-  if (dev.a16_mma != 0 && tokens > 16u && !swiglu && peers == 1u && wait_for == nullptr && a16mma_takes(k, x)) {
+  if (dev.a16_mma != 0 && tokens > 16u && peers == 1u && wait_for == nullptr && a16mma_takes(k, x)) {
     // beyond two token tiles the warp-level MMAs of the decode kernel are the limit: the weights
     // are decoded once per tile of up to 256 tokens and multiplied on the tensor cores
-    {
-      const uint32_t t0 = 0, pass = tokens;
-      GemvWeight gw[kMaxGroup];
-      for (uint32_t i = 0; i < count; ++i) {
-        gw[i].codes = static_cast<const uint8_t *>(w[i]->codes);
-        gw[i].scales = static_cast<const uint8_t *>(w[i]->scales);
-        gw[i].y[0] = static_cast<uint8_t *>(y[i]) + static_cast<size_t>(t0) * ldy[i] * out_elem;
-        gw[i].peers = 1;
-        gw[i].n = w[i]->n;
-        gw[i].ldy = ldy[i];
-        gw[i].inv_dw = 1.0f / w[i]->weight_scale_divisor;
-        gw[i].block_begin = 0;
-      }
-      if (a16mma_launch(slot, dev, gw, count, static_cast<const uint16_t *>(x) + static_cast<size_t>(t0) * k, k, pass, epilogue,
-                        stream) != 0) {
-        return -1;
-      }
+    GemvWeight gw[kMaxGroup];
+    for (uint32_t i = 0; i < count; ++i) {
+      gw[i].codes = static_cast<const uint8_t *>(w[i]->codes);
+      gw[i].scales = static_cast<const uint8_t *>(w[i]->scales);
+      gw[i].y[0] = y[i];
+      gw[i].peers = 1;
+      gw[i].n = w[i]->n;
+      gw[i].ldy = ldy[i];
+      gw[i].inv_dw = 1.0f / w[i]->weight_scale_divisor;
+      gw[i].block_begin = 0;
     }
-    return 0;
+    return a16mma_launch(slot, dev, gw, count, static_cast<const uint16_t *>(x), k, tokens, epilogue, stream);
   }
   for (uint32_t t0 = 0; t0 < tokens; t0 += B200Q_NVFP4_DECODE_MAX_TOKENS) {
     const uint32_t pass = tokens - t0 < B200Q_NVFP4_DECODE_MAX_TOKENS ? tokens - t0 : B200Q_NVFP4_DECODE_MAX_TOKENS;

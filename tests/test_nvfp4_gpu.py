@@ -143,7 +143,8 @@ def test_linear_a16(nv, oracle, n, k, tokens):
     check_bf16(nv.linear(x.cuda(), w), ref)
 
 
-@pytest.mark.parametrize("tokens,n,k", [(17, 128, 64), (24, 256, 320), (40, 384, 1024), (100, 1024, 5120), (300, 256, 2048), (64, 5120, 6144)])
+@pytest.mark.parametrize("tokens,n,k", [(17, 128, 64), (24, 256, 320), (40, 384, 1024), (100, 1024, 5120), (300, 256, 2048), (64, 5120, 6144),
+                                        (97, 1280, 576), (257, 640, 512), (530, 1024, 1024)])
 def test_a16_tensor_core_route(nv, oracle, tokens, n, k):
     """A16 calls of more than 8 tokens: weights decoded to fp16 in shared memory, BF16 activations as
     they are, tcgen05 kind::f16 with FP32 accumulation. Token tiles 32 / 64 / 128 / 256, two passes at
@@ -400,6 +401,28 @@ def test_swiglu(nv, oracle):
         got = nv.linear_swiglu(x.cuda(), w).double().cpu().numpy()
         assert np.abs(got - want).max() <= 2.0 ** -7 * np.abs(want).max()
         assert np.linalg.norm(got - want) <= 2.0 ** -8 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("tokens,inter,k", [(17, 128, 64), (33, 256, 320), (77, 384, 1024), (300, 128, 4096), (600, 1024, 256)])
+def test_swiglu_on_the_a16_tensor_core_route(nv, oracle, tokens, inter, k):
+    """Gate and up tiles side by side in one CTA, with and without a K split, ragged token tiles; and the
+    MLP entry built on it."""
+    rng = np.random.default_rng(tokens + inter)
+    codes, scales, d_w = make_weight(rng, 2 * inter, k, d_w=2000.0)
+    w = nv.Weight.from_planes(codes, scales, d_w)
+    x = torch.randn(tokens, k, generator=torch.Generator().manual_seed(tokens)).to(torch.bfloat16)
+    ref = ref_product(oracle, codes, scales, 2 * inter, k, d_w, x)
+    g, u = ref[:, :inter], ref[:, inter:]
+    want = g / (1.0 + np.exp(-g)) * u
+    h = nv.linear_swiglu(x.cuda(), w)
+    assert nv.device_status() == 0
+    got = h.double().cpu().numpy()
+    assert np.abs(got - want).max() <= 2.0 ** -7 * np.abs(want).max()
+    assert np.linalg.norm(got - want) <= 2.0 ** -8 * np.linalg.norm(want)
+    dc, ds, _ = make_weight(rng, 256, inter)
+    down = nv.Weight.from_planes(dc, ds, d_w)
+    ws = nv.Workspace(nv.mlp_workspace_bytes(2 * inter, k, nv.A16_ONLY, tokens))
+    assert torch.equal(nv.mlp(x.cuda(), w, down, ws), nv.linear(h, down))
 
 
 def test_every_launch_plan_gives_the_same_answer_within_tolerance(nv, oracle):
