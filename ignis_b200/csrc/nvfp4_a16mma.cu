@@ -76,14 +76,6 @@ struct CodeStage {
 constexpr uint32_t kRawCodes = 128 * 128;                   // four stages of a tile's codes: 128 rows x 256 values
 constexpr uint32_t kRawTileBytes = kRawCodes + 4 * 512;     // and its scale tiles
 
-// A position in a ring of `depth` slots: the slot and the parity of its current use.
-struct RingAt {
-  uint32_t slot = 0, phase = 0;
-  __device__ __forceinline__ void advance(uint32_t by, uint32_t depth) {
-    for (slot += by; slot >= depth; slot -= depth) phase ^= 1u;
-  }
-};
-
 constexpr int kGroups = 4, kDecoders = 4 * kGroups;   // groups of four decoder warps
 constexpr int kA16Threads = (kDecoders + 3) * 32;
 constexpr float kWeightScale = 128.0f;                // the A tiles hold weights times 2^-7

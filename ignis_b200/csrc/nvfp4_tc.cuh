@@ -88,6 +88,14 @@ __device__ __forceinline__ bool elect_one() {
   return is != 0u;
 }
 
+// A position in a ring of `depth` slots: the slot and the parity of its current use.
+struct RingAt {
+  uint32_t slot = 0, phase = 0;
+  __device__ __forceinline__ void advance(uint32_t by, uint32_t depth) {
+    for (slot += by; slot >= depth; slot -= depth) phase ^= 1u;
+  }
+};
+
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }

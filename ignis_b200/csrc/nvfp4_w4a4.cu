@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(256, 1) w4a4_gemm_pair_kernel(const __grid_con
   const uint32_t bar_acc_full = bars + 8 * 2 * kStages, bar_acc_empty = bar_acc_full + 8;
   const uint32_t bar_sf_ready = bar_acc_empty + 8;   // [5], the first CTA's: a stage's scales are in both CTAs' tensor memory
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(base_ptr + kStages * kPairStageBytes + 128);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();        // 0: the pair's first CTA, which issues the MMAs
   const uint32_t k_iters = p.k / 256u, k_atoms = p.k / 64u;
   const bool swiglu = (p.epilogue & kEpilogueSwiglu) != 0u;
@@ -484,97 +484,113 @@ __global__ void __launch_bounds__(256, 1) w4a4_gemm_pair_kernel(const __grid_con
   __syncthreads();
   cluster_sync_all();   // the peer's barriers exist before anything is sent to them
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *tmem_slot, 0);
 
   griddep_launch_dependents();
   griddep_wait();  // the quantized activations come from the previous kernel in the stream
 
-  if (warp == 4 && lane == 0) {
+  // The issuing roles run in whole warps with an elected lane (elect_one, nvfp4_tc.cuh): 12 copies, 4 MMAs and 2 commits
+  // a stage were each a loop over operand values inside a branch on the lane.
+  if (warp == 4) {
     // ---- producer (both CTAs): own tokens, own half of the weight rows, the scales of both halves ----
-    uint32_t git = 0;
+    RingAt at;
+    const uint32_t full0 = in_cta(bars, 0u);   // the first CTA's barriers collect both CTAs' bytes
     bool ok = true;
     for (uint32_t tile = first; tile < tiles && ok; tile += step) {
       const uint32_t m_tile = 2u * (tile % m_pairs) + rank, n_tile = tile / m_pairs;
       const uint32_t row_a = swiglu ? n_tile * 128u : n_tile * kBN;
       const uint32_t row_b = swiglu ? p.n / 2u + n_tile * 128u : n_tile * kBN + 128u;
-      for (uint32_t it = 0; it < k_iters; ++it, ++git) {
-        const uint32_t s = git % kStages;
-        if (!mbar_wait(bars + 8 * (kStages + s), ((git / kStages) & 1u) ^ 1u)) {
-          atomicOr(p.status, kStatusProducerTimeout);
+      const int32_t row = static_cast<int32_t>(rank == 0u ? row_a : row_b);
+      const uint32_t sfa0 = m_tile * k_atoms, sfb0 = row_a / 128u * k_atoms, sfb1 = row_b / 128u * k_atoms;
+      for (uint32_t it = 0; it < k_iters; ++it, at.advance(1u, kStages)) {
+        if (!mbar_wait(bars + 8 * (kStages + at.slot), at.phase ^ 1u)) {
+          if (lane == 0) atomicOr(p.status, kStatusProducerTimeout);
           ok = false;
           break;
         }
-        const uint32_t full = in_cta(bars + 8 * s, 0u);   // the first CTA's barrier collects both CTAs' bytes
-        const uint32_t stage = base + s * kPairStageBytes;
-        if (rank == 0u) mbar_expect_tx(bars + 8 * s, 2u * kPairStageBytes);
-        tma_load_2d_pair(stage, &map_a, full, static_cast<int32_t>(it * kBKBytes), static_cast<int32_t>(m_tile * kBM));
-        tma_load_2d_pair(stage + kABytes, &map_b, full, static_cast<int32_t>(it * kBKBytes), static_cast<int32_t>(rank == 0u ? row_a : row_b));
-        tma_load_2d_pair(stage + kABytes + kPairBBytes, &map_sfa, full, 0, static_cast<int32_t>(m_tile * k_atoms + it * 4u));
-        tma_load_2d_pair(stage + kABytes + kPairBBytes + kSfaBytes, &map_sfb, full, 0,
-                         static_cast<int32_t>((row_a / 128u) * k_atoms + it * 4u));
-        tma_load_2d_pair(stage + kABytes + kPairBBytes + kSfaBytes + 2048u, &map_sfb, full, 0,
-                         static_cast<int32_t>((row_b / 128u) * k_atoms + it * 4u));
+        if (elect_one()) {
+          const uint32_t full = full0 + 8 * at.slot, stage = base + at.slot * kPairStageBytes;
+          if (rank == 0u) mbar_expect_tx(bars + 8 * at.slot, 2u * kPairStageBytes);
+          tma_load_2d_pair(stage, &map_a, full, static_cast<int32_t>(it * kBKBytes), static_cast<int32_t>(m_tile * kBM));
+          tma_load_2d_pair(stage + kABytes, &map_b, full, static_cast<int32_t>(it * kBKBytes), row);
+          tma_load_2d_pair(stage + kABytes + kPairBBytes, &map_sfa, full, 0, static_cast<int32_t>(sfa0 + it * 4u));
+          tma_load_2d_pair(stage + kABytes + kPairBBytes + kSfaBytes, &map_sfb, full, 0, static_cast<int32_t>(sfb0 + it * 4u));
+          tma_load_2d_pair(stage + kABytes + kPairBBytes + kSfaBytes + 2048u, &map_sfb, full, 0, static_cast<int32_t>(sfb1 + it * 4u));
+        }
+        __syncwarp();
       }
     }
-  } else if (warp == 5 && lane == 0 && rank == 0u) {
+  } else if (warp == 5) {
     // ---- MMA issuer of the pair: M 256 (128 per CTA), N 256, K 64 ----
-    const uint32_t idesc = (1u << 7) | (1u << 10) | ((kBN >> 3) << 17) | ((256u >> 4) << 24);
-    uint32_t git = 0, tile_i = 0;
-    bool ok = true;
-    for (uint32_t tile = first; tile < tiles && ok; tile += step, ++tile_i) {
-      if (!mbar_wait(bar_acc_empty, (tile_i & 1u) ^ 1u)) {   // both CTAs have pulled the previous tile out of tensor memory
-        atomicOr(p.status, kStatusMmaTimeout);
-        break;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      for (uint32_t it = 0; it < k_iters; ++it, ++git) {
-        const uint32_t s = git % kStages;
-        if (!mbar_wait(bar_sf_ready + 8 * s, (git / kStages) & 1u)) {   // operands landed in both CTAs and scales copied
-          atomicOr(p.status, kStatusMmaTimeout);
-          ok = false;
+    if (rank == 0u) {
+      const uint32_t idesc = (1u << 7) | (1u << 10) | ((kBN >> 3) << 17) | ((256u >> 4) << 24);
+      const uint32_t own_empty = in_cta(bars + 8 * kStages, 0u), peer_empty = in_cta(bars + 8 * kStages, 1u);
+      const uint32_t own_acc = in_cta(bar_acc_full, 0u), peer_acc = in_cta(bar_acc_full, 1u);
+      const uint64_t desc0 = smem_desc(base, 1024u, 2u);
+      RingAt at;
+      uint32_t tile_i = 0;
+      bool ok = true;
+      for (uint32_t tile = first; tile < tiles && ok; tile += step, ++tile_i) {
+        if (!mbar_wait(bar_acc_empty, (tile_i & 1u) ^ 1u)) {   // both CTAs have pulled the previous tile out of tensor memory
+          if (lane == 0) atomicOr(p.status, kStatusMmaTimeout);
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t stage = base + s * kPairStageBytes;
-        const uint32_t sf_cols = tmem + kBN + s * kPairSfCols;
-        const uint64_t a_desc = smem_desc(stage, 1024u, 2u);
-        const uint64_t b_desc = smem_desc(stage + kABytes, 1024u, 2u);
+        for (uint32_t it = 0; it < k_iters; ++it, at.advance(1u, kStages)) {
+          if (!mbar_wait(bar_sf_ready + 8 * at.slot, at.phase)) {   // operands landed in both CTAs and scales copied
+            if (lane == 0) atomicOr(p.status, kStatusMmaTimeout);
+            ok = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          if (elect_one()) {
+            const uint32_t sf_cols = tmem + kBN + at.slot * kPairSfCols;
+            const uint64_t a_desc = desc0 + at.slot * (kPairStageBytes >> 4), b_desc = a_desc + (kABytes >> 4);
 #pragma unroll
-        for (uint32_t kb = 0; kb < 4; ++kb) {
-          mma_mxf4nvf4_pair(tmem, a_desc + 2u * kb, b_desc + 2u * kb, idesc, sf_cols + kb * 4u, sf_cols + 16u + kb * 8u,
-                            (it | kb) != 0u ? 1u : 0u);
+            for (uint32_t kb = 0; kb < 4; ++kb) {
+              mma_mxf4nvf4_pair(tmem, a_desc + 2u * kb, b_desc + 2u * kb, idesc, sf_cols + kb * 4u, sf_cols + 16u + kb * 8u,
+                                (it | kb) != 0u ? 1u : 0u);
+            }
+            mma_commit_pair(own_empty + 8 * at.slot);    // this CTA's stage ...
+            mma_commit_pair(peer_empty + 8 * at.slot);   // ... and the peer's
+          }
+          __syncwarp();
         }
-        mma_commit_pair(in_cta(bars + 8 * (kStages + s), 0u));   // this CTA's stage ...
-        mma_commit_pair(in_cta(bars + 8 * (kStages + s), 1u));   // ... and the peer's
-      }
-      if (ok) {
-        mma_commit_pair(in_cta(bar_acc_full, 0u));
-        mma_commit_pair(in_cta(bar_acc_full, 1u));
+        if (ok && elect_one()) {
+          mma_commit_pair(own_acc);
+          mma_commit_pair(peer_acc);
+        }
+        __syncwarp();
       }
     }
-  } else if (warp >= 6 && lane == 0 && rank == 0u) {
+  } else if (warp >= 6) {
     // ---- scale copiers of the pair (one copy instruction serves both CTAs): warp 6 the first two
     //      K-atoms of a stage, warp 7 the other two ----
-    const uint32_t kb0 = static_cast<uint32_t>(warp - 6) * 2u;
-    const uint32_t my_tiles = tiles > first ? (tiles - first + step - 1u) / step : 0u;
-    const uint32_t total = my_tiles * k_iters;
-    for (uint32_t g = 0; g < total; ++g) {
-      const uint32_t s = g % kStages;
-      if (!mbar_wait(bars + 8 * s, (g / kStages) & 1u)) {
-        atomicOr(p.status, kStatusMmaTimeout);
-        break;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t stage = base + s * kPairStageBytes;
-      const uint32_t sf_cols = tmem + kBN + s * kPairSfCols;
-      const uint32_t sfa_smem = stage + kABytes + kPairBBytes, sfb_smem = sfa_smem + kSfaBytes;
+    if (rank == 0u) {
+      const uint32_t kb0 = static_cast<uint32_t>(warp - 6) * 2u;
+      const uint32_t my_tiles = tiles > first ? (tiles - first + step - 1u) / step : 0u;
+      const uint32_t total = my_tiles * k_iters, ready = in_cta(bar_sf_ready, 0u);
+      const uint64_t sfa0 = smem_desc(base + kABytes + kPairBBytes, 128u, 0u);
+      RingAt at;
+      for (uint32_t g = 0; g < total; ++g, at.advance(1u, kStages)) {
+        if (!mbar_wait(bars + 8 * at.slot, at.phase)) {
+          if (lane == 0) atomicOr(p.status, kStatusMmaTimeout);
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (elect_one()) {
+          const uint32_t sf_cols = tmem + kBN + at.slot * kPairSfCols + kb0 * 4u;
+          const uint64_t sfa = sfa0 + at.slot * (kPairStageBytes >> 4) + kb0 * 32u, sfb = sfa + (kSfaBytes >> 4);
 #pragma unroll
-      for (uint32_t kb = kb0; kb < kb0 + 2u; ++kb) {
-        tmem_cp_sf_pair(sf_cols + kb * 4u, smem_desc(sfa_smem + kb * 512u, 128u, 0u));
-        tmem_cp_sf_pair(sf_cols + 16u + kb * 8u, smem_desc(sfb_smem + kb * 512u, 128u, 0u));
-        tmem_cp_sf_pair(sf_cols + 16u + kb * 8u + 4u, smem_desc(sfb_smem + 2048u + kb * 512u, 128u, 0u));
+          for (uint32_t kb = 0; kb < 2u; ++kb) {
+            tmem_cp_sf_pair(sf_cols + kb * 4u, sfa + kb * 32u);
+            tmem_cp_sf_pair(sf_cols + 16u + kb0 * 4u + kb * 8u, sfb + kb * 32u);
+            tmem_cp_sf_pair(sf_cols + 20u + kb0 * 4u + kb * 8u, sfb + 128u + kb * 32u);
+          }
+          mma_commit_pair(ready + 8 * at.slot);
+        }
+        __syncwarp();
       }
-      mma_commit_pair(in_cta(bar_sf_ready + 8 * s, 0u));
     }
   } else if (warp < 4) {
     // ---- epilogue (both CTAs): warp q owns this CTA's accumulator lanes (tokens) 32 q .. 32 q + 31 ----
