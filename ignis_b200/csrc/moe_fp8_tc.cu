@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kThreads) moe_fp8_tc_kernel(const __grid_const
   uint8_t *base_ptr = smem_raw + (base - raw);
   const uint32_t bars = base + p.stages * kStageBytes;   // full[stages], empty[stages], accumulator full; then the TMEM slot
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(base_ptr + p.stages * kStageBytes + 8u * (2u * p.stages + 1u) + 8u);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const uint32_t m_tile = blockIdx.x, tok0 = blockIdx.y * kBN;
   const uint32_t k_stages = p.cols / 64u;
 
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(kThreads) moe_fp8_tc_kernel(const __grid_const
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *tmem_slot, 0);
 
   if (warp < kDecoders) {
     // ---- decoder warps: widen 16 rows a warp into the A tiles; lane = 16 codes (piece) of rows first + 8 i ----
@@ -148,48 +148,49 @@ __global__ void __launch_bounds__(kThreads) moe_fp8_tc_kernel(const __grid_const
     // ---- producer of the activation tiles ----
     griddep_launch_dependents();
     griddep_wait();   // MODE 1 reads what MODE 0 wrote
-    if (lane == 0) {
-      for (uint32_t st = 0; st < k_stages; ++st) {
-        const uint32_t slot = st % p.stages;
-        if (!mbar_wait(bars + 8 * (p.stages + slot), ((st / p.stages) & 1u) ^ 1u)) {
-          atomicOr(&g_fp8_tc_status, kProducerTimeout);
-          break;
-        }
-        const uint32_t full = bars + 8 * slot;
-        mbar_expect_tx(full, kBBytes);
-        tma_load_2d(base + slot * kStageBytes + S * kABytes, &map_x, full, static_cast<int32_t>(st * 64u), static_cast<int32_t>(tok0));
+    RingAt at;
+    for (uint32_t st = 0; st < k_stages; ++st, at.advance(1u, p.stages)) {
+      if (!mbar_wait(bars + 8 * (p.stages + at.slot), at.phase ^ 1u)) {
+        if (lane == 0) atomicOr(&g_fp8_tc_status, kProducerTimeout);
+        break;
       }
+      if (elect_one()) {
+        mbar_expect_tx(bars + 8 * at.slot, kBBytes);
+        tma_load_2d(base + at.slot * kStageBytes + S * kABytes, &map_x, bars + 8 * at.slot, static_cast<int32_t>(st * 64u), static_cast<int32_t>(tok0));
+      }
+      __syncwarp();
     }
   } else {
-    // ---- MMA issuer ----
+    // ---- MMA issuer: the whole warp runs the loop, an elected lane issues (elect_one, nvfp4_tc.cuh) ----
     griddep_launch_dependents();
     griddep_wait();
-    if (lane == 0) {
-      // FP32 accumulator (bit 4), A and B BF16 (format 1 at bits 7 and 10), both K-major, N >> 3 at bit 17, M >> 4 at bit 24
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((kBN >> 3) << 17) | ((kBM >> 4) << 24);
-      bool ok = true;
-      for (uint32_t st = 0; st < k_stages; ++st) {
-        const uint32_t slot = st % p.stages;
-        if (!mbar_wait(bars + 8 * slot, (st / p.stages) & 1u)) {
-          atomicOr(&g_fp8_tc_status, kMmaTimeout);
-          ok = false;
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t stage = base + slot * kStageBytes;
-        const uint64_t b_desc = smem_desc_sw128(stage + S * kABytes);
+    // FP32 accumulator (bit 4), A and B BF16 (format 1 at bits 7 and 10), both K-major, N >> 3 at bit 17, M >> 4 at bit 24
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((kBN >> 3) << 17) | ((kBM >> 4) << 24);
+    const uint64_t desc0 = smem_desc_sw128(base);
+    bool ok = true;
+    RingAt at;
+    for (uint32_t st = 0; st < k_stages; ++st, at.advance(1u, p.stages)) {
+      if (!mbar_wait(bars + 8 * at.slot, at.phase)) {
+        if (lane == 0) atomicOr(&g_fp8_tc_status, kMmaTimeout);
+        ok = false;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (elect_one()) {
+        const uint64_t a_desc = desc0 + at.slot * (kStageBytes >> 4), b_desc = a_desc + S * (kABytes >> 4);
 #pragma unroll
         for (int s = 0; s < S; ++s) {
-          const uint64_t a_desc = smem_desc_sw128(stage + static_cast<uint32_t>(s) * kABytes);
 #pragma unroll
           for (uint32_t kb = 0; kb < 4; ++kb) {
-            mma_f16(tmem + static_cast<uint32_t>(s) * kBN, a_desc + 2u * kb, b_desc + 2u * kb, idesc, (st | kb) != 0u ? 1u : 0u);
+            mma_f16(tmem + static_cast<uint32_t>(s) * kBN, a_desc + s * (kABytes >> 4) + 2u * kb, b_desc + 2u * kb, idesc, (st | kb) != 0u ? 1u : 0u);
           }
         }
-        mma_commit(bars + 8 * (p.stages + slot));
+        mma_commit(bars + 8 * (p.stages + at.slot));
       }
-      if (ok) mma_commit(bars + 8 * 2 * p.stages);
+      __syncwarp();
     }
+    if (ok && elect_one()) mma_commit(bars + 8 * 2 * p.stages);
+    __syncwarp();
   }
 
   // ---- epilogue: a warp owns 32 accumulator lanes (weight rows) and half of the tokens ----

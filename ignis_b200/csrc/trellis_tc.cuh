@@ -217,7 +217,7 @@ __device__ __forceinline__ Core core_setup(uint8_t *smem_raw) {
   c.bars = c.base + kStages * kStageBytes;       // full[kStages], empty[kStages], accumulator full
   c.bar_acc = c.bars + 8u * 2u * kStages;
   c.tmem_slot = reinterpret_cast<uint32_t *>(smem_raw + (c.base - raw) + kStages * kStageBytes + 128);
-  c.warp = threadIdx.x >> 5;
+  c.warp = threadIdx.x >> 5;   // not uniform_warp(): a uniform index moved the decoders' addressing to the uniform datapath and cost 27 %
   c.lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < kStages; ++s) {
@@ -234,7 +234,7 @@ __device__ __forceinline__ Core core_setup(uint8_t *smem_raw) {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  c.tmem = *c.tmem_slot;
+  c.tmem = __shfl_sync(0xFFFFFFFFu, *c.tmem_slot, 0);
   return c;
 }
 
@@ -273,50 +273,52 @@ __device__ __forceinline__ bool core_roles(const Core &c, const Job &job, const 
     // ---- producer of the activation tiles ----
     griddep_launch_dependents();
     griddep_wait();   // the rotated activations come from the kernel before
-    if (c.lane == 0) {
-      for (uint32_t it = 0; it < k_stages; ++it) {
-        const uint32_t slot = it % kStages;
-        if (!mbar_wait(c.bars + 8u * (kStages + slot), ((it / kStages) & 1u) ^ 1u)) {
-          atomicOr(status, kStatusProducer);
-          break;
-        }
-        const uint32_t full = c.bars + 8u * slot;
+    RingAt at;
+    for (uint32_t it = 0; it < k_stages; ++it, at.advance(1u, kStages)) {
+      if (!mbar_wait(c.bars + 8u * (kStages + at.slot), at.phase ^ 1u)) {
+        if (c.lane == 0) atomicOr(status, kStatusProducer);
+        break;
+      }
+      if (elect_one()) {
+        const uint32_t full = c.bars + 8u * at.slot, stage = c.base + at.slot * kStageBytes;
         mbar_expect_tx(full, row_tiles * kABytes);
-        const uint32_t stage = c.base + slot * kStageBytes;
         tma_load_2d(stage, map_a, full, static_cast<int32_t>(it * 64u), static_cast<int32_t>(job.row0));
         if (row_tiles == 2u) tma_load_2d(stage + kABytes, map_a, full, static_cast<int32_t>(it * 64u), static_cast<int32_t>(job.row0 + 128u));
       }
+      __syncwarp();
     }
     return false;
   }
-  // ---- MMA issuer ----
+  // ---- MMA issuer: the whole warp runs the loop, an elected lane issues (elect_one, nvfp4_tc.cuh) ----
   griddep_launch_dependents();
   griddep_wait();
-  if (c.lane == 0) {
-    // instruction descriptor: FP32 accumulator (bit 4), A and B FP16 (format 0), both K-major,
-    // N >> 3 at bit 17, M >> 4 at bit 24
-    const uint32_t mma_n = job.nblk * 128u;
-    const uint32_t idesc = (1u << 4) | ((mma_n >> 3) << 17) | ((128u >> 4) << 24);
-    bool ok = true;
-    for (uint32_t it = 0; it < k_stages; ++it) {
-      const uint32_t slot = it % kStages;
-      if (!mbar_wait(c.bars + 8u * slot, (it / kStages) & 1u)) {
-        atomicOr(status, kStatusMma);
-        ok = false;
-        break;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t stage = c.base + slot * kStageBytes;
-      const uint64_t a0 = smem_desc_sw128(stage), a1 = smem_desc_sw128(stage + kABytes), b = smem_desc_sw128(stage + 2u * kABytes);
+  // instruction descriptor: FP32 accumulator (bit 4), A and B FP16 (format 0), both K-major,
+  // N >> 3 at bit 17, M >> 4 at bit 24
+  const uint32_t mma_n = job.nblk * 128u;
+  const uint32_t idesc = (1u << 4) | ((mma_n >> 3) << 17) | ((128u >> 4) << 24);
+  const uint64_t desc0 = smem_desc_sw128(c.base);
+  bool ok = true;
+  RingAt at;
+  for (uint32_t it = 0; it < k_stages; ++it, at.advance(1u, kStages)) {
+    if (!mbar_wait(c.bars + 8u * at.slot, at.phase)) {
+      if (c.lane == 0) atomicOr(status, kStatusMma);
+      ok = false;
+      break;
+    }
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (elect_one()) {
+      const uint64_t a0 = desc0 + at.slot * (kStageBytes >> 4), a1 = a0 + (kABytes >> 4), b = a1 + (kABytes >> 4);
 #pragma unroll
       for (uint32_t kb = 0; kb < 4; ++kb) {   // 16 values along K are 32 bytes: two 16-byte units further
         mma_f16(c.tmem, a0 + 2u * kb, b + 2u * kb, idesc, (it | kb) != 0u ? 1u : 0u);
         if (row_tiles == 2u) mma_f16(c.tmem + Shape<DW>::kCols, a1 + 2u * kb, b + 2u * kb, idesc, (it | kb) != 0u ? 1u : 0u);
       }
-      mma_commit(c.bars + 8u * (kStages + slot));
+      mma_commit(c.bars + 8u * (kStages + at.slot));
     }
-    if (ok) mma_commit(c.bar_acc);
+    __syncwarp();
   }
+  if (ok && elect_one()) mma_commit(c.bar_acc);
+  __syncwarp();
   return false;
 }
 
