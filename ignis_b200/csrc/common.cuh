@@ -47,7 +47,7 @@ struct DeviceState {
   int a4_decode_kc = 0;      // B200Q_A4_DECODE_KC: cluster size of that kernel (0: planned)
   int a4_decode_groups = 0;  // B200Q_A4_DECODE_GROUPS: quantizer groups per CTA of that kernel (0: chosen by the token count)
   int a4_decode_ctas = 2;  // B200Q_A4_DECODE_CTAS: CTAs of that kernel per SM (1: one CTA with a ring twice as deep)
-  int w4a4_pair = 1;     // B200Q_W4A4_PAIR: the prefill GEMM on CTA pairs (cta_group::2, 256 x 256 tiles); 0: one CTA per 128 x 256 tile
+  int w4a4_pair = -1;    // B200Q_W4A4_PAIR: prefill products on CTA pairs (1), on the narrow kernel (0), or the cheaper of the two (-1)
   int gemv_xu = 8;       // B200Q_GEMV_XU: words per row of 8 decoded by the hardware E2M1 conversion
   int sm_cap = 0;        // IGNIS_TRELLIS_SM_CAP
   int moe_tc = 1;        // B200Q_MOE_TC: expert calls of more than 64 tokens take the tensor-core kernels

@@ -312,7 +312,7 @@ int32_t b200q_nvfp4_linear_split(const b200q_nvfp4_weight *parent, uint32_t coun
   if (!wide || count == 1) {
     return linear_group_impl(parts, count, x, tokens, y, ldy, epilogue, policy, workspace, stream, what);
   }
-  // wide: one quantization of x, then a tensor-core product per range over the same operand
+  // wide: one quantization of x, then the ranges' products over the same operand
   if (tokens == 0) return fail(slot, "%s: tokens must be positive", what);
   if (x == nullptr || !aligned(x, 16)) return fail(slot, "%s: x is NULL or not 16-byte aligned", what);
   if (!std::isfinite(parent->input_scale_divisor) || !(parent->input_scale_divisor > 0.0f)) {
@@ -329,19 +329,13 @@ int32_t b200q_nvfp4_linear_split(const b200q_nvfp4_weight *parent, uint32_t coun
       return fail(slot, "%s: output %u must be 16-byte aligned with ldy a multiple of 8 and at least its rows", what, i);
     }
   }
-  uint8_t *base = static_cast<uint8_t *>(workspace->base);
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  A4Item items[B200Q_NVFP4_MAX_GROUP];
   for (uint32_t i = 0; i < count; ++i) {
-    const b200q_nvfp4_weight &w = part[i];
-    const int32_t rc = i == 0 ? w4a4_launch(slot, *dev, static_cast<const uint8_t *>(w.codes), static_cast<const uint8_t *>(w.scales), w.n, w.k,
-                                            w.weight_scale_divisor, w.input_scale_divisor, static_cast<const uint16_t *>(x), tokens,
-                                            y[i], ldy[i], epilogue, base, s)
-                              : w4a4_launch_prequantized(slot, *dev, static_cast<const uint8_t *>(w.codes),
-                                                         static_cast<const uint8_t *>(w.scales), w.n, w.k, w.weight_scale_divisor,
-                                                         w.input_scale_divisor, tokens, y[i], ldy[i], epilogue, base, s);
-    if (rc != 0) return -1;
+    items[i] = A4Item{static_cast<const uint8_t *>(part[i].codes), static_cast<const uint8_t *>(part[i].scales), y[i], part[i].n, ldy[i],
+                      part[i].weight_scale_divisor, part[i].input_scale_divisor};
   }
-  return 0;
+  return w4a4_launch_parts(slot, *dev, items, count, parent->k, static_cast<const uint16_t *>(x), tokens, epilogue,
+                           static_cast<uint8_t *>(workspace->base), static_cast<cudaStream_t>(stream));
 }
 
 namespace {

@@ -92,6 +92,14 @@ int32_t w4a4_decode_launch(ErrorSlot &slot, const DeviceState &dev, const A4Item
                            uint32_t k, uint32_t tokens, uint32_t epilogue, cudaStream_t stream);
 int32_t w4a4_decode_status(ErrorSlot &slot, cudaStream_t stream, uint32_t *status);
 
+// W4A4 products of some dozens to some hundreds of tokens over activations quantized in the operand layout
+// (nvfp4_w4a4_narrow.cu); several weights may share one launch.
+int32_t w4a4_narrow_prepare(ErrorSlot &slot);
+bool w4a4_narrow_takes(const DeviceState &dev, uint32_t row_tiles, uint32_t k, uint32_t tokens, bool swiglu);
+int32_t w4a4_narrow_launch(ErrorSlot &slot, const DeviceState &dev, const A4Item *items, uint32_t count, uint32_t k, uint32_t tokens,
+                           uint32_t epilogue, const uint8_t *x_codes, const uint8_t *x_scales, uint32_t *status, uint8_t *q_codes,
+                           uint8_t *q_scales, float q_din, cudaStream_t stream);
+
 // The tensor-core prefill route (nvfp4_w4a4.cu).
 int32_t w4a4_prepare(ErrorSlot &slot);
 bool w4a4_shape_ok(uint32_t n, uint32_t k);
@@ -104,6 +112,9 @@ int32_t w4a4_launch(ErrorSlot &slot, const DeviceState &dev, const uint8_t *w_co
 int32_t w4a4_launch_prequantized(ErrorSlot &slot, const DeviceState &dev, const uint8_t *w_codes, const uint8_t *w_scales,
                                  uint32_t n, uint32_t k, float d_w, float d_in, uint32_t tokens, void *y, uint32_t ldy,
                                  uint32_t epilogue, uint8_t *workspace, cudaStream_t stream);
+// Row ranges of one parent over one quantization of x: a launch for all of them where the narrow kernel takes the call.
+int32_t w4a4_launch_parts(ErrorSlot &slot, const DeviceState &dev, const A4Item *parts, uint32_t count, uint32_t k, const uint16_t *x,
+                          uint32_t tokens, uint32_t epilogue, uint8_t *workspace, cudaStream_t stream);
 int32_t w4a4_quantize_range(ErrorSlot &slot, const DeviceState &dev, const uint16_t *x_rows, uint32_t tokens_total,
                             uint32_t token_begin, uint32_t token_count, uint32_t k, float d_in, uint8_t *workspace,
                             cudaStream_t stream);

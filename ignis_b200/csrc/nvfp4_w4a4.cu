@@ -9,16 +9,14 @@
 //     scales, bit for bit the reference's rule (nvfp4_codec.cuh:81-110), the scales written in the
 //     same 512-byte (128 rows x 4 groups) tiles the weight plane uses - which is the scale-factor
 //     atom the block-scaled MMA reads, so neither operand's scales are ever reshuffled.
-//  2. The product, in two forms that share the stage layout and the epilogue:
-//     `w4a4_gemm_persistent_kernel` - one CTA per SM walking 128-token x 256-row tiles: a producer
-//     thread streams K in stages of 256 (TMA 2-D tiles of codes with the 128-byte swizzle, bulk
-//     copies of the scale tiles) into an mbarrier ring that keeps running across tile boundaries;
-//     two threads copy each stage's scale atoms to tensor memory (tcgen05.cp); one thread issues
-//     tcgen05.mma kind::mxf4nvf4 block_scale scale_vec::4X (M 128, N 256, K 64) with the fp32
+//  2. `w4a4_gemm_pair_kernel` - clusters of two CTAs, one CTA per SM, walk 256-token x 256-row tiles
+//     (tcgen05 cta_group::2): a producer warp streams K in stages of 256 (TMA 2-D tiles of codes with the
+//     128-byte swizzle, scale tiles beside them) into an mbarrier ring that keeps running across tile
+//     boundaries; two warps copy each stage's scale atoms to tensor memory (tcgen05.cp); one issues
+//     tcgen05.mma kind::mxf4nvf4 block_scale scale_vec::4X (M 256, N 256, K 64) with the fp32
 //     accumulator in tensor memory; four warps pull the accumulator (tcgen05.ld), hand tensor
-//     memory back and store under the next tile's MMAs. Kept behind B200Q_W4A4_PAIR = 0.
-//     `w4a4_gemm_pair_kernel` (the default) - the same on clusters of two CTAs sharing 256 x 256
-//     tiles (cta_group::2): fewer operand bytes per FLOP.
+//     memory back and store under the next tile's MMAs. Calls whose tiles would leave most of the
+//     device idle take the narrow kernel instead (nvfp4_w4a4_narrow.cu).
 //
 // Every wait on an mbarrier is bounded: after the limit the thread records a status bit in the
 // workspace, stops issuing and the CTA tears down (tensor memory freed) instead of hanging.
@@ -37,21 +35,6 @@ constexpr int kBM = 128;          // tokens per tile (MMA M)
 constexpr int kBKBytes = 128;     // bytes of codes per row per stage: 256 values along K
 constexpr uint32_t kABytes = kBM * kBKBytes;        // 16 KB
 constexpr uint32_t kSfaBytes = 4 * 512;             // 4 K-atoms of one 128-row tile
-
-// Two tile shapes. 128 x 256 (one CTA per SM, 4 stages, all 512 tensor-memory columns) is the
-// fused-SwiGLU form: 128 gate rows and their 128 up rows side by side. 128 x 128 (3 stages, 256
-// columns) lets two CTAs share an SM, so one's pipeline fill and accumulator drain hide under the
-// other's MMAs: the plain product.
-template <int BN>
-struct Tile {
-  static constexpr int kStages = BN == 256 ? 4 : 3;
-  static constexpr uint32_t kBBytes = BN * kBKBytes;
-  static constexpr uint32_t kSfbBytes = (BN / 128) * 4 * 512;
-  static constexpr uint32_t kStageBytes = kABytes + kBBytes + kSfaBytes + kSfbBytes;
-  static constexpr uint32_t kSmemBytes = kStages * kStageBytes + 256 + 1024;  // + barriers + alignment slack
-  static constexpr uint32_t kTmemCols = BN == 256 ? 512 : 256;
-  static constexpr uint32_t kSfColsPerStage = 16 + (BN / 128) * 16;  // activations, then weights
-};
 
 constexpr uint32_t kStatusProducerTimeout = 1u, kStatusMmaTimeout = 2u, kStatusEpilogueTimeout = 4u;
 
@@ -108,14 +91,10 @@ struct W4A4Params {
   float q_din;        // the next weight's input divisor
 };
 
-// ---- the persistent form ------------------------------------------------------------------------
-// One CTA per SM walks 128 x 256 tiles (tile = blockIdx.x, + gridDim.x, ...; the token tile index
-// runs fastest, so the CTAs at work share weight rows in the L2). The producer keeps the 4-stage ring
-// full across tile boundaries, so a tile's first MMAs find their operands waiting; the epilogue
-// warps pull the whole accumulator into registers (as packed BF16: 128 registers a thread - the
-// CTA has the SM's register file to itself), hand tensor memory back to the MMA thread and only
-// then store, under the next tile's MMAs. What a tile costs beyond its MMAs is the pull alone.
-// ---- the persistent kernels' epilogue for one 128-token x 256-row tile ---------------------------
+// The epilogue pulls the whole accumulator into registers (as packed BF16: 128 registers a thread - the
+// CTA has the SM's register file to itself), hands tensor memory back to the MMA warp and only
+// then stores, under the next tile's MMAs. What a tile costs beyond its MMAs is the pull alone.
+// ---- the epilogue of one CTA's 128-token x 256-row half of a tile --------------------------------
 // The calling warp q owns accumulator lanes (tokens) 32 q .. 32 q + 31 at `lane_base`. `release()`
 // hands tensor memory back to the MMA thread; it is called as soon as the accumulator has been
 // read, so that whatever follows runs under the next tile's MMAs.
@@ -237,171 +216,12 @@ __device__ __forceinline__ void w4a4_epilogue_tile(const W4A4Params &p, uint32_t
   }
 }
 
-__global__ void __launch_bounds__(256, 1) w4a4_gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
-                                                                     const __grid_constant__ CUtensorMap map_b,
-                                                                     const __grid_constant__ W4A4Params p) {
-  constexpr int kBN = 256;
-  constexpr int kStages = Tile<256>::kStages;
-  constexpr uint32_t kBBytes = Tile<256>::kBBytes, kStageBytes = Tile<256>::kStageBytes;
-  constexpr uint32_t kTmemCols = Tile<256>::kTmemCols, kSfColsPerStage = Tile<256>::kSfColsPerStage;
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t raw = smem_u32(smem_raw);
-  const uint32_t base = (raw + 1023u) & ~1023u;
-  uint8_t *base_ptr = smem_raw + (base - raw);
-  // barriers: full[4], empty[4], accumulator full, accumulator empty; then the tensor-memory slot
-  const uint32_t bars = base + kStages * kStageBytes;
-  const uint32_t bar_acc_full = bars + 8 * 2 * kStages, bar_acc_empty = bar_acc_full + 8;
-  const uint32_t bar_sf_ready = bar_acc_empty + 8;   // [4]: a stage's scales are in tensor memory
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(base_ptr + kStages * kStageBytes + 128);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t k_iters = p.k / 256u, k_atoms = p.k / 64u;
-  const bool swiglu = (p.epilogue & kEpilogueSwiglu) != 0u;
-  const uint32_t m_tiles = (p.tokens + kBM - 1) / kBM;
-  const uint32_t n_tiles = swiglu ? p.n / 256u : (p.n + 255u) / 256u;
-  const uint32_t tiles = m_tiles * n_tiles;
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
-      mbar_init(bars + 8 * s, 1);
-      mbar_init(bars + 8 * (kStages + s), 1);
-    }
-    mbar_init(bar_acc_full, 1);
-    mbar_init(bar_acc_empty, 4);  // one arrival per epilogue warp
-    for (int s = 0; s < kStages; ++s) mbar_init(bar_sf_ready + 8 * s, 2);  // the two scale copiers' commits
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 5) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tmem_slot;
-
-  griddep_launch_dependents();
-  griddep_wait();  // the quantized activations come from the previous kernel in the stream
-
-  if (warp == 4 && lane == 0) {
-    // ---- producer ----
-    uint32_t git = 0;  // stage uses since the kernel began
-    bool ok = true;
-    for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-      const uint32_t m_tile = tile % m_tiles, n_tile = tile / m_tiles;
-      const uint32_t row_a = swiglu ? n_tile * 128u : n_tile * kBN;
-      const uint32_t row_b = swiglu ? p.n / 2u + n_tile * 128u : n_tile * kBN + 128u;
-      const bool second_half = row_b < p.n;
-      for (uint32_t it = 0; it < k_iters; ++it, ++git) {
-        const uint32_t s = git % kStages;
-        if (!mbar_wait(bars + 8 * (kStages + s), ((git / kStages) & 1u) ^ 1u)) {
-          atomicOr(p.status, kStatusProducerTimeout);
-          ok = false;
-          break;
-        }
-        const uint32_t full = bars + 8 * s;
-        const uint32_t stage = base + s * kStageBytes;
-        mbar_expect_tx(full, kABytes + kSfaBytes + (second_half ? 2u : 1u) * (128u * kBKBytes + 2048u));
-        tma_load_2d(stage, &map_a, full, static_cast<int32_t>(it * kBKBytes), static_cast<int32_t>(m_tile * kBM));
-        tma_load_2d(stage + kABytes, &map_b, full, static_cast<int32_t>(it * kBKBytes), static_cast<int32_t>(row_a));
-        if (second_half) {
-          tma_load_2d(stage + kABytes + 128u * kBKBytes, &map_b, full, static_cast<int32_t>(it * kBKBytes), static_cast<int32_t>(row_b));
-        }
-        bulk_load(stage + kABytes + kBBytes, p.sfa + (static_cast<uint64_t>(m_tile) * k_atoms + it * 4u) * 512u, kSfaBytes, full);
-        bulk_load(stage + kABytes + kBBytes + kSfaBytes, p.sfb + (static_cast<uint64_t>(row_a / 128u) * k_atoms + it * 4u) * 512u, 2048u, full);
-        if (second_half) {
-          bulk_load(stage + kABytes + kBBytes + kSfaBytes + 2048u, p.sfb + (static_cast<uint64_t>(row_b / 128u) * k_atoms + it * 4u) * 512u,
-                    2048u, full);
-        }
-      }
-    }
-  } else if (warp == 5 && lane == 0) {
-    // ---- MMA issuer ----
-    // The scale copies of a stage (twelve of 512 bytes) cost this thread more issue time than its four
-    // MMAs when it issues both (880 cycles a stage, measured with clock64), so they come from the
-    // two copier warps below and this thread only waits for their commits.
-    const uint32_t idesc = (1u << 7) | (1u << 10) | ((kBN >> 3) << 17) | ((kBM >> 4) << 24);
-    uint32_t git = 0, tile_i = 0;
-    bool ok = true;
-    for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++tile_i) {
-      // the epilogue warps have pulled the previous tile out of tensor memory
-      if (!mbar_wait(bar_acc_empty, (tile_i & 1u) ^ 1u)) {
-        atomicOr(p.status, kStatusMmaTimeout);
-        break;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      for (uint32_t it = 0; it < k_iters; ++it, ++git) {
-        const uint32_t s = git % kStages;
-        if (!mbar_wait(bar_sf_ready + 8 * s, (git / kStages) & 1u)) {   // operands landed and scales copied
-          atomicOr(p.status, kStatusMmaTimeout);
-          ok = false;
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t stage = base + s * kStageBytes;
-        const uint32_t sf_cols = tmem + kBN + s * kSfColsPerStage;
-        const uint64_t a_desc = smem_desc(stage, 1024u, 2u);
-        const uint64_t b_desc = smem_desc(stage + kABytes, 1024u, 2u);
-#pragma unroll
-        for (uint32_t kb = 0; kb < 4; ++kb) {
-          mma_mxf4nvf4(tmem, a_desc + 2u * kb, b_desc + 2u * kb, idesc, sf_cols + kb * 4u, sf_cols + 16u + kb * 8u,
-                       (it | kb) != 0u ? 1u : 0u);
-        }
-        mma_commit(bars + 8 * (kStages + s));
-      }
-      if (ok) mma_commit(bar_acc_full);
-    }
-  } else if (warp >= 6 && lane == 0) {
-    // ---- scale copiers: a stage's scale tiles go to tensor memory from threads of their own,
-    //      warp 6 the first two K-atoms, warp 7 the other two ----
-    const uint32_t kb0 = static_cast<uint32_t>(warp - 6) * 2u;
-    const uint32_t my_tiles = tiles > blockIdx.x ? (tiles - blockIdx.x + gridDim.x - 1u) / gridDim.x : 0u;
-    const uint32_t total = my_tiles * k_iters;
-    for (uint32_t g = 0; g < total; ++g) {
-      const uint32_t s = g % kStages;
-      if (!mbar_wait(bars + 8 * s, (g / kStages) & 1u)) {
-        atomicOr(p.status, kStatusMmaTimeout);
-        break;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t stage = base + s * kStageBytes;
-      const uint32_t sf_cols = tmem + kBN + s * kSfColsPerStage;
-      const uint32_t sfa_smem = stage + kABytes + kBBytes, sfb_smem = sfa_smem + kSfaBytes;
-#pragma unroll
-      for (uint32_t kb = kb0; kb < kb0 + 2u; ++kb) {
-        tmem_cp_sf(sf_cols + kb * 4u, smem_desc(sfa_smem + kb * 512u, 128u, 0u));
-        tmem_cp_sf(sf_cols + 16u + kb * 8u, smem_desc(sfb_smem + kb * 512u, 128u, 0u));
-        tmem_cp_sf(sf_cols + 16u + kb * 8u + 4u, smem_desc(sfb_smem + 2048u + kb * 512u, 128u, 0u));
-      }
-      mma_commit(bar_sf_ready + 8 * s);
-    }
-  } else if (warp < 4) {
-    // ---- epilogue: warp q owns accumulator lanes (tokens) 32 q .. 32 q + 31 ----
-    const uint32_t lane_base = tmem + (static_cast<uint32_t>(warp * 32) << 16);
-    uint32_t tile_i = 0;
-    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++tile_i) {
-      const uint32_t m_tile = tile % m_tiles, n_tile = tile / m_tiles;
-      if (!mbar_wait(bar_acc_full, tile_i & 1u)) {
-        if (lane == 0) atomicOr(p.status, kStatusEpilogueTimeout);
-        break;
-      }
-      w4a4_epilogue_tile(p, lane_base, warp, lane, m_tile, n_tile, swiglu, [&] {
-        if (lane == 0) mbar_arrive(bar_acc_empty);
-      });
-    }
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (warp == 5) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
-  }
-}
-
-// ---- the persistent form on CTA pairs ------------------------------------------------------------
+// ---- the product on CTA pairs --------------------------------------------------------------------
 // Two CTAs of a cluster share a 256-token x 256-row tile (tcgen05 cta_group::2): each CTA holds its
 // 128 tokens' codes and accumulator rows, and only half of the weight rows - the tensor cores read
-// the other half from the peer's shared memory - so a CTA brings 38 KB per K stage where the
-// single-CTA form brings 54 KB for the same FLOPs, and five stages fit where four did. Every load
-// of both CTAs reports to the barrier of the pair's first CTA, whose MMA thread issues for both;
+// the other half from the peer's shared memory - so a CTA brings 38 KB per K stage. The token tile index
+// runs fastest, so the pairs at work share weight rows in the L2. Every load
+// of both CTAs reports to the barrier of the pair's first CTA, whose MMA warp issues for both;
 // its commits arrive at both CTAs' barriers (two plain commits, one per CTA). The scale tiles
 // travel as TMA tiles too (a bulk copy cannot report to the peer's barrier): the scale planes as
 // [tile][128] words.
@@ -662,14 +482,10 @@ uint64_t w4a4_workspace_bytes(uint32_t k, uint32_t tokens) {
 bool w4a4_shape_ok(uint32_t n, uint32_t k) { return (k % 256u) == 0 && (n % 128u) == 0; }
 
 int32_t w4a4_prepare(ErrorSlot &slot) {
-  cudaError_t err = cudaFuncSetAttribute(w4a4_gemm_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(Tile<256>::kSmemBytes));
-  if (err == cudaSuccess) {
-    err = cudaFuncSetAttribute(w4a4_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kPairSmemBytes));
-  }
+  const cudaError_t err = cudaFuncSetAttribute(w4a4_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kPairSmemBytes));
   if (err != cudaSuccess) return fail(slot, "nvfp4 prefill kernel attributes: %s", cudaGetErrorString(err));
   if (encode_tiled_fn() == nullptr) return fail(slot, "cuTensorMapEncodeTiled is not available from this driver");
-  return 0;
+  return w4a4_narrow_prepare(slot);
 }
 
 namespace {
@@ -692,6 +508,11 @@ int32_t w4a4_product(ErrorSlot &slot, const DeviceState &dev, const uint8_t *w_c
                                    k, d_in, a_codes, a_scales);
     if (err != cudaSuccess) return fail(slot, "nvfp4 activation quantizer launch: %s", cudaGetErrorString(err));
   }
+  const bool swiglu = (epilogue & kEpilogueSwiglu) != 0u;
+  if (w4a4_narrow_takes(dev, n / (swiglu ? 256u : 128u), k, tokens, swiglu)) {
+    const A4Item item = {w_codes, w_scales, y, n, ldy, d_w, d_in};
+    return w4a4_narrow_launch(slot, dev, &item, 1, k, tokens, epilogue, a_codes, a_scales, status, q.codes, q.scales, q.d_in, stream);
+  }
   CUtensorMap map_a, map_b;
   if (!make_code_map(&map_a, a_codes, pad, k / 2u, kBM) || !make_code_map(&map_b, w_codes, n, k / 2u, 128u)) {
     return fail(slot, "nvfp4 prefill: tensor map encoding failed");
@@ -710,41 +531,30 @@ int32_t w4a4_product(ErrorSlot &slot, const DeviceState &dev, const uint8_t *w_c
   p.q_codes = q.codes;
   p.q_scales = q.scales;
   p.q_din = q.d_in;
-  const bool swiglu = (epilogue & kEpilogueSwiglu) != 0u;
-  // the fused SwiGLU needs the wide tile (gate and up boxes side by side); the plain product takes
-  // the narrow one, two CTAs per SM
-  if (dev.w4a4_pair != 0) {
-    // CTA pairs on 256-token x 256-row tiles
-    CUtensorMap map_sfa, map_sfb;
-    if (!make_scale_map(&map_sfa, a_scales, static_cast<uint64_t>(pad / kBM) * (k / 64u)) ||
-        !make_scale_map(&map_sfb, w_scales, static_cast<uint64_t>(n / 128u) * (k / 64u))) {
-      return fail(slot, "nvfp4 prefill: tensor map encoding failed");
-    }
-    const uint32_t m_pairs = (pad / kBM + 1u) / 2u;
-    const uint32_t tiles = m_pairs * (swiglu ? n / 256u : (n + 255u) / 256u);
-    const uint32_t pairs_max = static_cast<uint32_t>(dev.sm_count) / 2u;
-    cudaLaunchConfig_t config = {};
-    config.gridDim = dim3(2u * (tiles < pairs_max ? tiles : pairs_max), 1, 1);
-    config.blockDim = dim3(256, 1, 1);
-    config.dynamicSmemBytes = kPairSmemBytes;
-    config.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    config.attrs = attr;
-    config.numAttrs = dev.pdl ? 2 : 1;
-    const cudaError_t perr = cudaLaunchKernelEx(&config, w4a4_gemm_pair_kernel, map_a, map_b, map_sfa, map_sfb, p);
-    if (perr != cudaSuccess) return fail(slot, "nvfp4 prefill launch: %s", cudaGetErrorString(perr));
-    return 0;
+  // CTA pairs on 256-token x 256-row tiles
+  CUtensorMap map_sfa, map_sfb;
+  if (!make_scale_map(&map_sfa, a_scales, static_cast<uint64_t>(pad / kBM) * (k / 64u)) ||
+      !make_scale_map(&map_sfb, w_scales, static_cast<uint64_t>(n / 128u) * (k / 64u))) {
+    return fail(slot, "nvfp4 prefill: tensor map encoding failed");
   }
-  // B200Q_W4A4_PAIR = 0: the persistent form on single CTAs, 128-token x 256-row tiles
-  const uint32_t tiles = (pad / kBM) * (swiglu ? n / 256u : (n + 255u) / 256u);
-  const uint32_t ctas = tiles < static_cast<uint32_t>(dev.sm_count) ? tiles : static_cast<uint32_t>(dev.sm_count);
-  const cudaError_t perr = launch(w4a4_gemm_persistent_kernel, dim3(ctas), dim3(256), Tile<256>::kSmemBytes, stream, dev.pdl != 0, map_a, map_b, p);
+  const uint32_t m_pairs = (pad / kBM + 1u) / 2u;
+  const uint32_t tiles = m_pairs * (swiglu ? n / 256u : (n + 255u) / 256u);
+  const uint32_t pairs_max = static_cast<uint32_t>(dev.sm_count) / 2u;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(2u * (tiles < pairs_max ? tiles : pairs_max), 1, 1);
+  config.blockDim = dim3(256, 1, 1);
+  config.dynamicSmemBytes = kPairSmemBytes;
+  config.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = attr;
+  config.numAttrs = dev.pdl ? 2 : 1;
+  const cudaError_t perr = cudaLaunchKernelEx(&config, w4a4_gemm_pair_kernel, map_a, map_b, map_sfa, map_sfb, p);
   if (perr != cudaSuccess) return fail(slot, "nvfp4 prefill launch: %s", cudaGetErrorString(perr));
   return 0;
 }
@@ -768,6 +578,26 @@ int32_t w4a4_launch_prequantized(ErrorSlot &slot, const DeviceState &dev, const 
   uint8_t *a_scales = a_codes + static_cast<uint64_t>(pad) * (k / 2u);
   return w4a4_product(slot, dev, w_codes, w_scales, n, k, d_w, d_in, nullptr, tokens, y, ldy, epilogue,
                       reinterpret_cast<uint32_t *>(workspace), a_codes, a_scales, QuantTarget(), stream);
+}
+
+int32_t w4a4_launch_parts(ErrorSlot &slot, const DeviceState &dev, const A4Item *parts, uint32_t count, uint32_t k, const uint16_t *x,
+                          uint32_t tokens, uint32_t epilogue, uint8_t *workspace, cudaStream_t stream) {
+  const uint32_t pad = w4a4_tokens_pad(tokens);
+  uint32_t row_tiles = 0;
+  for (uint32_t i = 0; i < count; ++i) row_tiles += parts[i].n / 128u;
+  uint8_t *a_codes = workspace + 256, *a_scales = a_codes + static_cast<uint64_t>(pad) * (k / 2u);
+  uint32_t *status = reinterpret_cast<uint32_t *>(workspace);
+  if (w4a4_narrow_takes(dev, row_tiles, k, tokens, false)) {
+    if (w4a4_quantize_range(slot, dev, x, tokens, 0, tokens, k, parts[0].d_in, workspace, stream) != 0) return -1;
+    return w4a4_narrow_launch(slot, dev, parts, count, k, tokens, epilogue, a_codes, a_scales, status, nullptr, nullptr, 1.0f, stream);
+  }
+  for (uint32_t i = 0; i < count; ++i) {
+    if (w4a4_product(slot, dev, parts[i].codes, parts[i].scales, parts[i].n, k, parts[i].d_w, parts[i].d_in, i == 0 ? x : nullptr, tokens,
+                     parts[i].y, parts[i].ldy, epilogue, status, a_codes, a_scales, QuantTarget(), stream) != 0) {
+      return -1;
+    }
+  }
+  return 0;
 }
 
 // Quantizes tokens [token_begin, token_begin + token_count) of a call of `tokens_total` tokens into
