@@ -520,9 +520,10 @@ int32_t b200q_nvfp4_linear_prequantized(const b200q_nvfp4_weight *w, uint32_t to
   }
   const DeviceState *dev = prepared_state(slot, what);
   if (dev == nullptr) return -1;
-  return w4a4_launch_prequantized(slot, *dev, static_cast<const uint8_t *>(w->codes), static_cast<const uint8_t *>(w->scales), w->n, w->k,
-                                  w->weight_scale_divisor, w->input_scale_divisor, tokens, y, ldy, epilogue,
-                                  static_cast<uint8_t *>(workspace->base), static_cast<cudaStream_t>(stream));
+  const A4Item item = {static_cast<const uint8_t *>(w->codes), static_cast<const uint8_t *>(w->scales), y, w->n, ldy, w->weight_scale_divisor,
+                       w->input_scale_divisor};
+  return w4a4_launch_parts(slot, *dev, &item, 1, w->k, nullptr, tokens, epilogue, static_cast<uint8_t *>(workspace->base),
+                           static_cast<cudaStream_t>(stream));
 }
 
 const char *b200q_nvfp4_last_error(void) { return nvfp4_error().text; }

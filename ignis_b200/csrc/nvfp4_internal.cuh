@@ -95,7 +95,8 @@ int32_t w4a4_decode_status(ErrorSlot &slot, cudaStream_t stream, uint32_t *statu
 // W4A4 products of some dozens to some hundreds of tokens over activations quantized in the operand layout
 // (nvfp4_w4a4_narrow.cu); several weights may share one launch.
 int32_t w4a4_narrow_prepare(ErrorSlot &slot);
-bool w4a4_narrow_takes(const DeviceState &dev, uint32_t row_tiles, uint32_t k, uint32_t tokens, bool swiglu);
+// What a product over `row_tiles` tiles of 128 output rows is expected to cost there, in SM cycles.
+double w4a4_narrow_cycles(const DeviceState &dev, uint32_t row_tiles, uint32_t k, uint32_t tokens, bool swiglu);
 int32_t w4a4_narrow_launch(ErrorSlot &slot, const DeviceState &dev, const A4Item *items, uint32_t count, uint32_t k, uint32_t tokens,
                            uint32_t epilogue, const uint8_t *x_codes, const uint8_t *x_scales, uint32_t *status, uint8_t *q_codes,
                            uint8_t *q_scales, float q_din, cudaStream_t stream);
@@ -107,12 +108,8 @@ uint64_t w4a4_workspace_bytes(uint32_t k, uint32_t tokens);
 int32_t w4a4_launch(ErrorSlot &slot, const DeviceState &dev, const uint8_t *w_codes, const uint8_t *w_scales, uint32_t n,
                     uint32_t k, float d_w, float d_in, const uint16_t *x, uint32_t tokens, void *y, uint32_t ldy,
                     uint32_t epilogue, uint8_t *workspace, cudaStream_t stream);
-// The same product over activations already quantized in `workspace` by an earlier w4a4_launch of
-// the same x, k and token count (split-output parents: one quantization, a product per range).
-int32_t w4a4_launch_prequantized(ErrorSlot &slot, const DeviceState &dev, const uint8_t *w_codes, const uint8_t *w_scales,
-                                 uint32_t n, uint32_t k, float d_w, float d_in, uint32_t tokens, void *y, uint32_t ldy,
-                                 uint32_t epilogue, uint8_t *workspace, cudaStream_t stream);
-// Row ranges of one parent over one quantization of x: a launch for all of them where the narrow kernel takes the call.
+// Weights that share k and the input divisor (row ranges of one parent), in one launch; x nullptr: over the
+// activations already quantized in `workspace` by an earlier call of the same k and token count.
 int32_t w4a4_launch_parts(ErrorSlot &slot, const DeviceState &dev, const A4Item *parts, uint32_t count, uint32_t k, const uint16_t *x,
                           uint32_t tokens, uint32_t epilogue, uint8_t *workspace, cudaStream_t stream);
 int32_t w4a4_quantize_range(ErrorSlot &slot, const DeviceState &dev, const uint16_t *x_rows, uint32_t tokens_total,

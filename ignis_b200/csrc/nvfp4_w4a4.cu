@@ -78,18 +78,35 @@ __global__ void __launch_bounds__(256, 5) quantize_swizzled_kernel(const uint16_
   }
 }
 
-struct W4A4Params {
-  const uint8_t *sfa;   // activation scales, tile order
-  const uint8_t *sfb;   // weight scales, tile order
+// One weight of a launch (row ranges of one parent share the activations), with its first 256-row tile in the grid's walk.
+struct W4A4Weight {
   void *y;
-  uint32_t *status;
-  uint32_t tokens, n, k, ldy;
+  uint32_t n, ldy;
   float alpha;
+  uint32_t tile_begin;
+};
+struct W4A4Params {
+  W4A4Weight w[kMaxGroup];
+  uint32_t count, n_tiles;   // n_tiles: 256-row tiles of all weights
+  uint32_t *status;
+  uint32_t tokens, k;
   uint32_t epilogue;  // STORE / ADD / OUT_F32, or the fused SwiGLU (the tile's columns 0..127 are gate rows, 128..255 the up rows)
   uint8_t *q_codes;   // kEpilogueQuant: h as the next product's operand, codes [pad tokens][n / 4] ...
   uint8_t *q_scales;  // ... and scales in 512-byte tiles
   float q_din;        // the next weight's input divisor
 };
+struct W4A4Maps {
+  CUtensorMap b[kMaxGroup], sfb[kMaxGroup];   // the weights' codes and scales
+};
+
+// The weight that 256-row tile `n_tile` of the launch belongs to.
+__device__ __forceinline__ uint32_t weight_of(const W4A4Params &p, uint32_t n_tile) {
+  uint32_t wi = 0;
+  for (uint32_t i = 1; i < p.count; ++i) {
+    if (n_tile >= p.w[i].tile_begin) wi = i;
+  }
+  return wi;
+}
 
 // The epilogue pulls the whole accumulator into registers (as packed BF16: 128 registers a thread - the
 // CTA has the SM's register file to itself), hands tensor memory back to the MMA warp and only
@@ -99,9 +116,10 @@ struct W4A4Params {
 // hands tensor memory back to the MMA thread; it is called as soon as the accumulator has been
 // read, so that whatever follows runs under the next tile's MMAs.
 template <class Release>
-__device__ __forceinline__ void w4a4_epilogue_tile(const W4A4Params &p, uint32_t lane_base, int warp, int lane, uint32_t m_tile,
+__device__ __forceinline__ void w4a4_epilogue_tile(const W4A4Params &p, const W4A4Weight &w, uint32_t lane_base, int warp, int lane, uint32_t m_tile,
                                                    uint32_t n_tile, bool swiglu, Release release) {
   constexpr int kBN = 256;
+  const float alpha = w.alpha;
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t token = m_tile * kBM + warp * 32 + lane;
   if (p.epilogue & (kEpilogueF32 | kEpilogueAdd)) {
@@ -113,14 +131,14 @@ __device__ __forceinline__ void w4a4_epilogue_tile(const W4A4Params &p, uint32_t
       tmem_ld32(lane_base + c, r);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       const uint32_t row0 = n_tile * kBN + c;
-      if (token < p.tokens && row0 < p.n) {
+      if (token < p.tokens && row0 < w.n) {
         const bool add = (p.epilogue & kEpilogueAdd) != 0u;
         if (p.epilogue & kEpilogueF32) {
-          float4 *dst = reinterpret_cast<float4 *>(static_cast<float *>(p.y) + static_cast<size_t>(token) * p.ldy + row0);
+          float4 *dst = reinterpret_cast<float4 *>(static_cast<float *>(w.y) + static_cast<size_t>(token) * w.ldy + row0);
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            float4 o = make_float4(__uint_as_float(r[4 * j]) * p.alpha, __uint_as_float(r[4 * j + 1]) * p.alpha,
-                                   __uint_as_float(r[4 * j + 2]) * p.alpha, __uint_as_float(r[4 * j + 3]) * p.alpha);
+            float4 o = make_float4(__uint_as_float(r[4 * j]) * alpha, __uint_as_float(r[4 * j + 1]) * alpha,
+                                   __uint_as_float(r[4 * j + 2]) * alpha, __uint_as_float(r[4 * j + 3]) * alpha);
             if (add) {
               const float4 old = dst[j];
               o.x += old.x, o.y += old.y, o.z += old.z, o.w += old.w;
@@ -128,7 +146,7 @@ __device__ __forceinline__ void w4a4_epilogue_tile(const W4A4Params &p, uint32_t
             dst[j] = o;
           }
         } else {
-          uint4 *dst = reinterpret_cast<uint4 *>(static_cast<__nv_bfloat16 *>(p.y) + static_cast<size_t>(token) * p.ldy + row0);
+          uint4 *dst = reinterpret_cast<uint4 *>(static_cast<__nv_bfloat16 *>(w.y) + static_cast<size_t>(token) * w.ldy + row0);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const uint4 old = dst[j];
@@ -137,8 +155,8 @@ __device__ __forceinline__ void w4a4_epilogue_tile(const W4A4Params &p, uint32_t
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const __nv_bfloat162 h = __floats2bfloat162_rn(
-                  __uint_as_float(r[8 * j + 2 * e]) * p.alpha + bf16_bits_to_f32(ow[e] & 0xFFFFu),
-                  __uint_as_float(r[8 * j + 2 * e + 1]) * p.alpha + __uint_as_float(ow[e] & 0xFFFF0000u));
+                  __uint_as_float(r[8 * j + 2 * e]) * alpha + bf16_bits_to_f32(ow[e] & 0xFFFFu),
+                  __uint_as_float(r[8 * j + 2 * e + 1]) * alpha + __uint_as_float(ow[e] & 0xFFFF0000u));
               o[e] = *reinterpret_cast<const uint32_t *>(&h);
             }
             dst[j] = make_uint4(o[0], o[1], o[2], o[3]);
@@ -161,7 +179,7 @@ __device__ __forceinline__ void w4a4_epilogue_tile(const W4A4Params &p, uint32_t
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-      const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[2 * j]) * p.alpha, __uint_as_float(r[2 * j + 1]) * p.alpha);
+      const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[2 * j]) * alpha, __uint_as_float(r[2 * j + 1]) * alpha);
       out[c / 2 + j] = *reinterpret_cast<const uint32_t *>(&h);
     }
   }
@@ -169,6 +187,9 @@ __device__ __forceinline__ void w4a4_epilogue_tile(const W4A4Params &p, uint32_t
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncwarp();
   release();
+  // Rows past the call's tokens: nothing of them is read (as operand rows of the next product they only reach output rows
+  // that are not stored), and their zeros would take the divisions' slow paths (242 -> 175 us a layer at 300 tokens).
+  if (token >= p.tokens) return;
   if (swiglu) {
     // h = BF16(silu(BF16(g)) * BF16(u)), in place over the gate half
 #pragma unroll
@@ -181,8 +202,8 @@ __device__ __forceinline__ void w4a4_epilogue_tile(const W4A4Params &p, uint32_t
   }
   if (swiglu && (p.epilogue & kEpilogueQuant)) {
     // h leaves as the down product's operand: 8 blocks of 16 along its K, quantized as the
-    // standalone quantizer would from the BF16 values (padding rows are zeros and stay zeros)
-    const uint32_t inter = p.n / 2u, g0 = n_tile * 8u;
+    // standalone quantizer would from the BF16 values
+    const uint32_t inter = w.n / 2u, g0 = n_tile * 8u;
     uint32_t sc[2] = {0u, 0u};
     uint4 *code_dst = reinterpret_cast<uint4 *>(p.q_codes + static_cast<uint64_t>(token) * (inter / 2u) + n_tile * 64u);
 #pragma unroll
@@ -202,16 +223,14 @@ __device__ __forceinline__ void w4a4_epilogue_tile(const W4A4Params &p, uint32_t
     *reinterpret_cast<uint32_t *>(p.q_scales + atom + 512u) = sc[1];
     return;
   }
-  if (token < p.tokens) {
-    const uint32_t width = swiglu ? 128u : kBN;
-    const uint32_t col0 = n_tile * width;
-    const uint32_t limit = swiglu ? p.n / 2u : p.n;
-    __nv_bfloat16 *row = static_cast<__nv_bfloat16 *>(p.y) + static_cast<size_t>(token) * p.ldy + col0;
+  const uint32_t width = swiglu ? 128u : kBN;
+  const uint32_t col0 = n_tile * width;
+  const uint32_t limit = swiglu ? w.n / 2u : w.n;
+  __nv_bfloat16 *row = static_cast<__nv_bfloat16 *>(w.y) + static_cast<size_t>(token) * w.ldy + col0;
 #pragma unroll
-    for (uint32_t c = 0; c < kBN; c += 8) {
-      if (c < width && col0 + c < limit) {  // n is a multiple of 128: an 8-column piece is whole
-        *reinterpret_cast<uint4 *>(row + c) = make_uint4(out[c / 2], out[c / 2 + 1], out[c / 2 + 2], out[c / 2 + 3]);
-      }
+  for (uint32_t c = 0; c < kBN; c += 8) {
+    if (c < width && col0 + c < limit) {  // n is a multiple of 128: an 8-column piece is whole
+      *reinterpret_cast<uint4 *>(row + c) = make_uint4(out[c / 2], out[c / 2 + 1], out[c / 2 + 2], out[c / 2 + 3]);
     }
   }
 }
@@ -261,9 +280,8 @@ __device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
 }
 
 __global__ void __launch_bounds__(256, 1) w4a4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
-                                                               const __grid_constant__ CUtensorMap map_b,
                                                                const __grid_constant__ CUtensorMap map_sfa,
-                                                               const __grid_constant__ CUtensorMap map_sfb,
+                                                               const __grid_constant__ W4A4Maps maps,
                                                                const __grid_constant__ W4A4Params p) {
   constexpr int kBN = 256;
   constexpr int kStages = kPairStages;
@@ -282,8 +300,7 @@ __global__ void __launch_bounds__(256, 1) w4a4_gemm_pair_kernel(const __grid_con
   const uint32_t k_iters = p.k / 256u, k_atoms = p.k / 64u;
   const bool swiglu = (p.epilogue & kEpilogueSwiglu) != 0u;
   const uint32_t m_tiles = (p.tokens + kBM - 1) / kBM, m_pairs = (m_tiles + 1u) / 2u;
-  const uint32_t n_tiles = swiglu ? p.n / 256u : (p.n + 255u) / 256u;
-  const uint32_t tiles = m_pairs * n_tiles;
+  const uint32_t tiles = m_pairs * p.n_tiles;
   const uint32_t first = blockIdx.x / 2u, step = gridDim.x / 2u;
 
   if (threadIdx.x == 0) {
@@ -317,9 +334,10 @@ __global__ void __launch_bounds__(256, 1) w4a4_gemm_pair_kernel(const __grid_con
     const uint32_t full0 = in_cta(bars, 0u);   // the first CTA's barriers collect both CTAs' bytes
     bool ok = true;
     for (uint32_t tile = first; tile < tiles && ok; tile += step) {
-      const uint32_t m_tile = 2u * (tile % m_pairs) + rank, n_tile = tile / m_pairs;
+      const uint32_t m_tile = 2u * (tile % m_pairs) + rank, wi = weight_of(p, tile / m_pairs), n_tile = tile / m_pairs - p.w[wi].tile_begin;
+      const CUtensorMap *map_b = &maps.b[wi], *map_sfb = &maps.sfb[wi];
       const uint32_t row_a = swiglu ? n_tile * 128u : n_tile * kBN;
-      const uint32_t row_b = swiglu ? p.n / 2u + n_tile * 128u : n_tile * kBN + 128u;
+      const uint32_t row_b = swiglu ? p.w[wi].n / 2u + n_tile * 128u : n_tile * kBN + 128u;
       const int32_t row = static_cast<int32_t>(rank == 0u ? row_a : row_b);
       const uint32_t sfa0 = m_tile * k_atoms, sfb0 = row_a / 128u * k_atoms, sfb1 = row_b / 128u * k_atoms;
       for (uint32_t it = 0; it < k_iters; ++it, at.advance(1u, kStages)) {
@@ -332,10 +350,10 @@ __global__ void __launch_bounds__(256, 1) w4a4_gemm_pair_kernel(const __grid_con
           const uint32_t full = full0 + 8 * at.slot, stage = base + at.slot * kPairStageBytes;
           if (rank == 0u) mbar_expect_tx(bars + 8 * at.slot, 2u * kPairStageBytes);
           tma_load_2d_pair(stage, &map_a, full, static_cast<int32_t>(it * kBKBytes), static_cast<int32_t>(m_tile * kBM));
-          tma_load_2d_pair(stage + kABytes, &map_b, full, static_cast<int32_t>(it * kBKBytes), row);
+          tma_load_2d_pair(stage + kABytes, map_b, full, static_cast<int32_t>(it * kBKBytes), row);
           tma_load_2d_pair(stage + kABytes + kPairBBytes, &map_sfa, full, 0, static_cast<int32_t>(sfa0 + it * 4u));
-          tma_load_2d_pair(stage + kABytes + kPairBBytes + kSfaBytes, &map_sfb, full, 0, static_cast<int32_t>(sfb0 + it * 4u));
-          tma_load_2d_pair(stage + kABytes + kPairBBytes + kSfaBytes + 2048u, &map_sfb, full, 0, static_cast<int32_t>(sfb1 + it * 4u));
+          tma_load_2d_pair(stage + kABytes + kPairBBytes + kSfaBytes, map_sfb, full, 0, static_cast<int32_t>(sfb0 + it * 4u));
+          tma_load_2d_pair(stage + kABytes + kPairBBytes + kSfaBytes + 2048u, map_sfb, full, 0, static_cast<int32_t>(sfb1 + it * 4u));
         }
         __syncwarp();
       }
@@ -418,7 +436,7 @@ __global__ void __launch_bounds__(256, 1) w4a4_gemm_pair_kernel(const __grid_con
     const uint32_t acc_empty_first = in_cta(bar_acc_empty, 0u);
     uint32_t tile_i = 0;
     for (uint32_t tile = first; tile < tiles; tile += step, ++tile_i) {
-      const uint32_t m_tile = 2u * (tile % m_pairs) + rank, n_tile = tile / m_pairs;
+      const uint32_t m_tile = 2u * (tile % m_pairs) + rank, wi = weight_of(p, tile / m_pairs), n_tile = tile / m_pairs - p.w[wi].tile_begin;
       if (!mbar_wait(bar_acc_full, tile_i & 1u)) {
         if (lane == 0) atomicOr(p.status, kStatusEpilogueTimeout);
         break;
@@ -429,7 +447,7 @@ __global__ void __launch_bounds__(256, 1) w4a4_gemm_pair_kernel(const __grid_con
         if (lane == 0) mbar_arrive_cluster(acc_empty_first);
         continue;
       }
-      w4a4_epilogue_tile(p, lane_base, warp, lane, m_tile, n_tile, swiglu, [&] {
+      w4a4_epilogue_tile(p, p.w[wi], lane_base, warp, lane, m_tile, n_tile, swiglu, [&] {
         if (lane == 0) mbar_arrive_cluster(acc_empty_first);
       });
     }
@@ -495,50 +513,66 @@ struct QuantTarget {
   float d_in = 1.0f;
 };
 
-// One product over activations at `a_codes` / `a_scales`; `x` non-NULL quantizes them there first.
-int32_t w4a4_product(ErrorSlot &slot, const DeviceState &dev, const uint8_t *w_codes, const uint8_t *w_scales, uint32_t n,
-                     uint32_t k, float d_w, float d_in, const uint16_t *x, uint32_t tokens, void *y, uint32_t ldy,
-                     uint32_t epilogue, uint32_t *status, uint8_t *a_codes, uint8_t *a_scales, const QuantTarget &q,
-                     cudaStream_t stream) {
+// Which kernel a product takes: the cheaper by what each is expected to cost, in SM cycles. The pair kernel: waves of
+// 256 x 256 tiles on half as many pairs as SMs, 820 cycles a stage of 256 (its loads) and 3000 a tile, never faster than
+// the weights come from HBM; `w4a4_narrow_cycles` beside its kernel. Measured (27B-style shapes): gate|up at 77 tokens
+// 22 us narrow, 28 pair; at 512 67 against 50; down at 200 tokens 24 against 33.
+bool narrow_is_cheaper(const DeviceState &dev, const A4Item *items, uint32_t count, uint32_t k, uint32_t tokens, bool swiglu) {
+  if (dev.w4a4_pair >= 0) return dev.w4a4_pair == 0;
+  uint32_t row_tiles = 0, n_tiles = 0;
+  for (uint32_t i = 0; i < count; ++i) {
+    row_tiles += items[i].n / (swiglu ? 256u : 128u);
+    n_tiles += (items[i].n + 255u) / 256u;
+  }
+  const double tiles = static_cast<double>(n_tiles) * ((tokens + 255u) / 256u);
+  const double walk = ceil(tiles / (dev.sm_count / 2)) * ((k / 256u) * 820.0 + 3000.0);
+  const double stream = row_tiles * (swiglu ? 144.0 : 72.0) * k / 3150.0;
+  return w4a4_narrow_cycles(dev, row_tiles, k, tokens, swiglu) < 5000.0 + (walk > stream ? walk : stream);
+}
+
+int32_t quantize_rows(ErrorSlot &slot, const DeviceState &dev, const uint16_t *x, uint32_t tokens, uint32_t k, float d_in, uint8_t *codes,
+                      uint8_t *scales, cudaStream_t stream) {
   const uint32_t pad = w4a4_tokens_pad(tokens);
-  if (x != nullptr) {
-    const uint64_t total = static_cast<uint64_t>(pad) * (k / 32u);
-    const uint32_t grid = static_cast<uint32_t>(total / 256u < 148u * 24u ? (total + 255u) / 256u : 148u * 24u);
-    const cudaError_t err = launch(quantize_swizzled_kernel, dim3(grid), dim3(256), 0, stream, dev.pdl != 0, x, tokens, pad,
-                                   k, d_in, a_codes, a_scales);
-    if (err != cudaSuccess) return fail(slot, "nvfp4 activation quantizer launch: %s", cudaGetErrorString(err));
-  }
+  const uint64_t total = static_cast<uint64_t>(pad) * (k / 32u);
+  const uint32_t grid = static_cast<uint32_t>(total / 256u < 148u * 24u ? (total + 255u) / 256u : 148u * 24u);
+  const cudaError_t err = launch(quantize_swizzled_kernel, dim3(grid), dim3(256), 0, stream, dev.pdl != 0, x, tokens, pad, k, d_in, codes, scales);
+  if (err != cudaSuccess) return fail(slot, "nvfp4 activation quantizer launch: %s", cudaGetErrorString(err));
+  return 0;
+}
+
+// The products of `count` weights that share k over the operand at `a_codes` / `a_scales`, in one launch; `x` non-NULL
+// is quantized there first.
+int32_t w4a4_products(ErrorSlot &slot, const DeviceState &dev, const A4Item *items, uint32_t count, uint32_t k, const uint16_t *x,
+                      uint32_t tokens, uint32_t epilogue, uint32_t *status, uint8_t *a_codes, uint8_t *a_scales, const QuantTarget &q,
+                      cudaStream_t stream) {
+  const uint32_t pad = w4a4_tokens_pad(tokens);
+  if (x != nullptr && quantize_rows(slot, dev, x, tokens, k, items[0].d_in, a_codes, a_scales, stream) != 0) return -1;
   const bool swiglu = (epilogue & kEpilogueSwiglu) != 0u;
-  if (w4a4_narrow_takes(dev, n / (swiglu ? 256u : 128u), k, tokens, swiglu)) {
-    const A4Item item = {w_codes, w_scales, y, n, ldy, d_w, d_in};
-    return w4a4_narrow_launch(slot, dev, &item, 1, k, tokens, epilogue, a_codes, a_scales, status, q.codes, q.scales, q.d_in, stream);
-  }
-  CUtensorMap map_a, map_b;
-  if (!make_code_map(&map_a, a_codes, pad, k / 2u, kBM) || !make_code_map(&map_b, w_codes, n, k / 2u, 128u)) {
-    return fail(slot, "nvfp4 prefill: tensor map encoding failed");
+  if (narrow_is_cheaper(dev, items, count, k, tokens, swiglu)) {
+    return w4a4_narrow_launch(slot, dev, items, count, k, tokens, epilogue, a_codes, a_scales, status, q.codes, q.scales, q.d_in, stream);
   }
   W4A4Params p = {};
-  p.sfa = a_scales;
-  p.sfb = w_scales;
-  p.y = y;
+  W4A4Maps maps = {};
+  CUtensorMap map_a, map_sfa;
+  bool encoded = make_code_map(&map_a, a_codes, pad, k / 2u, kBM) &&
+                 make_scale_map(&map_sfa, a_scales, static_cast<uint64_t>(pad / kBM) * (k / 64u));
+  p.count = count;
+  for (uint32_t i = 0; i < count; ++i) {
+    const A4Item &it = items[i];
+    p.w[i] = W4A4Weight{it.y, it.n, it.ldy, 1.0f / (it.d_in * it.d_w), p.n_tiles};
+    p.n_tiles += (it.n + 255u) / 256u;
+    encoded = encoded && make_code_map(&maps.b[i], it.codes, it.n, k / 2u, 128u) &&
+              make_scale_map(&maps.sfb[i], it.scales, static_cast<uint64_t>(it.n / 128u) * (k / 64u));
+  }
+  if (!encoded) return fail(slot, "nvfp4 prefill: tensor map encoding failed");
   p.status = status;
   p.tokens = tokens;
-  p.n = n;
   p.k = k;
-  p.ldy = ldy;
-  p.alpha = 1.0f / (d_in * d_w);
   p.epilogue = epilogue;
   p.q_codes = q.codes;
   p.q_scales = q.scales;
   p.q_din = q.d_in;
-  // CTA pairs on 256-token x 256-row tiles
-  CUtensorMap map_sfa, map_sfb;
-  if (!make_scale_map(&map_sfa, a_scales, static_cast<uint64_t>(pad / kBM) * (k / 64u)) ||
-      !make_scale_map(&map_sfb, w_scales, static_cast<uint64_t>(n / 128u) * (k / 64u))) {
-    return fail(slot, "nvfp4 prefill: tensor map encoding failed");
-  }
-  const uint32_t m_pairs = (pad / kBM + 1u) / 2u;
-  const uint32_t tiles = m_pairs * (swiglu ? n / 256u : (n + 255u) / 256u);
+  const uint32_t tiles = (pad / kBM + 1u) / 2u * p.n_tiles;
   const uint32_t pairs_max = static_cast<uint32_t>(dev.sm_count) / 2u;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(2u * (tiles < pairs_max ? tiles : pairs_max), 1, 1);
@@ -554,50 +588,25 @@ int32_t w4a4_product(ErrorSlot &slot, const DeviceState &dev, const uint8_t *w_c
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attr;
   config.numAttrs = dev.pdl ? 2 : 1;
-  const cudaError_t perr = cudaLaunchKernelEx(&config, w4a4_gemm_pair_kernel, map_a, map_b, map_sfa, map_sfb, p);
-  if (perr != cudaSuccess) return fail(slot, "nvfp4 prefill launch: %s", cudaGetErrorString(perr));
+  const cudaError_t err = cudaLaunchKernelEx(&config, w4a4_gemm_pair_kernel, map_a, map_sfa, maps, p);
+  if (err != cudaSuccess) return fail(slot, "nvfp4 prefill launch: %s", cudaGetErrorString(err));
   return 0;
 }
 }  // namespace
 
+int32_t w4a4_launch_parts(ErrorSlot &slot, const DeviceState &dev, const A4Item *parts, uint32_t count, uint32_t k, const uint16_t *x,
+                          uint32_t tokens, uint32_t epilogue, uint8_t *workspace, cudaStream_t stream) {
+  uint8_t *a_codes = workspace + 256;
+  uint8_t *a_scales = a_codes + static_cast<uint64_t>(w4a4_tokens_pad(tokens)) * (k / 2u);
+  return w4a4_products(slot, dev, parts, count, k, x, tokens, epilogue, reinterpret_cast<uint32_t *>(workspace), a_codes, a_scales, QuantTarget(),
+                       stream);
+}
+
 int32_t w4a4_launch(ErrorSlot &slot, const DeviceState &dev, const uint8_t *w_codes, const uint8_t *w_scales, uint32_t n,
                     uint32_t k, float d_w, float d_in, const uint16_t *x, uint32_t tokens, void *y, uint32_t ldy,
                     uint32_t epilogue, uint8_t *workspace, cudaStream_t stream) {
-  const uint32_t pad = w4a4_tokens_pad(tokens);
-  uint8_t *a_codes = workspace + 256;
-  uint8_t *a_scales = a_codes + static_cast<uint64_t>(pad) * (k / 2u);
-  return w4a4_product(slot, dev, w_codes, w_scales, n, k, d_w, d_in, x, tokens, y, ldy, epilogue,
-                      reinterpret_cast<uint32_t *>(workspace), a_codes, a_scales, QuantTarget(), stream);
-}
-
-int32_t w4a4_launch_prequantized(ErrorSlot &slot, const DeviceState &dev, const uint8_t *w_codes, const uint8_t *w_scales,
-                                 uint32_t n, uint32_t k, float d_w, float d_in, uint32_t tokens, void *y, uint32_t ldy,
-                                 uint32_t epilogue, uint8_t *workspace, cudaStream_t stream) {
-  const uint32_t pad = w4a4_tokens_pad(tokens);
-  uint8_t *a_codes = workspace + 256;
-  uint8_t *a_scales = a_codes + static_cast<uint64_t>(pad) * (k / 2u);
-  return w4a4_product(slot, dev, w_codes, w_scales, n, k, d_w, d_in, nullptr, tokens, y, ldy, epilogue,
-                      reinterpret_cast<uint32_t *>(workspace), a_codes, a_scales, QuantTarget(), stream);
-}
-
-int32_t w4a4_launch_parts(ErrorSlot &slot, const DeviceState &dev, const A4Item *parts, uint32_t count, uint32_t k, const uint16_t *x,
-                          uint32_t tokens, uint32_t epilogue, uint8_t *workspace, cudaStream_t stream) {
-  const uint32_t pad = w4a4_tokens_pad(tokens);
-  uint32_t row_tiles = 0;
-  for (uint32_t i = 0; i < count; ++i) row_tiles += parts[i].n / 128u;
-  uint8_t *a_codes = workspace + 256, *a_scales = a_codes + static_cast<uint64_t>(pad) * (k / 2u);
-  uint32_t *status = reinterpret_cast<uint32_t *>(workspace);
-  if (w4a4_narrow_takes(dev, row_tiles, k, tokens, false)) {
-    if (w4a4_quantize_range(slot, dev, x, tokens, 0, tokens, k, parts[0].d_in, workspace, stream) != 0) return -1;
-    return w4a4_narrow_launch(slot, dev, parts, count, k, tokens, epilogue, a_codes, a_scales, status, nullptr, nullptr, 1.0f, stream);
-  }
-  for (uint32_t i = 0; i < count; ++i) {
-    if (w4a4_product(slot, dev, parts[i].codes, parts[i].scales, parts[i].n, k, parts[i].d_w, parts[i].d_in, i == 0 ? x : nullptr, tokens,
-                     parts[i].y, parts[i].ldy, epilogue, status, a_codes, a_scales, QuantTarget(), stream) != 0) {
-      return -1;
-    }
-  }
-  return 0;
+  const A4Item item = {w_codes, w_scales, y, n, ldy, d_w, d_in};
+  return w4a4_launch_parts(slot, dev, &item, 1, k, x, tokens, epilogue, workspace, stream);
 }
 
 // Quantizes tokens [token_begin, token_begin + token_count) of a call of `tokens_total` tokens into
@@ -608,15 +617,9 @@ int32_t w4a4_quantize_range(ErrorSlot &slot, const DeviceState &dev, const uint1
                             uint32_t token_begin, uint32_t token_count, uint32_t k, float d_in, uint8_t *workspace,
                             cudaStream_t stream) {
   const uint64_t pad_total = w4a4_tokens_pad(tokens_total);
-  const uint32_t pad = w4a4_tokens_pad(token_count);
   uint8_t *codes = workspace + 256 + static_cast<uint64_t>(token_begin) * (k / 2u);
   uint8_t *scales = workspace + 256 + pad_total * (k / 2u) + static_cast<uint64_t>(token_begin / 128u) * (k / 64u) * 512u;
-  const uint64_t total = static_cast<uint64_t>(pad) * (k / 32u);
-  const uint32_t grid = static_cast<uint32_t>(total / 256u < 148u * 24u ? (total + 255u) / 256u : 148u * 24u);
-  const cudaError_t err = launch(quantize_swizzled_kernel, dim3(grid), dim3(256), 0, stream, dev.pdl != 0, x_rows, token_count, pad, k,
-                                 d_in, codes, scales);
-  if (err != cudaSuccess) return fail(slot, "nvfp4 activation quantizer launch: %s", cudaGetErrorString(err));
-  return 0;
+  return quantize_rows(slot, dev, x_rows, token_count, k, d_in, codes, scales, stream);
 }
 
 // Workspace of the MLP: the status line, x quantized (K = k), h quantized (K = inter).
@@ -638,12 +641,9 @@ int32_t w4a4_mlp_launch(ErrorSlot &slot, const DeviceState &dev, const uint8_t *
   h.codes = x_scales + pad * (k / 16u);
   h.scales = h.codes + pad * (inter / 2u);
   h.d_in = dn_din;
-  if (w4a4_product(slot, dev, gu_codes, gu_scales, gu_n, k, gu_dw, gu_din, x, tokens, nullptr, 0, kEpilogueSwiglu | kEpilogueQuant,
-                   status, x_codes, x_scales, h, stream) != 0) {
-    return -1;
-  }
-  return w4a4_product(slot, dev, dn_codes, dn_scales, dn_n, inter, dn_dw, dn_din, nullptr, tokens, y, ldy, epilogue, status,
-                      h.codes, h.scales, QuantTarget(), stream);
+  const A4Item gate_up = {gu_codes, gu_scales, nullptr, gu_n, 0, gu_dw, gu_din}, down = {dn_codes, dn_scales, y, dn_n, ldy, dn_dw, dn_din};
+  if (w4a4_products(slot, dev, &gate_up, 1, k, x, tokens, kEpilogueSwiglu | kEpilogueQuant, status, x_codes, x_scales, h, stream) != 0) return -1;
+  return w4a4_products(slot, dev, &down, 1, inter, nullptr, tokens, epilogue, status, h.codes, h.scales, QuantTarget(), stream);
 }
 
 }  // namespace b200q

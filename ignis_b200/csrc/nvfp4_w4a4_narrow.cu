@@ -3,8 +3,8 @@
 // The pair GEMM's 256 x 256 tiles leave most of the device idle there - 20 tiles for a 5120-row weight
 // on 74 CTA pairs, each walking all of K - while the weights still bound the call: 48 to 100 MB of them.
 //
-//  * The weights are the MMA's A operand: a CTA owns 128 weight rows (M) and up to 128 or 256 tokens (N, as few as
-//    the call has, in steps of 16) and walks a slice of K in stages of 256 values; the CTAs of a cluster
+//  * The weights are the MMA's A operand: a CTA owns 128 weight rows (M) and up to 128 tokens (N, as few as the
+//    call has, in steps of 16) and walks a slice of K in stages of 256 values; the CTAs of a cluster
 //    split K, so that narrow weights fill the device too, and add their sums through distributed
 //    shared memory in rank order.
 //  * Warp 8 brings a stage's weight codes and token codes by TMA (128-byte swizzle) and their scale tiles by
@@ -19,7 +19,7 @@
 #include "nvfp4_internal.cuh"
 #include "nvfp4_tc.cuh"
 
-#include <cstdlib>
+#include <cmath>
 
 namespace b200q {
 namespace {
@@ -46,10 +46,9 @@ struct NarrowParams {
   const uint8_t *sfx;    // the tokens' scale tiles
   uint32_t *status;
   uint32_t count, k, tokens;
-  uint32_t tile;         // tokens per CTA: a multiple of 16 up to 128, or 256
+  uint32_t tile;         // tokens per CTA: a multiple of 16 up to 128
   uint32_t stages, kc, tmem_cols;
   uint32_t acc_stride;   // tensor-memory columns from the first accumulator to the second
-  uint32_t sf_bufs;      // stages of scales in tensor memory: 1 or 2
   uint32_t epilogue;     // STORE / ADD / OUT_F32, the fused SwiGLU, or the fused SwiGLU quantized
   uint8_t *q_codes;      // kEpilogueQuant: h as the next product's operand
   uint8_t *q_scales;
@@ -84,10 +83,10 @@ __global__ void __launch_bounds__(kNarrowThreads, 2) w4a4_narrow_kernel(const __
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t *base_ptr = smem_raw + (base - raw);
-  const uint32_t x_bytes = p.tile * 128u, x_tiles = p.tile > 128u ? 2u : 1u;   // scale tiles of 128 tokens
-  // a stage: weight codes [TILES] | token codes | weight scales [TILES] | token scales [x_tiles]
+  const uint32_t x_bytes = p.tile * 128u;
+  // a stage: weight codes [TILES] | token codes | weight scales [TILES] | token scales
   const uint32_t sf_off = TILES * kABytes + x_bytes;
-  const uint32_t stage_bytes = sf_off + (TILES + x_tiles) * kSfBytes, stage_pitch = (stage_bytes + 1023u) & ~1023u;
+  const uint32_t stage_bytes = sf_off + (TILES + 1) * kSfBytes, stage_pitch = (stage_bytes + 1023u) & ~1023u;
   const uint32_t bars = base + p.stages * stage_pitch;   // full[stages], empty[stages], accumulator full; then the TMEM slot
   const uint32_t bar_empty = bars + 8u * p.stages, bar_acc = bar_empty + 8u * p.stages;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(base_ptr + (bar_acc - base) + 8u);
@@ -156,11 +155,7 @@ __global__ void __launch_bounds__(kNarrowThreads, 2) w4a4_narrow_kernel(const __
     auto tokens = [&](uint32_t s, uint32_t slot) {
       const uint32_t full = bars + 8 * slot, stage = base + slot * stage_pitch;
       tma_load_2d(stage + TILES * kABytes, &maps.x, full, static_cast<int32_t>(s * 128u), static_cast<int32_t>(tok0));
-      for (uint32_t t = 0; t < x_tiles; ++t) {
-        // the second scale tile of a last, short token tile need not exist: the first stands in for it
-        const uint32_t tile = tok0 + t * 128u < p.tokens ? t : 0u;
-        bulk_load(stage + sf_off + (TILES + t) * kSfBytes, sfx + (static_cast<size_t>(tile) * k_atoms + s * 4u) * 512u, kSfBytes, full);
-      }
+      bulk_load(stage + sf_off + TILES * kSfBytes, sfx + static_cast<size_t>(s) * kSfBytes, kSfBytes, full);
     };
     // the weights never depend on the previous kernel, the tokens come from it
     const uint32_t ahead = min(p.stages, s1 - s0);
@@ -191,7 +186,7 @@ __global__ void __launch_bounds__(kNarrowThreads, 2) w4a4_narrow_kernel(const __
     // E2M1 x E2M1 (format 1 at bits 7 and 10), both K-major, N >> 3 at bit 17, UE4M3 scales, M >> 4 at bit 24
     const uint32_t idesc = (1u << 7) | (1u << 10) | ((mma_n >> 3) << 17) | ((128u >> 4) << 24);
     const uint64_t desc0 = smem_desc(base, 1024u, 2u), sf_desc0 = smem_desc(base + sf_off, 128u, 0u);
-    const uint32_t pitch = stage_pitch >> 4, buf_cols = TILES * 16u + x_tiles * 16u, x_cols = x_tiles * 4u;   // x_cols: per K-atom
+    const uint32_t pitch = stage_pitch >> 4, buf_cols = (TILES + 1) * 16u;
     bool ok = true;
     RingAt at;
     for (uint32_t it = 0; it < s1 - s0; ++it, at.advance(1u, p.stages)) {
@@ -202,14 +197,13 @@ __global__ void __launch_bounds__(kNarrowThreads, 2) w4a4_narrow_kernel(const __
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (elect_one()) {
-        const uint32_t sfw_cols = sf_cols0 + (it & (p.sf_bufs - 1u)) * buf_cols, sfx_cols = sfw_cols + TILES * 16u;
+        const uint32_t sfw_cols = sf_cols0 + (it & 1u) * buf_cols, sfx_cols = sfw_cols + TILES * 16u;
         const uint64_t sf = sf_desc0 + at.slot * pitch;
 #pragma unroll
         for (uint32_t kb = 0; kb < 4; ++kb) {
 #pragma unroll
           for (uint32_t t = 0; t < TILES; ++t) tmem_cp_sf(sfw_cols + t * 16u + kb * 4u, sf + t * (kSfBytes >> 4) + kb * 32u);
-          tmem_cp_sf(sfx_cols + kb * x_cols, sf + TILES * (kSfBytes >> 4) + kb * 32u);
-          if (x_tiles == 2u) tmem_cp_sf(sfx_cols + kb * x_cols + 4u, sf + (TILES + 1) * (kSfBytes >> 4) + kb * 32u);
+          tmem_cp_sf(sfx_cols + kb * 4u, sf + TILES * (kSfBytes >> 4) + kb * 32u);
         }
         const uint64_t a_desc = desc0 + at.slot * pitch, b_desc = a_desc + TILES * (kABytes >> 4);
 #pragma unroll
@@ -217,7 +211,7 @@ __global__ void __launch_bounds__(kNarrowThreads, 2) w4a4_narrow_kernel(const __
 #pragma unroll
           for (uint32_t t = 0; t < TILES; ++t) {
             mma_mxf4nvf4(tmem + t * p.acc_stride, a_desc + t * (kABytes >> 4) + 2u * kb, b_desc + 2u * kb, idesc, sfw_cols + t * 16u + kb * 4u,
-                         sfx_cols + kb * x_cols, (it | kb) != 0u ? 1u : 0u);
+                         sfx_cols + kb * 4u, (it | kb) != 0u ? 1u : 0u);
           }
         }
         mma_commit(bar_empty + 8 * at.slot);
@@ -347,39 +341,26 @@ __global__ void __launch_bounds__(kNarrowThreads, 2) w4a4_narrow_kernel(const __
 constexpr size_t kNarrowMaxSmem = 222 * 1024;
 
 struct NarrowPlan {
-  uint32_t tiles, tile, kc, stages, acc_stride, sf_bufs, tmem_cols;
+  uint32_t tiles, tile, kc, stages, acc_stride, tmem_cols;
 };
 
-uint32_t narrow_pitch(const NarrowPlan &pl) {
-  const uint32_t bytes = pl.tiles * (kABytes + kSfBytes) + pl.tile * 128u + (pl.tile > 128u ? 2u : 1u) * kSfBytes;
-  return (bytes + 1023u) & ~1023u;
-}
+uint32_t narrow_pitch(const NarrowPlan &pl) { return (pl.tiles * (kABytes + kSfBytes) + pl.tile * 128u + kSfBytes + 1023u) & ~1023u; }
 size_t narrow_smem(const NarrowPlan &pl) { return static_cast<size_t>(pl.stages) * narrow_pitch(pl) + 16u * pl.stages + 32u + 1024u; }
 
-NarrowPlan narrow_plan(const DeviceState &dev, uint32_t row_tiles, uint32_t k_stages, uint32_t tokens, bool swiglu, bool quant) {
+// One CTA per SM with as deep a ring as fits (two with half the ring each: 80 us against 72 a layer at 77 tokens), K split
+// while the CTAs still run as one wave and a CTA keeps four stages.
+NarrowPlan narrow_plan(const DeviceState &dev, uint32_t row_tiles, uint32_t k_stages, uint32_t tokens, bool swiglu) {
   NarrowPlan pl = {};
   pl.tiles = swiglu ? 2u : 1u;
-  pl.tile = tokens <= 128u ? (tokens + 15u) / 16u * 16u : (swiglu ? 128u : 256u);
-  if (const char *e = getenv("NW_TILE")) { if (tokens > 128u) pl.tile = atoi(e); }
+  pl.tile = tokens <= 128u ? (tokens + 15u) / 16u * 16u : 128u;   // several token tiles start on whole scale tiles
   pl.acc_stride = (pl.tile + 31u) / 32u * 32u;
-  const uint32_t sf_cols = pl.tiles * 16u + (pl.tile > 128u ? 32u : 16u), acc = pl.tiles * pl.acc_stride;
   pl.tmem_cols = 64u;
-  while (pl.tmem_cols < acc + sf_cols) pl.tmem_cols <<= 1;
-  pl.sf_bufs = acc + 2u * sf_cols <= pl.tmem_cols ? 2u : 1u;
-  uint32_t per_sm = pl.tmem_cols <= 256u ? 2u : 1u;
-  if (const char *e = getenv("NW_PERSM")) { if (atoi(e) == 1) per_sm = 1; }
+  while (pl.tmem_cols < pl.tiles * pl.acc_stride + 2u * (pl.tiles + 1u) * 16u) pl.tmem_cols <<= 1;   // two stages of scales behind the accumulators
+  const uint32_t blocks = row_tiles * ((tokens + pl.tile - 1u) / pl.tile), sms = static_cast<uint32_t>(dev.sm_count);
   pl.kc = 1;
-  const uint32_t token_tiles = (tokens + pl.tile - 1u) / pl.tile;
-  const uint32_t slots = dev.sm_count * per_sm;
-  while (pl.kc < 8u && row_tiles * token_tiles * (pl.kc + 1u) <= slots && k_stages / (pl.kc + 1u) >= 4u) ++pl.kc;
-  if (const char *e = getenv("NW_KC")) pl.kc = atoi(e);
-  pl.stages = 1;
-  const size_t budget = per_sm == 2u ? 113u * 1024u : kNarrowMaxSmem;
-  while (pl.stages < 8u) {
-    ++pl.stages;
-    if (narrow_smem(pl) > budget) { --pl.stages; break; }
-  }
-  (void)quant;
+  // clusters are placed inside one GPC: wide ones leave some SMs out
+  while (pl.kc < 8u && blocks * (pl.kc + 1u) <= (pl.kc + 1u <= 4u ? sms : sms * 7u / 8u) && k_stages / (pl.kc + 1u) >= 4u) ++pl.kc;
+  for (pl.stages = 8u; narrow_smem(pl) > kNarrowMaxSmem;) --pl.stages;
   return pl;
 }
 
@@ -408,9 +389,14 @@ int32_t w4a4_narrow_prepare(ErrorSlot &slot) {
   return 0;
 }
 
-bool w4a4_narrow_takes(const DeviceState &dev, uint32_t row_tiles, uint32_t k, uint32_t tokens, bool swiglu) {
-  (void)row_tiles; (void)k; (void)swiglu;
-  return dev.w4a4_pair == 0 || (dev.w4a4_pair != 1 && tokens <= 512u);
+double w4a4_narrow_cycles(const DeviceState &dev, uint32_t row_tiles, uint32_t k, uint32_t tokens, bool swiglu) {
+  const uint32_t k_stages = k / 256u;
+  const NarrowPlan pl = narrow_plan(dev, row_tiles, k_stages, tokens, swiglu);
+  const double ctas = static_cast<double>(row_tiles) * ((tokens + pl.tile - 1u) / pl.tile) * pl.kc;
+  const double stage = narrow_pitch(pl) / 42.0;   // what an SM brings from the L2 in a cycle
+  const double walk = ceil(ctas / dev.sm_count) * (ceil(static_cast<double>(k_stages) / pl.kc) * (stage > 350.0 ? stage : 350.0) + 4000.0 + (pl.kc > 1u ? 2000.0 : 0.0));
+  const double stream = row_tiles * pl.tiles * 72.0 * k / 3150.0;   // the weights at the rate of HBM, per cycle of 1.9 GHz
+  return 4000.0 + (walk > stream ? walk : stream);
 }
 
 int32_t w4a4_narrow_launch(ErrorSlot &slot, const DeviceState &dev, const A4Item *items, uint32_t count, uint32_t k, uint32_t tokens,
@@ -419,7 +405,7 @@ int32_t w4a4_narrow_launch(ErrorSlot &slot, const DeviceState &dev, const A4Item
   const bool swiglu = (epilogue & kEpilogueSwiglu) != 0u, quant = (epilogue & kEpilogueQuant) != 0u;
   uint32_t row_tiles = 0;
   for (uint32_t i = 0; i < count; ++i) row_tiles += items[i].n / (swiglu ? 256u : 128u);
-  const NarrowPlan pl = narrow_plan(dev, row_tiles, k / 256u, tokens, swiglu, quant);
+  const NarrowPlan pl = narrow_plan(dev, row_tiles, k / 256u, tokens, swiglu);
   NarrowParams p = {};
   NarrowMaps maps = {};
   p.sfx = x_scales;
@@ -432,7 +418,6 @@ int32_t w4a4_narrow_launch(ErrorSlot &slot, const DeviceState &dev, const A4Item
   p.kc = pl.kc;
   p.tmem_cols = pl.tmem_cols;
   p.acc_stride = pl.acc_stride;
-  p.sf_bufs = pl.sf_bufs;
   p.epilogue = epilogue;
   p.q_codes = q_codes;
   p.q_scales = q_scales;
