@@ -4,6 +4,8 @@ from __future__ import annotations
 import ctypes as C
 import os
 
+import torch
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libignis_b200.so")
 
@@ -227,3 +229,9 @@ def load() -> C.CDLL:
         fn.argtypes = argtypes
     _lib = lib
     return lib
+
+
+def current_stream() -> int:
+    """The handle of the current device's current CUDA stream. (``torch.cuda.current_stream()`` builds a
+    Stream object around it, which took 1.6 us of a call that enqueues one kernel.)"""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())

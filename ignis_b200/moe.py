@@ -35,8 +35,7 @@ def _check(rc: int) -> None:
         raise MoeError(_lib.load().ignis_moe_last_error().decode())
 
 
-def _stream() -> C.c_void_p:
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+_stream = _lib.current_stream
 
 
 @dataclass(frozen=True)
@@ -47,7 +46,11 @@ class Geometry:
     top_k: int = 10
 
     def c_struct(self) -> _lib.MoeGeometry:
-        return _lib.MoeGeometry(self.hidden, self.inter, self.experts, self.top_k)
+        """The C struct, built once (the fields are frozen)."""
+        struct = self.__dict__.get("_struct")
+        if struct is None:
+            struct = self.__dict__["_struct"] = _lib.MoeGeometry(self.hidden, self.inter, self.experts, self.top_k)
+        return struct
 
 
 _geometry = Geometry()
@@ -172,9 +175,9 @@ def router(x: torch.Tensor, w_router: torch.Tensor, geometry: Geometry | None = 
     """(ids int32 [tokens, top_k], weights fp32 [tokens, top_k], logits fp32 [tokens, experts])."""
     g = geometry or _geometry
     tokens = x.shape[0]
-    ids = torch.empty((tokens, g.top_k), dtype=torch.int32, device=x.device)
-    weights = torch.empty((tokens, g.top_k), dtype=torch.float32, device=x.device)
-    logits = torch.empty((tokens, g.experts), dtype=torch.float32, device=x.device)
+    ids = x.new_empty((tokens, g.top_k), dtype=torch.int32)
+    weights = x.new_empty((tokens, g.top_k), dtype=torch.float32)
+    logits = x.new_empty((tokens, g.experts), dtype=torch.float32)
     gs = g.c_struct()
     _check(_lib.load().b200q_moe_router(C.byref(gs), x.data_ptr(), tokens, w_router.data_ptr(), ids.data_ptr(), weights.data_ptr(),
                                          logits.data_ptr(), _stream()))
@@ -237,8 +240,8 @@ def fp8_row_scale_payload(w: torch.Tensor) -> np.ndarray:
 def shared_expert(gate: torch.Tensor, up: torch.Tensor, down: torch.Tensor, x: torch.Tensor, geometry: Geometry | None = None):
     g = geometry or _geometry
     tokens = x.shape[0]
-    h = torch.empty((tokens, g.inter), dtype=torch.bfloat16, device=x.device)
-    shared = torch.empty((tokens, g.hidden), dtype=torch.float32, device=x.device)
+    h = x.new_empty((tokens, g.inter), dtype=torch.bfloat16)
+    shared = x.new_empty((tokens, g.hidden), dtype=torch.float32)
     gs = g.c_struct()
     _check(_lib.load().b200q_moe_shared_expert(C.byref(gs), gate.data_ptr(), up.data_ptr(), down.data_ptr(), x.data_ptr(), tokens,
                                                 h.data_ptr(), shared.data_ptr(), _stream()))
@@ -251,7 +254,7 @@ def combine(ws: Workspace | None, shared: torch.Tensor, x: torch.Tensor, w_gate:
     (`acc` when given, else the workspace's)."""
     g = geometry or (ws.geometry if ws is not None else _geometry)
     tokens = x.shape[0]
-    out = torch.empty((tokens, g.hidden), dtype=torch.bfloat16, device=x.device)
+    out = x.new_empty((tokens, g.hidden), dtype=torch.bfloat16)
     acc = ws.acc if acc is None else acc
     gs = g.c_struct()
     _check(_lib.load().b200q_moe_combine(C.byref(gs), acc.data_ptr(), shared.data_ptr(), x.data_ptr(), w_gate.data_ptr(), tokens,

@@ -119,6 +119,17 @@ class Weight:
         return _lib.Nvfp4Weight(self.codes.data_ptr(), self.scales.data_ptr(), self.n, self.k,
                                 self.weight_scale_divisor, self.input_scale_divisor)
 
+    def __setattr__(self, name, value) -> None:
+        object.__setattr__(self, name, value)
+        self.__dict__.pop("_ref", None)   # a field was replaced: the struct is built anew
+
+    def ref(self):
+        """``byref`` of the C struct, built once: a decode call enqueues one kernel, and building it took a fifth of that call."""
+        ref = self.__dict__.get("_ref")
+        if ref is None:
+            ref = self.__dict__["_ref"] = C.byref(self.c_struct())
+        return ref
+
     @property
     def payload_bytes(self) -> int:
         """Bytes the linear streams: codes, scales and the divisor."""
@@ -136,8 +147,7 @@ def workspace_bytes(n: int, k: int, policy: int, tokens: int) -> int:
     return int(_lib.load().b200q_nvfp4_workspace_bytes(n, k, policy, tokens))
 
 
-def _stream() -> C.c_void_p:
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+_stream = _lib.current_stream
 
 
 class Workspace:
@@ -146,6 +156,7 @@ class Workspace:
     def __init__(self, nbytes: int, device: str | torch.device = "cuda") -> None:
         self.buffer = torch.empty(max(256, int(nbytes)), dtype=torch.uint8, device=device)
         self.c = _lib.Workspace(self.buffer.data_ptr(), self.buffer.numel())
+        self.ref = C.byref(self.c)
         _check(_lib.load().b200q_nvfp4_workspace_init(C.byref(self.c), _stream()))
 
     def status(self) -> int:
@@ -156,17 +167,17 @@ class Workspace:
 
 
 def _check_x(x: torch.Tensor, k: int) -> None:
-    if x.dtype != torch.bfloat16 or x.dim() != 2 or x.shape[1] != k or not x.is_contiguous() or not x.is_cuda:
+    if x.dtype is not torch.bfloat16 or x.dim() != 2 or x.size(1) != k or not x.is_contiguous() or not x.is_cuda:
         raise Nvfp4Error("x must be a contiguous CUDA BF16 [tokens, k] tensor")
 
 
-def _out(tokens: int, width: int, epilogue: int, out: torch.Tensor | None, device) -> torch.Tensor:
+def _out(tokens: int, width: int, epilogue: int, out: torch.Tensor | None, like: torch.Tensor) -> torch.Tensor:
     dtype = torch.float32 if epilogue & OUT_F32 else torch.bfloat16
     if out is None:
         if epilogue & ADD:
             raise Nvfp4Error("the ADD epilogue accumulates into `out`, which must be given")
-        return torch.empty((tokens, width), dtype=dtype, device=device)
-    if out.dtype != dtype or out.dim() != 2 or out.shape[0] != tokens or out.shape[1] < width or out.stride(1) != 1:
+        return like.new_empty((tokens, width), dtype=dtype)
+    if out.dtype is not dtype or out.dim() != 2 or out.size(0) != tokens or out.size(1) < width or out.stride(1) != 1:
         raise Nvfp4Error("`out` has the wrong dtype or shape")
     return out
 
@@ -176,11 +187,10 @@ def linear(x: torch.Tensor, w: Weight, out: torch.Tensor | None = None, policy: 
     """``out[t, r] = sum_c w[r, c] x[t, c]``: ninfer::ops::linear; with ``ADD``, linear_add. Under
     ``ALLOW_A4`` wide calls take the tensor-core W4A4 route and need `workspace`."""
     _check_x(x, w.k)
-    tokens = x.shape[0]
-    y = _out(tokens, w.n, epilogue, out, x.device)
-    ws = w.c_struct()
-    _check(_lib.load().b200q_nvfp4_linear(C.byref(ws), x.data_ptr(), tokens, y.data_ptr(), y.stride(0), epilogue, policy,
-                                           C.byref(workspace.c) if workspace is not None else None, _stream()))
+    tokens = x.size(0)
+    y = _out(tokens, w.n, epilogue, out, x)
+    _check(_lib.load().b200q_nvfp4_linear(w.ref(), x.data_ptr(), tokens, y.data_ptr(), y.stride(0), epilogue, policy,
+                                           workspace.ref if workspace is not None else None, _stream()))
     return y
 
 
@@ -192,9 +202,8 @@ def linear_noalloc(x: torch.Tensor, w: Weight, out: torch.Tensor, epilogue: int 
     caller passes the output too, so nothing is allocated anywhere on this path."""
     _check_x(x, w.k)
     tokens = x.shape[0]
-    y = _out(tokens, w.n, epilogue, out, x.device)
-    ws = w.c_struct()
-    _check(_lib.load().b200q_nvfp4_linear_noalloc(C.byref(ws), x.data_ptr(), tokens, y.data_ptr(), y.stride(0), epilogue,
+    y = _out(tokens, w.n, epilogue, out, x)
+    _check(_lib.load().b200q_nvfp4_linear_noalloc(w.ref(), x.data_ptr(), tokens, y.data_ptr(), y.stride(0), epilogue,
                                                    _stream()))
     return y
 
@@ -206,7 +215,7 @@ def linear_group(x: torch.Tensor, weights: list[Weight], outs: list[torch.Tensor
         raise Nvfp4Error("linear_group needs at least one weight")
     _check_x(x, weights[0].k)
     tokens = x.shape[0]
-    ys = [_out(tokens, w.n, epilogue, None if outs is None else outs[i], x.device) for i, w in enumerate(weights)]
+    ys = [_out(tokens, w.n, epilogue, None if outs is None else outs[i], x) for i, w in enumerate(weights)]
     structs = [w.c_struct() for w in weights]
     count = len(weights)
     wp = (C.POINTER(_lib.Nvfp4Weight) * count)(*[C.pointer(s) for s in structs])
@@ -229,17 +238,19 @@ def linear_split(x: torch.Tensor, parent: Weight, row_counts: list[int], outs: l
     NVFP4 parent): consecutive row ranges of `parent`, `row_counts[i]` rows each, every range into
     its own contiguous output."""
     _check_x(x, parent.k)
-    tokens = x.shape[0]
+    tokens = x.size(0)
     count = len(row_counts)
-    begins = [sum(row_counts[:i]) for i in range(count)]
-    ys = [_out(tokens, r, epilogue, None if outs is None else outs[i], x.device) for i, r in enumerate(row_counts)]
-    ws = parent.c_struct()
-    rb = (C.c_uint32 * count)(*begins)
-    rc = (C.c_uint32 * count)(*row_counts)
-    yp = (C.c_void_p * count)(*[y.data_ptr() for y in ys])
-    ld = (C.c_uint32 * count)(*[y.stride(0) for y in ys])
-    _check(_lib.load().b200q_nvfp4_linear_split(C.byref(ws), count, rb, rc, x.data_ptr(), tokens, yp, ld, epilogue, policy,
-                                                 C.byref(workspace.c) if workspace is not None else None, _stream()))
+    key = tuple(row_counts)
+    ranges = parent.__dict__.get("_ranges")
+    if ranges is None or ranges[0] != key:   # the ranges' C arrays, kept with the parent
+        u32s = C.c_uint32 * count
+        ranges = parent.__dict__["_ranges"] = (key, u32s(*[sum(key[:i]) for i in range(count)]), u32s(*key), u32s, C.c_void_p * count)
+    _, rb, rc, u32s, ptrs = ranges
+    ys = [_out(tokens, r, epilogue, None if outs is None else outs[i], x) for i, r in enumerate(row_counts)]
+    yp = ptrs(*[y.data_ptr() for y in ys])
+    ld = u32s(*[y.stride(0) for y in ys])
+    _check(_lib.load().b200q_nvfp4_linear_split(parent.ref(), count, rb, rc, x.data_ptr(), tokens, yp, ld, epilogue, policy,
+                                                 workspace.ref if workspace is not None else None, _stream()))
     return ys
 
 
@@ -286,10 +297,9 @@ def linear_swiglu(x: torch.Tensor, gate_up: Weight, out: torch.Tensor | None = N
     (prefill_swiglu::gate_up_swiglu, kernel/src/prefill_swiglu.h:73-107) and need `workspace`."""
     _check_x(x, gate_up.k)
     tokens = x.shape[0]
-    h = _out(tokens, gate_up.n // 2, STORE, out, x.device)
-    ws = gate_up.c_struct()
-    _check(_lib.load().b200q_nvfp4_linear_swiglu(C.byref(ws), x.data_ptr(), tokens, h.data_ptr(), h.stride(0), policy,
-                                                  C.byref(workspace.c) if workspace is not None else None, _stream()))
+    h = _out(tokens, gate_up.n // 2, STORE, out, x)
+    _check(_lib.load().b200q_nvfp4_linear_swiglu(gate_up.ref(), x.data_ptr(), tokens, h.data_ptr(), h.stride(0), policy,
+                                                  workspace.ref if workspace is not None else None, _stream()))
     return h
 
 
@@ -304,18 +314,16 @@ def mlp(x: torch.Tensor, gate_up: Weight, down: Weight, workspace: Workspace, ou
     quantizes it straight into the down product's operand."""
     _check_x(x, gate_up.k)
     tokens = x.shape[0]
-    y = _out(tokens, down.n, epilogue, out, x.device)
-    gu, dn = gate_up.c_struct(), down.c_struct()
-    _check(_lib.load().b200q_nvfp4_mlp(C.byref(gu), C.byref(dn), x.data_ptr(), tokens, y.data_ptr(), y.stride(0), epilogue, policy,
-                                        C.byref(workspace.c), _stream()))
+    y = _out(tokens, down.n, epilogue, out, x)
+    _check(_lib.load().b200q_nvfp4_mlp(gate_up.ref(), down.ref(), x.data_ptr(), tokens, y.data_ptr(), y.stride(0), epilogue, policy,
+                                        workspace.ref, _stream()))
     return y
 
 
 def dequantize(w: Weight) -> torch.Tensor:
     """The logical weight as float32 ``[n, k]`` (the bit-exact dequant seam)."""
     out = torch.empty((w.n, w.k), dtype=torch.float32, device=w.codes.device)
-    ws = w.c_struct()
-    _check(_lib.load().b200q_nvfp4_dequantize(C.byref(ws), out.data_ptr(), _stream()))
+    _check(_lib.load().b200q_nvfp4_dequantize(w.ref(), out.data_ptr(), _stream()))
     return out
 
 
@@ -337,7 +345,7 @@ def quantize_operand(x_rows: torch.Tensor, tokens_total: int, token_begin: int, 
     ``token_begin ..`` of a call of `tokens_total`) into their place of the W4A4 operand in `workspace`."""
     _check_x(x_rows, k)
     _check(_lib.load().b200q_nvfp4_quantize_operand(x_rows.data_ptr(), tokens_total, token_begin, x_rows.shape[0], k,
-                                                     float(input_scale_divisor), C.byref(workspace.c), _stream()))
+                                                     float(input_scale_divisor), workspace.ref, _stream()))
 
 
 def operand_ranges(k: int, tokens_total: int, token_begin: int, token_count: int) -> tuple[tuple[int, int], tuple[int, int]]:
@@ -354,10 +362,9 @@ def operand_ranges(k: int, tokens_total: int, token_begin: int, token_count: int
 def linear_prequantized(w: Weight, tokens: int, workspace: Workspace, out: torch.Tensor | None = None,
                         epilogue: int = STORE) -> torch.Tensor:
     """``b200q_nvfp4_linear_prequantized``: the tensor-core product over the operand in `workspace`."""
-    y = _out(tokens, w.n, epilogue, out, w.codes.device)
-    ws = w.c_struct()
-    _check(_lib.load().b200q_nvfp4_linear_prequantized(C.byref(ws), tokens, y.data_ptr(), y.stride(0), epilogue,
-                                                        C.byref(workspace.c), _stream()))
+    y = _out(tokens, w.n, epilogue, out, w.codes)
+    _check(_lib.load().b200q_nvfp4_linear_prequantized(w.ref(), tokens, y.data_ptr(), y.stride(0), epilogue,
+                                                        workspace.ref, _stream()))
     return y
 
 

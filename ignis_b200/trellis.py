@@ -84,6 +84,17 @@ class Weight:
         return _lib.TrellisWeight(self.trellis.data_ptr(), self.suh.data_ptr(), self.svh.data_ptr(), self.k2, self.in_,
                                   self.out, self.tile_stride)
 
+    def __setattr__(self, name, value) -> None:
+        object.__setattr__(self, name, value)
+        self.__dict__.pop("_struct", None)   # a field was replaced: the struct is built anew
+
+    def struct(self) -> _lib.TrellisWeight:
+        """The C struct, built once."""
+        struct = self.__dict__.get("_struct")
+        if struct is None:
+            struct = self.__dict__["_struct"] = self.c_struct()
+        return struct
+
 
 def prepare() -> None:
     _check(_lib.load().ignis_trellis_prepare())
@@ -97,8 +108,7 @@ def workspace_bytes(in_: int, out: int, weights: int, tokens: int) -> int:
     return int(_lib.load().ignis_trellis_workspace_bytes(in_, out, weights, tokens))
 
 
-def _stream() -> C.c_void_p:
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+_stream = _lib.current_stream
 
 
 class WorkspaceBuffer:
@@ -107,11 +117,12 @@ class WorkspaceBuffer:
     def __init__(self, nbytes: int, device="cuda") -> None:
         self.buffer = torch.empty(max(256, nbytes), dtype=torch.uint8, device=device)
         self.c = _lib.Workspace(self.buffer.data_ptr(), self.buffer.numel())
+        self.ref = C.byref(self.c)
         _check(_lib.load().ignis_trellis_workspace_init(C.byref(self.c), _stream()))
 
 
 def _check_x(x: torch.Tensor, in_: int) -> None:
-    if x.dtype != torch.bfloat16 or x.dim() != 2 or x.shape[1] != in_ or not x.is_contiguous() or not x.is_cuda:
+    if x.dtype is not torch.bfloat16 or x.dim() != 2 or x.size(1) != in_ or not x.is_contiguous() or not x.is_cuda:
         raise TrellisError("x must be a contiguous CUDA BF16 [tokens, in] tensor")
 
 
@@ -123,10 +134,9 @@ def linear(w: Weight, x: torch.Tensor, out: torch.Tensor | None = None, epilogue
     if out is None:
         if epilogue == ADD:
             raise TrellisError("the ADD epilogue accumulates into `out`, which must be given")
-        out = torch.empty((tokens, w.out), dtype=torch.bfloat16, device=x.device)
-    ws = w.c_struct()
-    _check(_lib.load().ignis_trellis_linear(C.byref(ws), x.data_ptr(), tokens, out.data_ptr(), out.stride(0), epilogue,
-                                             C.byref(workspace.c) if workspace else None, _stream()))
+        out = x.new_empty((tokens, w.out))
+    _check(_lib.load().ignis_trellis_linear(C.byref(w.struct()), x.data_ptr(), tokens, out.data_ptr(), out.stride(0), epilogue,
+                                             workspace.ref if workspace else None, _stream()))
     return out
 
 
@@ -141,10 +151,9 @@ def linear_group(weights: list[Weight], x: torch.Tensor, outs: list[torch.Tensor
     if outs is None:
         if epilogue == ADD:
             raise TrellisError("the ADD epilogue accumulates into `outs`, which must be given")
-        outs = [torch.empty((tokens, w.out), dtype=torch.bfloat16, device=x.device) for w in weights]
-    structs = [w.c_struct() for w in weights]
+        outs = [x.new_empty((tokens, w.out)) for w in weights]
     count = len(weights)
-    wp = (C.POINTER(_lib.TrellisWeight) * count)(*[C.pointer(s) for s in structs])
+    wp = (C.POINTER(_lib.TrellisWeight) * count)(*[C.pointer(w.struct()) for w in weights])
     yp = (C.c_void_p * count)(*[y.data_ptr() for y in outs])
     ld = (C.c_uint32 * count)(*[y.stride(0) for y in outs])
     _check(_lib.load().b200q_trellis_linear_group(wp, count, x.data_ptr(), tokens, yp, ld, epilogue, _stream()))
@@ -157,10 +166,9 @@ def linear_swiglu(gate: Weight, up: Weight, x: torch.Tensor, out: torch.Tensor |
     _check_x(x, gate.in_)
     tokens = x.shape[0]
     if out is None:
-        out = torch.empty((tokens, gate.out), dtype=torch.bfloat16, device=x.device)
-    g, u = gate.c_struct(), up.c_struct()
-    _check(_lib.load().ignis_trellis_linear_swiglu(C.byref(g), C.byref(u), x.data_ptr(), tokens, out.data_ptr(),
-                                                    out.stride(0), C.byref(workspace.c) if workspace else None,
+        out = x.new_empty((tokens, gate.out))
+    _check(_lib.load().ignis_trellis_linear_swiglu(C.byref(gate.struct()), C.byref(up.struct()), x.data_ptr(), tokens, out.data_ptr(),
+                                                    out.stride(0), workspace.ref if workspace else None,
                                                     _stream()))
     return out
 
