@@ -35,6 +35,54 @@ using namespace trellis_dev;
 
 constexpr int kThreads = 256;
 constexpr int kWarps = 8;
+constexpr int kLinearThreads = 288;   // the linear: eight decoding warps and the producer's
+
+__device__ uint32_t g_linear_status = 0;   // bounded waits of the linear's word ring that ran out
+constexpr uint32_t kLinearProducer = 0x10u, kLinearDecoder = 0x20u;
+
+// CTAs of the linear kernel an SM holds at once, by (token tiles x weights).
+constexpr int linear_ctas_per_sm(int nt, int sides) { return nt * sides <= 2 ? 3 : (nt * sides <= 8 ? 2 : 1); }
+
+// ---- the word ring: mbarriers and bulk copies ----
+__device__ __forceinline__ uint32_t smem_address(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ void ring_init(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory"); }
+__device__ __forceinline__ void ring_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void ring_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ bool ring_wait(uint32_t bar, uint32_t parity) {
+  for (uint32_t spin = 0; spin < (1u << 22); ++spin) {
+    uint32_t done;
+    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ void ring_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t address) {
+  uint32_t v;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(address));
+  return v;
+}
+// A position in a ring of `depth` slots: the slot and the parity of its current use.
+struct RingAt {
+  uint32_t slot = 0, phase = 0;
+  __device__ __forceinline__ void advance(uint32_t by, uint32_t depth) {
+    for (slot += by; slot >= depth; slot -= depth) phase ^= 1u;
+  }
+};
+
+// The power of two that brings the largest magnitude of a warp's 128 values (four a lane) into [2^13, 2^14): from the
+// maximum's exponent bits, held to what a float carries; 0 for zeros and for what is not finite.
+__device__ __forceinline__ int block_shift(const float (&v)[4]) {
+  const uint32_t m = max(max(__float_as_uint(v[0]) & 0x7FFFFFFFu, __float_as_uint(v[1]) & 0x7FFFFFFFu),
+                         max(__float_as_uint(v[2]) & 0x7FFFFFFFu, __float_as_uint(v[3]) & 0x7FFFFFFFu));
+  const float top = __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, m));
+  if (!(top > 0.0f && top <= 3.0e38f)) return 0;
+  return max(-126, min(126, 140 - static_cast<int>(__float_as_uint(top) >> 23)));
+}
 
 // ---- reconstruct: one warp per tile ---------------------------------------------------------
 __global__ void __launch_bounds__(kThreads) trellis_reconstruct_kernel(const uint32_t *__restrict__ trellis, uint32_t k2,
@@ -92,16 +140,13 @@ struct TrellisParams {
   uint32_t epilogue;    // 0 store, 1 add, 2 SwiGLU
   uint32_t kc;          // cluster size: slices of the input blocks
   uint32_t chunk;       // 128-input blocks of rotated activations shared memory holds at a time
+  uint32_t ring;        // 128-input blocks of words in the ring
+  uint32_t slot_bytes;  // one of them: 1024 k2 bytes per weight
 };
 
 constexpr uint32_t kEpiAdd = 1, kEpiSwiglu = 2;  // 0 stores
 
-// The lane's words of the 8 steps of one 128-input block of one tile column.
-struct BlockWords {
-  uint32_t w[8][3];
-};
-
-// K2 = 0 decodes with the side's runtime k2 (a SwiGLU pair whose weights differ in width).
+// K2 = 0 decodes with the side's runtime k2 (weights of one call that differ in width).
 template <int K2>
 __device__ __forceinline__ void decode_tile(uint32_t k2, uint32_t a, uint32_t b, uint32_t c, uint32_t off, uint32_t (&frag)[4]) {
   if (K2 == 0) {
@@ -114,18 +159,19 @@ __device__ __forceinline__ void decode_tile(uint32_t k2, uint32_t a, uint32_t b,
 // Work split. A CTA serves one block of 128 output columns and a slice of the 128-input blocks
 // (the cluster splits the inputs); warp j owns tile column j of the block, all the way down the
 // slice, so the warps of a CTA never add into each other and the loop body is one tile: a few
-// hundred bytes of code that stay in the instruction cache. The words of the next 128-input block
-// are requested as the current block's are consumed (24 registers per weight in flight per lane).
-// NT token tiles of 8 share every decoded tile (up to 64 tokens a pass).
+// hundred bytes of code that stay in the instruction cache. NT token tiles of 8 share every decoded
+// tile (up to 64 tokens a pass).
+// Warp 8 brings the words: per 128-input block and weight eight rows of eight tiles (a contiguous 128 k2 bytes each) by
+// bulk copies into a ring in shared memory, ahead of the previous kernel's end. The kernel is bound by instruction issue
+// (ALU pipe first), and words read straight from global memory cost each lane three loads of 64-bit addresses with
+// a runtime stride per tile: about 20 of 75 instructions; from the ring they are three loads at constant offsets.
 template <int K2, int NT, int SIDES, bool GROUP>
-__global__ void __launch_bounds__(kThreads, (SIDES == 1 && NT <= 2) ? 3 : ((NT * SIDES <= 8) ? 2 : 1))
+__global__ void __launch_bounds__(kLinearThreads, linear_ctas_per_sm(NT, SIDES))
     trellis_linear_kernel(const __grid_constant__ TrellisParams p) {
-  extern __shared__ __align__(16) uint8_t smem_raw[];
+  extern __shared__ __align__(128) uint8_t smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank(), kc = p.kc;
-  // The target this CTA serves. A plain call (GROUP false) reads target[0] straight from the launch
-  // constants, which keeps the walk's address arithmetic on the uniform datapath; a grouped call
-  // selects a copy, and pays about 5 % more instructions per tile for it.
+  // The target this CTA serves. A plain call (GROUP false) reads target[0] straight from the launch constants.
   TrellisTarget picked = {};
   if (GROUP) {
     picked = p.target[0];
@@ -142,40 +188,44 @@ __global__ void __launch_bounds__(kThreads, (SIDES == 1 && NT <= 2) ? 3 : ((NT *
   const uint32_t b0 = static_cast<uint32_t>(static_cast<uint64_t>(nblk) * rank / kc);
   const uint32_t b1 = static_cast<uint32_t>(static_cast<uint64_t>(nblk) * (rank + 1) / kc);
 
-  // shared memory: [fragments (side, block, step, token tile, lane)] [part] [inverse scales] [scales]
-  const size_t frag_bytes = static_cast<size_t>(SIDES) * p.chunk * NT * 2048u;
-  uint2 *xs = reinterpret_cast<uint2 *>(smem_raw);
-  float4 *part = reinterpret_cast<float4 *>(smem_raw + frag_bytes);                       // [side][tile column 8][NT][lane 32]
-  float *inv_s = reinterpret_cast<float *>(smem_raw + frag_bytes + static_cast<size_t>(SIDES) * 8 * NT * 32 * 16);
-  float *scale_s = inv_s + static_cast<size_t>(SIDES) * p.chunk * NT * 8;                  // [side][block][token]
+  // shared memory: [word ring: slot (side, tile row, tile column)] [fragments (side, block, step, token tile, lane)] [part]
+  // [inverse scales] [scales] [ring barriers: full, empty]
+  const uint32_t ring_bytes = p.ring * p.slot_bytes;
+  const uint32_t frag_bytes = SIDES * p.chunk * NT * 2048u;
+  uint2 *xs = reinterpret_cast<uint2 *>(smem_raw + ring_bytes);
+  float4 *part = reinterpret_cast<float4 *>(smem_raw + ring_bytes + frag_bytes);           // [side][tile column 8][NT][lane 32]
+  float *inv_s = reinterpret_cast<float *>(part + SIDES * 8 * NT * 32);
+  float *scale_s = inv_s + SIDES * p.chunk * NT * 8;                                        // [side][block][token]
+  const uint32_t bars = smem_address(scale_s + SIDES * p.chunk * NT * 8), empties = bars + 8u * p.ring;
 
-  // the lane's word pointers of this warp's tile column, at the slice's first step
-  LaneWindow win[SIDES];
-  const uint32_t *q[SIDES][3];
-  int64_t step_words[SIDES];
-#pragma unroll
-  for (int sd = 0; sd < SIDES; ++sd) {
-    const TrellisSide &S = sd == 0 ? side0 : p.up;
-    win[sd] = lane_window(K2 != 0 ? static_cast<uint32_t>(K2) : S.k2, lane);
-    const uint32_t tile_words = 4u * S.k2;
-    step_words[sd] = static_cast<int64_t>(S.tile_stride) * tile_words;
-    const uint32_t *base = S.trellis + (static_cast<uint64_t>(col_block) * 8u + static_cast<uint32_t>(warp)) * tile_words +
-                           static_cast<uint64_t>(b0) * 8u * static_cast<uint64_t>(step_words[sd]);
-    q[sd][0] = base + win[sd].w0;
-    q[sd][1] = base + win[sd].w1;
-    q[sd][2] = base + win[sd].w2;
+  if (threadIdx.x == 0) {
+    for (uint32_t d = 0; d < p.ring; ++d) {
+      ring_init(bars + 8u * d, 1);            // the producer's expect_tx arrival
+      ring_init(empties + 8u * d, kWarps);    // one arrival per decoding warp
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  BlockWords bw[SIDES];
-  if (b0 < b1) {  // the weights never depend on the previous kernel: request the first block now
-#pragma unroll
-    for (int sd = 0; sd < SIDES; ++sd)
-#pragma unroll
-      for (int kt = 0; kt < 8; ++kt)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) bw[sd].w[kt][c] = __ldg(q[sd][c] + kt * step_words[sd]);
-  }
-
+  __syncthreads();
   griddep_launch_dependents();
+
+  if (warp == kWarps) {
+    // ---- producer of the words: lane (side, tile row) copies its row; the weights never depend on the previous kernel ----
+    const uint32_t sd = static_cast<uint32_t>(lane) >> 3, row = static_cast<uint32_t>(lane) & 7u;
+    const TrellisSide &S = SIDES == 2 && sd == 1u ? p.up : side0;
+    const uint32_t row_bytes = 128u * S.k2, side_at = sd == 1u ? 1024u * side0.k2 : 0u;
+    const uint64_t row_pitch = static_cast<uint64_t>(S.tile_stride) * 16u * S.k2;   // bytes from a tile row to the next
+    const uint8_t *src = reinterpret_cast<const uint8_t *>(S.trellis) + static_cast<uint64_t>(col_block) * row_bytes + (static_cast<uint64_t>(b0) * 8u + row) * row_pitch;
+    RingAt at;
+    for (uint32_t blk = b0; blk < b1; ++blk, at.advance(1u, p.ring), src += 8u * row_pitch) {
+      if (!ring_wait(empties + 8u * at.slot, at.phase ^ 1u)) {
+        if (lane == 0) atomicOr(&g_linear_status, kLinearProducer);
+        break;
+      }
+      if (lane == 0) ring_expect(bars + 8u * at.slot, 1024u * (side0.k2 + (SIDES == 2 ? p.up.k2 : 0u)));
+      __syncwarp();
+      if (lane < 8 * SIDES) ring_load(smem_address(smem_raw) + at.slot * p.slot_bytes + side_at + row * row_bytes, src, row_bytes, bars + 8u * at.slot);
+    }
+  }
   griddep_wait();
 
   float tot[SIDES][NT][4];
@@ -191,62 +241,86 @@ __global__ void __launch_bounds__(kThreads, (SIDES == 1 && NT <= 2) ? 3 : ((NT *
 #pragma unroll
     for (int tt = 0; tt < NT; ++tt) carry[sd][tt][0] = carry[sd][tt][1] = 0.0f;
   const int t2 = (lane & 3) * 2;
-
-  for (uint32_t cb = b0; cb < b1; cb += p.chunk) {
-    const uint32_t ce = min(cb + p.chunk, b1), nb = ce - cb;
-    if (cb != b0) __syncthreads();  // the previous chunk's fragments are no longer read
-    // ---- rotate the chunk of the activations into B fragments (each weight has its own suh) ----
-    {
-      const uint32_t items = nb * 8u * NT * SIDES;  // (side, block, token), dealt to the warps
-      for (uint32_t item = static_cast<uint32_t>(warp); item < items; item += kWarps) {
-        const uint32_t tok = item % (8u * NT), rest = item / (8u * NT), bl = rest % nb, sd = rest / nb;
-        float v[4] = {0.f, 0.f, 0.f, 0.f};
-        if (tok < p.tokens) {
-          const size_t k0 = static_cast<size_t>(cb + bl) * 128u + 4u * lane;
-          const uint2 xb = ldg64_coherent(p.x + static_cast<size_t>(tok) * p.in + k0);
-          const uint2 sb = *reinterpret_cast<const uint2 *>((sd == 0 ? side0.suh : p.up.suh) + k0);
-          const __half2 s01 = *reinterpret_cast<const __half2 *>(&sb.x), s23 = *reinterpret_cast<const __half2 *>(&sb.y);
-          v[0] = bf16_bits_to_f32(xb.x & 0xFFFFu) * __low2float(s01);
-          v[1] = __uint_as_float(xb.x & 0xFFFF0000u) * __high2float(s01);
-          v[2] = bf16_bits_to_f32(xb.y & 0xFFFFu) * __low2float(s23);
-          v[3] = __uint_as_float(xb.y & 0xFFFF0000u) * __high2float(s23);
-        }
-        hadamard128(v, lane);
-        float m = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
+  // the lane's words of this warp's tile column inside a ring slot, as byte addresses
+  LaneWindow win[SIDES];
+  uint32_t word_at[SIDES][3];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
-        int shift = 0;
-        if (m > 0.0f && m <= 3.0e38f) {
-          int e;
-          (void)frexpf(m, &e);
-          shift = max(-126, min(126, 14 - e));
-        }
-        const float scale = ldexpf(1.0f, shift);
-        const __half2 h01 = __floats2half2_rn(v[0] * scale, v[1] * scale);
-        const __half2 h23 = __floats2half2_rn(v[2] * scale, v[3] * scale);
-        // element e = 4 lane + i of the block: step kt = e / 16, inside it k16 = e % 16; the reader
-        // lane (g = token slot, t) keeps k16 in {2t, 2t+1} in .x and {2t+8, 2t+9} in .y
-        const int kt = lane >> 2, k16 = (lane & 3) * 4;
-        const int t_first = (k16 & 7) >> 1, reg = k16 >> 3;
-        const uint32_t tt = tok >> 3, slot = tok & 7u;
-        const size_t blk_slot = static_cast<size_t>(sd) * p.chunk + bl;
-        uint32_t *dst = reinterpret_cast<uint32_t *>(xs + ((blk_slot * 8 + kt) * NT + tt) * 32 + slot * 4);
-        dst[t_first * 2 + reg] = *reinterpret_cast<const uint32_t *>(&h01);
-        dst[(t_first + 1) * 2 + reg] = *reinterpret_cast<const uint32_t *>(&h23);
-        if (lane == 0) {
-          inv_s[blk_slot * 8 * NT + tok] = tok < p.tokens ? ldexpf(1.0f, -shift) : 0.0f;
-          scale_s[blk_slot * 8 * NT + tok] = scale;
-        }
+  for (int sd = 0; sd < SIDES; ++sd) {
+    const uint32_t k2 = K2 != 0 ? static_cast<uint32_t>(K2) : (sd == 0 ? side0.k2 : p.up.k2);
+    win[sd] = lane_window(k2, lane);
+    const uint32_t base = smem_address(smem_raw) + (sd == 1 ? 1024u * (K2 != 0 ? static_cast<uint32_t>(K2) : side0.k2) : 0u) + static_cast<uint32_t>(warp & 7) * 16u * k2;
+    word_at[sd][0] = base + 4u * win[sd].w0;
+    word_at[sd][1] = base + 4u * win[sd].w1;
+    word_at[sd][2] = base + 4u * win[sd].w2;
+  }
+  RingAt at;
+  bool ok = true;
+
+  // The producer's warp waits for this loop's warps; they meet at a barrier of their own.
+  for (uint32_t cb = b0; cb < b1 && warp < kWarps; cb += p.chunk) {
+    const uint32_t ce = min(cb + p.chunk, b1), nb = ce - cb;
+    if (cb != b0) asm volatile("bar.sync 1, 256;" ::: "memory");  // the previous chunk's fragments are no longer read
+    // ---- rotate the chunk of the activations into B fragments (each weight has its own suh): items (side, block, token) dealt to
+    //      the warps, token fastest, an item's place carried along instead of divided out ----
+    const uint32_t step_q = kWarps / p.tokens, step_r = kWarps % p.tokens;
+    uint32_t tok = static_cast<uint32_t>(warp) % p.tokens, rest = static_cast<uint32_t>(warp) / p.tokens;
+    for (; rest < nb * SIDES; tok += step_r, rest += step_q) {
+      if (tok >= p.tokens) {
+        tok -= p.tokens;
+        if (++rest >= nb * SIDES) break;
+      }
+      const uint32_t sd = SIDES == 2 && rest >= nb ? 1u : 0u, bl = rest - sd * nb;
+      float v[4];
+      const size_t k0 = static_cast<size_t>(cb + bl) * 128u + 4u * lane;
+      const uint2 xb = ldg64_coherent(p.x + static_cast<size_t>(tok) * p.in + k0);
+      const uint2 sb = __ldg(reinterpret_cast<const uint2 *>((sd == 0 ? side0.suh : p.up.suh) + k0));
+      const __half2 s01 = *reinterpret_cast<const __half2 *>(&sb.x), s23 = *reinterpret_cast<const __half2 *>(&sb.y);
+      v[0] = bf16_bits_to_f32(xb.x & 0xFFFFu) * __low2float(s01);
+      v[1] = __uint_as_float(xb.x & 0xFFFF0000u) * __high2float(s01);
+      v[2] = bf16_bits_to_f32(xb.y & 0xFFFFu) * __low2float(s23);
+      v[3] = __uint_as_float(xb.y & 0xFFFF0000u) * __high2float(s23);
+      hadamard128(v, lane);
+      const int shift = block_shift(v);
+      const float scale = __uint_as_float(static_cast<uint32_t>(shift + 127) << 23);
+      const __half2 h01 = __floats2half2_rn(v[0] * scale, v[1] * scale);
+      const __half2 h23 = __floats2half2_rn(v[2] * scale, v[3] * scale);
+      // element e = 4 lane + i of the block: step kt = e / 16, inside it k16 = e % 16; the reader
+      // lane (g = token slot, t) keeps k16 in {2t, 2t+1} in .x and {2t+8, 2t+9} in .y
+      const int kt = lane >> 2, k16 = (lane & 3) * 4;
+      const int t_first = (k16 & 7) >> 1, reg = k16 >> 3;
+      const uint32_t tt = tok >> 3, slot = tok & 7u;
+      const uint32_t blk_slot = sd * p.chunk + bl;
+      uint32_t *dst = reinterpret_cast<uint32_t *>(xs + ((blk_slot * 8 + kt) * NT + tt) * 32 + slot * 4);
+      dst[t_first * 2 + reg] = *reinterpret_cast<const uint32_t *>(&h01);
+      dst[(t_first + 1) * 2 + reg] = *reinterpret_cast<const uint32_t *>(&h23);
+      if (lane == 0) {
+        inv_s[blk_slot * 8 * NT + tok] = __uint_as_float(static_cast<uint32_t>(127 - shift) << 23);
+        scale_s[blk_slot * 8 * NT + tok] = scale;
       }
     }
-    __syncthreads();
+    if (cb == b0 && p.tokens < 8u * NT) {   // token slots past the pass: zero fragments, once (nothing writes them later)
+      const uint32_t pad = 8u * NT - p.tokens, rows = SIDES * p.chunk;
+      for (uint32_t i = threadIdx.x; i < rows * 8u * pad * 4u; i += kThreads) {   // (block, step, token, uint2 of 4)
+        const uint32_t q = i & 3u, pad_tok = p.tokens + (i >> 2) % pad, step = (i >> 2) / pad;
+        xs[(step * NT + (pad_tok >> 3)) * 32 + (pad_tok & 7u) * 4 + q] = make_uint2(0u, 0u);
+      }
+      for (uint32_t i = threadIdx.x; i < rows * pad; i += kThreads) {
+        const uint32_t at_tok = i / pad * 8u * NT + p.tokens + i % pad;
+        inv_s[at_tok] = 0.0f;
+        scale_s[at_tok] = 1.0f;
+      }
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");
 
     // ---- this warp's tile column down the chunk ----
-    for (uint32_t bl = 0; bl < nb; ++bl) {
-      const bool more = cb + bl + 1 < b1;  // uniform: another block follows in this CTA's slice
+    for (uint32_t bl = 0; bl < nb; ++bl, at.advance(1u, p.ring)) {
+      if (ok && !ring_wait(bars + 8u * at.slot, at.phase)) {
+        if (lane == 0) atomicOr(&g_linear_status, kLinearDecoder);
+        ok = false;
+      }
 #pragma unroll
       for (int sd = 0; sd < SIDES; ++sd) {
-        const size_t blk_slot = static_cast<size_t>(sd) * p.chunk + bl;
+        const uint32_t blk_slot = sd * p.chunk + bl;
         // into this block's units: accumulators were in the previous block's
 #pragma unroll
         for (int tt = 0; tt < NT; ++tt) {
@@ -260,19 +334,17 @@ __global__ void __launch_bounds__(kThreads, (SIDES == 1 && NT <= 2) ? 3 : ((NT *
           carry[sd][tt][0] = iv.x;
           carry[sd][tt][1] = iv.y;
         }
-        if (more) q[sd][0] += 8 * step_words[sd], q[sd][1] += 8 * step_words[sd], q[sd][2] += 8 * step_words[sd];
       }
+      const uint32_t slot_at = at.slot * p.slot_bytes;
 #pragma unroll
       for (int kt = 0; kt < 8; ++kt) {
 #pragma unroll
         for (int sd = 0; sd < SIDES; ++sd) {
+          const uint32_t k2 = K2 != 0 ? static_cast<uint32_t>(K2) : (sd == 0 ? side0.k2 : p.up.k2);
+          const uint32_t row_at = slot_at + kt * 128u * k2;
           uint32_t frag[4];
-          decode_tile<K2>(sd == 0 ? side0.k2 : p.up.k2, bw[sd].w[kt][0], bw[sd].w[kt][1], bw[sd].w[kt][2], win[sd].off, frag);
-          if (more) {  // the same step of the next block, into the registers just consumed
-#pragma unroll
-            for (int c = 0; c < 3; ++c) bw[sd].w[kt][c] = __ldg(q[sd][c] + kt * step_words[sd]);
-          }
-          const uint2 *xb = xs + ((static_cast<size_t>(sd) * p.chunk + bl) * 8 + kt) * NT * 32 + lane;
+          decode_tile<K2>(k2, lds32(word_at[sd][0] + row_at), lds32(word_at[sd][1] + row_at), lds32(word_at[sd][2] + row_at), win[sd].off, frag);
+          const uint2 *xb = xs + ((sd * p.chunk + bl) * 8 + kt) * NT * 32 + lane;
 #pragma unroll
           for (int tt = 0; tt < NT; ++tt) {
             const uint2 b = xb[tt * 32];
@@ -280,6 +352,8 @@ __global__ void __launch_bounds__(kThreads, (SIDES == 1 && NT <= 2) ? 3 : ((NT *
           }
         }
       }
+      __syncwarp();
+      if (lane == 0) ring_arrive(empties + 8u * at.slot);
     }
   }
   // back to the activations' own units, and out to the cluster
@@ -291,12 +365,12 @@ __global__ void __launch_bounds__(kThreads, (SIDES == 1 && NT <= 2) ? 3 : ((NT *
       tot[sd][tt][1] *= carry[sd][tt][1];
       tot[sd][tt][2] *= carry[sd][tt][0];
       tot[sd][tt][3] *= carry[sd][tt][1];
-      part[((sd * 8 + warp) * NT + tt) * 32 + lane] = make_float4(tot[sd][tt][0], tot[sd][tt][1], tot[sd][tt][2], tot[sd][tt][3]);
+      if (warp < kWarps) part[((sd * 8 + warp) * NT + tt) * 32 + lane] = make_float4(tot[sd][tt][0], tot[sd][tt][1], tot[sd][tt][2], tot[sd][tt][3]);
     }
   cluster_barrier();
 
   // ---- finish: tokens dealt over the cluster's CTAs and their warps; lane = 4 output columns ----
-  for (uint32_t tok = rank + kc * static_cast<uint32_t>(warp); tok < p.tokens; tok += kc * kWarps) {
+  for (uint32_t tok = rank + kc * static_cast<uint32_t>(warp); tok < p.tokens; tok += kc * (kWarps + 1)) {
     const uint32_t tt = tok >> 3, slot = tok & 7u;
     const int tq = static_cast<int>(slot >> 1), te = static_cast<int>(slot & 1u);
     float v[SIDES][4];
@@ -340,17 +414,10 @@ __global__ void __launch_bounds__(kThreads, (SIDES == 1 && NT <= 2) ? 3 : ((NT *
 }
 
 constexpr size_t kLinearMaxSmem = 200 * 1024;
+constexpr size_t kLinearSmBytes = 226 * 1024;   // shared memory of an SM for resident CTAs
 
-size_t linear_smem_bytes(uint32_t chunk, int nt, int sides) {
-  return static_cast<size_t>(sides) * chunk * nt * 2048u + static_cast<size_t>(sides) * 8 * nt * 32 * 16 +
-         static_cast<size_t>(sides) * chunk * nt * 8 * 4 * 2;
-}
-
-// Blocks of rotated activations that fit the kernel's shared memory.
-uint32_t chunk_cap(int nt, int sides) {
-  const size_t fixed = static_cast<size_t>(sides) * 8 * nt * 32 * 16;
-  const size_t per_block = static_cast<size_t>(sides) * nt * (2048u + 64u);
-  return static_cast<uint32_t>((kLinearMaxSmem - fixed) / per_block);
+size_t linear_smem_bytes(uint32_t chunk, int nt, int sides, uint32_t ring, uint32_t slot_bytes) {
+  return static_cast<size_t>(ring) * (slot_bytes + 16u) + static_cast<size_t>(sides) * chunk * nt * (2048u + 64u) + static_cast<size_t>(sides) * 8 * nt * 32 * 16;
 }
 
 bool aligned(const void *p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
@@ -391,15 +458,12 @@ TrellisSide make_side(const ignis_trellis_weight *w) {
   return s;
 }
 
-// CTAs of the linear kernel an SM holds at once, by (token tiles x weights).
-int ctas_per_sm(int nt, int sides) { return (sides == 1 && nt <= 2) ? 3 : (nt * sides <= 8 ? 2 : 1); }
-
 // Cluster size for (in, out): the one that costs least in waves of CTAs, each costing its warps'
 // walk down the slice (one tile per 16 inputs), the rotation of the slice and a fixed part.
 uint32_t plan_kc(const DeviceState &dev, uint32_t in, uint32_t out, int nt, int sides) {
   const uint32_t nblk = in / 128u, col_blocks = out / 128u;
   const uint32_t sms = dev.sm_cap > 0 ? static_cast<uint32_t>(dev.sm_cap) : static_cast<uint32_t>(dev.sm_count);
-  const double slots = static_cast<double>(ctas_per_sm(nt, sides)) * sms;
+  const double slots = static_cast<double>(linear_ctas_per_sm(nt, sides)) * sms;
   uint32_t best = 1;
   double best_cost = 1e30;
   for (uint32_t kc = 1; kc <= 8; ++kc) {
@@ -536,9 +600,18 @@ int32_t run_linear(ErrorSlot &slot, const ignis_trellis_weight *const *w, uint32
     const int nt = p.tokens <= 8 ? 1 : (p.tokens <= 16 ? 2 : (p.tokens <= 32 ? 4 : 8));
     const uint32_t kc = plan_kc(*dev, in, out_total, nt, sides);
     const uint32_t slice = (in / 128u + kc - 1) / kc;
-    const uint32_t cap = chunk_cap(nt, sides);
     p.kc = kc;
-    p.chunk = slice < cap ? slice : cap;
+    // What an SM has for each of its CTAs: the ring takes up to four blocks, the rotated activations as much of the slice as fits
+    // beside it.
+    size_t budget = kLinearSmBytes / linear_ctas_per_sm(nt, sides) - 1024u;
+    if (budget > kLinearMaxSmem) budget = kLinearMaxSmem;
+    p.slot_bytes = 0;
+    for (uint32_t i = 0; i < count; ++i) p.slot_bytes = w[i]->k2 * 1024u > p.slot_bytes ? w[i]->k2 * 1024u : p.slot_bytes;
+    if (swiglu) p.slot_bytes += up->k2 * 1024u;
+    p.ring = slice < 4u ? slice : 4u;
+    for (p.chunk = slice; p.chunk > 4u && linear_smem_bytes(p.chunk, nt, sides, p.ring, p.slot_bytes) > budget;) --p.chunk;
+    while (p.ring > 2u && linear_smem_bytes(p.chunk, nt, sides, p.ring, p.slot_bytes) > budget) --p.ring;
+    while (p.chunk > 1u && linear_smem_bytes(p.chunk, nt, sides, p.ring, p.slot_bytes) > budget) --p.chunk;
     p.x = static_cast<const uint16_t *>(x) + static_cast<size_t>(t0) * in;
     uint32_t ctas = 0;
     for (uint32_t i = 0; i < count; ++i) {
@@ -550,8 +623,8 @@ int32_t run_linear(ErrorSlot &slot, const ignis_trellis_weight *const *w, uint32
     }
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(ctas, 1, 1);
-    config.blockDim = dim3(kThreads, 1, 1);
-    config.dynamicSmemBytes = linear_smem_bytes(p.chunk, nt, sides);
+    config.blockDim = dim3(kLinearThreads, 1, 1);
+    config.dynamicSmemBytes = linear_smem_bytes(p.chunk, nt, sides, p.ring, p.slot_bytes);
     config.stream = static_cast<cudaStream_t>(stream);
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -671,7 +744,12 @@ int32_t ignis_trellis_reconstruct(const ignis_trellis_weight *w, void *w_f16, vo
 int32_t b200q_trellis_device_status(void *stream, uint32_t *status) {
   ErrorSlot &slot = trellis_error();
   if (status == nullptr) return fail(slot, "b200q_trellis_device_status: status is NULL");
-  return trellis_tc_status(slot, static_cast<cudaStream_t>(stream), status);
+  uint32_t linear = 0, wide = 0;
+  if (trellis_tc_status(slot, static_cast<cudaStream_t>(stream), &wide) != 0) return -1;
+  const cudaError_t err = cudaMemcpyFromSymbol(&linear, g_linear_status, sizeof(uint32_t));   // the stream is idle
+  if (err != cudaSuccess) return fail(slot, "b200q_trellis_device_status: %s", cudaGetErrorString(err));
+  *status = linear | wide;
+  return 0;
 }
 
 const char *ignis_trellis_last_error(void) { return trellis_error().text; }
