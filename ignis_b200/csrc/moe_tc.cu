@@ -134,6 +134,8 @@ __global__ void __launch_bounds__(Shape<DW>::kThreads, DW == 16 ? 1 : 2) moe_tc_
   job.k2 = slot.k2;
   job.tile_stride = out_plane / 16u;
   job.in = in;
+  job.stage0 = 0u;
+  job.stage1 = in / 64u;
   job.blk0 = kBlocks * col_tile;
   job.blk1 = kBlocks * col_tile + 1u;
   job.nblk = kBlocks == 2u && job.blk1 < out_plane / 128u ? 2u : 1u;

@@ -99,6 +99,8 @@ __global__ void __launch_bounds__(Shape<DW>::kThreads, DW == 16 ? 1 : 2) trellis
   job.k2 = p.k2;
   job.tile_stride = p.tile_stride;
   job.in = p.in;
+  job.stage0 = 0u;
+  job.stage1 = p.in / 64u;
   job.blk0 = kBlocks * col_tile;
   job.blk1 = kBlocks * col_tile + 1u;
   job.nblk = kBlocks == 2u && job.blk1 < p.out / 128u ? 2u : 1u;

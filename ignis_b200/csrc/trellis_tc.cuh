@@ -57,7 +57,8 @@ struct Shape {
   static constexpr uint32_t kStages = DW == 16 ? 3 : 2;
   static constexpr uint32_t kBBytes = kCols * 128;  // one stage of decoded weights: kCols columns x 64 fp16
   static constexpr uint32_t kStageBytes = 2 * kABytes + kBBytes;
-  static constexpr uint32_t kSmemBytes = kStages * kStageBytes + 256 + 1024;   // + barriers and the tensor-memory slot + alignment slack
+  static constexpr uint32_t kRawBytes = kBlocks * 15360;          // ring of packed words
+  static constexpr uint32_t kSmemBytes = kStages * kStageBytes + kRawBytes + 256 + 1024;   // + barriers and the tensor-memory slot + alignment slack
   static constexpr uint32_t kTmemCols = 2 * kCols;
 };
 constexpr uint32_t kStatusProducer = 1u, kStatusMma = 2u, kStatusEpilogue = 4u, kStatusDecoder = 8u;
@@ -72,19 +73,23 @@ struct Job {
   uint32_t blk0, blk1;      // the 128-column blocks behind accumulator columns 0..127 and 128..255
   uint32_t nblk;            // 1: blk1 does not exist (the MMA's N is 128)
   uint32_t row0, rows;      // row0 is also the TMA row coordinate
+  uint32_t stage0, stage1;  // the K stages of 64 inputs it walks
 };
 
-// The raw words of the 4 tiles a decoder warp owns in one stage (1 tile column x 4 tile rows), one
-// word per lane and tile (two for the widths whose tiles have more than 32 words): lane l holds
-// word l of the tile, and the three words a lane's window needs come from its neighbours by shuffle.
-// A 16 x 16 tile is 4 k2 words, so one coalesced load of up to 128 bytes fetches a whole tile.
-template <int K2>
-struct StageWords {
-  static constexpr int kPerTile = (4 * K2 + 31) / 32;
-  uint32_t w[4][kPerTile];
-};
-
-constexpr int kWordRing = 4;   // stages of raw words a decoder warp keeps in flight in registers
+// The ring of packed words: a slot is one K stage of the CTA's tile columns, four tile rows of a contiguous 128 k2 bytes per
+// column block. Three to seven stages fit, by the width (of DW = 16 as many: twice the columns, twice the bytes).
+__host__ __device__ constexpr uint32_t raw_slot_bytes(uint32_t k2, uint32_t blocks) { return 512u * k2 * blocks; }
+constexpr uint32_t kMaxRaw = 7;
+template <int DW>
+__device__ __forceinline__ uint32_t raw_slots(uint32_t k2) {
+  const uint32_t fit = Shape<DW>::kRawBytes / raw_slot_bytes(k2, Shape<DW>::kBlocks);
+  return fit < kMaxRaw ? fit : kMaxRaw;
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t address) {
+  uint32_t v;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(address));
+  return v;
+}
 
 // Six stages of the in-register Sylvester Hadamard (natural order) on 64 values: one half of a
 // 128-wide transform, whose seventh stage pairs value i of one half with value i of the other.
@@ -102,98 +107,63 @@ __device__ __forceinline__ void hadamard64_regs(float (&v)[64]) {
   }
 }
 
-template <int K2>
-__device__ __forceinline__ void load_stage_words(StageWords<K2> &sw, const uint32_t *col0, int lane, uint64_t row_words, uint32_t ks) {
-  // tile rows 4 ks .. 4 ks + 3 of the warp's tile column
-  const uint32_t *base = col0 + static_cast<uint64_t>(ks) * 4u * row_words + lane;
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const uint32_t *t = base + static_cast<uint64_t>(r) * row_words;
-#pragma unroll
-    for (int h = 0; h < StageWords<K2>::kPerTile; ++h) {
-      sw.w[r][h] = (32 * h + lane < 4 * K2) ? __ldg(t + 32 * h) : 0u;
-    }
-  }
-}
-
-// Word `index` of a tile whose words lie one per lane (and, beyond 32, in the second register).
-template <int K2>
-__device__ __forceinline__ uint32_t tile_word(const uint32_t (&w)[(4 * K2 + 31) / 32], uint32_t index) {
-  if ((4 * K2 + 31) / 32 == 1) return __shfl_sync(0xFFFFFFFFu, w[0], static_cast<int>(index));
-  const uint32_t lo = __shfl_sync(0xFFFFFFFFu, w[0], static_cast<int>(index & 31u));
-  const uint32_t hi = __shfl_sync(0xFFFFFFFFu, w[(4 * K2 + 31) / 32 - 1], static_cast<int>(index & 31u));
-  return index < 32u ? lo : hi;
-}
-
 // The decoder warps' loop over the job's K stages. `stages_base` is the shared-memory address of
-// stage 0; `bars`: full[kStages], empty[kStages].
+// stage 0; `bars`: full[kStages], empty[kStages]; `raw_base`, `raw_bars`: the packed words' ring and its full barriers. (Words
+// requested ahead into registers have to arrive before the proxy fence that hands a stage to the tensor core lets a thread go
+// on, whichever stage they belong to; from shared memory the fence finds nothing in flight.)
 template <int K2, int DW>
-__device__ __forceinline__ bool decode_stages(const Job &job, uint32_t stages_base, uint32_t bars, int warp, int lane, uint32_t *status) {
-  constexpr uint32_t kStages = Shape<DW>::kStages, kStageBytes = Shape<DW>::kStageBytes;
+__device__ __forceinline__ bool decode_stages(const Job &job, uint32_t stages_base, uint32_t bars, uint32_t raw_base, uint32_t raw_bars, int warp,
+                                              int lane, uint32_t *status) {
+  constexpr uint32_t kStages = Shape<DW>::kStages, kStageBytes = Shape<DW>::kStageBytes, kSlot = raw_slot_bytes(K2, Shape<DW>::kBlocks);
   const LaneWindow win = lane_window(K2, lane);
-  const uint32_t k_stages = job.in / 64u;
   const uint32_t cb = static_cast<uint32_t>(warp) >> 3;                    // which of the job's two column blocks
-  const uint32_t blk = cb == 0u ? job.blk0 : job.blk1;
-  const uint32_t tn = blk * 8u + (static_cast<uint32_t>(warp) & 7u);        // the warp's tile column in the plane
-  const uint64_t row_words = static_cast<uint64_t>(job.tile_stride) * 4u * K2;
-  const uint32_t *col0 = job.trellis + static_cast<uint64_t>(tn) * 4u * K2;
   const bool live = cb < job.nblk;
   const uint32_t c0 = static_cast<uint32_t>(lane) >> 2, t = static_cast<uint32_t>(lane) & 3u;
   // row n = 16 warp + c0 (+ 8) of the B tile: 8-row group 2 warp (+ 1)
   const uint32_t lane_off = kABytes * 2u + (2u * static_cast<uint32_t>(warp)) * 1024u + c0 * 128u + 4u * t;
-  // The words of the next kWordRing stages are in flight in registers: a load issued when its
-  // stage's slot of the ring was last decoded has several stage times to arrive (one stage ahead is
-  // not enough: a stage is shorter than the latency of HBM).
-  StageWords<K2> ring[kWordRing];
-#pragma unroll
-  for (int d = 0; d < kWordRing; ++d) {   // the weights never depend on the previous kernel
-    if (live && static_cast<uint32_t>(d) < k_stages) load_stage_words<K2>(ring[d], col0, lane, row_words, static_cast<uint32_t>(d));
-  }
+  // the lane's words of the warp's tile column in a slot: tile row r is 128 K2 bytes further
+  const uint32_t col = raw_base + cb * 512u * K2 + (static_cast<uint32_t>(warp) & 7u) * 16u * K2;
+  const uint32_t at0 = col + 4u * win.w0, at1 = col + 4u * win.w1, at2 = col + 4u * win.w2;
+  const uint32_t raws = raw_slots<DW>(K2);
   griddep_launch_dependents();
-  griddep_wait();   // from here on the warp may also touch what an earlier kernel wrote
-  for (uint32_t it0 = 0; it0 < k_stages; it0 += kWordRing) {
-#pragma unroll
-    for (int d = 0; d < kWordRing; ++d) {
-      const uint32_t it = it0 + static_cast<uint32_t>(d);
-      if (it >= k_stages) break;
-      const uint32_t slot = it % kStages;
-      if (!mbar_wait(bars + 8u * (kStages + slot), ((it / kStages) & 1u) ^ 1u)) {
-        if (lane == 0) atomicOr(status, kStatusDecoder);
-        return false;
-      }
-      if (live) {
-        const uint32_t tile = stages_base + slot * kStageBytes + lane_off;
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const uint32_t w0 = tile_word<K2>(ring[d].w[r], win.w0), w1 = tile_word<K2>(ring[d].w[r], win.w1),
-                         w2 = tile_word<K2>(ring[d].w[r], win.w2);
-          uint32_t frag[4];
-          decode8<K2>(w0, w1, w2, win.off, frag);
-          const uint32_t lo = ((2u * r) ^ c0) << 4, hi = ((2u * r + 1u) ^ c0) << 4;
-          asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + lo), "r"(frag[0]) : "memory");
-          asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + hi), "r"(frag[1]) : "memory");
-          asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + 1024u + lo), "r"(frag[2]) : "memory");
-          asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + 1024u + hi), "r"(frag[3]) : "memory");
-        }
-        // the tile is read by the tensor core (async proxy): order these writes before it
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      }
-      mbar_arrive(bars + 8u * slot);
-      if (live && it + kWordRing < k_stages) load_stage_words<K2>(ring[d], col0, lane, row_words, it + kWordRing);
+  griddep_wait();   // the epilogue touches what an earlier kernel wrote
+  RingAt at, from;
+  for (uint32_t it = job.stage0; it < job.stage1; ++it, at.advance(1u, kStages), from.advance(1u, raws)) {
+    if (!mbar_wait(raw_bars + 8u * from.slot, from.phase) || !mbar_wait(bars + 8u * (kStages + at.slot), at.phase ^ 1u)) {
+      if (lane == 0) atomicOr(status, kStatusDecoder);
+      return false;
     }
+    if (live) {
+      const uint32_t tile = stages_base + at.slot * kStageBytes + lane_off, raw = from.slot * kSlot;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        uint32_t frag[4];
+        decode8<K2>(lds32(at0 + raw + r * 128u * K2), lds32(at1 + raw + r * 128u * K2), lds32(at2 + raw + r * 128u * K2), win.off, frag);
+        const uint32_t lo = ((2u * r) ^ c0) << 4, hi = ((2u * r + 1u) ^ c0) << 4;
+        asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + lo), "r"(frag[0]) : "memory");
+        asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + hi), "r"(frag[1]) : "memory");
+        asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + 1024u + lo), "r"(frag[2]) : "memory");
+        asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + 1024u + hi), "r"(frag[3]) : "memory");
+      }
+      // the tile is read by the tensor core (async proxy): order these writes before it
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bars + 8u * at.slot);
   }
   return true;
 }
 
 template <int DW>
-__device__ __forceinline__ bool decode_stages_any(const Job &job, uint32_t stages_base, uint32_t bars, int warp, int lane, uint32_t *status) {
+__device__ __forceinline__ bool decode_stages_any(const Job &job, uint32_t stages_base, uint32_t bars, uint32_t raw_base, uint32_t raw_bars, int warp, int lane,
+                                                  uint32_t *status) {
   switch (job.k2) {
-    case 4: return decode_stages<4, DW>(job, stages_base, bars, warp, lane, status);
-    case 5: return decode_stages<5, DW>(job, stages_base, bars, warp, lane, status);
-    case 6: return decode_stages<6, DW>(job, stages_base, bars, warp, lane, status);
-    case 8: return decode_stages<8, DW>(job, stages_base, bars, warp, lane, status);
-    case 10: return decode_stages<10, DW>(job, stages_base, bars, warp, lane, status);
-    default: return decode_stages<12, DW>(job, stages_base, bars, warp, lane, status);
+    case 4: return decode_stages<4, DW>(job, stages_base, bars, raw_base, raw_bars, warp, lane, status);
+    case 5: return decode_stages<5, DW>(job, stages_base, bars, raw_base, raw_bars, warp, lane, status);
+    case 6: return decode_stages<6, DW>(job, stages_base, bars, raw_base, raw_bars, warp, lane, status);
+    case 8: return decode_stages<8, DW>(job, stages_base, bars, raw_base, raw_bars, warp, lane, status);
+    case 10: return decode_stages<10, DW>(job, stages_base, bars, raw_base, raw_bars, warp, lane, status);
+    default: return decode_stages<12, DW>(job, stages_base, bars, raw_base, raw_bars, warp, lane, status);
   }
 }
 
@@ -202,7 +172,7 @@ __device__ __forceinline__ bool decode_stages_any(const Job &job, uint32_t stage
 // hold row tile tt, lanes = rows, the job's block 0 in the first 128 columns of a tile. The caller
 // ends with core_finish().
 struct Core {
-  uint32_t base, bars, bar_acc, tmem;
+  uint32_t base, bars, bar_acc, raw, raw_bars, tmem;
   uint32_t *tmem_slot;
   int warp, lane;
 };
@@ -214,17 +184,20 @@ __device__ __forceinline__ Core core_setup(uint8_t *smem_raw) {
   Core c;
   const uint32_t raw = smem_u32(smem_raw);
   c.base = (raw + 1023u) & ~1023u;   // the 128-byte swizzle wants 1024-byte aligned tiles
-  c.bars = c.base + kStages * kStageBytes;       // full[kStages], empty[kStages], accumulator full
+  c.raw = c.base + kStages * kStageBytes;        // the packed words' ring
+  c.bars = c.raw + Shape<DW>::kRawBytes;         // full[kStages], empty[kStages], accumulator full, words full[kMaxRaw]
   c.bar_acc = c.bars + 8u * 2u * kStages;
-  c.tmem_slot = reinterpret_cast<uint32_t *>(smem_raw + (c.base - raw) + kStages * kStageBytes + 128);
+  c.raw_bars = c.bar_acc + 8u;
+  c.tmem_slot = reinterpret_cast<uint32_t *>(smem_raw + (c.bars - raw) + 128);
   c.warp = threadIdx.x >> 5;   // not uniform_warp(): a uniform index moved the decoders' addressing to the uniform datapath and cost 27 %
   c.lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < kStages; ++s) {
-      mbar_init(c.bars + 8u * s, kDecoderWarps * 32 + 1);   // every decoder thread and the producer's expect_tx arrival
+      mbar_init(c.bars + 8u * s, kDecoderWarps + 1);        // every decoder warp and the producer's expect_tx arrival
       mbar_init(c.bars + 8u * (kStages + s), 1);            // the MMA thread's commit
     }
     mbar_init(c.bar_acc, 1);
+    for (uint32_t s = 0; s < kMaxRaw; ++s) mbar_init(c.raw_bars + 8u * s, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (c.warp == kDecoderWarps + 1) {
@@ -266,26 +239,49 @@ template <int DW>
 __device__ __forceinline__ bool core_roles(const Core &c, const Job &job, const CUtensorMap *map_a, uint32_t *status) {
   constexpr uint32_t kStages = Shape<DW>::kStages, kStageBytes = Shape<DW>::kStageBytes;
   constexpr int kDecoderWarps = DW;
-  const uint32_t k_stages = job.in / 64u;
+  const uint32_t k_stages = job.stage1 - job.stage0;
   const uint32_t row_tiles = job.rows > 128u ? 2u : 1u;
-  if (c.warp < kDecoderWarps) return decode_stages_any<DW>(job, c.base, c.bars, c.warp, c.lane, status);
+  if (c.warp < kDecoderWarps) return decode_stages_any<DW>(job, c.base, c.bars, c.raw, c.raw_bars, c.warp, c.lane, status);
   if (c.warp == kDecoderWarps) {
-    // ---- producer of the activation tiles ----
+    // ---- producer: the packed words (they never depend on the previous kernel) and the activation tiles ----
+    const uint32_t raws = raw_slots<DW>(job.k2), slot_bytes = raw_slot_bytes(job.k2, Shape<DW>::kBlocks), row_bytes = 128u * job.k2;
+    const uint64_t row_pitch = static_cast<uint64_t>(job.tile_stride) * 16u * job.k2;   // bytes from a tile row to the next
+    const uint8_t *plane = reinterpret_cast<const uint8_t *>(job.trellis) + static_cast<uint64_t>(job.stage0) * 4u * row_pitch;
+    auto words = [&](uint32_t it, uint32_t slot) {   // stage `it` of the job into `slot`: four tile rows per column block
+      const uint32_t full = c.raw_bars + 8u * slot, dst = c.raw + slot * slot_bytes;
+      mbar_expect_tx(full, 4u * row_bytes * job.nblk);
+      const uint8_t *src = plane + static_cast<uint64_t>(it) * 4u * row_pitch;
+      for (uint32_t b = 0; b < job.nblk; ++b) {
+        const uint8_t *block = src + static_cast<uint64_t>(b == 0u ? job.blk0 : job.blk1) * row_bytes;
+#pragma unroll
+        for (uint32_t r = 0; r < 4u; ++r) bulk_load(dst + b * 512u * job.k2 + r * row_bytes, block + r * row_pitch, row_bytes, full);
+      }
+    };
+    const uint32_t ahead = raws < k_stages ? raws : k_stages;
+    if (elect_one()) {
+      for (uint32_t it = 0; it < ahead; ++it) words(it, it);
+    }
+    __syncwarp();
     griddep_launch_dependents();
     griddep_wait();   // the rotated activations come from the kernel before
-    RingAt at;
+    RingAt at, next;
     for (uint32_t it = 0; it < k_stages; ++it, at.advance(1u, kStages)) {
       if (!mbar_wait(c.bars + 8u * (kStages + at.slot), at.phase ^ 1u)) {
         if (c.lane == 0) atomicOr(status, kStatusProducer);
         break;
       }
+      // The MMAs of stage it - kStages have retired, so its words were decoded: their slot takes the stage `raws` further on.
+      const bool refill = it >= kStages && it - kStages + raws < k_stages;
       if (elect_one()) {
         const uint32_t full = c.bars + 8u * at.slot, stage = c.base + at.slot * kStageBytes;
+        const int32_t x = static_cast<int32_t>((job.stage0 + it) * 64u);
         mbar_expect_tx(full, row_tiles * kABytes);
-        tma_load_2d(stage, map_a, full, static_cast<int32_t>(it * 64u), static_cast<int32_t>(job.row0));
-        if (row_tiles == 2u) tma_load_2d(stage + kABytes, map_a, full, static_cast<int32_t>(it * 64u), static_cast<int32_t>(job.row0 + 128u));
+        tma_load_2d(stage, map_a, full, x, static_cast<int32_t>(job.row0));
+        if (row_tiles == 2u) tma_load_2d(stage + kABytes, map_a, full, x, static_cast<int32_t>(job.row0 + 128u));
+        if (refill) words(it - kStages + raws, next.slot);
       }
       __syncwarp();
+      if (refill) next.advance(1u, raws);
     }
     return false;
   }
