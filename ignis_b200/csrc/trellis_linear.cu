@@ -336,14 +336,22 @@ __global__ void __launch_bounds__(kLinearThreads, linear_ctas_per_sm(NT, SIDES))
         }
       }
       const uint32_t slot_at = at.slot * p.slot_bytes;
+      uint32_t w[SIDES][3];   // the next tile's words, read while the current one is decoded
+      auto read_words = [&](int sd, int kt) {
+        const uint32_t k2 = K2 != 0 ? static_cast<uint32_t>(K2) : (sd == 0 ? side0.k2 : p.up.k2);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) w[sd][c] = lds32(word_at[sd][c] + slot_at + kt * 128u * k2);
+      };
+#pragma unroll
+      for (int sd = 0; sd < SIDES; ++sd) read_words(sd, 0);
 #pragma unroll
       for (int kt = 0; kt < 8; ++kt) {
 #pragma unroll
         for (int sd = 0; sd < SIDES; ++sd) {
-          const uint32_t k2 = K2 != 0 ? static_cast<uint32_t>(K2) : (sd == 0 ? side0.k2 : p.up.k2);
-          const uint32_t row_at = slot_at + kt * 128u * k2;
+          const uint32_t w0 = w[sd][0], w1 = w[sd][1], w2 = w[sd][2];
+          if (kt < 7) read_words(sd, kt + 1);
           uint32_t frag[4];
-          decode_tile<K2>(k2, lds32(word_at[sd][0] + row_at), lds32(word_at[sd][1] + row_at), lds32(word_at[sd][2] + row_at), win[sd].off, frag);
+          decode_tile<K2>(K2 != 0 ? static_cast<uint32_t>(K2) : (sd == 0 ? side0.k2 : p.up.k2), w0, w1, w2, win[sd].off, frag);
           const uint2 *xb = xs + ((sd * p.chunk + bl) * 8 + kt) * NT * 32 + lane;
 #pragma unroll
           for (int tt = 0; tt < NT; ++tt) {

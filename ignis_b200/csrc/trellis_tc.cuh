@@ -128,26 +128,51 @@ __device__ __forceinline__ bool decode_stages(const Job &job, uint32_t stages_ba
   griddep_launch_dependents();
   griddep_wait();   // the epilogue touches what an earlier kernel wrote
   RingAt at, from;
-  for (uint32_t it = job.stage0; it < job.stage1; ++it, at.advance(1u, kStages), from.advance(1u, raws)) {
-    if (!mbar_wait(raw_bars + 8u * from.slot, from.phase) || !mbar_wait(bars + 8u * (kStages + at.slot), at.phase ^ 1u)) {
+  // A stage's twelve words are read while the stage before is handed over: their latency, and the wait for the copies behind
+  // them, run under the fence.
+  uint32_t w[4][3];
+  auto read_words = [&]() {
+    const uint32_t raw = from.slot * kSlot;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      w[r][0] = lds32(at0 + raw + r * 128u * K2);
+      w[r][1] = lds32(at1 + raw + r * 128u * K2);
+      w[r][2] = lds32(at2 + raw + r * 128u * K2);
+    }
+  };
+  if (!mbar_wait(raw_bars, 0u)) {
+    if (lane == 0) atomicOr(status, kStatusDecoder);
+    return false;
+  }
+  if (live) read_words();
+  for (uint32_t it = job.stage0; it < job.stage1; ++it, at.advance(1u, kStages)) {
+    if (!mbar_wait(bars + 8u * (kStages + at.slot), at.phase ^ 1u)) {
       if (lane == 0) atomicOr(status, kStatusDecoder);
       return false;
     }
     if (live) {
-      const uint32_t tile = stages_base + at.slot * kStageBytes + lane_off, raw = from.slot * kSlot;
+      const uint32_t tile = stages_base + at.slot * kStageBytes + lane_off;
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
         uint32_t frag[4];
-        decode8<K2>(lds32(at0 + raw + r * 128u * K2), lds32(at1 + raw + r * 128u * K2), lds32(at2 + raw + r * 128u * K2), win.off, frag);
+        decode8<K2>(w[r][0], w[r][1], w[r][2], win.off, frag);
         const uint32_t lo = ((2u * r) ^ c0) << 4, hi = ((2u * r + 1u) ^ c0) << 4;
         asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + lo), "r"(frag[0]) : "memory");
         asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + hi), "r"(frag[1]) : "memory");
         asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + 1024u + lo), "r"(frag[2]) : "memory");
         asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + 1024u + hi), "r"(frag[3]) : "memory");
       }
-      // the tile is read by the tensor core (async proxy): order these writes before it
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    from.advance(1u, raws);
+    if (it + 1u < job.stage1) {
+      if (!mbar_wait(raw_bars + 8u * from.slot, from.phase)) {
+        if (lane == 0) atomicOr(status, kStatusDecoder);
+        return false;
+      }
+      if (live) read_words();
+    }
+    // the tile is read by the tensor core (async proxy): order these writes before it
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
     if (lane == 0) mbar_arrive(bars + 8u * at.slot);
   }
