@@ -133,7 +133,6 @@ __global__ void __launch_bounds__(Shape<DW>::kThreads, DW == 16 ? 1 : 2) moe_tc_
   job.trellis = static_cast<const uint32_t *>(slot.record);
   job.k2 = slot.k2;
   job.tile_stride = out_plane / 16u;
-  job.in = in;
   job.stage0 = 0u;
   job.stage1 = in / 64u;
   job.blk0 = kBlocks * col_tile;
@@ -165,36 +164,36 @@ __global__ void __launch_bounds__(Shape<DW>::kThreads, DW == 16 ? 1 : 2) moe_tc_
     // the lane's own row (PHASE 1): which assignment (token, rank) it is and its routing weight
     const uint32_t my_a = PHASE == 1 && valid ? p.sorted[row] : 0u;
     const float my_weight = PHASE == 1 && valid ? p.weights[my_a] : 0.0f;
-    float sv[2][2];   // svh of the four columns a lane writes: [pass][lo, hi] = columns 64 pass + lane, + 32
+    const uint32_t col = 4u * (lane & 15u);
+    float4 sv[2];   // svh of the columns a lane writes: 64 pass + 4 (lane % 16) .. + 3
 #pragma unroll
-    for (int ps = 0; ps < 2; ++ps) {
-      sv[ps][0] = live ? __half2float(__ushort_as_half(__ldg(svh + col0 + 64u * ps + lane))) : 0.0f;
-      sv[ps][1] = live ? __half2float(__ushort_as_half(__ldg(svh + col0 + 64u * ps + 32u + lane))) : 0.0f;
-    }
+    for (int ps = 0; ps < 2; ++ps) sv[ps] = live ? four_halves(svh + col0 + 64u * ps + col) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (core_accumulator<DW>(c, decoded, p.status + 1) && (split || live)) {
       float *areas = reinterpret_cast<float *>(smem_raw + (c.base - smem_u32(smem_raw)));
-      float *mine = areas + group * 8192u;
-      const float *other = areas + (group ^ kBlocks) * 8192u;
+      float *mine = areas + group * kArea;
+      const float *other = areas + (group ^ kBlocks) * kArea;
       const uint32_t taddr = c.tmem + ((quad * 32u) << 16) + tt * kCols + cb * 128u;
       if (PHASE == 0) {
-        float *out = p.gu + static_cast<size_t>(item.first + first) * 2u * p.inter + col0 + lane;
-        auto emit = [&](uint32_t ps, uint32_t r, float lo, float hi) {
-          float *dst = out + static_cast<size_t>(r) * 2u * p.inter + 64u * ps;
-          dst[0] = lo * sv[ps][0];
-          dst[32] = hi * sv[ps][1];
+        float *out = p.gu + static_cast<size_t>(item.first + first) * 2u * p.inter + col0 + col;
+        auto emit = [&](uint32_t ps, uint32_t r, bool there, const float4 &v) {
+          if (there) {
+            *reinterpret_cast<float4 *>(out + static_cast<size_t>(r) * 2u * p.inter + 64u * ps) =
+                make_float4(v.x * sv[ps].x, v.y * sv[ps].y, v.z * sv[ps].z, v.w * sv[ps].w);
+          }
         };
-        if (split) half_epilogue<DW>(taddr, half, live, inv, valid, mine, other, quad, lane, rows, emit);
-        else block_epilogue(taddr, inv, valid, mine, quad, lane, rows, emit);
+        if (split) half_epilogue<DW>(taddr, half, live, inv, valid, mine, other, quad, lane, rows, kWhole, emit);
+        else block_epilogue(taddr, inv, valid, mine, quad, lane, rows, kWhole, emit);
       } else {
-        auto emit = [&](uint32_t ps, uint32_t r, float lo, float hi) {   // the row's assignment and weight, handed round by shuffle
+        auto emit = [&](uint32_t ps, uint32_t r, bool there, const float4 &v) {   // the row's assignment and weight, handed round by shuffle
           const uint32_t a = __shfl_sync(0xFFFFFFFFu, my_a, static_cast<int>(r));
           const float wr = __shfl_sync(0xFFFFFFFFu, my_weight, static_cast<int>(r));
-          float *dst = p.down_rows + static_cast<size_t>(a) * p.hidden + col0 + 64u * ps + lane;
-          dst[0] = wr * (lo * sv[ps][0]);
-          dst[32] = wr * (hi * sv[ps][1]);
+          if (there) {
+            *reinterpret_cast<float4 *>(p.down_rows + static_cast<size_t>(a) * p.hidden + col0 + 64u * ps + col) =
+                make_float4(wr * (v.x * sv[ps].x), wr * (v.y * sv[ps].y), wr * (v.z * sv[ps].z), wr * (v.w * sv[ps].w));
+          }
         };
-        if (split) half_epilogue<DW>(taddr, half, live, inv, valid, mine, other, quad, lane, rows, emit);
-        else block_epilogue(taddr, inv, valid, mine, quad, lane, rows, emit);
+        if (split) half_epilogue<DW>(taddr, half, live, inv, valid, mine, other, quad, lane, rows, kWhole, emit);
+        else block_epilogue(taddr, inv, valid, mine, quad, lane, rows, kWhole, emit);
       }
     }
   }

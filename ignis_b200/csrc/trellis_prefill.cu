@@ -80,6 +80,7 @@ struct DenseParams {
   const float *inv;      // the tokens' inverse scales
   uint16_t *y;           // BF16 [tokens][ldy]
   uint32_t k2, tile_stride, in, out, tokens, ldy, epilogue;
+  uint32_t ranks;        // the CTAs of a cluster share an item's K stages (1: no cluster)
 };
 
 // DW: the core's shape - 16 (256 columns a CTA, one CTA per SM) or 8 (128 columns, two per SM).
@@ -93,14 +94,15 @@ __global__ void __launch_bounds__(Shape<DW>::kThreads, DW == 16 ? 1 : 2) trellis
   // Token tiles run fastest over the grid, so the CTAs at work at one time decode the same columns
   // of the plane (read from HBM once, then from the L2).
   const uint32_t row_tiles = (p.tokens + 255u) / 256u;
-  const uint32_t col_tile = blockIdx.x / row_tiles, row_tile = blockIdx.x % row_tiles;
+  const Split split_k = {p.ranks, p.ranks == 1u ? 0u : cluster_rank()};
+  const uint32_t item = blockIdx.x / p.ranks, col_tile = item / row_tiles, row_tile = item % row_tiles;
   Job job;
   job.trellis = p.trellis;
   job.k2 = p.k2;
   job.tile_stride = p.tile_stride;
-  job.in = p.in;
-  job.stage0 = 0u;
-  job.stage1 = p.in / 64u;
+  const uint32_t stages = p.in / 64u;
+  job.stage0 = stages * split_k.rank / p.ranks;
+  job.stage1 = stages * (split_k.rank + 1u) / p.ranks;
   job.blk0 = kBlocks * col_tile;
   job.blk1 = kBlocks * col_tile + 1u;
   job.nblk = kBlocks == 2u && job.blk1 < p.out / 128u ? 2u : 1u;
@@ -125,33 +127,36 @@ __global__ void __launch_bounds__(Shape<DW>::kThreads, DW == 16 ? 1 : 2) trellis
     const uint32_t token0 = job.row0 + first;
     const uint32_t col0 = (cb == 0u ? job.blk0 : job.blk1) * 128u;
     const float inv = valid ? p.inv[token0 + lane] : 0.0f;
-    float sv[2][2];   // svh of the four columns a lane writes: [pass][lo, hi] = columns 64 pass + lane, + 32
+    const uint32_t col = 4u * (lane & 15u);
+    float4 sv[2];   // svh of the columns a lane writes: 64 pass + 4 (lane % 16) .. + 3
 #pragma unroll
-    for (int ps = 0; ps < 2; ++ps) {
-      sv[ps][0] = live ? __half2float(__ushort_as_half(__ldg(p.svh + col0 + 64u * ps + lane))) : 0.0f;
-      sv[ps][1] = live ? __half2float(__ushort_as_half(__ldg(p.svh + col0 + 64u * ps + 32u + lane))) : 0.0f;
-    }
+    for (int ps = 0; ps < 2; ++ps) sv[ps] = live ? four_halves(p.svh + col0 + 64u * ps + col) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (core_accumulator<kDenseDw>(c, decoded, &g_trellis_tc_status) && (split || live)) {
       float *areas = reinterpret_cast<float *>(smem_raw + (c.base - smem_u32(smem_raw)));
-      uint16_t *out = p.y + static_cast<size_t>(token0) * p.ldy + col0 + lane;
-      auto emit = [&](uint32_t ps, uint32_t r, float lo, float hi) {
-        uint16_t *dst = out + static_cast<size_t>(r) * p.ldy + 64u * ps;
-        float v[2] = {lo * sv[ps][0], hi * sv[ps][1]};
+      uint16_t *out = p.y + static_cast<size_t>(token0) * p.ldy + col0 + col;
+      auto emit = [&](uint32_t ps, uint32_t r, bool there, const float4 &o) {
+        if (!there) return;
+        uint2 *dst = reinterpret_cast<uint2 *>(out + static_cast<size_t>(r) * p.ldy + 64u * ps);
+        float v[4] = {o.x * sv[ps].x, o.y * sv[ps].y, o.z * sv[ps].z, o.w * sv[ps].w};
         if (p.epilogue != kEpiStore) {
+          const uint2 old = *dst;
+          const float was[4] = {bf16_bits_to_f32(old.x & 0xFFFFu), __uint_as_float(old.x & 0xFFFF0000u), bf16_bits_to_f32(old.y & 0xFFFFu),
+                                __uint_as_float(old.y & 0xFFFF0000u)};
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const float o = bf16_bits_to_f32(dst[32 * e]);
-            v[e] = p.epilogue == kEpiAdd ? v[e] + o : o / (1.0f + __expf(-o)) * v[e];
-          }
+          for (int e = 0; e < 4; ++e) v[e] = p.epilogue == kEpiAdd ? v[e] + was[e] : was[e] / (1.0f + __expf(-was[e])) * v[e];
         }
-#pragma unroll
-        for (int e = 0; e < 2; ++e) dst[32 * e] = __bfloat16_as_ushort(__float2bfloat16_rn(v[e]));
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
+        *dst = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
       };
       const uint32_t taddr = c.tmem + ((quad * 32u) << 16) + tt * kCols + cb * 128u;
-      float *mine = areas + group * 8192u;
-      if (split) half_epilogue<kDenseDw>(taddr, half, live, inv, valid, mine, areas + (group ^ kBlocks) * 8192u, quad, lane, rows, emit);
-      else block_epilogue(taddr, inv, valid, mine, quad, lane, rows, emit);
+      float *mine = areas + group * kArea;
+      if (split) half_epilogue<kDenseDw>(taddr, half, live, inv, valid, mine, areas + (group ^ kBlocks) * kArea, quad, lane, rows, split_k, emit);
+      else block_epilogue(taddr, inv, valid, mine, quad, lane, rows, split_k, emit);
+    } else {
+      split_meetings(split_k, tiles);
     }
+  } else {
+    split_meetings(split_k, job.rows > 128u ? 2u : 1u);
   }
   core_finish<kDenseDw>(c);
 }
@@ -174,6 +179,40 @@ uint64_t trellis_tc_workspace_bytes(uint32_t in, uint32_t weights, uint32_t toke
 // narrow CTAs overlap each other's fill, drain and epilogue); B200Q_TRELLIS_TC_SHAPE = 16 selects
 // the wide one (read when the kernels are prepared).
 int g_dense_dw = 8;
+
+// The CTAs of a cluster that share the K stages of an item (the narrow shape).
+constexpr uint32_t kMaxRanks = 8;
+
+namespace {
+cudaLaunchConfig_t dense_config(uint32_t items, uint32_t ranks, cudaStream_t stream, bool pdl, cudaLaunchAttribute (&attr)[2]) {
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(items * ranks);
+  config.blockDim = dim3(Shape<8>::kThreads);
+  config.dynamicSmemBytes = Shape<8>::kSmemBytes;
+  config.stream = stream;
+  unsigned n = 0;
+  if (pdl) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (ranks > 1u) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = ranks;
+    attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  config.attrs = attr;
+  config.numAttrs = n;
+  return config;
+}
+
+uint32_t dense_ranks(const DeviceState &dev, uint32_t items, uint32_t stages) {
+  (void)dev; (void)items; (void)stages;
+  const char *e = getenv("XR");
+  if (e) { uint32_t r = atoi(e); return stages / r >= 8 ? r : 1; }
+  return 1;
+}
+}  // namespace
 
 int32_t trellis_tc_prepare(ErrorSlot &slot) {
   const char *shape = getenv("B200Q_TRELLIS_TC_SHAPE");
@@ -218,10 +257,17 @@ int32_t one_product(ErrorSlot &slot, const DeviceState &dev, const ignis_trellis
   p.ldy = ldy;
   p.epilogue = epilogue;
   const uint32_t row_tiles = (tokens + 255u) / 256u;
-  const uint32_t wide_ctas = (w->out + 255u) / 256u * row_tiles;
-  err = g_dense_dw == 16 ? launch(trellis_tc_dense_kernel<16>, dim3(wide_ctas), dim3(Shape<16>::kThreads), Shape<16>::kSmemBytes, stream, dev.pdl != 0, map_a, p)
-                 : launch(trellis_tc_dense_kernel<8>, dim3((w->out + 127u) / 128u * row_tiles), dim3(Shape<8>::kThreads), Shape<8>::kSmemBytes, stream,
-                          dev.pdl != 0, map_a, p);
+  if (g_dense_dw == 16) {
+    p.ranks = 1u;
+    err = launch(trellis_tc_dense_kernel<16>, dim3((w->out + 255u) / 256u * row_tiles), dim3(Shape<16>::kThreads), Shape<16>::kSmemBytes, stream,
+                 dev.pdl != 0, map_a, p);
+  } else {
+    const uint32_t items = w->out / 128u * row_tiles;
+    p.ranks = dense_ranks(dev, items, w->in / 64u);
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t config = dense_config(items, p.ranks, stream, dev.pdl != 0, attr);
+    err = cudaLaunchKernelEx(&config, trellis_tc_dense_kernel<8>, map_a, p);
+  }
   if (err != cudaSuccess) return fail(slot, "%s: launch failed: %s", what, cudaGetErrorString(err));
   return 0;
 }

@@ -57,8 +57,7 @@ struct Shape {
   static constexpr uint32_t kStages = DW == 16 ? 3 : 2;
   static constexpr uint32_t kBBytes = kCols * 128;  // one stage of decoded weights: kCols columns x 64 fp16
   static constexpr uint32_t kStageBytes = 2 * kABytes + kBBytes;
-  static constexpr uint32_t kRawBytes = kBlocks * 15360;          // ring of packed words
-  static constexpr uint32_t kSmemBytes = kStages * kStageBytes + kRawBytes + 256 + 1024;   // + barriers and the tensor-memory slot + alignment slack
+  static constexpr uint32_t kSmemBytes = kStages * kStageBytes + 256 + 1024;   // + barriers and the tensor-memory slot + alignment slack
   static constexpr uint32_t kTmemCols = 2 * kCols;
 };
 constexpr uint32_t kStatusProducer = 1u, kStatusMma = 2u, kStatusEpilogue = 4u, kStatusDecoder = 8u;
@@ -69,27 +68,23 @@ struct Job {
   const uint32_t *trellis;  // the plane: tile (tk, tn) at word (tk * tile_stride + tn) * 4 k2
   uint32_t k2;
   uint32_t tile_stride;     // tiles per stored row of the plane
-  uint32_t in;              // a multiple of 128
   uint32_t blk0, blk1;      // the 128-column blocks behind accumulator columns 0..127 and 128..255
   uint32_t nblk;            // 1: blk1 does not exist (the MMA's N is 128)
   uint32_t row0, rows;      // row0 is also the TMA row coordinate
-  uint32_t stage0, stage1;  // the K stages of 64 inputs it walks
+  uint32_t stage0, stage1;  // the K stages of 64 inputs it walks: all of `in`, or the CTA's share of a cluster's
 };
 
-// The ring of packed words: a slot is one K stage of the CTA's tile columns, four tile rows of a contiguous 128 k2 bytes per
-// column block. Three to seven stages fit, by the width (of DW = 16 as many: twice the columns, twice the bytes).
-__host__ __device__ constexpr uint32_t raw_slot_bytes(uint32_t k2, uint32_t blocks) { return 512u * k2 * blocks; }
-constexpr uint32_t kMaxRaw = 7;
-template <int DW>
-__device__ __forceinline__ uint32_t raw_slots(uint32_t k2) {
-  const uint32_t fit = Shape<DW>::kRawBytes / raw_slot_bytes(k2, Shape<DW>::kBlocks);
-  return fit < kMaxRaw ? fit : kMaxRaw;
-}
-__device__ __forceinline__ uint32_t lds32(uint32_t address) {
-  uint32_t v;
-  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(address));
-  return v;
-}
+// The raw words of the 4 tiles a decoder warp owns in one stage (1 tile column x 4 tile rows), one
+// word per lane and tile (two for the widths whose tiles have more than 32 words): lane l holds
+// word l of the tile, and the three words a lane's window needs come from its neighbours by shuffle.
+// A 16 x 16 tile is 4 k2 words, so one coalesced load of up to 128 bytes fetches a whole tile.
+template <int K2>
+struct StageWords {
+  static constexpr int kPerTile = (4 * K2 + 31) / 32;
+  uint32_t w[4][kPerTile];
+};
+
+constexpr int kWordRing = 4;   // stages of raw words a decoder warp keeps in flight in registers
 
 // Six stages of the in-register Sylvester Hadamard (natural order) on 64 values: one half of a
 // 128-wide transform, whose seventh stage pairs value i of one half with value i of the other.
@@ -107,88 +102,98 @@ __device__ __forceinline__ void hadamard64_regs(float (&v)[64]) {
   }
 }
 
+template <int K2>
+__device__ __forceinline__ void load_stage_words(StageWords<K2> &sw, const uint32_t *col0, int lane, uint64_t row_words, uint32_t ks) {
+  // tile rows 4 ks .. 4 ks + 3 of the warp's tile column
+  const uint32_t *base = col0 + static_cast<uint64_t>(ks) * 4u * row_words + lane;
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const uint32_t *t = base + static_cast<uint64_t>(r) * row_words;
+#pragma unroll
+    for (int h = 0; h < StageWords<K2>::kPerTile; ++h) {
+      sw.w[r][h] = (32 * h + lane < 4 * K2) ? __ldg(t + 32 * h) : 0u;
+    }
+  }
+}
+
+// Word `index` of a tile whose words lie one per lane (and, beyond 32, in the second register).
+template <int K2>
+__device__ __forceinline__ uint32_t tile_word(const uint32_t (&w)[(4 * K2 + 31) / 32], uint32_t index) {
+  if ((4 * K2 + 31) / 32 == 1) return __shfl_sync(0xFFFFFFFFu, w[0], static_cast<int>(index));
+  const uint32_t lo = __shfl_sync(0xFFFFFFFFu, w[0], static_cast<int>(index & 31u));
+  const uint32_t hi = __shfl_sync(0xFFFFFFFFu, w[(4 * K2 + 31) / 32 - 1], static_cast<int>(index & 31u));
+  return index < 32u ? lo : hi;
+}
+
 // The decoder warps' loop over the job's K stages. `stages_base` is the shared-memory address of
-// stage 0; `bars`: full[kStages], empty[kStages]; `raw_base`, `raw_bars`: the packed words' ring and its full barriers. (Words
-// requested ahead into registers have to arrive before the proxy fence that hands a stage to the tensor core lets a thread go
-// on, whichever stage they belong to; from shared memory the fence finds nothing in flight.)
+// stage 0; `bars`: full[kStages], empty[kStages].
 template <int K2, int DW>
-__device__ __forceinline__ bool decode_stages(const Job &job, uint32_t stages_base, uint32_t bars, uint32_t raw_base, uint32_t raw_bars, int warp,
-                                              int lane, uint32_t *status) {
-  constexpr uint32_t kStages = Shape<DW>::kStages, kStageBytes = Shape<DW>::kStageBytes, kSlot = raw_slot_bytes(K2, Shape<DW>::kBlocks);
+__device__ __forceinline__ bool decode_stages(const Job &job, uint32_t stages_base, uint32_t bars, int warp, int lane, uint32_t *status) {
+  constexpr uint32_t kStages = Shape<DW>::kStages, kStageBytes = Shape<DW>::kStageBytes;
   const LaneWindow win = lane_window(K2, lane);
+  const uint32_t k_stages = job.stage1 - job.stage0;
   const uint32_t cb = static_cast<uint32_t>(warp) >> 3;                    // which of the job's two column blocks
+  const uint32_t blk = cb == 0u ? job.blk0 : job.blk1;
+  const uint32_t tn = blk * 8u + (static_cast<uint32_t>(warp) & 7u);        // the warp's tile column in the plane
+  const uint64_t row_words = static_cast<uint64_t>(job.tile_stride) * 4u * K2;
+  const uint32_t *col0 = job.trellis + static_cast<uint64_t>(tn) * 4u * K2 + static_cast<uint64_t>(job.stage0) * 4u * row_words;
   const bool live = cb < job.nblk;
   const uint32_t c0 = static_cast<uint32_t>(lane) >> 2, t = static_cast<uint32_t>(lane) & 3u;
   // row n = 16 warp + c0 (+ 8) of the B tile: 8-row group 2 warp (+ 1)
   const uint32_t lane_off = kABytes * 2u + (2u * static_cast<uint32_t>(warp)) * 1024u + c0 * 128u + 4u * t;
-  // the lane's words of the warp's tile column in a slot: tile row r is 128 K2 bytes further
-  const uint32_t col = raw_base + cb * 512u * K2 + (static_cast<uint32_t>(warp) & 7u) * 16u * K2;
-  const uint32_t at0 = col + 4u * win.w0, at1 = col + 4u * win.w1, at2 = col + 4u * win.w2;
-  const uint32_t raws = raw_slots<DW>(K2);
-  griddep_launch_dependents();
-  griddep_wait();   // the epilogue touches what an earlier kernel wrote
-  RingAt at, from;
-  // A stage's twelve words are read while the stage before is handed over: their latency, and the wait for the copies behind
-  // them, run under the fence.
-  uint32_t w[4][3];
-  auto read_words = [&]() {
-    const uint32_t raw = from.slot * kSlot;
+  // The words of the next kWordRing stages are in flight in registers: a load issued when its
+  // stage's slot of the ring was last decoded has several stage times to arrive (one stage ahead is
+  // not enough: a stage is shorter than the latency of HBM).
+  StageWords<K2> ring[kWordRing];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      w[r][0] = lds32(at0 + raw + r * 128u * K2);
-      w[r][1] = lds32(at1 + raw + r * 128u * K2);
-      w[r][2] = lds32(at2 + raw + r * 128u * K2);
-    }
-  };
-  if (!mbar_wait(raw_bars, 0u)) {
-    if (lane == 0) atomicOr(status, kStatusDecoder);
-    return false;
+  for (int d = 0; d < kWordRing; ++d) {   // the weights never depend on the previous kernel
+    if (live && static_cast<uint32_t>(d) < k_stages) load_stage_words<K2>(ring[d], col0, lane, row_words, static_cast<uint32_t>(d));
   }
-  if (live) read_words();
-  for (uint32_t it = job.stage0; it < job.stage1; ++it, at.advance(1u, kStages)) {
-    if (!mbar_wait(bars + 8u * (kStages + at.slot), at.phase ^ 1u)) {
-      if (lane == 0) atomicOr(status, kStatusDecoder);
-      return false;
-    }
-    if (live) {
-      const uint32_t tile = stages_base + at.slot * kStageBytes + lane_off;
+  griddep_launch_dependents();
+  griddep_wait();   // from here on the warp may also touch what an earlier kernel wrote
+  for (uint32_t it0 = 0; it0 < k_stages; it0 += kWordRing) {
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        uint32_t frag[4];
-        decode8<K2>(w[r][0], w[r][1], w[r][2], win.off, frag);
-        const uint32_t lo = ((2u * r) ^ c0) << 4, hi = ((2u * r + 1u) ^ c0) << 4;
-        asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + lo), "r"(frag[0]) : "memory");
-        asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + hi), "r"(frag[1]) : "memory");
-        asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + 1024u + lo), "r"(frag[2]) : "memory");
-        asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + 1024u + hi), "r"(frag[3]) : "memory");
-      }
-    }
-    from.advance(1u, raws);
-    if (it + 1u < job.stage1) {
-      if (!mbar_wait(raw_bars + 8u * from.slot, from.phase)) {
+    for (int d = 0; d < kWordRing; ++d) {
+      const uint32_t it = it0 + static_cast<uint32_t>(d);
+      if (it >= k_stages) break;
+      const uint32_t slot = it % kStages;
+      if (!mbar_wait(bars + 8u * (kStages + slot), ((it / kStages) & 1u) ^ 1u)) {
         if (lane == 0) atomicOr(status, kStatusDecoder);
         return false;
       }
-      if (live) read_words();
+      if (live) {
+        const uint32_t tile = stages_base + slot * kStageBytes + lane_off;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const uint32_t w0 = tile_word<K2>(ring[d].w[r], win.w0), w1 = tile_word<K2>(ring[d].w[r], win.w1),
+                         w2 = tile_word<K2>(ring[d].w[r], win.w2);
+          uint32_t frag[4];
+          decode8<K2>(w0, w1, w2, win.off, frag);
+          const uint32_t lo = ((2u * r) ^ c0) << 4, hi = ((2u * r + 1u) ^ c0) << 4;
+          asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + lo), "r"(frag[0]) : "memory");
+          asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + hi), "r"(frag[1]) : "memory");
+          asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + 1024u + lo), "r"(frag[2]) : "memory");
+          asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + 1024u + hi), "r"(frag[3]) : "memory");
+        }
+        // the tile is read by the tensor core (async proxy): order these writes before it
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      }
+      mbar_arrive(bars + 8u * slot);
+      if (live && it + kWordRing < k_stages) load_stage_words<K2>(ring[d], col0, lane, row_words, it + kWordRing);
     }
-    // the tile is read by the tensor core (async proxy): order these writes before it
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncwarp();
-    if (lane == 0) mbar_arrive(bars + 8u * at.slot);
   }
   return true;
 }
 
 template <int DW>
-__device__ __forceinline__ bool decode_stages_any(const Job &job, uint32_t stages_base, uint32_t bars, uint32_t raw_base, uint32_t raw_bars, int warp, int lane,
-                                                  uint32_t *status) {
+__device__ __forceinline__ bool decode_stages_any(const Job &job, uint32_t stages_base, uint32_t bars, int warp, int lane, uint32_t *status) {
   switch (job.k2) {
-    case 4: return decode_stages<4, DW>(job, stages_base, bars, raw_base, raw_bars, warp, lane, status);
-    case 5: return decode_stages<5, DW>(job, stages_base, bars, raw_base, raw_bars, warp, lane, status);
-    case 6: return decode_stages<6, DW>(job, stages_base, bars, raw_base, raw_bars, warp, lane, status);
-    case 8: return decode_stages<8, DW>(job, stages_base, bars, raw_base, raw_bars, warp, lane, status);
-    case 10: return decode_stages<10, DW>(job, stages_base, bars, raw_base, raw_bars, warp, lane, status);
-    default: return decode_stages<12, DW>(job, stages_base, bars, raw_base, raw_bars, warp, lane, status);
+    case 4: return decode_stages<4, DW>(job, stages_base, bars, warp, lane, status);
+    case 5: return decode_stages<5, DW>(job, stages_base, bars, warp, lane, status);
+    case 6: return decode_stages<6, DW>(job, stages_base, bars, warp, lane, status);
+    case 8: return decode_stages<8, DW>(job, stages_base, bars, warp, lane, status);
+    case 10: return decode_stages<10, DW>(job, stages_base, bars, warp, lane, status);
+    default: return decode_stages<12, DW>(job, stages_base, bars, warp, lane, status);
   }
 }
 
@@ -197,7 +202,7 @@ __device__ __forceinline__ bool decode_stages_any(const Job &job, uint32_t stage
 // hold row tile tt, lanes = rows, the job's block 0 in the first 128 columns of a tile. The caller
 // ends with core_finish().
 struct Core {
-  uint32_t base, bars, bar_acc, raw, raw_bars, tmem;
+  uint32_t base, bars, bar_acc, tmem;
   uint32_t *tmem_slot;
   int warp, lane;
 };
@@ -209,20 +214,17 @@ __device__ __forceinline__ Core core_setup(uint8_t *smem_raw) {
   Core c;
   const uint32_t raw = smem_u32(smem_raw);
   c.base = (raw + 1023u) & ~1023u;   // the 128-byte swizzle wants 1024-byte aligned tiles
-  c.raw = c.base + kStages * kStageBytes;        // the packed words' ring
-  c.bars = c.raw + Shape<DW>::kRawBytes;         // full[kStages], empty[kStages], accumulator full, words full[kMaxRaw]
+  c.bars = c.base + kStages * kStageBytes;       // full[kStages], empty[kStages], accumulator full
   c.bar_acc = c.bars + 8u * 2u * kStages;
-  c.raw_bars = c.bar_acc + 8u;
-  c.tmem_slot = reinterpret_cast<uint32_t *>(smem_raw + (c.bars - raw) + 128);
+  c.tmem_slot = reinterpret_cast<uint32_t *>(smem_raw + (c.base - raw) + kStages * kStageBytes + 128);
   c.warp = threadIdx.x >> 5;   // not uniform_warp(): a uniform index moved the decoders' addressing to the uniform datapath and cost 27 %
   c.lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < kStages; ++s) {
-      mbar_init(c.bars + 8u * s, kDecoderWarps + 1);        // every decoder warp and the producer's expect_tx arrival
+      mbar_init(c.bars + 8u * s, kDecoderWarps * 32 + 1);   // every decoder thread and the producer's expect_tx arrival
       mbar_init(c.bars + 8u * (kStages + s), 1);            // the MMA thread's commit
     }
     mbar_init(c.bar_acc, 1);
-    for (uint32_t s = 0; s < kMaxRaw; ++s) mbar_init(c.raw_bars + 8u * s, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (c.warp == kDecoderWarps + 1) {
@@ -266,47 +268,25 @@ __device__ __forceinline__ bool core_roles(const Core &c, const Job &job, const 
   constexpr int kDecoderWarps = DW;
   const uint32_t k_stages = job.stage1 - job.stage0;
   const uint32_t row_tiles = job.rows > 128u ? 2u : 1u;
-  if (c.warp < kDecoderWarps) return decode_stages_any<DW>(job, c.base, c.bars, c.raw, c.raw_bars, c.warp, c.lane, status);
+  if (c.warp < kDecoderWarps) return decode_stages_any<DW>(job, c.base, c.bars, c.warp, c.lane, status);
   if (c.warp == kDecoderWarps) {
-    // ---- producer: the packed words (they never depend on the previous kernel) and the activation tiles ----
-    const uint32_t raws = raw_slots<DW>(job.k2), slot_bytes = raw_slot_bytes(job.k2, Shape<DW>::kBlocks), row_bytes = 128u * job.k2;
-    const uint64_t row_pitch = static_cast<uint64_t>(job.tile_stride) * 16u * job.k2;   // bytes from a tile row to the next
-    const uint8_t *plane = reinterpret_cast<const uint8_t *>(job.trellis) + static_cast<uint64_t>(job.stage0) * 4u * row_pitch;
-    auto words = [&](uint32_t it, uint32_t slot) {   // stage `it` of the job into `slot`: four tile rows per column block
-      const uint32_t full = c.raw_bars + 8u * slot, dst = c.raw + slot * slot_bytes;
-      mbar_expect_tx(full, 4u * row_bytes * job.nblk);
-      const uint8_t *src = plane + static_cast<uint64_t>(it) * 4u * row_pitch;
-      for (uint32_t b = 0; b < job.nblk; ++b) {
-        const uint8_t *block = src + static_cast<uint64_t>(b == 0u ? job.blk0 : job.blk1) * row_bytes;
-#pragma unroll
-        for (uint32_t r = 0; r < 4u; ++r) bulk_load(dst + b * 512u * job.k2 + r * row_bytes, block + r * row_pitch, row_bytes, full);
-      }
-    };
-    const uint32_t ahead = raws < k_stages ? raws : k_stages;
-    if (elect_one()) {
-      for (uint32_t it = 0; it < ahead; ++it) words(it, it);
-    }
-    __syncwarp();
+    // ---- producer of the activation tiles ----
     griddep_launch_dependents();
     griddep_wait();   // the rotated activations come from the kernel before
-    RingAt at, next;
+    RingAt at;
     for (uint32_t it = 0; it < k_stages; ++it, at.advance(1u, kStages)) {
       if (!mbar_wait(c.bars + 8u * (kStages + at.slot), at.phase ^ 1u)) {
         if (c.lane == 0) atomicOr(status, kStatusProducer);
         break;
       }
-      // The MMAs of stage it - kStages have retired, so its words were decoded: their slot takes the stage `raws` further on.
-      const bool refill = it >= kStages && it - kStages + raws < k_stages;
       if (elect_one()) {
         const uint32_t full = c.bars + 8u * at.slot, stage = c.base + at.slot * kStageBytes;
         const int32_t x = static_cast<int32_t>((job.stage0 + it) * 64u);
         mbar_expect_tx(full, row_tiles * kABytes);
         tma_load_2d(stage, map_a, full, x, static_cast<int32_t>(job.row0));
         if (row_tiles == 2u) tma_load_2d(stage + kABytes, map_a, full, x, static_cast<int32_t>(job.row0 + 128u));
-        if (refill) words(it - kStages + raws, next.slot);
       }
       __syncwarp();
-      if (refill) next.advance(1u, raws);
     }
     return false;
   }
@@ -352,22 +332,75 @@ __device__ __forceinline__ bool core_run(const Core &c, const Job &job, const CU
 
 // ---- epilogue ------------------------------------------------------------------------------------
 // A warp group (warp / 4: four warps, 128 threads = the 128 rows of a row tile, a warp's lanes the
-// rows 32 (warp % 4) .. + 31) owns 32 KB of the idle stage ring as [value 64][row 128] floats. The
-// row's low five bits are XORed with the value index, so a warp's accesses are free of bank
-// conflicts both when its lanes are 32 rows of one value (a thread parking its row) and when they
-// are 32 values of one row (the warp writing a row out).
-__device__ __forceinline__ uint32_t stash_at(uint32_t i, uint32_t t) { return i * 128u + (t & 96u) + ((t ^ i) & 31u); }
+// rows 32 (warp % 4) .. + 31) owns an area of the idle stage ring: 128 rows of 64 floats, 68 apart, so
+// that 16-byte accesses are free of bank conflicts both when a warp's lanes are 32 rows (a thread
+// parking its row) and when they are one row's values (the warp writing rows out).
+constexpr uint32_t kPitch = 68;
+constexpr uint32_t kArea = 128 * kPitch;   // floats
+static_assert(2 * kArea * 4 <= Shape<8>::kStages * Shape<8>::kStageBytes && 4 * kArea * 4 <= Shape<16>::kStages * Shape<16>::kStageBytes,
+              "the areas of all warp groups fit into the stage ring");
 
-// Hands the calling warp's first `rows` rows of 64 parked values to `emit(r, lo, hi)`: lane l gets
-// values l and l + 32 of row r, so what the caller stores per row is contiguous across the warp.
-// (A thread storing its own row touches 32 different lines per instruction, and the memory pipe
-// takes them one per cycle: the row-wise form is what makes the epilogue short.)
+// A cluster that shares a job's K stages parks every CTA's share of the sums (the transform is linear);
+// the rows are dealt over the ranks, and a row's owner adds what the ranks parked for it, its own first.
+struct Split {
+  uint32_t ranks, rank;
+};
+constexpr Split kWhole = {1u, 0u};
+
+// The cluster meetings of one job's epilogue, for the threads that do not run it.
+__device__ __forceinline__ void split_meetings(const Split split, uint32_t row_tiles) {
+  if (split.ranks == 1u) return;
+  for (uint32_t i = 0; i < 2u * row_tiles; ++i) cluster_barrier();
+}
+
+__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t local, uint32_t rank) {
+  uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
+  return v;
+}
+
+// Hands the calling warp's first `rows` rows of 64 parked values to `emit(r, there, v)`, two rows at a
+// time: a half-warp per row, lane l its values 4 (l % 16) .. + 3, so what the caller stores per row is
+// contiguous. (A thread storing its own row touches 32 different lines per instruction, and the memory
+// pipe takes them one per cycle: the row-wise form is what makes the epilogue short.) All lanes call
+// `emit` together; `there` is false in the half whose row does not exist.
+//
+// With a cluster the row pairs are dealt over the ranks between two meetings: everything is parked, and
+// nothing is parked over it before every rank has read it.
 template <class RowEmit>
-__device__ __forceinline__ void emit_rows(const float *area, uint32_t quad, uint32_t lane, uint32_t rows, RowEmit emit) {
-  for (uint32_t r = 0; r < rows; ++r) {
-    const uint32_t t = quad * 32u + r;
-    emit(r, area[stash_at(lane, t)], area[stash_at(lane + 32u, t)]);
+__device__ __forceinline__ void emit_rows(const float *area, uint32_t quad, uint32_t lane, uint32_t rows, const Split split, RowEmit emit) {
+  const uint32_t up = lane >> 4, pairs = (rows + 1u) / 2u;
+  const float *base = area + (quad * 32u + up) * kPitch + 4u * (lane & 15u);
+  if (split.ranks == 1u) {
+    for (uint32_t i = 0; i < pairs; ++i) emit(2u * i + up, 2u * i + up < rows, *reinterpret_cast<const float4 *>(base + 2u * i * kPitch));
+    return;
   }
+  cluster_barrier();
+  const uint32_t mine = smem_u32(base);
+  for (uint32_t i0 = split.rank; i0 < pairs; i0 += 4u * split.ranks) {   // four pairs at a time: their loads travel together
+    float4 sum[4];
+    for (uint32_t k = 0, q = split.rank; k < split.ranks; ++k, q = q + 1u == split.ranks ? 0u : q + 1u) {   // no rank is read by all at once
+      float4 v[4];
+#pragma unroll
+      for (uint32_t j = 0; j < 4u; ++j) {
+        const uint32_t i = i0 + j * split.ranks;
+        v[j] = i < pairs ? ld_cluster_f32x4(mine + 8u * kPitch * i, q) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      }
+#pragma unroll
+      for (uint32_t j = 0; j < 4u; ++j) {
+        if (k == 0u) sum[j] = v[j];
+        else sum[j].x += v[j].x, sum[j].y += v[j].y, sum[j].z += v[j].z, sum[j].w += v[j].w;
+      }
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 4u; ++j) {
+      const uint32_t i = i0 + j * split.ranks;
+      if (i < pairs) emit(2u * i + up, 2u * i + up < rows, sum[j]);
+    }
+  }
+  cluster_barrier();
 }
 
 __device__ __forceinline__ void load_half_row(uint32_t taddr, float inv, float (&v)[64]) {
@@ -381,46 +414,54 @@ __device__ __forceinline__ void load_half_row(uint32_t taddr, float inv, float (
   }
 }
 
+__device__ __forceinline__ float4 four_halves(const uint16_t *p) {
+  const uint2 raw = __ldg(reinterpret_cast<const uint2 *>(p));
+  const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&raw.x)), b = __half22float2(*reinterpret_cast<const __half2 *>(&raw.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void park_row(float *row, const float (&v)[64]) {
+#pragma unroll
+  for (int i = 0; i < 64; i += 4) *reinterpret_cast<float4 *>(row + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+}
+
 // The epilogue of one (row tile, block) item for the calling warp: a thread owns one row (lane =
 // row 32 quad + lane of the row tile; `rows` of the warp's 32 exist, `valid` = lane < rows) and
 // `taddr` is the tensor-memory address of the block's first column in those lanes. The thread
 // applies `inv` and six Hadamard stages to each half of its 128 columns in registers, the seventh
-// stage combines the halves through `area`, and `emit(pass, r, lo, hi)` receives, a row at a
-// time, columns 64 pass + lane (lo) and 64 pass + 32 + lane (hi), 1 / sqrt(128) included.
+// stage combines the halves through `area`, and `emit(pass, r, there, v)` receives, two rows at a
+// time, columns 64 pass + 4 (lane % 16) .. + 3 of row r, 1 / sqrt(128) included.
 template <class RowEmit>
 __device__ __forceinline__ void block_epilogue(uint32_t taddr, float inv, bool valid, float *area, uint32_t quad, uint32_t lane,
-                                               uint32_t rows, RowEmit emit) {
-  const uint32_t t = quad * 32u + lane;
+                                               uint32_t rows, const Split split, RowEmit emit) {
+  float *row = area + (quad * 32u + lane) * kPitch;
   float v[64];
 #pragma unroll
   for (int half = 0; half < 2; ++half) {
     load_half_row(taddr + 64u * half, inv, v);
     if (valid) {
       hadamard64_regs(v);
-      if (half == 0) {
-#pragma unroll
-        for (int i = 0; i < 64; ++i) area[stash_at(i, t)] = v[i];
-      }
+      if (half == 0) park_row(row, v);
     }
   }
   const float c = 0.08838834764831845f;   // 1 / sqrt(128)
   if (valid) {   // the seventh stage: columns i (sum, parked) and 64 + i (difference, kept)
 #pragma unroll
-    for (int i = 0; i < 64; ++i) {
-      const float a = area[stash_at(i, t)], b = v[i];
-      area[stash_at(i, t)] = (a + b) * c;
-      v[i] = (a - b) * c;
+    for (int i = 0; i < 64; i += 4) {
+      float4 a = *reinterpret_cast<const float4 *>(row + i);
+      const float b0 = v[i], b1 = v[i + 1], b2 = v[i + 2], b3 = v[i + 3];
+      *reinterpret_cast<float4 *>(row + i) = make_float4((a.x + b0) * c, (a.y + b1) * c, (a.z + b2) * c, (a.w + b3) * c);
+      v[i] = (a.x - b0) * c;
+      v[i + 1] = (a.y - b1) * c;
+      v[i + 2] = (a.z - b2) * c;
+      v[i + 3] = (a.w - b3) * c;
     }
   }
   __syncwarp();
-  emit_rows(area, quad, lane, rows, [&](uint32_t r, float lo, float hi) { emit(0u, r, lo, hi); });
+  emit_rows(area, quad, lane, rows, split, [&](uint32_t r, bool there, const float4 &o) { emit(0u, r, there, o); });
   __syncwarp();
-  if (valid) {
-#pragma unroll
-    for (int i = 0; i < 64; ++i) area[stash_at(i, t)] = v[i];
-  }
+  if (valid) park_row(row, v);
   __syncwarp();
-  emit_rows(area, quad, lane, rows, [&](uint32_t r, float lo, float hi) { emit(1u, r, lo, hi); });
+  emit_rows(area, quad, lane, rows, split, [&](uint32_t r, bool there, const float4 &o) { emit(1u, r, there, o); });
 }
 
 // The same for a job of one row tile, where only two of the four warp groups would have a block:
@@ -428,38 +469,37 @@ __device__ __forceinline__ void block_epilogue(uint32_t taddr, float inv, bool v
 // transforms its half and parks it in its group's area (`mine`); all decoder warps meet at barrier 1;
 // the seventh stage gives the first half's owner columns 0..63 (sums) and the other's columns
 // 64..127 (differences), parked again after a second meeting and written out row-wise:
-// `emit(half, r, lo, hi)` as above. Every decoder warp calls this exactly once (`live`: the group's
+// `emit(half, r, there, v)` as above. Every decoder warp calls this exactly once (`live`: the group's
 // block exists - warp-uniform).
 template <int DW, class RowEmit>
 __device__ __forceinline__ void half_epilogue(uint32_t taddr_block, uint32_t half, bool live, float inv, bool valid, float *mine,
-                                              const float *other, uint32_t quad, uint32_t lane, uint32_t rows, RowEmit emit) {
-  const uint32_t t = quad * 32u + lane;
+                                              const float *other, uint32_t quad, uint32_t lane, uint32_t rows, const Split split, RowEmit emit) {
+  const uint32_t at = (quad * 32u + lane) * kPitch;
   float v[64];
   if (live) {
     load_half_row(taddr_block + 64u * half, inv, v);
     if (valid) {
       hadamard64_regs(v);
-#pragma unroll
-      for (int i = 0; i < 64; ++i) mine[stash_at(i, t)] = v[i];
+      park_row(mine + at, v);
     }
   }
   asm volatile("bar.sync 1, %0;" ::"n"(DW * 32) : "memory");
   const float c = 0.08838834764831845f;   // 1 / sqrt(128)
   if (live && valid) {
 #pragma unroll
-    for (int i = 0; i < 64; ++i) {
-      const float o = other[stash_at(i, t)];
-      v[i] = half == 0u ? (v[i] + o) * c : (o - v[i]) * c;
+    for (int i = 0; i < 64; i += 4) {
+      const float4 o = *reinterpret_cast<const float4 *>(other + at + i);
+      v[i] = half == 0u ? (v[i] + o.x) * c : (o.x - v[i]) * c;
+      v[i + 1] = half == 0u ? (v[i + 1] + o.y) * c : (o.y - v[i + 1]) * c;
+      v[i + 2] = half == 0u ? (v[i + 2] + o.z) * c : (o.z - v[i + 2]) * c;
+      v[i + 3] = half == 0u ? (v[i + 3] + o.w) * c : (o.w - v[i + 3]) * c;
     }
   }
   asm volatile("bar.sync 1, %0;" ::"n"(DW * 32) : "memory");
   if (!live) return;
-  if (valid) {
-#pragma unroll
-    for (int i = 0; i < 64; ++i) mine[stash_at(i, t)] = v[i];
-  }
+  if (valid) park_row(mine + at, v);
   __syncwarp();
-  emit_rows(mine, quad, lane, rows, [&](uint32_t r, float lo, float hi) { emit(half, r, lo, hi); });
+  emit_rows(mine, quad, lane, rows, split, [&](uint32_t r, bool there, const float4 &o) { emit(half, r, there, o); });
 }
 
 template <int DW>
