@@ -182,6 +182,7 @@ int g_dense_dw = 8;
 
 // The CTAs of a cluster that share the K stages of an item (the narrow shape).
 constexpr uint32_t kMaxRanks = 8;
+uint32_t g_dense_clusters[kMaxRanks + 1] = {};   // clusters of so many CTAs that the device runs at once (0: none)
 
 namespace {
 cudaLaunchConfig_t dense_config(uint32_t items, uint32_t ranks, cudaStream_t stream, bool pdl, cudaLaunchAttribute (&attr)[2]) {
@@ -206,11 +207,28 @@ cudaLaunchConfig_t dense_config(uint32_t items, uint32_t ranks, cudaStream_t str
   return config;
 }
 
-uint32_t dense_ranks(const DeviceState &dev, uint32_t items, uint32_t stages) {
-  (void)dev; (void)items; (void)stages;
-  const char *e = getenv("XR");
-  if (e) { uint32_t r = atoi(e); return stages / r >= 8 ? r : 1; }
-  return 1;
+// How many CTAs share an item: the count for which a model of the launch gives the least time. In microseconds, from
+// measurements of four shapes at 70 to 2000 tokens: a stage takes 1.17 with two CTAs on the SM, 0.72 alone (0.95 in a cluster,
+// whose CTAs may share an SM all the same); the epilogue 3 per row tile of 128 and 0.9 more per rank (its reads from the other
+// CTAs' shared memory). The last wave is counted for what is left in it. Few items leave SMs idle and walk all of K alone
+// (17408 -> 5120 at 128 tokens: 40 items of 272 stages, 190 us; six ranks each: 63), a last wave that is nearly empty costs as
+// much as a full one (the same at 1000 tokens: 160 items, 306 us; three ranks: 250); many items need no sharing. At least eight
+// stages per rank: what a CTA spends before its first and after its last stage is as long.
+uint32_t dense_ranks(const DeviceState &dev, uint32_t items, uint32_t stages, uint32_t row_tiles128) {
+  uint32_t best = 1u;
+  float least = 0.0f;
+  for (uint32_t ranks = 1; ranks <= kMaxRanks && (ranks == 1u || stages / ranks >= 8u); ++ranks) {
+    const uint32_t at_once = ranks == 1u ? 2u * static_cast<uint32_t>(dev.sm_count) : g_dense_clusters[ranks];
+    if (at_once == 0u) continue;
+    const uint32_t waves = items / at_once, left = items % at_once;
+    const float epilogue = static_cast<float>(row_tiles128) * (3.0f + 0.9f * static_cast<float>(ranks));
+    const float walked = static_cast<float>((stages + ranks - 1u) / ranks);
+    const bool alone = left * ranks <= static_cast<uint32_t>(dev.sm_count);
+    float t = static_cast<float>(waves) * (1.17f * walked + epilogue);
+    if (left != 0u) t += (!alone ? 1.17f : ranks == 1u ? 0.72f : 0.95f) * walked + epilogue;
+    if (ranks == 1u || t < least) least = t, best = ranks;
+  }
+  return best;
 }
 }  // namespace
 
@@ -223,6 +241,16 @@ int32_t trellis_tc_prepare(ErrorSlot &slot) {
     err = cudaFuncSetAttribute(trellis_rotate_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRotateMaxSmem));
   }
   if (err != cudaSuccess) return fail(slot, "trellis prefill kernel attributes: %s", cudaGetErrorString(err));
+  for (uint32_t ranks = 2; ranks <= kMaxRanks; ++ranks) {
+    cudaLaunchAttribute attr[2];
+    const cudaLaunchConfig_t config = dense_config(1u, ranks, nullptr, false, attr);
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, trellis_tc_dense_kernel<8>, &config) != cudaSuccess) {
+      (void)cudaGetLastError();
+      clusters = 0;
+    }
+    g_dense_clusters[ranks] = static_cast<uint32_t>(clusters);
+  }
   if (encode_tiled_fn() == nullptr) return fail(slot, "cuTensorMapEncodeTiled is not available from this driver");
   return 0;
 }
@@ -263,7 +291,7 @@ int32_t one_product(ErrorSlot &slot, const DeviceState &dev, const ignis_trellis
                  dev.pdl != 0, map_a, p);
   } else {
     const uint32_t items = w->out / 128u * row_tiles;
-    p.ranks = dense_ranks(dev, items, w->in / 64u);
+    p.ranks = dense_ranks(dev, items, w->in / 64u, tokens > 128u ? 2u : 1u);
     cudaLaunchAttribute attr[2];
     cudaLaunchConfig_t config = dense_config(items, p.ranks, stream, dev.pdl != 0, attr);
     err = cudaLaunchKernelEx(&config, trellis_tc_dense_kernel<8>, map_a, p);
