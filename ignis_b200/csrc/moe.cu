@@ -299,110 +299,121 @@ __global__ void __launch_bounds__(kThreads) moe_rotate_kernel(const __grid_const
   }
 }
 
-// The lane's words of the 8 steps of one 128-input block of one tile column.
-struct BlockWords {
-  uint32_t w[8][3];
-};
-
 __device__ __forceinline__ void cp_async16(void *smem_dst, const void *src) {
   const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// The item's fragments and scales of one 128-input block, copied asynchronously into the CTA's
-// staging buffers: 2 KB per live row tile and 64 bytes of (inverse scale, scale) pairs.
+// What a CTA has staged of the item: kDepth slots, each one 128-input block - the packed words of the column block's 8 x 8 tiles
+// (eight contiguous rows of 128 k2 bytes), the fragments (2 KB per live row tile) and the (inverse scale, scale) pairs.
 template <int NT>
-__device__ __forceinline__ void stage_block(uint2 *frag_buf, float2 *scale_buf, const uint2 *frag, const float2 *scales,
-                                            uint32_t nblk, uint32_t bl, uint32_t ntiles) {
-  for (uint32_t c = threadIdx.x; c < ntiles * 128u; c += kThreads) {
-    const uint32_t tt = c >> 7, off = c & 127u;  // 16-byte chunk `off` of tile tt's fragment
-    cp_async16(frag_buf + tt * 256u + off * 2u, frag + (static_cast<size_t>(tt) * nblk + bl) * 256u + off * 2u);
-  }
-  if (threadIdx.x < ntiles * 4u) {
-    const uint32_t tt = threadIdx.x >> 2, off = threadIdx.x & 3u;
-    cp_async16(scale_buf + tt * 8u + off * 2u, scales + (static_cast<size_t>(tt) * nblk + bl) * 8u + off * 2u);
-  }
-  cp_async_commit();
-}
+struct Staging {
+  static constexpr int kDepth = NT == 1 ? 4 : 3;
+  static constexpr uint32_t kFrag = 8192, kScale = kFrag + NT * 2048, kSlot = kScale + NT * 64;
+  static constexpr uint32_t kBytes = kDepth * kSlot;
+};
 
 // Warp j of the CTA walks tile column j of the item's column block down all the inputs: one tile
 // per 16 inputs, decoded once and multiplied with every live row tile of the item (up to NT tiles
-// of 8 rows). The words of the next 128-input block are requested as the current block's are
-// consumed; the rows' fragments and scales of the next block are copied to shared memory while
-// the current block is multiplied (one CTA barrier per block). Sums are in the units of the
-// current block's per-row scale and carried exactly into the next block's.
+// of 8 rows). The blocks to come are copied into the staging slots by all threads (one CTA barrier
+// per block). Sums are in the units of the current block's per-row scale and carried exactly into the
+// next block's. Bound by instruction issue: words that every lane read from global memory itself were
+// three loads with addresses of a runtime stride per tile, and one block ahead of their use.
 template <int K2, int NT>
-__device__ __forceinline__ void walk_tile_column(const uint32_t *tile_base, int64_t step_words, uint32_t nblk, const uint2 *frag,
-                                                 const float2 *scales, uint32_t ntiles, int lane, uint2 (*frag_buf)[NT * 256],
-                                                 float2 (*scale_buf)[NT * 8], float (&tot)[NT][4]) {
+__device__ __forceinline__ void walk_tile_column(const uint8_t *col, uint64_t row_pitch, uint32_t nblk, const uint2 *frag,
+                                                 const float2 *scales, uint32_t ntiles, int warp, int lane, uint8_t *smem, float (&tot)[NT][4]) {
+  using S = Staging<NT>;
+  constexpr uint32_t kRowChunks = 8u * K2;   // 16-byte pieces of a tile row
   const LaneWindow win = lane_window(K2, lane);
-  const uint32_t *q0 = tile_base + win.w0, *q1 = tile_base + win.w1, *q2 = tile_base + win.w2;
-  BlockWords bw;
+  auto stage = [&](uint32_t bl, uint32_t slot) {
+    uint8_t *to = smem + slot * S::kSlot;
+    const uint8_t *from = col + static_cast<uint64_t>(bl) * 8u * row_pitch;
 #pragma unroll
-  for (int kt = 0; kt < 8; ++kt) {
-    bw.w[kt][0] = __ldg(q0 + kt * step_words);
-    bw.w[kt][1] = __ldg(q1 + kt * step_words);
-    bw.w[kt][2] = __ldg(q2 + kt * step_words);
+    for (uint32_t c0 = 0; c0 < 8u * kRowChunks; c0 += kThreads) {
+      const uint32_t c = c0 + threadIdx.x;
+      if (8u * kRowChunks % kThreads == 0u || c < 8u * kRowChunks) {
+        cp_async16(to + c * 16u, from + static_cast<uint64_t>(c / kRowChunks) * row_pitch + c % kRowChunks * 16u);
+      }
+    }
+    for (uint32_t c = threadIdx.x; c < ntiles * 128u; c += kThreads) {
+      const uint32_t tt = c >> 7, off = c & 127u;  // 16-byte chunk `off` of tile tt's fragment
+      cp_async16(to + S::kFrag + c * 16u, frag + (static_cast<size_t>(tt) * nblk + bl) * 256u + off * 2u);
+    }
+    if (threadIdx.x < ntiles * 4u) {
+      const uint32_t tt = threadIdx.x >> 2, off = threadIdx.x & 3u;
+      cp_async16(to + S::kScale + threadIdx.x * 16u, scales + (static_cast<size_t>(tt) * nblk + bl) * 8u + off * 2u);
+    }
+  };
+#pragma unroll
+  for (uint32_t d = 0; d + 1u < S::kDepth; ++d) {
+    if (d < nblk) stage(d, d);
+    cp_async_commit();
   }
-  stage_block<NT>(frag_buf[0], scale_buf[0], frag, scales, nblk, 0, ntiles);
   const int t2 = (lane & 3) * 2;
+  // the lane's words of the warp's tile column in a slot: tile row kt is 128 K2 bytes further
+  const uint8_t *w0 = smem + warp * 16 * K2 + 4u * win.w0, *w1 = smem + warp * 16 * K2 + 4u * win.w1, *w2 = smem + warp * 16 * K2 + 4u * win.w2;
+  float carry[NT][2];   // the previous block's inverse scales (nothing to carry at block 0)
+#pragma unroll
+  for (int tt = 0; tt < NT; ++tt) carry[tt][0] = carry[tt][1] = 0.0f;
+  uint32_t slot = 0, fill = S::kDepth - 1u;
   for (uint32_t bl = 0; bl < nblk; ++bl) {
-    const bool more = bl + 1 < nblk;
-    cp_async_wait_all();
-    __syncthreads();  // this block's copies are visible; nobody still reads the buffers refilled next
-    if (more) stage_block<NT>(frag_buf[(bl + 1) & 1], scale_buf[(bl + 1) % 3], frag, scales, nblk, bl + 1, ntiles);
-    const uint2 *fb = frag_buf[bl & 1] + lane;
-    const float2 *cur = scale_buf[bl % 3] + t2, *prev = scale_buf[(bl + 2) % 3] + t2;
+    cp_async_wait<S::kDepth - 2>();
+    __syncthreads();  // this block's copies are visible; nobody still reads the slot refilled next
+    if (bl + S::kDepth - 1u < nblk) stage(bl + S::kDepth - 1u, fill);
+    cp_async_commit();
+    const uint32_t at = slot * S::kSlot;
+    const uint2 *fb = reinterpret_cast<const uint2 *>(smem + at + S::kFrag) + lane;
+    const float2 *cur = reinterpret_cast<const float2 *>(smem + at + S::kScale) + t2;
+    uint32_t w[3];   // the next tile's words, read while the current one is decoded
+    w[0] = *reinterpret_cast<const uint32_t *>(w0 + at);
+    w[1] = *reinterpret_cast<const uint32_t *>(w1 + at);
+    w[2] = *reinterpret_cast<const uint32_t *>(w2 + at);
     // into this block's units: the sums so far are in the previous block's (inverse scale of the
-    // previous block times scale of this one, an exact power of two; nothing to carry at block 0)
+    // previous block times scale of this one, an exact power of two)
 #pragma unroll
     for (int tt = 0; tt < NT; ++tt) {
-      float f0 = 0.0f, f1 = 0.0f;
-      if (bl > 0 && static_cast<uint32_t>(tt) < ntiles) {
-        const float4 c = *reinterpret_cast<const float4 *>(cur + tt * 8), pv = *reinterpret_cast<const float4 *>(prev + tt * 8);
-        f0 = pv.x * c.y;
-        f1 = pv.z * c.w;
+      if (static_cast<uint32_t>(tt) < ntiles) {  // uniform over the CTA
+        const float4 c = *reinterpret_cast<const float4 *>(cur + tt * 8);
+        const float f0 = carry[tt][0] * c.y, f1 = carry[tt][1] * c.w;
+        carry[tt][0] = c.x;
+        carry[tt][1] = c.z;
+        tot[tt][0] *= f0;
+        tot[tt][1] *= f1;
+        tot[tt][2] *= f0;
+        tot[tt][3] *= f1;
       }
-      tot[tt][0] *= f0;
-      tot[tt][1] *= f1;
-      tot[tt][2] *= f0;
-      tot[tt][3] *= f1;
     }
-    if (more) q0 += 8 * step_words, q1 += 8 * step_words, q2 += 8 * step_words;
 #pragma unroll
     for (int kt = 0; kt < 8; ++kt) {
-      uint32_t a[4];
-      decode8<K2>(bw.w[kt][0], bw.w[kt][1], bw.w[kt][2], win.off, a);
-      if (more) {
-        bw.w[kt][0] = __ldg(q0 + kt * step_words);
-        bw.w[kt][1] = __ldg(q1 + kt * step_words);
-        bw.w[kt][2] = __ldg(q2 + kt * step_words);
+      const uint32_t a0 = w[0], a1 = w[1], a2 = w[2];
+      if (kt < 7) {
+        w[0] = *reinterpret_cast<const uint32_t *>(w0 + at + (kt + 1) * 128 * K2);
+        w[1] = *reinterpret_cast<const uint32_t *>(w1 + at + (kt + 1) * 128 * K2);
+        w[2] = *reinterpret_cast<const uint32_t *>(w2 + at + (kt + 1) * 128 * K2);
       }
+      uint32_t a[4];
+      decode8<K2>(a0, a1, a2, win.off, a);
 #pragma unroll
       for (int tt = 0; tt < NT; ++tt) {
-        if (static_cast<uint32_t>(tt) < ntiles) {  // uniform over the CTA
+        if (static_cast<uint32_t>(tt) < ntiles) {
           const uint2 b = fb[tt * 256 + kt * 32];
           mma_f16_f32(tot[tt], a[0], a[2], a[1], a[3], b.x, b.y);
         }
       }
     }
+    slot = slot + 1u == S::kDepth ? 0u : slot + 1u;
+    fill = fill + 1u == S::kDepth ? 0u : fill + 1u;
   }
   // back to the rows' own units
-  const float2 *last = scale_buf[(nblk - 1u) % 3] + t2;
 #pragma unroll
   for (int tt = 0; tt < NT; ++tt) {
-    float i0 = 0.0f, i1 = 0.0f;
-    if (static_cast<uint32_t>(tt) < ntiles) {
-      const float4 c = *reinterpret_cast<const float4 *>(last + tt * 8);
-      i0 = c.x;
-      i1 = c.z;
-    }
-    tot[tt][0] *= i0;
-    tot[tt][1] *= i1;
-    tot[tt][2] *= i0;
-    tot[tt][3] *= i1;
+    tot[tt][0] *= carry[tt][0];
+    tot[tt][1] *= carry[tt][1];
+    tot[tt][2] *= carry[tt][0];
+    tot[tt][3] *= carry[tt][1];
   }
 }
 
@@ -410,11 +421,9 @@ __device__ __forceinline__ void walk_tile_column(const uint32_t *tile_base, int6
 // One CTA per (item, block of 128 output columns); no CTA waits for another.
 template <int PHASE, int NT>
 __global__ void __launch_bounds__(kThreads, NT <= 2 ? 3 : 2) moe_experts_kernel(const __grid_constant__ ExpertParams p) {
-  // staging for two blocks of fragments, aliased after the walk by the partial sums
-  // [tile column 8][row tile NT][lane 32]; three blocks of scales
-  __shared__ __align__(16) uint2 frag_buf[2][NT * 256];
-  __shared__ __align__(16) float2 scale_buf[3][NT * 8];
-  float4 *part = reinterpret_cast<float4 *>(&frag_buf[0][0]);
+  // the staging slots, taken over after the walk by the partial sums [tile column 8][row tile NT][lane 32]
+  extern __shared__ __align__(128) uint8_t staging[];
+  float4 *part = reinterpret_cast<float4 *>(staging);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t in = PHASE == 0 ? p.hidden : p.inter;
   const uint32_t out_plane = PHASE == 0 ? 2u * p.inter : p.hidden;   // columns of the stored plane
@@ -447,14 +456,13 @@ __global__ void __launch_bounds__(kThreads, NT <= 2 ? 3 : 2) moe_experts_kernel(
 #pragma unroll
     for (int e = 0; e < 4; ++e) tot[tt][e] = 0.0f;
   {
-    const uint32_t tile_words = 4u * k2;
-    const uint32_t *tile_base = trellis + (static_cast<uint64_t>(col_block) * 8u + static_cast<uint32_t>(warp)) * tile_words;
-    const int64_t step_words = static_cast<int64_t>(out_plane / 16u) * tile_words;
+    const uint8_t *col = reinterpret_cast<const uint8_t *>(trellis) + static_cast<uint64_t>(col_block) * 128u * k2;
+    const uint64_t pitch = static_cast<uint64_t>(out_plane) * k2;   // bytes from a tile row to the next
     switch (k2) {
-      case 4: walk_tile_column<4, NT>(tile_base, step_words, nblk, frag, scales, ntiles, lane, frag_buf, scale_buf, tot); break;
-      case 5: walk_tile_column<5, NT>(tile_base, step_words, nblk, frag, scales, ntiles, lane, frag_buf, scale_buf, tot); break;
-      case 6: walk_tile_column<6, NT>(tile_base, step_words, nblk, frag, scales, ntiles, lane, frag_buf, scale_buf, tot); break;
-      default: walk_tile_column<8, NT>(tile_base, step_words, nblk, frag, scales, ntiles, lane, frag_buf, scale_buf, tot); break;
+      case 4: walk_tile_column<4, NT>(col, pitch, nblk, frag, scales, ntiles, warp, lane, staging, tot); break;
+      case 5: walk_tile_column<5, NT>(col, pitch, nblk, frag, scales, ntiles, warp, lane, staging, tot); break;
+      case 6: walk_tile_column<6, NT>(col, pitch, nblk, frag, scales, ntiles, warp, lane, staging, tot); break;
+      default: walk_tile_column<8, NT>(col, pitch, nblk, frag, scales, ntiles, warp, lane, staging, tot); break;
     }
   }
   __syncthreads();  // every warp is done with the staging buffers: the partial sums take their place
@@ -670,11 +678,11 @@ int32_t run_experts(const Geometry &g, const void *x, uint32_t tokens, const int
     if (err != cudaSuccess) return fail(slot, "%s: rotation launch failed: %s", what, cudaGetErrorString(err));
     const dim3 grid(items_max * col_blocks);
     if (phase == 0) {
-      err = wide ? launch(moe_experts_kernel<0, 8>, grid, dim3(kThreads), 0, stream, pdl, p)
-                 : launch(moe_experts_kernel<0, 1>, grid, dim3(kThreads), 0, stream, pdl, p);
+      err = wide ? launch(moe_experts_kernel<0, 8>, grid, dim3(kThreads), Staging<8>::kBytes, stream, pdl, p)
+                 : launch(moe_experts_kernel<0, 1>, grid, dim3(kThreads), Staging<1>::kBytes, stream, pdl, p);
     } else {
-      err = wide ? launch(moe_experts_kernel<1, 8>, grid, dim3(kThreads), 0, stream, pdl, p)
-                 : launch(moe_experts_kernel<1, 1>, grid, dim3(kThreads), 0, stream, pdl, p);
+      err = wide ? launch(moe_experts_kernel<1, 8>, grid, dim3(kThreads), Staging<8>::kBytes, stream, pdl, p)
+                 : launch(moe_experts_kernel<1, 1>, grid, dim3(kThreads), Staging<1>::kBytes, stream, pdl, p);
     }
     if (err != cudaSuccess) return fail(slot, "%s: expert launch failed: %s", what, cudaGetErrorString(err));
   }
@@ -685,6 +693,9 @@ int32_t run_experts(const Geometry &g, const void *x, uint32_t tokens, const int
 
 int32_t prepare_moe_kernels(ErrorSlot &slot) {
   if (moe_rows_prepare(slot) != 0) return -1;
+  cudaError_t err = cudaFuncSetAttribute(moe_experts_kernel<0, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Staging<8>::kBytes));
+  if (err == cudaSuccess) err = cudaFuncSetAttribute(moe_experts_kernel<1, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Staging<8>::kBytes));
+  if (err != cudaSuccess) return fail(slot, "expert kernel attributes: %s", cudaGetErrorString(err));
   if (moe_tc_prepare(slot) != 0) return -1;
   return moe_fp8_tc_prepare(slot);
 }

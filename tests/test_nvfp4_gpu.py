@@ -771,6 +771,33 @@ def test_w4a4_tensor_core_route(nv, oracle, tokens, n, k):
         nv.linear(x.cuda(), w, policy=nv.ALLOW_A4)
 
 
+@pytest.mark.parametrize("tokens,n,k", [(33, 128, 256), (47, 384, 1792), (112, 128, 4352), (128, 256, 768), (129, 640, 1024), (145, 128, 2304),
+                                        (257, 128, 512)])
+def test_w4a4_few_tokens(nv, oracle, tokens, n, k):
+    """Calls that leave the pair GEMM idle (nvfp4_w4a4_narrow.cu): token tiles of 48 to 128 with ragged ends, one row tile to
+    five, K slices of unequal length over a cluster, and residual ADD and the fused SwiGLU on top of them."""
+    rng = np.random.default_rng(3 * tokens + n + k)
+    codes, scales, d_w = make_weight(rng, n, k)
+    d_in = 448.0
+    w = nv.Weight.from_planes(codes, scales, d_w, d_in)
+    gen = torch.Generator().manual_seed(k + tokens)
+    x = torch.randn(tokens, k, generator=gen).to(torch.bfloat16)
+    ref = w4a4_reference(oracle, codes, scales, n, k, d_w, d_in, x)
+    ws = nv.Workspace(nv.workspace_bytes(n, k, nv.ALLOW_A4, tokens))
+    check_f32(nv.linear(x.cuda(), w, policy=nv.ALLOW_A4, epilogue=nv.OUT_F32, workspace=ws), ref)
+    base = torch.randn(tokens, n, generator=gen).to(torch.bfloat16)
+    y = base.clone().cuda()
+    nv.linear(x.cuda(), w, y, policy=nv.ALLOW_A4, epilogue=nv.ADD, workspace=ws)
+    check_bf16(y, ref + base.double().numpy())
+    if n % 256 == 0:
+        g = torch.from_numpy(ref[:, : n // 2]).to(torch.bfloat16).double()
+        u = torch.from_numpy(ref[:, n // 2:]).to(torch.bfloat16).double()
+        want = (g / (1 + torch.exp(-g)) * u).numpy()
+        got = nv.linear_swiglu(x.cuda(), w, policy=nv.ALLOW_A4, workspace=ws).double().cpu().numpy()
+        assert np.linalg.norm(got - want) <= 2.0 ** -7 * np.linalg.norm(want)
+    assert ws.status() == 0
+
+
 def test_w4a4_one_cta_forms_agree_with_the_pair_form(nv, oracle, tmp_path):
     """The prefill GEMM form kept behind an environment switch (one CTA per tile, persistent) runs in
     a child process - the switch is read once per process - on the same operands as this process's

@@ -141,6 +141,22 @@ def test_linear_shapes_and_token_counts(tr, oracle, in_, out, k2, tokens):
     assert torch.equal(y, tr.linear(w, x.cuda()))   # deterministic run to run
 
 
+@pytest.mark.parametrize("in_,out,k2", [(128, 1280, 12), (896, 128, 12), (2176, 128, 4), (4480, 128, 10)])
+@pytest.mark.parametrize("tokens", [1, 9, 33])
+def test_word_ring_edges(tr, oracle, in_, out, k2, tokens):
+    """The packed words' ring in shared memory: slices shorter than the ring, slices that wrap it, the widest and the narrowest
+    words."""
+    rng = np.random.default_rng(in_ + out + tokens)
+    words = oracle.hash_trellis_words(7300 + in_ + k2, in_, out, k2)
+    suh, svh = make_scales(rng, in_, 0.05), make_scales(rng, out, 0.03)
+    inner = oracle.trellis_decode(words, k2, in_, out)
+    x = torch.randn(tokens, in_, generator=torch.Generator().manual_seed(tokens + in_)).to(torch.bfloat16)
+    x64 = x.double().numpy()
+    w = tr.Weight.from_numpy(words, suh, svh, k2, in_, out)
+    check_linear(tr.linear(w, x.cuda()), oracle.trellis_project(inner, suh, svh, x64), tolerance(oracle, inner, suh, svh, x64))
+    assert tr.device_status() == 0
+
+
 def test_loud_channels_and_tiny_tokens(tr, oracle):
     """A few inputs 1000x louder than the rest, and tokens of very different scale: the per-block
     power-of-two scaling keeps every block in fp16 range (test_trellis_linear.cu:80-89)."""
@@ -291,6 +307,33 @@ def test_real_shapes_at_wide_token_counts(tr, oracle, in_, out, tokens):
         assert tr.device_status() == 0
         check_linear(y[pick], ref, s)
         assert torch.equal(y, tr.linear(w, x.cuda(), workspace=ws))   # the same bits again
+
+
+@pytest.mark.parametrize("in_,out,k2", [(1024, 128, 4), (1152, 256, 12), (4096, 384, 5), (8704, 128, 8)])
+@pytest.mark.parametrize("tokens", [65, 128, 129, 257])
+def test_k_shared_by_a_cluster(tr, oracle, in_, out, k2, tokens):
+    """Few items beyond 64 tokens: two to eight CTAs of a cluster share an item's K stages, in unequal shares too, and deal its
+    rows; one row tile and two, a last row pair with one row, residual ADD on top."""
+    from oracle import oracle as orc
+
+    rng = np.random.default_rng(in_ + tokens)
+    words = oracle.hash_trellis_words(6100 + in_ + k2, in_, out, k2)
+    suh, svh = make_scales(rng, in_, 0.05), make_scales(rng, out, 0.03)
+    inner = oracle.trellis_decode(words, k2, in_, out)
+    w = tr.Weight.from_numpy(words, suh, svh, k2, in_, out)
+    gen = torch.Generator().manual_seed(tokens)
+    x = torch.randn(tokens, in_, generator=gen).to(torch.bfloat16)
+    ref, s = orc.trellis_project_rows(inner, suh, svh, x.double().numpy())
+    ws = tr.WorkspaceBuffer(tr.workspace_bytes(in_, out, 1, tokens))
+    y = tr.linear(w, x.cuda(), workspace=ws)
+    check_linear(y, ref, s)
+    assert torch.equal(y, tr.linear(w, x.cuda(), workspace=ws))   # the same bits again
+    base = torch.randn(tokens, out, generator=gen).to(torch.bfloat16)
+    z = base.clone().cuda()
+    tr.linear(w, x.cuda(), out=z, epilogue=tr.ADD, workspace=ws)
+    b64 = base.double().numpy()
+    check_linear(z, ref + b64, s + 2.0 * np.abs(b64))
+    assert tr.device_status() == 0
 
 
 @pytest.mark.parametrize("tokens", [64, 130, 300])
