@@ -1,6 +1,6 @@
 // Device-side pieces shared by the dense trellis linear and the MoE expert kernels: the tile
-// decode (format: kernel/src/trellis_decode.cuh:6-24 of the reference), the warp Hadamard, the
-// cluster helpers and a warp's walk over its 128-input blocks.
+// decode (format: kernel/src/trellis_decode.cuh:6-24 of the reference), the warp Hadamard and the
+// cluster helpers.
 #ifndef B200Q_TRELLIS_DEVICE_CUH
 #define B200Q_TRELLIS_DEVICE_CUH
 
@@ -109,94 +109,6 @@ __device__ __forceinline__ float ld_cluster_f32(const float *local_smem, uint32_
   float v;
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
   return v;
-}
-
-struct TileWords {
-  uint32_t w[8][3];
-};
-
-// The lane's three words of each of the 8 tiles of one 16-input step. `p0/p1/p2` point at the
-// lane's words w0/w1/w2 of the step's first tile; tiles are 4 K2 words apart (a compile-time
-// distance, so the loads carry immediate offsets).
-template <int K2>
-__device__ __forceinline__ void load_step(TileWords &tw, const uint32_t *p0, const uint32_t *p1, const uint32_t *p2) {
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    tw.w[j][0] = __ldg(p0 + j * 4 * K2);
-    tw.w[j][1] = __ldg(p1 + j * 4 * K2);
-    tw.w[j][2] = __ldg(p2 + j * 4 * K2);
-  }
-}
-
-// One step of 16 inputs: the 8 tiles of the column block, decoded and multiplied.
-template <int K2>
-__device__ __forceinline__ void step_tiles(const TileWords &tw, uint32_t off, const uint2 bfrag, float (&acc)[8][4]) {
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    uint32_t frag[4];
-    decode8<K2>(tw.w[j][0], tw.w[j][1], tw.w[j][2], off, frag);
-    mma_f16_f32(acc[j], frag[0], frag[2], frag[1], frag[3], bfrag.x, bfrag.y);
-  }
-}
-
-// A warp's walk over its 128-input blocks [blk, b1) in strides of `stride` blocks: 8 steps per
-// block, the words of the next step in flight while the current one is decoded (two register
-// buffers, alternating). Accumulators live in the units of the current block's per-token scale
-// and are carried into the next block's units by an exact power-of-two factor.
-template <int K2>
-__device__ __forceinline__ void walk_blocks(const uint32_t *col_base, uint64_t tk_stride, const LaneWindow &win, uint32_t blk,
-                                            uint32_t b0, uint32_t b1, uint32_t stride, const uint2 *xs_side,
-                                            const float *inv_side, const float *scale_side, int lane, float (&tot)[8][4]) {
-  if (blk >= b1) return;
-  const int t2 = (lane & 3) * 2;
-  // Three running pointers (the lane's words w0, w1, w2 of the step to load next); every load is
-  // pointer + compile-time offset. Inside a block the next step is one tile row further; after a
-  // block's last step the pointers jump to the warp's next block.
-  const uint32_t *q0 = col_base + win.w0 + static_cast<uint64_t>(blk) * 8u * tk_stride;
-  const uint32_t *q1 = q0 + (static_cast<int64_t>(win.w1) - static_cast<int64_t>(win.w0));
-  const uint32_t *q2 = q0 + (static_cast<int64_t>(win.w2) - static_cast<int64_t>(win.w0));
-  const int64_t step = static_cast<int64_t>(tk_stride);
-  const int64_t jump = static_cast<int64_t>(static_cast<uint64_t>(stride) * 8u - 7u) * step;
-  TileWords even, odd;
-  load_step<K2>(even, q0, q1, q2);
-  q0 += step, q1 += step, q2 += step;
-  float carry0 = 0.0f, carry1 = 0.0f;
-  for (; blk < b1; blk += stride) {
-    const uint32_t bl = blk - b0;
-    const float f0 = carry0 * scale_side[bl * 8 + t2], f1 = carry1 * scale_side[bl * 8 + t2 + 1];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      tot[j][0] *= f0;
-      tot[j][1] *= f1;
-      tot[j][2] *= f0;
-      tot[j][3] *= f1;
-    }
-    // after this block's last step: on to the next block, or (last block) back one step, so the
-    // final prefetch re-reads the last step instead of running past the tensor
-    const int64_t after = blk + stride < b1 ? jump : -step;
-    const uint2 *xb = xs_side + static_cast<size_t>(bl) * 8 * 32 + lane;
-#pragma unroll
-    for (int kt = 0; kt < 8; kt += 2) {
-      load_step<K2>(odd, q0, q1, q2);  // step kt + 1
-      {
-        const int64_t d = kt + 1 == 7 ? after : step;
-        q0 += d, q1 += d, q2 += d;
-      }
-      step_tiles<K2>(even, win.off, xb[kt * 32], tot);
-      load_step<K2>(even, q0, q1, q2);  // step kt + 2, or the first step of the next block
-      q0 += step, q1 += step, q2 += step;
-      step_tiles<K2>(odd, win.off, xb[(kt + 1) * 32], tot);
-    }
-    carry0 = inv_side[bl * 8 + t2];
-    carry1 = inv_side[bl * 8 + t2 + 1];
-  }
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    tot[j][0] *= carry0;
-    tot[j][1] *= carry1;
-    tot[j][2] *= carry0;
-    tot[j][3] *= carry1;
-  }
 }
 
 }  // namespace trellis_dev

@@ -324,13 +324,6 @@ __device__ __forceinline__ bool core_roles(const Core &c, const Job &job, const 
   return false;
 }
 
-// Both steps back to back.
-template <int DW>
-__device__ __forceinline__ bool core_run(const Core &c, const Job &job, const CUtensorMap *map_a, uint32_t *status) {
-  const bool decoded = core_roles<DW>(c, job, map_a, status);
-  return c.warp < DW ? core_accumulator<DW>(c, decoded, status) : false;
-}
-
 // ---- epilogue ------------------------------------------------------------------------------------
 // A warp group (warp / 4: four warps, 128 threads = the 128 rows of a row tile, a warp's lanes the
 // rows 32 (warp % 4) .. + 31) owns an area of the idle stage ring: 128 rows of 64 floats, 68 apart, so
