@@ -123,6 +123,10 @@ class Weight:
         object.__setattr__(self, name, value)
         self.__dict__.pop("_ref", None)   # a field was replaced: the struct is built anew
 
+    def __getstate__(self) -> dict:
+        """The fields, without what calls keep beside them: C objects hold addresses and cannot be copied or pickled."""
+        return {name: value for name, value in self.__dict__.items() if name not in ("_ref", "_ranges")}
+
     def ref(self):
         """``byref`` of the C struct, built once: a decode call enqueues one kernel, and building it took a fifth of that call."""
         ref = self.__dict__.get("_ref")

@@ -88,6 +88,10 @@ class Weight:
         object.__setattr__(self, name, value)
         self.__dict__.pop("_struct", None)   # a field was replaced: the struct is built anew
 
+    def __getstate__(self) -> dict:
+        """The fields, without the C struct that calls keep beside them: it holds addresses and cannot be copied or pickled."""
+        return {name: value for name, value in self.__dict__.items() if name != "_struct"}
+
     def struct(self) -> _lib.TrellisWeight:
         """The C struct, built once."""
         struct = self.__dict__.get("_struct")

@@ -1,0 +1,92 @@
+"""No-GPU checks of the Python mirror's weights and workspaces: what a call keeps with an object it was
+given must not change what that object is afterwards. The planes are CPU tensors that say they are on a
+device; nothing here launches a kernel."""
+from __future__ import annotations
+
+import copy
+import pickle
+
+import pytest
+import torch
+
+from ignis_b200 import _lib, moe, nvfp4, trellis
+
+
+class OnDevice(torch.Tensor):
+    """A CPU tensor that answers ``is_cuda`` as a device tensor would."""
+
+    is_cuda = True
+
+    def __deepcopy__(self, memo):
+        return on_device(self.as_subclass(torch.Tensor).clone())
+
+
+def on_device(t: torch.Tensor) -> torch.Tensor:
+    return t.as_subclass(OnDevice)
+
+
+def nvfp4_weight() -> nvfp4.Weight:
+    n, k = 128, 256
+    return nvfp4.Weight(on_device(torch.arange(n * k // 2, dtype=torch.int64).to(torch.uint8).reshape(n, k // 2)),
+                        on_device(torch.ones(n * k // 16, dtype=torch.uint8)), n, k, 448.0, 96.0)
+
+
+def trellis_weight() -> trellis.Weight:
+    in_ = out = 128
+    return trellis.Weight(on_device(torch.arange(8 * 8 * trellis.tile_words16(6), dtype=torch.int16)), on_device(torch.ones(in_, dtype=torch.float16)),
+                          on_device(torch.ones(out, dtype=torch.float16)), 6, in_, out)
+
+
+class Recorder:
+    """Stands in for the library: every entry point succeeds, the last call's arguments are kept."""
+
+    def __init__(self) -> None:
+        self.args = ()
+
+    def __getattr__(self, name):
+        def entry(*args):
+            self.args = args
+            return 0
+        return entry
+
+
+@pytest.fixture
+def lib(monkeypatch):
+    lib = Recorder()
+    monkeypatch.setattr(_lib, "load", lambda: lib)
+    for module in (nvfp4, trellis, moe):
+        monkeypatch.setattr(module, "_stream", lambda: 0)
+    return lib
+
+
+def planes(w) -> list[torch.Tensor]:
+    return [w.codes, w.scales] if isinstance(w, nvfp4.Weight) else [w.trellis, w.suh, w.svh]
+
+
+def activations(w) -> torch.Tensor:
+    return on_device(torch.ones(2, w.k if isinstance(w, nvfp4.Weight) else w.in_, dtype=torch.bfloat16))
+
+
+def addresses_in_a_call(lib, w) -> list[int]:
+    """The plane addresses in the struct that the library is handed."""
+    if isinstance(w, nvfp4.Weight):
+        nvfp4.linear_split(activations(w), w, [w.n])
+        s = lib.args[0]._obj
+        return [s.codes, s.scales]
+    trellis.linear(w, activations(w))
+    s = lib.args[0]._obj
+    return [s.trellis, s.suh, s.svh]
+
+
+@pytest.mark.parametrize("make", [nvfp4_weight, trellis_weight])
+@pytest.mark.parametrize("duplicate", [copy.deepcopy, lambda w: pickle.loads(pickle.dumps(w)), copy.copy])
+def test_a_weight_that_was_called_can_be_copied(lib, make, duplicate):
+    w = make()
+    w.label = "layer 0"   # what a program adds goes along
+    before = addresses_in_a_call(lib, w)
+    assert before == [t.data_ptr() for t in planes(w)]
+    twin = duplicate(w)
+    assert type(twin) is type(w) and twin.label == "layer 0"
+    assert all(torch.equal(a, b) for a, b in zip(planes(w), planes(twin)))
+    assert addresses_in_a_call(lib, twin) == [t.data_ptr() for t in planes(twin)]   # its own planes
+    assert addresses_in_a_call(lib, w) == before
