@@ -128,11 +128,13 @@ class Weight:
         return {name: value for name, value in self.__dict__.items() if name not in ("_ref", "_ranges")}
 
     def ref(self):
-        """``byref`` of the C struct, built once: a decode call enqueues one kernel, and building it took a fifth of that call."""
-        ref = self.__dict__.get("_ref")
-        if ref is None:
-            ref = self.__dict__["_ref"] = C.byref(self.c_struct())
-        return ref
+        """``byref`` of the C struct. Kept between calls (a decode call enqueues one kernel, and building the struct took a
+        fifth of it) while both planes lie where it says: a plane may be re-seated in place, its field never assigned."""
+        at = (self.codes.data_ptr(), self.scales.data_ptr())
+        kept = self.__dict__.get("_ref")
+        if kept is None or kept[0] != at:
+            kept = self.__dict__["_ref"] = (at, C.byref(self.c_struct()))
+        return kept[1]
 
     @property
     def payload_bytes(self) -> int:

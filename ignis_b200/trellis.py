@@ -93,11 +93,13 @@ class Weight:
         return {name: value for name, value in self.__dict__.items() if name != "_struct"}
 
     def struct(self) -> _lib.TrellisWeight:
-        """The C struct, built once."""
-        struct = self.__dict__.get("_struct")
-        if struct is None:
-            struct = self.__dict__["_struct"] = self.c_struct()
-        return struct
+        """The C struct, kept between calls while the three planes lie where it says (a plane may be re-seated in place, its
+        field never assigned)."""
+        at = (self.trellis.data_ptr(), self.suh.data_ptr(), self.svh.data_ptr())
+        kept = self.__dict__.get("_struct")
+        if kept is None or kept[0] != at:
+            kept = self.__dict__["_struct"] = (at, self.c_struct())
+        return kept[1]
 
 
 def prepare() -> None:

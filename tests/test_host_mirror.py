@@ -90,3 +90,27 @@ def test_a_weight_that_was_called_can_be_copied(lib, make, duplicate):
     assert all(torch.equal(a, b) for a, b in zip(planes(w), planes(twin)))
     assert addresses_in_a_call(lib, twin) == [t.data_ptr() for t in planes(twin)]   # its own planes
     assert addresses_in_a_call(lib, w) == before
+
+
+@pytest.mark.parametrize("make", [nvfp4_weight, trellis_weight])
+def test_planes_reseated_in_place_are_the_ones_a_call_reads(lib, make):
+    """A plane can get another memory without its field being assigned: through ``.data``, ``set_`` or ``resize_``."""
+    w = make()
+    for i in range(len(planes(w))):
+        addresses_in_a_call(lib, w)
+        kept = planes(w)[i].data   # keeps the old memory alive: the new one lies elsewhere
+        planes(w)[i].data = on_device(planes(w)[i].as_subclass(torch.Tensor).clone())
+        assert planes(w)[i].data_ptr() != kept.data_ptr()
+        assert addresses_in_a_call(lib, w) == [t.data_ptr() for t in planes(w)]
+    planes(w)[1].set_(on_device(planes(w)[1].as_subclass(torch.Tensor).clone()))
+    assert addresses_in_a_call(lib, w) == [t.data_ptr() for t in planes(w)]
+
+
+@pytest.mark.parametrize("make", [nvfp4_weight, trellis_weight])
+def test_a_weight_moved_off_the_device_is_refused(lib, make):
+    w = make()
+    addresses_in_a_call(lib, w)
+    name = "codes" if isinstance(w, nvfp4.Weight) else "trellis"
+    setattr(w, name, getattr(w, name).as_subclass(torch.Tensor).clone())
+    with pytest.raises((nvfp4.Nvfp4Error, trellis.TrellisError)):
+        addresses_in_a_call(lib, w)
