@@ -162,7 +162,6 @@ class Workspace:
     def __init__(self, nbytes: int, device: str | torch.device = "cuda") -> None:
         self.buffer = torch.empty(max(256, int(nbytes)), dtype=torch.uint8, device=device)
         self.c = _lib.Workspace(self.buffer.data_ptr(), self.buffer.numel())
-        self.ref = C.byref(self.c)
         _check(_lib.load().b200q_nvfp4_workspace_init(C.byref(self.c), _stream()))
 
     def status(self) -> int:
@@ -196,7 +195,7 @@ def linear(x: torch.Tensor, w: Weight, out: torch.Tensor | None = None, policy: 
     tokens = x.size(0)
     y = _out(tokens, w.n, epilogue, out, x)
     _check(_lib.load().b200q_nvfp4_linear(w.ref(), x.data_ptr(), tokens, y.data_ptr(), y.stride(0), epilogue, policy,
-                                           workspace.ref if workspace is not None else None, _stream()))
+                                           C.byref(workspace.c) if workspace is not None else None, _stream()))
     return y
 
 
@@ -256,7 +255,7 @@ def linear_split(x: torch.Tensor, parent: Weight, row_counts: list[int], outs: l
     yp = ptrs(*[y.data_ptr() for y in ys])
     ld = u32s(*[y.stride(0) for y in ys])
     _check(_lib.load().b200q_nvfp4_linear_split(parent.ref(), count, rb, rc, x.data_ptr(), tokens, yp, ld, epilogue, policy,
-                                                 workspace.ref if workspace is not None else None, _stream()))
+                                                 C.byref(workspace.c) if workspace is not None else None, _stream()))
     return ys
 
 
@@ -305,7 +304,7 @@ def linear_swiglu(x: torch.Tensor, gate_up: Weight, out: torch.Tensor | None = N
     tokens = x.shape[0]
     h = _out(tokens, gate_up.n // 2, STORE, out, x)
     _check(_lib.load().b200q_nvfp4_linear_swiglu(gate_up.ref(), x.data_ptr(), tokens, h.data_ptr(), h.stride(0), policy,
-                                                  workspace.ref if workspace is not None else None, _stream()))
+                                                  C.byref(workspace.c) if workspace is not None else None, _stream()))
     return h
 
 
@@ -322,7 +321,7 @@ def mlp(x: torch.Tensor, gate_up: Weight, down: Weight, workspace: Workspace, ou
     tokens = x.shape[0]
     y = _out(tokens, down.n, epilogue, out, x)
     _check(_lib.load().b200q_nvfp4_mlp(gate_up.ref(), down.ref(), x.data_ptr(), tokens, y.data_ptr(), y.stride(0), epilogue, policy,
-                                        workspace.ref, _stream()))
+                                        C.byref(workspace.c), _stream()))
     return y
 
 
@@ -351,7 +350,7 @@ def quantize_operand(x_rows: torch.Tensor, tokens_total: int, token_begin: int, 
     ``token_begin ..`` of a call of `tokens_total`) into their place of the W4A4 operand in `workspace`."""
     _check_x(x_rows, k)
     _check(_lib.load().b200q_nvfp4_quantize_operand(x_rows.data_ptr(), tokens_total, token_begin, x_rows.shape[0], k,
-                                                     float(input_scale_divisor), workspace.ref, _stream()))
+                                                     float(input_scale_divisor), C.byref(workspace.c), _stream()))
 
 
 def operand_ranges(k: int, tokens_total: int, token_begin: int, token_count: int) -> tuple[tuple[int, int], tuple[int, int]]:
@@ -370,7 +369,7 @@ def linear_prequantized(w: Weight, tokens: int, workspace: Workspace, out: torch
     """``b200q_nvfp4_linear_prequantized``: the tensor-core product over the operand in `workspace`."""
     y = _out(tokens, w.n, epilogue, out, w.codes)
     _check(_lib.load().b200q_nvfp4_linear_prequantized(w.ref(), tokens, y.data_ptr(), y.stride(0), epilogue,
-                                                        workspace.ref, _stream()))
+                                                        C.byref(workspace.c), _stream()))
     return y
 
 

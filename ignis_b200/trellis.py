@@ -123,7 +123,6 @@ class WorkspaceBuffer:
     def __init__(self, nbytes: int, device="cuda") -> None:
         self.buffer = torch.empty(max(256, nbytes), dtype=torch.uint8, device=device)
         self.c = _lib.Workspace(self.buffer.data_ptr(), self.buffer.numel())
-        self.ref = C.byref(self.c)
         _check(_lib.load().ignis_trellis_workspace_init(C.byref(self.c), _stream()))
 
 
@@ -142,7 +141,7 @@ def linear(w: Weight, x: torch.Tensor, out: torch.Tensor | None = None, epilogue
             raise TrellisError("the ADD epilogue accumulates into `out`, which must be given")
         out = x.new_empty((tokens, w.out))
     _check(_lib.load().ignis_trellis_linear(C.byref(w.struct()), x.data_ptr(), tokens, out.data_ptr(), out.stride(0), epilogue,
-                                             workspace.ref if workspace else None, _stream()))
+                                             C.byref(workspace.c) if workspace else None, _stream()))
     return out
 
 
@@ -174,7 +173,7 @@ def linear_swiglu(gate: Weight, up: Weight, x: torch.Tensor, out: torch.Tensor |
     if out is None:
         out = x.new_empty((tokens, gate.out))
     _check(_lib.load().ignis_trellis_linear_swiglu(C.byref(gate.struct()), C.byref(up.struct()), x.data_ptr(), tokens, out.data_ptr(),
-                                                    out.stride(0), workspace.ref if workspace else None,
+                                                    out.stride(0), C.byref(workspace.c) if workspace else None,
                                                     _stream()))
     return out
 

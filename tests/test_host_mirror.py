@@ -114,3 +114,15 @@ def test_a_weight_moved_off_the_device_is_refused(lib, make):
     setattr(w, name, getattr(w, name).as_subclass(torch.Tensor).clone())
     with pytest.raises((nvfp4.Nvfp4Error, trellis.TrellisError)):
         addresses_in_a_call(lib, w)
+
+
+@pytest.mark.parametrize("make,module,kind", [(nvfp4_weight, nvfp4, nvfp4.Workspace), (trellis_weight, trellis, trellis.WorkspaceBuffer)])
+def test_a_call_takes_the_workspace_struct_that_is_there_now(lib, make, module, kind):
+    ws = kind(512, device="cpu")
+    w = make()
+    x = activations(w)
+    for base in (ws.c.base, ws.c.base + 256):   # another struct put in its place: a part of a larger region
+        ws.c = _lib.Workspace(base, 256)
+        module.linear(*((x, w) if module is nvfp4 else (w, x)), workspace=ws)
+        seen = next(a._obj for a in lib.args if isinstance(getattr(a, "_obj", None), _lib.Workspace))
+        assert seen.base == base and seen.bytes == 256
