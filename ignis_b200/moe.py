@@ -46,11 +46,7 @@ class Geometry:
     top_k: int = 10
 
     def c_struct(self) -> _lib.MoeGeometry:
-        """The C struct, built once (the fields are frozen)."""
-        struct = self.__dict__.get("_struct")
-        if struct is None:
-            struct = self.__dict__["_struct"] = _lib.MoeGeometry(self.hidden, self.inter, self.experts, self.top_k)
-        return struct
+        return _lib.MoeGeometry(self.hidden, self.inter, self.experts, self.top_k)
 
 
 _geometry = Geometry()

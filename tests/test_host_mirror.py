@@ -126,3 +126,10 @@ def test_a_call_takes_the_workspace_struct_that_is_there_now(lib, make, module, 
         module.linear(*((x, w) if module is nvfp4 else (w, x)), workspace=ws)
         seen = next(a._obj for a in lib.args if isinstance(getattr(a, "_obj", None), _lib.Workspace))
         assert seen.base == base and seen.bytes == 256
+
+
+def test_a_geometry_struct_is_the_callers_own():
+    g = moe.Geometry(256, 128, 8, 2)
+    g.c_struct().hidden = 512
+    assert g.c_struct().hidden == 256
+    assert pickle.loads(pickle.dumps(g)) == g and set(vars(g)) == {"hidden", "inter", "experts", "top_k"}
