@@ -753,9 +753,10 @@ int32_t b200q_trellis_device_status(void *stream, uint32_t *status) {
   ErrorSlot &slot = trellis_error();
   if (status == nullptr) return fail(slot, "b200q_trellis_device_status: status is NULL");
   uint32_t linear = 0, wide = 0;
-  if (trellis_tc_status(slot, static_cast<cudaStream_t>(stream), &wide) != 0) return -1;
-  const cudaError_t err = cudaMemcpyFromSymbol(&linear, g_linear_status, sizeof(uint32_t));   // the stream is idle
+  // both words in the caller's stream: a synchronous copy would wait for the other blocking streams too
+  const cudaError_t err = cudaMemcpyFromSymbolAsync(&linear, g_linear_status, sizeof(uint32_t), 0, cudaMemcpyDeviceToHost, static_cast<cudaStream_t>(stream));
   if (err != cudaSuccess) return fail(slot, "b200q_trellis_device_status: %s", cudaGetErrorString(err));
+  if (trellis_tc_status(slot, static_cast<cudaStream_t>(stream), &wide) != 0) return -1;   // waits for the stream
   *status = linear | wide;
   return 0;
 }

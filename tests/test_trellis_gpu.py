@@ -486,3 +486,32 @@ def test_workspace_and_rejects(tr):
     with pytest.raises(tr.TrellisError):
         tr.linear(w, x, epilogue=5)
     assert tr.sm_cap() == 0
+
+
+def test_status_waits_for_its_own_stream_only(tr):
+    """The status words are read in the caller's stream: a blocking stream with work in flight (which the
+    legacy stream, and with it a synchronous copy, waits for) is still at it when the answer is there."""
+    import ctypes
+
+    cudart, handle = torch.cuda.cudart(), ctypes.c_size_t(0)
+    assert int(cudart.cudaStreamCreate(ctypes.addressof(handle))) == 0
+    busy, own, done = torch.cuda.ExternalStream(handle.value), torch.cuda.Stream(), torch.cuda.Event()
+
+    def status():
+        with torch.cuda.stream(own):
+            return tr.device_status()
+
+    def work(cycles):
+        with torch.cuda.stream(busy):
+            torch.cuda._sleep(cycles)
+            done.record()
+
+    work(1000)   # first uses may wait for the whole device
+    assert status() == 0
+    torch.cuda.synchronize()
+    work(500_000_000)   # a quarter of a second
+    assert status() == 0
+    waited = done.query()
+    busy.synchronize()
+    assert int(cudart.cudaStreamDestroy(handle.value)) == 0
+    assert not waited
