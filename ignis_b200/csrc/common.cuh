@@ -33,15 +33,19 @@ inline int32_t fail(ErrorSlot &slot, const char *fmt, ...) {
 // ---- per-device state --------------------------------------------------------------------------
 struct DeviceState {
   bool prepared = false;
+  // What is a function of the device alone: asked when it is prepared first, and never written again. How much of a
+  // kernel the device holds at once goes by cluster size (0: unknown).
+  bool counted = false;
   int sm_count = 0;
+  int gemv_slots[9] = {};        // CTAs of the NVFP4 decode kernel
+  int a4_slots[9] = {};          // CTAs of the W4A4 decode kernel, one per SM
+  int trellis_clusters[9] = {};  // clusters of the dense trellis tensor-core kernel
   int pdl = 1;           // programmatic dependent launch between the kernels of a call chain
   int gemv_rb = 0;       // B200Q_GEMV_RM: 32-row groups per CTA of the NVFP4 decode kernel (0: auto)
   int gemv_kc = 0;       // B200Q_GEMV_KC: its cluster size (0: auto)
   int gemv_ctas_per_sm = 2;
-  int gemv_slots[9] = {};  // CTAs of the NVFP4 decode kernel resident at once, by cluster size (0: unknown)
   int a16_mma = 1;       // B200Q_A16_MMA: A16 calls of more than 8 tokens take the tensor-core kernel
   int a4_decode = 1;     // B200Q_A4_DECODE: AllowA4 calls of up to 32 tokens take the W4A4 decode kernel (0: the A16 route)
-  int a4_slots[9] = {};      // CTAs of the W4A4 decode kernel placed at one per SM, by cluster size (0: unknown)
   int trellis_kc_max = 8;    // B200Q_TRELLIS_KC_MAX: largest cluster the trellis linear plans (measurement knob)
   int a4_decode_pair = -1;   // B200Q_A4_DECODE_PAIR: two row tiles per CTA of that kernel (-1: by the token count)
   int a4_decode_kc = 0;      // B200Q_A4_DECODE_KC: cluster size of that kernel (0: planned)
@@ -51,16 +55,17 @@ struct DeviceState {
   int gemv_xu = 8;       // B200Q_GEMV_XU: words per row of 8 decoded by the hardware E2M1 conversion
   int sm_cap = 0;        // IGNIS_TRELLIS_SM_CAP
   int moe_tc = 1;        // B200Q_MOE_TC: expert calls of more than 64 tokens take the tensor-core kernels
+  int trellis_dw = 8;    // B200Q_TRELLIS_TC_SHAPE: decoder warps of a dense trellis tensor-core CTA, 8 or 16
+  int moe_dw = 8;        // B200Q_MOE_TC_WIDE: the same for the MoE expert products (1: 16)
   int trellis_tc = 1;    // B200Q_TRELLIS_TC: dense trellis calls of more than 64 tokens with a workspace take the tensor-core route
   int peer_barrier_polls = 1 << 22;  // B200Q_PEER_BARRIER_POLLS: looks at a flag before b200q_peer_barrier gives up (400 ns apart)
 };
 // State of the current device, nullptr (and `slot` filled) when the device query fails.
 DeviceState *device_state(ErrorSlot &slot);
-// Prepares the current device once (thread-safe). 0 on success.
-int32_t prepare_device(ErrorSlot &slot);
-// Kernel attributes of one family each (defined beside the kernels), and all of them behind
-// prepare_device: what every *_prepare entry point runs, so that a process that prepared through one
-// family's entry can call the others' ops too.
+// Kernel attributes and occupancy counts of one family each (defined beside the kernels; called under the
+// lock of prepare_all), and all of them for the current device: what every *_prepare entry point runs
+// (thread-safe; 0 on success), so that a process that prepared through one family's entry can call the
+// others' ops too.
 int32_t prepare_nvfp4_kernels(ErrorSlot &slot);
 int32_t prepare_trellis_kernels(ErrorSlot &slot);
 int32_t prepare_moe_kernels(ErrorSlot &slot);

@@ -256,11 +256,6 @@ __global__ void __launch_bounds__(256) moe_tc_fold_kernel(const __grid_constant_
 
 constexpr size_t kRotateSmemMax = 200 * 1024;
 
-
-// Which shape the expert products take: 8 decoder warps and two CTAs per SM unless B200Q_MOE_TC_WIDE
-// is set to 1 (read when the kernels are prepared).
-int g_moe_dw = 8;
-
 template <int DW>
 cudaError_t set_gemm_attrs() {
   cudaError_t err = cudaFuncSetAttribute(moe_tc_gemm_kernel<0, DW>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Shape<DW>::kSmemBytes));
@@ -279,8 +274,6 @@ cudaError_t launch_gemm(int phase, uint32_t items_max, uint32_t out_plane, cudaS
 }  // namespace
 
 int32_t moe_tc_prepare(ErrorSlot &slot) {
-  const char *wide = getenv("B200Q_MOE_TC_WIDE");
-  g_moe_dw = wide != nullptr && wide[0] == '1' ? 16 : 8;
   cudaError_t err = set_gemm_attrs<16>();
   if (err == cudaSuccess) err = set_gemm_attrs<8>();
   if (err == cudaSuccess) err = cudaFuncSetAttribute(moe_tc_rotate_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRotateSmemMax));
@@ -306,7 +299,8 @@ int32_t moe_tc_experts(ErrorSlot &slot, const DeviceState &dev, const ExpertPara
     if (!make_rows_map(&map_a, phase == 0 ? static_cast<const void *>(p.frag_in) : static_cast<const void *>(p.frag_h), rows, in)) {
       return fail(slot, "%s: tensor map encoding failed", what);
     }
-    err = g_moe_dw == 16 ? launch_gemm<16>(phase, items_max, out_plane, stream, pdl, map_a, p) : launch_gemm<8>(phase, items_max, out_plane, stream, pdl, map_a, p);
+    // 8 decoder warps and two CTAs per SM unless B200Q_MOE_TC_WIDE is set
+    err = dev.moe_dw == 16 ? launch_gemm<16>(phase, items_max, out_plane, stream, pdl, map_a, p) : launch_gemm<8>(phase, items_max, out_plane, stream, pdl, map_a, p);
     if (err != cudaSuccess) return fail(slot, "%s: expert launch failed: %s", what, cudaGetErrorString(err));
   }
   const cudaError_t err = launch(moe_tc_fold_kernel, dim3(tokens), dim3(256), 0, stream, pdl, p, tokens);

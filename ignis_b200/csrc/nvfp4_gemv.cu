@@ -679,7 +679,7 @@ int32_t gemv_prepare(ErrorSlot &slot) {
   // GPC, so the count is not simply slots / size. The plan uses it to tell one wave from two.
   DeviceState *dev = device_state(slot);
   if (dev == nullptr) return -1;
-  for (int kc = 1; kc <= 8; ++kc) {
+  for (int kc = 1; kc <= 8 && !dev->counted; ++kc) {
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(static_cast<unsigned>(kc) * 1024u, 1, 1);
     config.blockDim = dim3(kThreads, 1, 1);

@@ -422,7 +422,7 @@ int32_t w4a4_decode_prepare(ErrorSlot &slot) {
   // kernel whatever its shared memory; the plan scales the count by the CTAs that do share an SM.
   DeviceState *dev = device_state(slot);
   if (dev == nullptr) return -1;
-  for (int kc = 1; kc <= 8; ++kc) {
+  for (int kc = 1; kc <= 8 && !dev->counted; ++kc) {
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(static_cast<unsigned>(kc) * 1024u, 1, 1);
     config.blockDim = dim3(64 + 128 * 2, 1, 1);

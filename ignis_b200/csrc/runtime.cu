@@ -50,29 +50,22 @@ DeviceState *device_state(ErrorSlot &slot) {
   return &g_state[device];
 }
 
-int32_t prepare_all(ErrorSlot &slot) {
-  if (prepare_device(slot) != 0) return -1;
-  if (prepare_nvfp4_kernels(slot) != 0) return -1;
-  if (prepare_trellis_kernels(slot) != 0) return -1;
-  return prepare_moe_kernels(slot);
-}
-
-int32_t prepare_device(ErrorSlot &slot) {
-  std::lock_guard<std::mutex> lock(g_mutex);
-  DeviceState *state = device_state(slot);
-  if (state == nullptr) return -1;
-  // A repeated call re-reads the environment switches (tests and sweeps flip them between
-  // calls); everything else it computes is a function of the device alone.
-  int device = 0;
-  cudaGetDevice(&device);
-  cudaDeviceProp prop;
-  cudaError_t err = cudaGetDeviceProperties(&prop, device);
-  if (err != cudaSuccess) return fail(slot, "cudaGetDeviceProperties: %s", cudaGetErrorString(err));
-  if (prop.major != 10) {
-    return fail(slot, "this library is built for sm_100a only; device %d is sm_%d%d", device, prop.major, prop.minor);
+namespace {
+// The device's properties, once, and the switches of the environment, in every call (tests and sweeps flip them between
+// calls). What else is known of the device stays as it is.
+int32_t prepare_device(ErrorSlot &slot, DeviceState *state) {
+  DeviceState fresh = *state;
+  if (!state->counted) {
+    int device = 0;
+    cudaGetDevice(&device);
+    cudaDeviceProp prop;
+    const cudaError_t err = cudaGetDeviceProperties(&prop, device);
+    if (err != cudaSuccess) return fail(slot, "cudaGetDeviceProperties: %s", cudaGetErrorString(err));
+    if (prop.major != 10) {
+      return fail(slot, "this library is built for sm_100a only; device %d is sm_%d%d", device, prop.major, prop.minor);
+    }
+    fresh.sm_count = prop.multiProcessorCount;
   }
-  DeviceState fresh;
-  fresh.sm_count = prop.multiProcessorCount;
   fresh.pdl = env_int("B200Q_PDL", 1) != 0;
   fresh.gemv_rb = env_int("B200Q_GEMV_RM", 0);
   fresh.gemv_kc = env_int("B200Q_GEMV_KC", 0);
@@ -88,13 +81,27 @@ int32_t prepare_device(ErrorSlot &slot) {
   fresh.w4a4_pair = env_int("B200Q_W4A4_PAIR", -1);
   fresh.sm_cap = env_int("IGNIS_TRELLIS_SM_CAP", 0);
   if (fresh.sm_cap < 0 || fresh.sm_cap > fresh.sm_count) fresh.sm_cap = 0;
+  fresh.trellis_dw = env_int("B200Q_TRELLIS_TC_SHAPE", 8) == 16 ? 16 : 8;
+  fresh.moe_dw = env_int("B200Q_MOE_TC_WIDE", 0) == 1 ? 16 : 8;
   fresh.trellis_tc = env_int("B200Q_TRELLIS_TC", 1);
   fresh.moe_tc = env_int("B200Q_MOE_TC", 1);
   fresh.peer_barrier_polls = env_int("B200Q_PEER_BARRIER_POLLS", 1 << 22);
   if (fresh.peer_barrier_polls < 1) fresh.peer_barrier_polls = 1;
-  for (int i = 0; i < 9; ++i) fresh.gemv_slots[i] = state->gemv_slots[i];
-  fresh.prepared = true;
   *state = fresh;
+  return 0;
+}
+}  // namespace
+
+int32_t prepare_all(ErrorSlot &slot) {
+  std::lock_guard<std::mutex> lock(g_mutex);
+  DeviceState *state = device_state(slot);
+  if (state == nullptr) return -1;
+  if (prepare_device(slot, state) != 0) return -1;
+  if (prepare_nvfp4_kernels(slot) != 0) return -1;
+  if (prepare_trellis_kernels(slot) != 0) return -1;
+  if (prepare_moe_kernels(slot) != 0) return -1;
+  state->counted = true;
+  state->prepared = true;
   return 0;
 }
 

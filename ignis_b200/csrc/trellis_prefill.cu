@@ -177,14 +177,11 @@ uint64_t trellis_tc_workspace_bytes(uint32_t in, uint32_t weights, uint32_t toke
 // Which shape a dense product takes: the narrow one (8 decoder warps, two CTAs per SM), which
 // measured faster at 256, 1024 and 4096 tokens (a decoded tile serves 256 tokens in both, and the
 // narrow CTAs overlap each other's fill, drain and epilogue); B200Q_TRELLIS_TC_SHAPE = 16 selects
-// the wide one (read when the kernels are prepared).
-int g_dense_dw = 8;
-
+// the wide one (DeviceState::trellis_dw).
+namespace {
 // The CTAs of a cluster that share the K stages of an item (the narrow shape).
 constexpr uint32_t kMaxRanks = 8;
-uint32_t g_dense_clusters[kMaxRanks + 1] = {};   // clusters of so many CTAs that the device runs at once (0: none)
 
-namespace {
 cudaLaunchConfig_t dense_config(uint32_t items, uint32_t ranks, cudaStream_t stream, bool pdl, cudaLaunchAttribute (&attr)[2]) {
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(items * ranks);
@@ -218,7 +215,7 @@ uint32_t dense_ranks(const DeviceState &dev, uint32_t items, uint32_t stages, ui
   uint32_t best = 1u;
   float least = 0.0f;
   for (uint32_t ranks = 1; ranks <= kMaxRanks && (ranks == 1u || stages / ranks >= 8u); ++ranks) {
-    const uint32_t at_once = ranks == 1u ? 2u * static_cast<uint32_t>(dev.sm_count) : g_dense_clusters[ranks];
+    const uint32_t at_once = ranks == 1u ? 2u * static_cast<uint32_t>(dev.sm_count) : static_cast<uint32_t>(dev.trellis_clusters[ranks]);
     if (at_once == 0u) continue;
     const uint32_t waves = items / at_once, left = items % at_once;
     const float epilogue = static_cast<float>(row_tiles128) * (3.0f + 0.9f * static_cast<float>(ranks));
@@ -233,15 +230,15 @@ uint32_t dense_ranks(const DeviceState &dev, uint32_t items, uint32_t stages, ui
 }  // namespace
 
 int32_t trellis_tc_prepare(ErrorSlot &slot) {
-  const char *shape = getenv("B200Q_TRELLIS_TC_SHAPE");
-  g_dense_dw = shape != nullptr && atoi(shape) == 16 ? 16 : 8;
+  DeviceState *dev = device_state(slot);
+  if (dev == nullptr) return -1;
   cudaError_t err = cudaFuncSetAttribute(trellis_tc_dense_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Shape<16>::kSmemBytes));
   if (err == cudaSuccess) err = cudaFuncSetAttribute(trellis_tc_dense_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Shape<8>::kSmemBytes));
   if (err == cudaSuccess) {
     err = cudaFuncSetAttribute(trellis_rotate_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRotateMaxSmem));
   }
   if (err != cudaSuccess) return fail(slot, "trellis prefill kernel attributes: %s", cudaGetErrorString(err));
-  for (uint32_t ranks = 2; ranks <= kMaxRanks; ++ranks) {
+  for (uint32_t ranks = 2; ranks <= kMaxRanks && !dev->counted; ++ranks) {
     cudaLaunchAttribute attr[2];
     const cudaLaunchConfig_t config = dense_config(1u, ranks, nullptr, false, attr);
     int clusters = 0;
@@ -249,7 +246,7 @@ int32_t trellis_tc_prepare(ErrorSlot &slot) {
       (void)cudaGetLastError();
       clusters = 0;
     }
-    g_dense_clusters[ranks] = static_cast<uint32_t>(clusters);
+    dev->trellis_clusters[ranks] = clusters;
   }
   if (encode_tiled_fn() == nullptr) return fail(slot, "cuTensorMapEncodeTiled is not available from this driver");
   return 0;
@@ -285,7 +282,7 @@ int32_t one_product(ErrorSlot &slot, const DeviceState &dev, const ignis_trellis
   p.ldy = ldy;
   p.epilogue = epilogue;
   const uint32_t row_tiles = (tokens + 255u) / 256u;
-  if (g_dense_dw == 16) {
+  if (dev.trellis_dw == 16) {
     p.ranks = 1u;
     err = launch(trellis_tc_dense_kernel<16>, dim3((w->out + 255u) / 256u * row_tiles), dim3(Shape<16>::kThreads), Shape<16>::kSmemBytes, stream,
                  dev.pdl != 0, map_a, p);

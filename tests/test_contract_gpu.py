@@ -137,6 +137,23 @@ def test_moe_experts_are_reproducible_and_capturable(oracle):
         mo.set_geometry(2560, 640, 512, 10)
 
 
+def test_preparing_again_asks_nothing_of_the_device():
+    """A program prepares with every workspace or layer that it makes: what an occupancy query answers is a function of the
+    device alone and is asked once (the queries together took some 25 ms)."""
+    import time
+
+    from ignis_b200 import moe, nvfp4, trellis
+
+    for prepare in (nvfp4.prepare, trellis.prepare, moe.prepare):
+        prepare()
+        times = []
+        for _ in range(5):
+            start = time.perf_counter()
+            prepare()
+            times.append(time.perf_counter() - start)
+        assert min(times) < 5e-3
+
+
 def test_peer_barrier_gives_up_within_its_limit_and_reports_who_was_missing():
     """Failure detection without a fault: one GPU plays rank 0 of two, both ranks' flag arrays in
     its own memory, and nothing ever writes rank 1's flag. With the poll limit set to a few
