@@ -288,8 +288,17 @@ int32_t moe_fp8_tc_prepare(ErrorSlot &slot) {
   return 0;
 }
 
+// From 65 tokens: the row kernel (moe_rows.cu) reads and multiplies the weights once per 64 tokens, this one once in all up to 256,
+// but spends about 30 us on its two launches whatever the size. So the row kernel keeps the calls whose weights times token
+// groups are small, and none beyond 256 tokens. Both products from a cold L2, rows against this kernel in us (hidden x inter):
+// 4096 x 14336 at 72 tokens 282 / 191, at 256 609 / 200; 7168 x 2048 at 72 83 / 87, at 192 140 / 89; 2048 x 1408 at 192 44 / 42, at 256
+// 58 / 42; 2560 x 640 at 256 44, this kernel at 257 40; 2048 x 128 and 1024 x 512 at 256 25 and 17, at 257 32 and 26.
+constexpr uint32_t kFp8TcTokens = 256;
+constexpr uint64_t kFp8TcRowWork = 1ull << 23;
+
 bool moe_fp8_tc_takes(const DeviceState &dev, uint32_t hidden, uint32_t inter, uint32_t tokens, const void *x, const void *h) {
-  return dev.moe_tc != 0 && tokens > kFp8TcMinTokens && hidden % 128u == 0 && inter % 128u == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 &&
+  const uint64_t row_work = static_cast<uint64_t>(hidden) * inter * ((tokens + 63u) / 64u);
+  return dev.moe_tc != 0 && tokens > 64u && (tokens > kFp8TcTokens || row_work > kFp8TcRowWork) && hidden % 128u == 0 && inter % 128u == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 &&
          (reinterpret_cast<uintptr_t>(h) & 15u) == 0;
 }
 

@@ -54,7 +54,8 @@ int32_t moe_tc_experts(ErrorSlot &slot, const DeviceState &dev, const ExpertPara
 
 // The shared expert of a wide call on the tensor cores (moe_fp8_tc.cu): FP8 rows widened exactly to
 // BF16 in swizzled shared memory, BF16 activations by TMA, tcgen05 kind::f16. Takes calls of more
-// than 64 tokens whose widths are multiples of 128 and whose x and h are 16-byte aligned.
+// than 64 tokens, by the work they are (moe_fp8_tc.cu), whose widths are multiples of 128 and whose x and h are
+// 16-byte aligned.
 int32_t moe_fp8_tc_prepare(ErrorSlot &slot);
 bool moe_fp8_tc_takes(const DeviceState &dev, uint32_t hidden, uint32_t inter, uint32_t tokens, const void *x, const void *h);
 cudaError_t moe_fp8_tc_shared_expert(const DeviceState &dev, const uint8_t *gate, const uint8_t *up, const uint8_t *down, const uint16_t *x,
@@ -63,8 +64,6 @@ cudaError_t moe_fp8_tc_status(uint32_t *status, cudaStream_t stream);   // non-z
 
 // The narrow dense products of the block (moe_rows.cu): the router's logits and selection, and the
 // shared expert of calls the tensor-core kernels do not take.
-constexpr uint32_t kRouterTileMinTokens = 1536;
-constexpr uint32_t kFp8TcMinTokens = 256;
 int32_t moe_rows_prepare(ErrorSlot &slot);
 cudaError_t moe_router_logits_launch(const DeviceState &dev, const uint16_t *x, const uint16_t *w, uint32_t tokens, uint32_t hidden,
                                      uint32_t experts, float *logits, cudaStream_t stream);

@@ -377,12 +377,18 @@ int32_t moe_rows_prepare(ErrorSlot &slot) {
   return 0;
 }
 
+constexpr uint32_t kRouterRowCtas = 768;
+
 cudaError_t moe_router_logits_launch(const DeviceState &dev, const uint16_t *x, const uint16_t *w, uint32_t tokens, uint32_t hidden,
                                      uint32_t experts, float *logits, cudaStream_t stream) {
   const RowsParams p = {w, nullptr, x, logits, experts, hidden, tokens, 1u};
-  // The tile form re-reads its operands least, but has only experts / 128 x tokens / 128 CTAs: the row
-  // form grows with the tokens (25 us at 1000, 35 at 1500 of 512 x 2048), the tile form stays near 38.
-  if (tokens > kRouterTileMinTokens) {
+  // The tile form re-reads its operands least, but has only experts / 128 x tokens / 128 CTAs, each a walk down all of
+  // `hidden`: its time hardly depends on the call until they fill the device. The row form has 16 times as many, and its time
+  // grows with them. The line lies where they meet at 512 experts: five waves of the row form's CTAs, 1536 tokens there.
+  // Logits and selection from a cold L2, rows against tiles in us: 512 experts x 2048 at 1536 / 1537 tokens 60 / 52, 256 x 7168 at
+  // 2048 99 / 130, 128 x 2048 at 4096 42 / 48, 8 x 4096 at 2048 24 / 77.
+  const uint32_t row_ctas = (experts + kRowTile - 1u) / kRowTile * ((tokens + 63u) / 64u);
+  if (row_ctas > kRouterRowCtas) {
     return launch(moe_router_tile_kernel, dim3((experts + kTile - 1) / kTile, (tokens + kTile - 1) / kTile), dim3(kThreads), kTileSmem, stream,
                   dev.pdl != 0, p);
   }

@@ -459,6 +459,56 @@ def test_shared_expert_token_tiles(mo, tokens):
     assert torch.allclose(shared.double(), down, rtol=1e-4, atol=1e-5 * float(down.abs().max()))
 
 
+def fp8_weights(mo, shapes, gen):
+    payloads = [torch.from_numpy(mo.fp8_row_scale_payload(torch.randn(r, c, generator=gen) * 0.03)).cuda() for r, c in shapes]
+    wide = []
+    for p, (r, c) in zip(payloads, shapes):
+        pad = (r * c + 255) // 256 * 256
+        wide.append(p[: r * c].view(torch.float8_e4m3fn).double().reshape(r, c) * p[pad:].view(torch.bfloat16).double().unsqueeze(1))
+    return payloads, wide
+
+
+@pytest.mark.parametrize("tokens,inter", [(64, 4224), (65, 4224), (128, 1024), (192, 1408), (256, 1024), (256, 1152)])
+def test_shared_expert_on_both_sides_of_the_line_between_its_kernels(mo, tokens, inter):
+    """65 to 256 tokens take the row kernel or tcgen05 by the work they are: hidden x inter x groups of 64 tokens, at 2^23."""
+    mo.set_geometry(2048, inter, 8, 2)
+    gen = torch.Generator().manual_seed(tokens + inter)
+    payloads, wide = fp8_weights(mo, [(inter, 2048), (inter, 2048), (2048, inter)], gen)
+    x = (torch.randn(tokens, 2048, generator=gen) * 0.5).to(torch.bfloat16).cuda()
+    shared, h = mo.shared_expert(*payloads, x)
+    g, u = x.double() @ wide[0].T, x.double() @ wide[1].T
+    want = g / (1 + torch.exp(-g)) * u
+    assert torch.allclose(h.double(), want, rtol=2 ** -7, atol=1e-4 * float(want.abs().max()))
+    down = h.double() @ wide[2].T
+    assert torch.allclose(shared.double(), down, rtol=1e-4, atol=1e-5 * float(down.abs().max()))
+
+
+def test_wide_geometries_are_not_given_the_narrow_ones_kernels(mo):
+    """What a kernel costs goes with the geometry, not with the tokens alone: one token more must not make a call much cheaper
+    (a shared expert of 4096 x 14336 took 609 us at 256 tokens and 200 at 257) nor much dearer (a router of 8 experts 21 us
+    at 1536 and 79 at 1537)."""
+    geometry = mo.Geometry(4096, 14336, 8, 2)
+
+    def microseconds(call):
+        times = []
+        for _ in range(12):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            call()
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b) * 1e3)
+        return min(times[2:])
+
+    codes = torch.randint(0, 120, (14336 * 4096 + 2 * 14336,), dtype=torch.uint8, device="cuda")   # every byte a finite code
+    x = torch.randn(1537, 4096, device="cuda").to(torch.bfloat16)
+    shared = [microseconds(lambda: mo.shared_expert(codes, codes, codes, x[:t], geometry)) for t in (256, 257)]
+    assert shared[0] < 1.5 * shared[1], shared
+    w = torch.randn(8, 4096, device="cuda").to(torch.bfloat16)
+    router = [microseconds(lambda: mo.router(x[:t], w, geometry)) for t in (1536, 1537)]
+    assert router[1] < 2.0 * router[0], router
+
+
 @pytest.mark.parametrize("tokens", [5, 11, 17, 64, 130, 300])   # up to 256: warp-level MMAs, one to eight token tiles a CTA; above: tcgen05, ragged token tiles
 def test_shared_expert_and_combine(mo, tokens):
     mo.set_geometry(256, 128, 8, 2)
