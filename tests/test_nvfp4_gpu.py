@@ -771,11 +771,22 @@ def test_w4a4_tensor_core_route(nv, oracle, tokens, n, k):
         nv.linear(x.cuda(), w, policy=nv.ALLOW_A4)
 
 
+@pytest.fixture(params=["0", "1"], ids=["narrow", "pair"])
+def w4a4_kernel(nv, request, monkeypatch):
+    """Each of the two W4A4 kernels beyond 32 tokens (nvfp4_w4a4_narrow.cu, the pair GEMM), whichever the rule would choose."""
+    monkeypatch.setenv("B200Q_W4A4_PAIR", request.param)
+    nv.prepare()
+    yield request.param
+    monkeypatch.undo()
+    nv.prepare()
+
+
 @pytest.mark.parametrize("tokens,n,k", [(33, 128, 256), (47, 384, 1792), (112, 128, 4352), (128, 256, 768), (129, 640, 1024), (145, 128, 2304),
-                                        (257, 128, 512)])
-def test_w4a4_few_tokens(nv, oracle, tokens, n, k):
-    """Calls that leave the pair GEMM idle (nvfp4_w4a4_narrow.cu): token tiles of 48 to 128 with ragged ends, one row tile to
-    five, K slices of unequal length over a cluster, and residual ADD and the fused SwiGLU on top of them."""
+                                        (257, 128, 512), (33, 512, 1024), (77, 256, 4352), (145, 256, 2304), (300, 768, 1024)])
+def test_w4a4_few_tokens(nv, oracle, w4a4_kernel, tokens, n, k):
+    """33 to some hundreds of tokens on both kernels: token tiles of 48 to 128 with ragged ends, one row tile to six, K in one piece and in
+    slices of unequal length over a cluster (the narrow kernel's, from 2048), residual ADD, and the fused SwiGLU (gate and up
+    rows in one CTA) where n allows it."""
     rng = np.random.default_rng(3 * tokens + n + k)
     codes, scales, d_w = make_weight(rng, n, k)
     d_in = 448.0
@@ -798,43 +809,45 @@ def test_w4a4_few_tokens(nv, oracle, tokens, n, k):
     assert ws.status() == 0
 
 
-def test_w4a4_one_cta_forms_agree_with_the_pair_form(nv, oracle, tmp_path):
-    """The prefill GEMM form kept behind an environment switch (one CTA per tile, persistent) runs in
-    a child process - the switch is read once per process - on the same operands as this process's
-    CTA-pair form: K is walked in the same order, so the BF16 outputs agree bit for bit."""
-    import os
-    import subprocess
-    import sys
+@pytest.mark.parametrize("tokens,k,inter,n_out", [(33, 512, 256, 128), (77, 2304, 512, 384), (128, 4352, 256, 256), (145, 1024, 768, 128),
+                                                  (300, 2304, 2304, 256)])
+def test_w4a4_mlp_quantizes_as_its_parts_do(nv, w4a4_kernel, tokens, k, inter, n_out):
+    """The quantizing epilogue of the gate|up product on both kernels, with and without a K split (of either product): the MLP
+    equals linear(linear_swiglu(x)), whose operand the standalone quantizer writes, bit for bit, plain and with ADD."""
+    rng = np.random.default_rng(tokens + k)
+    gate_up = nv.Weight.from_planes(*make_weight(rng, 2 * inter, k), 448.0)
+    down = nv.Weight.from_planes(*make_weight(rng, n_out, inter), 96.0)
+    gen = torch.Generator().manual_seed(tokens)
+    x = torch.randn(tokens, k, generator=gen).to(torch.bfloat16).cuda()
+    residual = torch.randn(tokens, n_out, generator=gen).to(torch.bfloat16).cuda()
+    parts = nv.Workspace(max(nv.workspace_bytes(2 * inter, k, nv.ALLOW_A4, tokens), nv.workspace_bytes(n_out, inter, nv.ALLOW_A4, tokens)))
+    h = nv.linear_swiglu(x, gate_up, policy=nv.ALLOW_A4, workspace=parts)
+    ws = nv.Workspace(nv.mlp_workspace_bytes(2 * inter, k, nv.ALLOW_A4, tokens))
+    ws.buffer[256:].fill_(0xFF)   # rows past the tokens are not written: nothing of them may reach an output
+    assert torch.equal(nv.mlp(x, gate_up, down, ws, policy=nv.ALLOW_A4), nv.linear(h, down, policy=nv.ALLOW_A4, workspace=parts))
+    want = nv.linear(h, down, out=residual.clone(), policy=nv.ALLOW_A4, epilogue=nv.ADD, workspace=parts)
+    assert torch.equal(nv.mlp(x, gate_up, down, ws, out=residual.clone(), policy=nv.ALLOW_A4, epilogue=nv.ADD), want)
+    assert ws.status() == 0 and parts.status() == 0
 
-    script = (
-        "import sys, numpy as np, torch\n"
-        "sys.path.insert(0, sys.argv[1])\n"
-        "from ignis_b200 import nvfp4 as nv\n"
-        "nv.prepare()\n"
-        "d = np.load(sys.argv[2])\n"
-        "w = nv.Weight.from_planes(d['codes'], d['scales'], 448.0, 448.0)\n"
-        "x = torch.from_numpy(d['x']).view(torch.bfloat16).cuda()\n"
-        "ws = nv.Workspace(nv.workspace_bytes(w.n, w.k, nv.ALLOW_A4, x.shape[0]))\n"
-        "y = nv.linear(x, w, policy=nv.ALLOW_A4, workspace=ws)\n"
-        "assert ws.status() == 0\n"
-        "np.save(sys.argv[3], y.view(torch.int16).cpu().numpy())\n"
-    )
+
+def test_w4a4_kernels_agree_where_both_walk_k_in_one_piece(nv, oracle, monkeypatch):
+    """The narrow kernel without a K split and the pair GEMM add a product's K in the same order: the same BF16 outputs, bit for bit."""
     tokens, n, k = 300, 640, 1024
     rng = np.random.default_rng(5)
-    codes, scales, _ = make_weight(rng, n, k)
+    codes, scales, d_w = make_weight(rng, n, k)
     x = torch.randn(tokens, k, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16)
-    np.savez(tmp_path / "in.npz", codes=codes, scales=scales, x=x.view(torch.int16).numpy())
-    w = nv.Weight.from_planes(codes, scales, 448.0, 448.0)
+    w = nv.Weight.from_planes(codes, scales, d_w, 448.0)
     ws = nv.Workspace(nv.workspace_bytes(n, k, nv.ALLOW_A4, tokens))
-    here = nv.linear(x.cuda(), w, policy=nv.ALLOW_A4, workspace=ws).view(torch.int16).cpu().numpy()
-    check_bf16(torch.from_numpy(here).view(torch.bfloat16), w4a4_reference(oracle, codes, scales, n, k, 448.0, 448.0, x))
-    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-    for switches in ({"B200Q_W4A4_PAIR": "0"},):
-        out = tmp_path / ("out_" + "_".join(switches.values()) + ".npy")
-        subprocess.run([sys.executable, "-c", script, root, str(tmp_path / "in.npz"), str(out)], check=True,
-                       env={**os.environ, **switches}, timeout=600)
-        assert np.array_equal(np.load(out), here)
-
+    got = []
+    for kernel in ("0", "1"):
+        monkeypatch.setenv("B200Q_W4A4_PAIR", kernel)
+        nv.prepare()
+        got.append(nv.linear(x.cuda(), w, policy=nv.ALLOW_A4, workspace=ws))
+        assert ws.status() == 0
+    monkeypatch.undo()
+    nv.prepare()
+    assert torch.equal(got[0], got[1])
+    check_bf16(got[0], w4a4_reference(oracle, codes, scales, n, k, d_w, 448.0, x))
 
 
 def test_operand_quantized_in_token_ranges_equals_the_one_call_route(nv, oracle):
