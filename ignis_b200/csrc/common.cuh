@@ -116,13 +116,6 @@ __device__ __forceinline__ void ldg256_stream(const void *p, uint32_t (&r)[8], u
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                : "l"(p), "l"(policy));
 }
-// The same for a stream of which every reader takes one 32-byte sector at a time: the L2 fetches the
-// line's four sectors with the first of them.
-__device__ __forceinline__ void ldg256_stream_line(const void *p, uint32_t (&r)[8], uint64_t policy) {
-  asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.L2::128B.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8], %9;"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "l"(p), "l"(policy));
-}
 __device__ __forceinline__ uint4 ldg128_stream(const void *p, uint64_t policy) {
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.b32 {%0,%1,%2,%3}, [%4], %5;"

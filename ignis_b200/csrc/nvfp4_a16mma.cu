@@ -80,21 +80,6 @@ constexpr int kGroups = 4, kDecoders = 4 * kGroups;   // groups of four decoder 
 constexpr int kA16Threads = (kDecoders + 3) * 32;
 constexpr float kWeightScale = 128.0f;                // the A tiles hold weights times 2^-7
 
-// 16 accumulator columns of this thread's lane.
-__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&r)[16]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-                 "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-               : "r"(addr)
-               : "memory");
-}
-
-__device__ __forceinline__ void tma_load_2d_hint(uint32_t dst, const CUtensorMap *map, uint32_t bar, int32_t x, int32_t y, uint64_t policy) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
-      ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "l"(policy)
-      : "memory");
-}
 // One row's 64 weights of a stage, widened into its 128 bytes of the A tile (`tile`: the row's address,
 // `sw`: its low bits). Both operands of the MMA are BF16, so the weights leave as
 // BF16(code * scale * 2^-7): exact, at most 6 significant bits. A code's three magnitude bits on the
@@ -537,14 +522,7 @@ int32_t a16mma_launch(ErrorSlot &slot, const DeviceState &dev, const GemvWeight 
   EncodeTiledFn encode = encode_tiled_fn();
   A16Maps maps = {};
   for (uint32_t i = 0; i < count; ++i) {
-    const cuuint64_t dims[2] = {k / 2u, weights[i].n};
-    const cuuint64_t strides[1] = {k / 2u};
-    const cuuint32_t box[2] = {128u, 128u};
-    const cuuint32_t elem[2] = {1, 1};
-    if (encode == nullptr ||
-        encode(&maps.m[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t *>(weights[i].codes), dims, strides, box, elem,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
+    if (!make_code_map(&maps.m[i], weights[i].codes, weights[i].n, k / 2u, 128u)) {
       return fail(slot, "nvfp4 A16 tensor-core route: tensor map encoding failed");
     }
   }

@@ -461,19 +461,6 @@ __global__ void __launch_bounds__(256, 1) w4a4_gemm_pair_kernel(const __grid_con
 }
 
 // ---- host side --------------------------------------------------------------------------------
-// A [rows][k/2]-byte plane as a 2-D byte tensor with (128 bytes x box_rows) boxes, 128-byte swizzle.
-bool make_code_map(CUtensorMap *map, const void *codes, uint64_t rows, uint64_t row_bytes, uint32_t box_rows) {
-  EncodeTiledFn fn = encode_tiled_fn();
-  if (fn == nullptr) return false;
-  const cuuint64_t dims[2] = {row_bytes, rows};
-  const cuuint64_t strides[1] = {row_bytes};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(kBKBytes), box_rows};
-  const cuuint32_t elem[2] = {1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(codes), dims, strides, box, elem,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // A scale plane of 512-byte tiles as a 2-D tensor [tiles][128 words] with boxes of four tiles (one K stage).
 bool make_scale_map(CUtensorMap *map, const void *scales, uint64_t tiles) {
   EncodeTiledFn fn = encode_tiled_fn();

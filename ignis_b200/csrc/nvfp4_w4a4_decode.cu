@@ -66,13 +66,6 @@ struct A4Params {
   uint32_t epilogue;   // STORE / ADD / OUT_F32, or the fused SwiGLU
 };
 
-__device__ __forceinline__ void tma_load_2d_hint(uint32_t dst, const CUtensorMap *map, uint32_t bar, int32_t x, int32_t y,
-                                                 uint64_t policy) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
-      ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "l"(policy)
-      : "memory");
-}
 __device__ __forceinline__ void bulk_load_hint(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar, uint64_t policy) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
                ::"r"(dst), "l"(src), "r"(bytes), "r"(bar), "l"(policy)
@@ -501,7 +494,6 @@ int32_t w4a4_decode_launch(ErrorSlot &slot, const DeviceState &dev, const A4Item
   p.tmem_cols = cols <= 128u ? 128u : (cols <= 256u ? 256u : 512u);
   if (dev.a4_decode_kc > 0 && static_cast<uint32_t>(dev.a4_decode_kc) <= 8u && k_stages / dev.a4_decode_kc >= 1u) kc = dev.a4_decode_kc;
   p.kc = kc;
-  EncodeTiledFn encode = encode_tiled_fn();
   uint32_t ctas = 0;
   for (uint32_t i = 0; i < count; ++i) {
     A4Weight &g = p.w[i];
@@ -513,14 +505,7 @@ int32_t w4a4_decode_launch(ErrorSlot &slot, const DeviceState &dev, const A4Item
     g.d_in = items[i].d_in;
     g.block_begin = ctas;
     ctas += (two ? items[i].n / 2u : items[i].n) / 128u * kc;
-    const cuuint64_t dims[2] = {k / 2u, items[i].n};
-    const cuuint64_t strides[1] = {k / 2u};
-    const cuuint32_t box[2] = {128u, 128u};
-    const cuuint32_t elem[2] = {1, 1};
-    if (encode == nullptr ||
-        encode(&maps.m[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t *>(items[i].codes), dims, strides, box, elem,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
+    if (!make_code_map(&maps.m[i], items[i].codes, items[i].n, k / 2u, 128u)) {
       return fail(slot, "nvfp4 W4A4 decode route: tensor map encoding failed");
     }
   }

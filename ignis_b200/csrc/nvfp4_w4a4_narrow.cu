@@ -55,19 +55,6 @@ struct NarrowParams {
   float q_din;
 };
 
-__device__ __forceinline__ void tma_load_2d_hint(uint32_t dst, const CUtensorMap *map, uint32_t bar, int32_t x, int32_t y, uint64_t policy) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
-      ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "l"(policy)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&r)[16]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-                 "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-               : "r"(addr)
-               : "memory");
-}
 
 // Silu(g) u as the reference's formula rounds it: both products to BF16 first.
 __device__ __forceinline__ __nv_bfloat16 swiglu_bf16(float acc_g, float acc_u, float alpha) {
@@ -369,17 +356,6 @@ size_t narrow_epilogue_bytes(const NarrowPlan &pl, bool quant) {
   return (pl.kc > 1u ? static_cast<size_t>(pl.tiles) * pl.tile * 512u : 0u) + (quant ? static_cast<size_t>(pl.tile) * 272u : 0u);
 }
 
-bool narrow_code_map(CUtensorMap *map, const void *codes, uint64_t rows, uint64_t row_bytes, uint32_t box_rows) {
-  EncodeTiledFn fn = encode_tiled_fn();
-  if (fn == nullptr) return false;
-  const cuuint64_t dims[2] = {row_bytes, rows};
-  const cuuint64_t strides[1] = {row_bytes};
-  const cuuint32_t box[2] = {128u, box_rows};
-  const cuuint32_t elem[2] = {1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(codes), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 }  // namespace
 
 int32_t w4a4_narrow_prepare(ErrorSlot &slot) {
@@ -423,7 +399,7 @@ int32_t w4a4_narrow_launch(ErrorSlot &slot, const DeviceState &dev, const A4Item
   p.q_scales = q_scales;
   p.q_din = q_din;
   uint32_t ctas = 0;
-  bool encoded = narrow_code_map(&maps.x, x_codes, (static_cast<uint64_t>(tokens) + 127u) / 128u * 128u, k / 2u, pl.tile);
+  bool encoded = make_code_map(&maps.x, x_codes, (static_cast<uint64_t>(tokens) + 127u) / 128u * 128u, k / 2u, pl.tile);
   for (uint32_t i = 0; i < count; ++i) {
     NarrowWeight &g = p.w[i];
     g.scales = items[i].scales;
@@ -433,7 +409,7 @@ int32_t w4a4_narrow_launch(ErrorSlot &slot, const DeviceState &dev, const A4Item
     g.alpha = 1.0f / (items[i].d_in * items[i].d_w);
     g.block_begin = ctas;
     ctas += items[i].n / (swiglu ? 256u : 128u) * pl.kc;
-    encoded = encoded && narrow_code_map(&maps.w[i], items[i].codes, items[i].n, k / 2u, 128u);
+    encoded = encoded && make_code_map(&maps.w[i], items[i].codes, items[i].n, k / 2u, 128u);
   }
   if (!encoded) return fail(slot, "nvfp4 W4A4 narrow route: tensor map encoding failed");
   const size_t ring = narrow_smem(pl), need = narrow_epilogue_bytes(pl, quant) + 1024u;

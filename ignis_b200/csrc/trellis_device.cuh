@@ -93,24 +93,6 @@ __device__ __forceinline__ void hadamard128(float (&v)[4], int lane) {
   for (int i = 0; i < 4; ++i) v[i] *= 0.08838834764831845f;
 }
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n"
-               "barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float ld_cluster_f32(const float *local_smem, uint32_t rank) {
-  const uint32_t local = static_cast<uint32_t>(__cvta_generic_to_shared(local_smem));
-  uint32_t remote;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
-  return v;
-}
-
 }  // namespace trellis_dev
 }  // namespace b200q
 

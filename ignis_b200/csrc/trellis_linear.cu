@@ -25,6 +25,7 @@
 // stream.
 #include "../../include/ignis_trellis_linear.h"
 
+#include "nvfp4_tc.cuh"
 #include "trellis_device.cuh"
 #include "trellis_internal.cuh"
 
@@ -43,37 +44,11 @@ constexpr uint32_t kLinearProducer = 0x10u, kLinearDecoder = 0x20u;
 // CTAs of the linear kernel an SM holds at once, by (token tiles x weights).
 constexpr int linear_ctas_per_sm(int nt, int sides) { return nt * sides <= 2 ? 3 : (nt * sides <= 8 ? 2 : 1); }
 
-// ---- the word ring: mbarriers and bulk copies ----
-__device__ __forceinline__ uint32_t smem_address(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ void ring_init(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory"); }
-__device__ __forceinline__ void ring_expect(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void ring_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
-__device__ __forceinline__ bool ring_wait(uint32_t bar, uint32_t parity) {
-  for (uint32_t spin = 0; spin < (1u << 22); ++spin) {
-    uint32_t done;
-    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-__device__ __forceinline__ void ring_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
 __device__ __forceinline__ uint32_t lds32(uint32_t address) {
   uint32_t v;
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(address));
   return v;
 }
-// A position in a ring of `depth` slots: the slot and the parity of its current use.
-struct RingAt {
-  uint32_t slot = 0, phase = 0;
-  __device__ __forceinline__ void advance(uint32_t by, uint32_t depth) {
-    for (slot += by; slot >= depth; slot -= depth) phase ^= 1u;
-  }
-};
-
 // The power of two that brings the largest magnitude of a warp's 128 values (four a lane) into [2^13, 2^14): from the
 // maximum's exponent bits, held to what a float carries; 0 for zeros and for what is not finite.
 __device__ __forceinline__ int block_shift(const float (&v)[4]) {
@@ -170,7 +145,7 @@ __global__ void __launch_bounds__(kLinearThreads, linear_ctas_per_sm(NT, SIDES))
     trellis_linear_kernel(const __grid_constant__ TrellisParams p) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_rank(), kc = p.kc;
+  const uint32_t rank = cluster_ctarank(), kc = p.kc;
   // The target this CTA serves. A plain call (GROUP false) reads target[0] straight from the launch constants.
   TrellisTarget picked = {};
   if (GROUP) {
@@ -196,12 +171,12 @@ __global__ void __launch_bounds__(kLinearThreads, linear_ctas_per_sm(NT, SIDES))
   float4 *part = reinterpret_cast<float4 *>(smem_raw + ring_bytes + frag_bytes);           // [side][tile column 8][NT][lane 32]
   float *inv_s = reinterpret_cast<float *>(part + SIDES * 8 * NT * 32);
   float *scale_s = inv_s + SIDES * p.chunk * NT * 8;                                        // [side][block][token]
-  const uint32_t bars = smem_address(scale_s + SIDES * p.chunk * NT * 8), empties = bars + 8u * p.ring;
+  const uint32_t bars = smem_u32(scale_s + SIDES * p.chunk * NT * 8), empties = bars + 8u * p.ring;
 
   if (threadIdx.x == 0) {
     for (uint32_t d = 0; d < p.ring; ++d) {
-      ring_init(bars + 8u * d, 1);            // the producer's expect_tx arrival
-      ring_init(empties + 8u * d, kWarps);    // one arrival per decoding warp
+      mbar_init(bars + 8u * d, 1);            // the producer's expect_tx arrival
+      mbar_init(empties + 8u * d, kWarps);    // one arrival per decoding warp
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -217,13 +192,13 @@ __global__ void __launch_bounds__(kLinearThreads, linear_ctas_per_sm(NT, SIDES))
     const uint8_t *src = reinterpret_cast<const uint8_t *>(S.trellis) + static_cast<uint64_t>(col_block) * row_bytes + (static_cast<uint64_t>(b0) * 8u + row) * row_pitch;
     RingAt at;
     for (uint32_t blk = b0; blk < b1; ++blk, at.advance(1u, p.ring), src += 8u * row_pitch) {
-      if (!ring_wait(empties + 8u * at.slot, at.phase ^ 1u)) {
+      if (!mbar_wait(empties + 8u * at.slot, at.phase ^ 1u)) {
         if (lane == 0) atomicOr(&g_linear_status, kLinearProducer);
         break;
       }
-      if (lane == 0) ring_expect(bars + 8u * at.slot, 1024u * (side0.k2 + (SIDES == 2 ? p.up.k2 : 0u)));
+      if (lane == 0) mbar_expect_tx(bars + 8u * at.slot, 1024u * (side0.k2 + (SIDES == 2 ? p.up.k2 : 0u)));
       __syncwarp();
-      if (lane < 8 * SIDES) ring_load(smem_address(smem_raw) + at.slot * p.slot_bytes + side_at + row * row_bytes, src, row_bytes, bars + 8u * at.slot);
+      if (lane < 8 * SIDES) bulk_load(smem_u32(smem_raw) + at.slot * p.slot_bytes + side_at + row * row_bytes, src, row_bytes, bars + 8u * at.slot);
     }
   }
   griddep_wait();
@@ -248,7 +223,7 @@ __global__ void __launch_bounds__(kLinearThreads, linear_ctas_per_sm(NT, SIDES))
   for (int sd = 0; sd < SIDES; ++sd) {
     const uint32_t k2 = K2 != 0 ? static_cast<uint32_t>(K2) : (sd == 0 ? side0.k2 : p.up.k2);
     win[sd] = lane_window(k2, lane);
-    const uint32_t base = smem_address(smem_raw) + (sd == 1 ? 1024u * (K2 != 0 ? static_cast<uint32_t>(K2) : side0.k2) : 0u) + static_cast<uint32_t>(warp & 7) * 16u * k2;
+    const uint32_t base = smem_u32(smem_raw) + (sd == 1 ? 1024u * (K2 != 0 ? static_cast<uint32_t>(K2) : side0.k2) : 0u) + static_cast<uint32_t>(warp & 7) * 16u * k2;
     word_at[sd][0] = base + 4u * win[sd].w0;
     word_at[sd][1] = base + 4u * win[sd].w1;
     word_at[sd][2] = base + 4u * win[sd].w2;
@@ -314,7 +289,7 @@ __global__ void __launch_bounds__(kLinearThreads, linear_ctas_per_sm(NT, SIDES))
 
     // ---- this warp's tile column down the chunk ----
     for (uint32_t bl = 0; bl < nb; ++bl, at.advance(1u, p.ring)) {
-      if (ok && !ring_wait(bars + 8u * at.slot, at.phase)) {
+      if (ok && !mbar_wait(bars + 8u * at.slot, at.phase)) {
         if (lane == 0) atomicOr(&g_linear_status, kLinearDecoder);
         ok = false;
       }
@@ -361,7 +336,7 @@ __global__ void __launch_bounds__(kLinearThreads, linear_ctas_per_sm(NT, SIDES))
         }
       }
       __syncwarp();
-      if (lane == 0) ring_arrive(empties + 8u * at.slot);
+      if (lane == 0) mbar_arrive(empties + 8u * at.slot);
     }
   }
   // back to the activations' own units, and out to the cluster
@@ -375,7 +350,7 @@ __global__ void __launch_bounds__(kLinearThreads, linear_ctas_per_sm(NT, SIDES))
       tot[sd][tt][3] *= carry[sd][tt][1];
       if (warp < kWarps) part[((sd * 8 + warp) * NT + tt) * 32 + lane] = make_float4(tot[sd][tt][0], tot[sd][tt][1], tot[sd][tt][2], tot[sd][tt][3]);
     }
-  cluster_barrier();
+  cluster_sync_all();
 
   // ---- finish: tokens dealt over the cluster's CTAs and their warps; lane = 4 output columns ----
   for (uint32_t tok = rank + kc * static_cast<uint32_t>(warp); tok < p.tokens; tok += kc * (kWarps + 1)) {
@@ -418,7 +393,7 @@ __global__ void __launch_bounds__(kLinearThreads, linear_ctas_per_sm(NT, SIDES))
     packed.y = *reinterpret_cast<const uint32_t *>(&o23);
     *reinterpret_cast<uint2 *>(dst) = packed;
   }
-  cluster_barrier();  // peers keep their partial sums alive until every CTA has read them
+  cluster_sync_all();  // peers keep their partial sums alive until every CTA has read them
 }
 
 constexpr size_t kLinearMaxSmem = 200 * 1024;

@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(Shape<DW>::kThreads, DW == 16 ? 1 : 2) trellis
   // Token tiles run fastest over the grid, so the CTAs at work at one time decode the same columns
   // of the plane (read from HBM once, then from the L2).
   const uint32_t row_tiles = (p.tokens + 255u) / 256u;
-  const Split split_k = {p.ranks, p.ranks == 1u ? 0u : cluster_rank()};
+  const Split split_k = {p.ranks, p.ranks == 1u ? 0u : cluster_ctarank()};
   const uint32_t item = blockIdx.x / p.ranks, col_tile = item / row_tiles, row_tile = item % row_tiles;
   Job job;
   job.trellis = p.trellis;

@@ -344,7 +344,7 @@ constexpr Split kWhole = {1u, 0u};
 // The cluster meetings of one job's epilogue, for the threads that do not run it.
 __device__ __forceinline__ void split_meetings(const Split split, uint32_t row_tiles) {
   if (split.ranks == 1u) return;
-  for (uint32_t i = 0; i < 2u * row_tiles; ++i) cluster_barrier();
+  for (uint32_t i = 0; i < 2u * row_tiles; ++i) cluster_sync_all();
 }
 
 __device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t local, uint32_t rank) {
@@ -371,7 +371,7 @@ __device__ __forceinline__ void emit_rows(const float *area, uint32_t quad, uint
     for (uint32_t i = 0; i < pairs; ++i) emit(2u * i + up, 2u * i + up < rows, *reinterpret_cast<const float4 *>(base + 2u * i * kPitch));
     return;
   }
-  cluster_barrier();
+  cluster_sync_all();
   const uint32_t mine = smem_u32(base);
   for (uint32_t i0 = split.rank; i0 < pairs; i0 += 4u * split.ranks) {   // four pairs at a time: their loads travel together
     float4 sum[4];
@@ -394,7 +394,7 @@ __device__ __forceinline__ void emit_rows(const float *area, uint32_t quad, uint
       if (i < pairs) emit(2u * i + up, 2u * i + up < rows, sum[j]);
     }
   }
-  cluster_barrier();
+  cluster_sync_all();
 }
 
 __device__ __forceinline__ void load_half_row(uint32_t taddr, float inv, float (&v)[64]) {
