@@ -298,8 +298,8 @@ constexpr uint64_t kFp8TcRowWork = 1ull << 23;
 
 bool moe_fp8_tc_takes(const DeviceState &dev, uint32_t hidden, uint32_t inter, uint32_t tokens, const void *x, const void *h) {
   const uint64_t row_work = static_cast<uint64_t>(hidden) * inter * ((tokens + 63u) / 64u);
-  return dev.moe_tc != 0 && tokens > 64u && (tokens > kFp8TcTokens || row_work > kFp8TcRowWork) && hidden % 128u == 0 && inter % 128u == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 &&
-         (reinterpret_cast<uintptr_t>(h) & 15u) == 0;
+  if (dev.moe_tc == 0 || tokens <= 64u || (tokens <= kFp8TcTokens && row_work <= kFp8TcRowWork)) return false;
+  return hidden % 128u == 0 && inter % 128u == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(h) & 15u) == 0;
 }
 
 cudaError_t moe_fp8_tc_shared_expert(const DeviceState &dev, const uint8_t *gate, const uint8_t *up, const uint8_t *down, const uint16_t *x,

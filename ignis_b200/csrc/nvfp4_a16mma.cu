@@ -21,7 +21,7 @@
 //  * Warp 17 owns tensor memory and issues tcgen05.mma kind::f16 (A and B BF16, M 128, K 16, four per stage and
 //    tile), then commits the stage back to its writers. The issuing roles run in whole warps with an elected
 //    lane (nvfp4_tc.cuh, elect_one): with a branch on the lane the same kernel took 2.5 times as long.
-//    Measured on one 27B-style layer: 102 us at 17 tokens, 116 at 100, 424 at 600 (before: 156, 470, 1786).
+//    Measured on one 27B-style layer: 99 us at 17 tokens, 122 at 100, 458 at 600 (the kernel before: 156, 470, 1786).
 //  * K can be split over the CTAs of a cluster (narrow weights cannot fill the device otherwise):
 //    every CTA pulls its accumulators to shared memory, the cluster meets in distributed shared
 //    memory, and the tokens are dealt to the CTAs, which add the partial sums in rank order:

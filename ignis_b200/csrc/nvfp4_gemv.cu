@@ -729,7 +729,7 @@ GemvPlan gemv_plan(const DeviceState &dev, uint32_t groups, uint32_t ksteps, int
         // fitted on B200 (microseconds per launch): a warp's step costs about 1.6, a step of the
         // CTA's activation slice 0.3 per token tile, a wave of CTAs 3, the launch itself 2.4, and every
         // CTA of a cluster 0.35: clusters are placed inside one GPC, so the wider they are the more
-        // SMs stay empty and the later the last CTA starts (phase stamps of the four configs[1] calls)
+        // SMs stay empty and the later the last CTA starts (phase stamps of a 27B-style layer's four calls)
         const double cost = waves * (1.57 * steps + 0.3 * nt * slice + 3.0) + 2.4 + 0.35 * kc;
         if (cost < best_cost) {
           best_cost = cost;

@@ -92,7 +92,7 @@ int32_t w4a4_decode_launch(ErrorSlot &slot, const DeviceState &dev, const A4Item
                            uint32_t k, uint32_t tokens, uint32_t epilogue, cudaStream_t stream);
 int32_t w4a4_decode_status(ErrorSlot &slot, cudaStream_t stream, uint32_t *status);
 
-// W4A4 products of some dozens to some hundreds of tokens over activations quantized in the operand layout
+// W4A4 products of calls with few tokens over activations quantized in the operand layout
 // (nvfp4_w4a4_narrow.cu); several weights may share one launch.
 int32_t w4a4_narrow_prepare(ErrorSlot &slot);
 // What a product over `row_tiles` tiles of 128 output rows is expected to cost there, in SM cycles.

@@ -78,9 +78,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) { return static_cast
 
 // The warp's index as a value the compiler knows to be the same in all lanes, and one elected lane. A role
 // that issues tensor-core, TMA or commit instructions runs its loop in the whole warp and elects a lane
-// around them: their operands then live in uniform registers. Inside a branch on the lane index
-// the compiler wraps every such instruction in a loop over the distinct operand values (about 20
-// dependent instructions, 145 cycles an MMA where the tensor core needs 16 to 128).
+// around them. Issued from inside a branch on the lane index an MMA took about 145 cycles, where the tensor core
+// needs 16 to 128.
 __device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xFFFFFFFFu, static_cast<int>(threadIdx.x >> 5), 0); }
 __device__ __forceinline__ bool elect_one() {
   uint32_t is;

@@ -43,7 +43,7 @@ constexpr uint32_t kStatusProducerTimeout = 1u, kStatusMmaTimeout = 2u, kStatusE
 // 16 bytes of codes and two of the four scale bytes that lie side by side in a scale tile out. The
 // kernel is bound by instruction issue as much as by memory (about 13 instructions per value), so a
 // thread is kept small: 48 registers, five CTAs an SM, their load and arithmetic phases interleaved
-// (four blocks a thread at 65 registers and three CTAs: 2.6 % slower on the configs[2] step).
+// (four blocks a thread at 65 registers and three CTAs: 2.6 % slower on a step of 8192 tokens, 5120 -> 17408 -> 5120).
 // Rows at and beyond `tokens` get zero codes and zero scales.
 __global__ void __launch_bounds__(256, 5) quantize_swizzled_kernel(const uint16_t *x, uint32_t tokens, uint32_t tokens_pad,
                                                                    uint32_t k, float d_in, uint8_t *codes, uint8_t *scales) {
@@ -326,8 +326,7 @@ __global__ void __launch_bounds__(256, 1) w4a4_gemm_pair_kernel(const __grid_con
   griddep_launch_dependents();
   griddep_wait();  // the quantized activations come from the previous kernel in the stream
 
-  // The issuing roles run in whole warps with an elected lane (elect_one, nvfp4_tc.cuh): 12 copies, 4 MMAs and 2 commits
-  // a stage were each a loop over operand values inside a branch on the lane.
+  // The issuing roles run in whole warps with an elected lane (elect_one, nvfp4_tc.cuh).
   if (warp == 4) {
     // ---- producer (both CTAs): own tokens, own half of the weight rows, the scales of both halves ----
     RingAt at;
@@ -500,10 +499,21 @@ struct QuantTarget {
   float d_in = 1.0f;
 };
 
-// Which kernel a product takes: the cheaper by what each is expected to cost, in SM cycles. The pair kernel: waves of
-// 256 x 256 tiles on half as many pairs as SMs, 820 cycles a stage of 256 (its loads) and 3000 a tile, never faster than
-// the weights come from HBM; `w4a4_narrow_cycles` beside its kernel. Measured (27B-style shapes): gate|up at 77 tokens
-// 22 us narrow, 28 pair; at 512 67 against 50; down at 200 tokens 24 against 33.
+// Which kernel a product takes: the cheaper by a model of each, in SM cycles. The pair kernel: waves of
+// 256 x 256 tiles on half as many pairs as SMs, 820 cycles a stage of 256 and 3000 a tile, never faster than
+// the weights come from HBM; `w4a4_narrow_cycles` beside its kernel. Both forced, the products of a 27B-style layer with
+// their quantizer, in us, narrow / pair:
+//   tokens     q|k|v         o            gate|up       down
+//      33    9.9 / 14.0    8.3 / 15.2   19.5 / 36.7   13.5 / 31.2
+//     128   15.1 / 15.7   12.1 / 18.8   26.2 / 39.6   17.5 / 36.1
+//     200   13.1 / 16.9   13.7 / 19.4   42.9 / 39.8   24.2 / 36.5
+//     300   22.3 / 18.6   14.0 / 20.9   61.2 / 61.4   26.5 / 36.8
+//     384   24.1 / 18.8   14.6 / 21.3   63.2 / 62.0   27.5 / 38.4
+//     512   25.0 / 19.1   25.8 / 21.6   82.2 / 62.4   48.8 / 39.8
+// Up to 128 tokens the models take the narrow kernel for all four, beyond them the pair kernel. That is the faster one up to 128
+// and from 512; between them it is for gate|up and, from 300, q|k|v, but not for o and down (up to 1.5 times the
+// narrow kernel's time): the narrow model charges every CTA the share of the L2 that an SM has when all of them pull, also
+// where a launch has 80 CTAs.
 bool narrow_is_cheaper(const DeviceState &dev, const A4Item *items, uint32_t count, uint32_t k, uint32_t tokens, bool swiglu) {
   if (dev.w4a4_pair >= 0) return dev.w4a4_pair == 0;
   uint32_t row_tiles = 0, n_tiles = 0;

@@ -20,9 +20,9 @@
 // one tile per 16 inputs, decoded once and multiplied with every token tile of 8, fp32
 // accumulation, folded by the block's inverse scale every 128 inputs. The CTAs of a cluster (the
 // split of the inputs) meet in distributed shared memory in a fixed order; each applies the
-// output Hadamard, svh and the epilogue to its share of the tokens. Weight words are requested
-// one 128-input block ahead, the first block before the grid waits for its predecessor in the
-// stream.
+// output Hadamard, svh and the epilogue to its share of the tokens. A warp of its own brings the weight
+// words through a ring in shared memory, up to four 128-input blocks ahead, the first of them before the
+// grid waits for its predecessor in the stream.
 #include "../../include/ignis_trellis_linear.h"
 
 #include "nvfp4_tc.cuh"
@@ -41,7 +41,8 @@ constexpr int kLinearThreads = 288;   // the linear: eight decoding warps and th
 __device__ uint32_t g_linear_status = 0;   // bounded waits of the linear's word ring that ran out
 constexpr uint32_t kLinearProducer = 0x10u, kLinearDecoder = 0x20u;
 
-// CTAs of the linear kernel an SM holds at once, by (token tiles x weights).
+// CTAs of the linear kernel an SM holds at once, by (token tiles x weights). (plan_kc counts waves with it: it enters the split
+// of the inputs, and with that the order of a product's sums.)
 constexpr int linear_ctas_per_sm(int nt, int sides) { return nt * sides <= 2 ? 3 : (nt * sides <= 8 ? 2 : 1); }
 
 __device__ __forceinline__ uint32_t lds32(uint32_t address) {

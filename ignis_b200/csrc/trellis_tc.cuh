@@ -27,8 +27,7 @@
 //    the row's inverse scale and six Hadamard stages in registers and parks the 64 values in the
 //    (by then idle) stage ring, where the seventh stage combines the two halves; the results are
 //    parked once more and written out row-wise - half a warp per row, four columns a lane - with svh
-//    and the caller's epilogue. All of it moves 16 bytes per lane and access (4 bytes: 1155 us against
-//    1090 for a 27B-style layer of 1000 tokens, 1357 against 1295 for the MoE block of 4096).
+//    and the caller's epilogue. All of it moves 16 bytes per lane and access.
 //  * Every mbarrier wait is bounded; a wait that runs out sets a bit of a status word and the CTA
 //    falls through to the common exit and frees its tensor memory.
 #ifndef B200Q_TRELLIS_TC_CUH

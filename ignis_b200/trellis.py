@@ -148,7 +148,7 @@ def linear(w: Weight, x: torch.Tensor, out: torch.Tensor | None = None, epilogue
 def linear_group(weights: list[Weight], x: torch.Tensor, outs: list[torch.Tensor] | None = None,
                  epilogue: int = STORE) -> list[torch.Tensor]:
     """Up to four weights of the same `in` over one x in one launch (``b200q_trellis_linear_group``;
-    not in the reference's ABI): the bits of separate ``linear`` calls."""
+    not in the reference's ABI): separate ``linear`` calls, up to the order of the sums."""
     if not weights:
         raise TrellisError("linear_group needs at least one weight")
     _check_x(x, weights[0].in_)

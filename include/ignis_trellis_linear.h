@@ -97,8 +97,10 @@ int32_t ignis_trellis_linear_swiglu(const ignis_trellis_weight *gate, const igni
 
 /* Not in the reference's ABI: up to 4 weights of the same `in` applied to the same x in one launch,
  * weight i writing y[i][t][..ldy[i]] (q | k | v and the like: a narrow weight alone cannot fill
- * the device, and every launch has a fixed cost). Same arithmetic and bits as `count` separate
- * ignis_trellis_linear calls; STORE or ADD. Needs no workspace. */
+ * the device, and every launch has a fixed cost). Same arithmetic as `count` separate ignis_trellis_linear
+ * calls; how many CTAs share the inputs, and with it the order of the sums, goes by the widths of all
+ * weights together (q | k | v of a 27B-style layer: a value in a thousand lands on the next BF16). STORE
+ * or ADD. Needs no workspace. */
 int32_t b200q_trellis_linear_group(const ignis_trellis_weight *const *w, uint32_t count, const void *x,
                                    uint32_t tokens, void *const *y, const uint32_t *ldy, uint32_t epilogue,
                                    void *stream);

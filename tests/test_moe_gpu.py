@@ -126,7 +126,7 @@ def test_reference_geometry_decode_and_prefill_agree(mo, oracle):
 
 
 def zipf_routing(tokens, experts, top_k, seed):
-    """configs[4]'s routing: Zipf(1.1) popularity over a seeded permutation of the expert ids, top_k
+    """The benchmark's routing: Zipf(1.1) popularity over a seeded permutation of the expert ids, top_k
     distinct experts per token drawn in proportion to it, weights = BF16(softmax of normal logits)."""
     cpu = torch.Generator().manual_seed(seed)
     perm = torch.randperm(experts, generator=cpu)
@@ -137,9 +137,9 @@ def zipf_routing(tokens, experts, top_k, seed):
     return ids.numpy(), w.numpy()
 
 
-@pytest.mark.parametrize("k2s", [(5, 5, 5, 5), (4, 5, 6, 8)])   # configs[4]'s 2.5 bits per weight; the reference's mix of widths
+@pytest.mark.parametrize("k2s", [(5, 5, 5, 5), (4, 5, 6, 8)])   # 2.5 bits per weight; the reference's mix of widths
 def test_config4_geometry_under_zipf_routing(mo, oracle, k2s):
-    """The benchmark's configs[4]'s geometry - 512 experts of 2048 -> 768 -> 2048, top-10, Zipf(1.1) - at
+    """The benchmark's geometry - 512 experts of 2048 -> 768 -> 2048, top-10, Zipf(1.1) - at
     1024 tokens through the prefill entry, the routed sum held to the fp64 reference on a sample of
     tokens chosen for the shapes of work the skew produces (kernel/tests/test_moe_experts.cu:75-91):
     the token of one singleton expert, 24 tokens of an expert that fills one 64-row item and part of

@@ -27,7 +27,7 @@ def nv():
 
 
 def make_weight(rng, n, k, d_w=448.0):
-    """configs[0]'s distribution: uniform codes, scales = E4M3(|N(0,1)| + 0.1)."""
+    """The benchmark's distribution: uniform codes, scales = E4M3(|N(0,1)| + 0.1)."""
     codes = rng.integers(0, 256, (n, k // 2)).astype(np.uint8)
     natural = torch.from_numpy((np.abs(rng.standard_normal((n, k // 16))) + 0.1).astype(np.float32))
     natural = natural.to(torch.float8_e4m3fn).view(torch.uint8).numpy()
@@ -171,7 +171,7 @@ def test_a16_tensor_core_route(nv, oracle, tokens, n, k):
 
 
 def test_config0_full_size(nv, oracle):
-    """The benchmark's configs[0]: M = 1, K = 5120, N = 17408, tensor scale 1/448."""
+    """One MLP up-projection at one token: M = 1, K = 5120, N = 17408, tensor scale 1/448."""
     n, k = 17408, 5120
     rng = np.random.default_rng(20261125)
     codes, scales, d_w = make_weight(rng, n, k)
@@ -183,7 +183,7 @@ def test_config0_full_size(nv, oracle):
 
 
 def test_config2_full_size_sampled(nv, oracle):
-    """The benchmark's configs[2] at its full size (M = 8192, up 5120 -> 17408, W4A4): the whole product on
+    """The benchmark's prefill at its full size (M = 8192, up 5120 -> 17408, W4A4): the whole product on
     the device, checked against the host arithmetic on sampled row tiles x tokens (first, last and
     interior tiles of both dimensions), and through a size-independent property - a product over
     the same weights with the tokens reversed is the reversed product, bit for bit."""
@@ -209,7 +209,7 @@ def test_config2_full_size_sampled(nv, oracle):
 
 
 def test_config2_down_full_size_sampled(nv, oracle):
-    """The benchmark's configs[2]'s second product at its full size (M = 8192, down 17408 -> 5120, W4A4):
+    """The benchmark's second prefill product at its full size (M = 8192, down 17408 -> 5120, W4A4):
     sampled row tiles x tokens against the host arithmetic (first, last and interior tiles of both
     dimensions; K = 17408 is 68 stages of the ring), and the token-reversal property."""
     tokens, n, k = 8192, 5120, 17408
@@ -235,7 +235,7 @@ def test_config2_down_full_size_sampled(nv, oracle):
 
 @pytest.mark.parametrize("name,n,k", [("down", 5120, 17408), ("gate_up", 34816, 5120), ("qkv", 8192, 5120)])
 def test_config1_products_full_size_under_a16(nv, oracle, name, n, k):
-    """configs[1]'s widest and longest products at 8 tokens under the A16 policy (the headline
+    """A 27B-style layer's widest and longest products at 8 tokens under the A16 policy (the headline
     benchmark's kernel and launch plans at their real sizes): down 17408 -> 5120, the fused gate|up
     parent 5120 -> 34816 and q|k|v as one parent, sampled row tiles against the fp64 product of the
     exactly decoded weights, float32 and BF16 outputs; plus the token-order property."""
@@ -267,7 +267,7 @@ def test_config1_products_full_size_under_a16(nv, oracle, name, n, k):
 
 @pytest.mark.parametrize("world", [4, 8])
 def test_config1_row_shards_of_four_and_eight_ranks(nv, oracle, world):
-    """The launches one rank of `world` makes for configs[1] at 8 tokens - the q | k | v shards as one
+    """The launches one rank of `world` makes for a 27B-style layer at 8 tokens - the q | k | v shards as one
     group, o, the gate | up shards as one group, down - at the first and
     the last rank's rows: every output column against the fp64 product of the exactly decoded
     rows it stands for."""
@@ -682,7 +682,7 @@ def test_w4a4_decode_route(nv, oracle, tokens, n, k):
 
 
 def test_config1_gate_up_full_size_under_allow_a4(nv, oracle):
-    """configs[1]'s widest product (gate|up, 34816 x 5120, 8 tokens) under ALLOW_A4 at full size: sampled
+    """A 27B-style layer's widest product (gate|up, 34816 x 5120, 8 tokens) under ALLOW_A4 at full size: sampled
     row tiles against the host arithmetic, and the token-order property (the same tokens in reverse
     give the reversed outputs, bit for bit: every token is quantized and multiplied on its own)."""
     tokens, n, k = 8, 34816, 5120
