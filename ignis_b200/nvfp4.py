@@ -119,22 +119,24 @@ class Weight:
         return _lib.Nvfp4Weight(self.codes.data_ptr(), self.scales.data_ptr(), self.n, self.k,
                                 self.weight_scale_divisor, self.input_scale_divisor)
 
+    _struct = (None, None, None)   # where the planes lay when the C struct was built, and the struct
+
     def __setattr__(self, name, value) -> None:
         object.__setattr__(self, name, value)
-        self.__dict__.pop("_ref", None)   # a field was replaced: the struct is built anew
+        self.__dict__.pop("_struct", None)   # a field was replaced: the struct is built anew
 
     def __getstate__(self) -> dict:
         """The fields, without what calls keep beside them: C objects hold addresses and cannot be copied or pickled."""
-        return {name: value for name, value in self.__dict__.items() if name not in ("_ref", "_ranges")}
+        return {name: value for name, value in self.__dict__.items() if name not in ("_struct", "_ranges")}
 
-    def ref(self):
-        """``byref`` of the C struct. Kept between calls (a decode call enqueues one kernel, and building the struct took a
-        fifth of it) while both planes lie where it says: a plane may be re-seated in place, its field never assigned."""
-        at = (self.codes.data_ptr(), self.scales.data_ptr())
-        kept = self.__dict__.get("_ref")
-        if kept is None or kept[0] != at:
-            kept = self.__dict__["_ref"] = (at, C.byref(self.c_struct()))
-        return kept[1]
+    def struct(self) -> _lib.Nvfp4Weight:
+        """The C struct. Kept between calls (a decode call enqueues one kernel, and building the struct took a fifth of it)
+        while both planes lie where it says: a plane may be re-seated in place, its field never assigned."""
+        codes, scales, struct = self._struct
+        if codes != self.codes.data_ptr() or scales != self.scales.data_ptr():
+            struct = self.c_struct()
+            self.__dict__["_struct"] = (struct.codes, struct.scales, struct)
+        return struct
 
     @property
     def payload_bytes(self) -> int:
@@ -194,8 +196,8 @@ def linear(x: torch.Tensor, w: Weight, out: torch.Tensor | None = None, policy: 
     _check_x(x, w.k)
     tokens = x.size(0)
     y = _out(tokens, w.n, epilogue, out, x)
-    _check(_lib.load().b200q_nvfp4_linear(w.ref(), x.data_ptr(), tokens, y.data_ptr(), y.stride(0), epilogue, policy,
-                                           C.byref(workspace.c) if workspace is not None else None, _stream()))
+    _check(_lib.load().b200q_nvfp4_linear(w.struct(), x.data_ptr(), tokens, y.data_ptr(), y.stride(0), epilogue, policy,
+                                           workspace.c if workspace is not None else None, _stream()))
     return y
 
 
@@ -208,7 +210,7 @@ def linear_noalloc(x: torch.Tensor, w: Weight, out: torch.Tensor, epilogue: int 
     _check_x(x, w.k)
     tokens = x.shape[0]
     y = _out(tokens, w.n, epilogue, out, x)
-    _check(_lib.load().b200q_nvfp4_linear_noalloc(w.ref(), x.data_ptr(), tokens, y.data_ptr(), y.stride(0), epilogue,
+    _check(_lib.load().b200q_nvfp4_linear_noalloc(w.struct(), x.data_ptr(), tokens, y.data_ptr(), y.stride(0), epilogue,
                                                    _stream()))
     return y
 
@@ -254,8 +256,8 @@ def linear_split(x: torch.Tensor, parent: Weight, row_counts: list[int], outs: l
     ys = [_out(tokens, r, epilogue, None if outs is None else outs[i], x) for i, r in enumerate(row_counts)]
     yp = ptrs(*[y.data_ptr() for y in ys])
     ld = u32s(*[y.stride(0) for y in ys])
-    _check(_lib.load().b200q_nvfp4_linear_split(parent.ref(), count, rb, rc, x.data_ptr(), tokens, yp, ld, epilogue, policy,
-                                                 C.byref(workspace.c) if workspace is not None else None, _stream()))
+    _check(_lib.load().b200q_nvfp4_linear_split(parent.struct(), count, rb, rc, x.data_ptr(), tokens, yp, ld, epilogue, policy,
+                                                 workspace.c if workspace is not None else None, _stream()))
     return ys
 
 
@@ -303,8 +305,8 @@ def linear_swiglu(x: torch.Tensor, gate_up: Weight, out: torch.Tensor | None = N
     _check_x(x, gate_up.k)
     tokens = x.shape[0]
     h = _out(tokens, gate_up.n // 2, STORE, out, x)
-    _check(_lib.load().b200q_nvfp4_linear_swiglu(gate_up.ref(), x.data_ptr(), tokens, h.data_ptr(), h.stride(0), policy,
-                                                  C.byref(workspace.c) if workspace is not None else None, _stream()))
+    _check(_lib.load().b200q_nvfp4_linear_swiglu(gate_up.struct(), x.data_ptr(), tokens, h.data_ptr(), h.stride(0), policy,
+                                                  workspace.c if workspace is not None else None, _stream()))
     return h
 
 
@@ -320,15 +322,15 @@ def mlp(x: torch.Tensor, gate_up: Weight, down: Weight, workspace: Workspace, ou
     _check_x(x, gate_up.k)
     tokens = x.shape[0]
     y = _out(tokens, down.n, epilogue, out, x)
-    _check(_lib.load().b200q_nvfp4_mlp(gate_up.ref(), down.ref(), x.data_ptr(), tokens, y.data_ptr(), y.stride(0), epilogue, policy,
-                                        C.byref(workspace.c), _stream()))
+    _check(_lib.load().b200q_nvfp4_mlp(gate_up.struct(), down.struct(), x.data_ptr(), tokens, y.data_ptr(), y.stride(0), epilogue, policy,
+                                        workspace.c, _stream()))
     return y
 
 
 def dequantize(w: Weight) -> torch.Tensor:
     """The logical weight as float32 ``[n, k]`` (the bit-exact dequant seam)."""
     out = torch.empty((w.n, w.k), dtype=torch.float32, device=w.codes.device)
-    _check(_lib.load().b200q_nvfp4_dequantize(w.ref(), out.data_ptr(), _stream()))
+    _check(_lib.load().b200q_nvfp4_dequantize(w.struct(), out.data_ptr(), _stream()))
     return out
 
 
@@ -350,7 +352,7 @@ def quantize_operand(x_rows: torch.Tensor, tokens_total: int, token_begin: int, 
     ``token_begin ..`` of a call of `tokens_total`) into their place of the W4A4 operand in `workspace`."""
     _check_x(x_rows, k)
     _check(_lib.load().b200q_nvfp4_quantize_operand(x_rows.data_ptr(), tokens_total, token_begin, x_rows.shape[0], k,
-                                                     float(input_scale_divisor), C.byref(workspace.c), _stream()))
+                                                     float(input_scale_divisor), workspace.c, _stream()))
 
 
 def operand_ranges(k: int, tokens_total: int, token_begin: int, token_count: int) -> tuple[tuple[int, int], tuple[int, int]]:
@@ -368,8 +370,8 @@ def linear_prequantized(w: Weight, tokens: int, workspace: Workspace, out: torch
                         epilogue: int = STORE) -> torch.Tensor:
     """``b200q_nvfp4_linear_prequantized``: the tensor-core product over the operand in `workspace`."""
     y = _out(tokens, w.n, epilogue, out, w.codes)
-    _check(_lib.load().b200q_nvfp4_linear_prequantized(w.ref(), tokens, y.data_ptr(), y.stride(0), epilogue,
-                                                        C.byref(workspace.c), _stream()))
+    _check(_lib.load().b200q_nvfp4_linear_prequantized(w.struct(), tokens, y.data_ptr(), y.stride(0), epilogue,
+                                                        workspace.c, _stream()))
     return y
 
 

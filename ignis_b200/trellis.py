@@ -84,6 +84,8 @@ class Weight:
         return _lib.TrellisWeight(self.trellis.data_ptr(), self.suh.data_ptr(), self.svh.data_ptr(), self.k2, self.in_,
                                   self.out, self.tile_stride)
 
+    _struct = (None, None, None, None)   # where the planes lay when the C struct was built, and the struct
+
     def __setattr__(self, name, value) -> None:
         object.__setattr__(self, name, value)
         self.__dict__.pop("_struct", None)   # a field was replaced: the struct is built anew
@@ -95,11 +97,11 @@ class Weight:
     def struct(self) -> _lib.TrellisWeight:
         """The C struct, kept between calls while the three planes lie where it says (a plane may be re-seated in place, its
         field never assigned)."""
-        at = (self.trellis.data_ptr(), self.suh.data_ptr(), self.svh.data_ptr())
-        kept = self.__dict__.get("_struct")
-        if kept is None or kept[0] != at:
-            kept = self.__dict__["_struct"] = (at, self.c_struct())
-        return kept[1]
+        trellis, suh, svh, struct = self._struct
+        if trellis != self.trellis.data_ptr() or suh != self.suh.data_ptr() or svh != self.svh.data_ptr():
+            struct = self.c_struct()
+            self.__dict__["_struct"] = (struct.trellis, struct.suh, struct.svh, struct)
+        return struct
 
 
 def prepare() -> None:
@@ -140,8 +142,8 @@ def linear(w: Weight, x: torch.Tensor, out: torch.Tensor | None = None, epilogue
         if epilogue == ADD:
             raise TrellisError("the ADD epilogue accumulates into `out`, which must be given")
         out = x.new_empty((tokens, w.out))
-    _check(_lib.load().ignis_trellis_linear(C.byref(w.struct()), x.data_ptr(), tokens, out.data_ptr(), out.stride(0), epilogue,
-                                             C.byref(workspace.c) if workspace else None, _stream()))
+    _check(_lib.load().ignis_trellis_linear(w.struct(), x.data_ptr(), tokens, out.data_ptr(), out.stride(0), epilogue,
+                                             workspace.c if workspace else None, _stream()))
     return out
 
 
@@ -172,8 +174,8 @@ def linear_swiglu(gate: Weight, up: Weight, x: torch.Tensor, out: torch.Tensor |
     tokens = x.shape[0]
     if out is None:
         out = x.new_empty((tokens, gate.out))
-    _check(_lib.load().ignis_trellis_linear_swiglu(C.byref(gate.struct()), C.byref(up.struct()), x.data_ptr(), tokens, out.data_ptr(),
-                                                    out.stride(0), C.byref(workspace.c) if workspace else None,
+    _check(_lib.load().ignis_trellis_linear_swiglu(gate.struct(), up.struct(), x.data_ptr(), tokens, out.data_ptr(),
+                                                    out.stride(0), workspace.c if workspace else None,
                                                     _stream()))
     return out
 

@@ -71,10 +71,10 @@ def addresses_in_a_call(lib, w) -> list[int]:
     """The plane addresses in the struct that the library is handed."""
     if isinstance(w, nvfp4.Weight):
         nvfp4.linear_split(activations(w), w, [w.n])
-        s = lib.args[0]._obj
+        s = lib.args[0]
         return [s.codes, s.scales]
     trellis.linear(w, activations(w))
-    s = lib.args[0]._obj
+    s = lib.args[0]
     return [s.trellis, s.suh, s.svh]
 
 
@@ -124,7 +124,7 @@ def test_a_call_takes_the_workspace_struct_that_is_there_now(lib, make, module, 
     for base in (ws.c.base, ws.c.base + 256):   # another struct put in its place: a part of a larger region
         ws.c = _lib.Workspace(base, 256)
         module.linear(*((x, w) if module is nvfp4 else (w, x)), workspace=ws)
-        seen = next(a._obj for a in lib.args if isinstance(getattr(a, "_obj", None), _lib.Workspace))
+        seen = next(a for a in lib.args if isinstance(a, _lib.Workspace))
         assert seen.base == base and seen.bytes == 256
 
 
