@@ -205,6 +205,26 @@ __device__ __forceinline__ float ld_cluster_f32(const float *local_smem, uint32_
   return v;
 }
 
+// The address of this CTA's shared-memory address `local` in CTA `rank` of the cluster, and a store there that
+// counts its bytes at an mbarrier of the same CTA.
+__device__ __forceinline__ uint32_t cluster_map(uint32_t local, uint32_t rank) {
+  uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
+  return remote;
+}
+__device__ __forceinline__ void push_f32(uint32_t remote, float v, uint32_t remote_bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];"
+               ::"r"(remote), "r"(__float_as_uint(v)), "r"(remote_bar) : "memory");
+}
+// The wait for what the other CTAs of a cluster push: longer than the waits that can hold each of them up together,
+// so that no CTA leaves while a push to it is still to come.
+__device__ __forceinline__ bool mbar_wait_pushed(uint32_t bar) {
+  for (int i = 0; i < 4; ++i) {
+    if (mbar_wait(bar, 0u)) return true;
+  }
+  return false;
+}
+
 // ---- host: the driver's tensor-map encoder ----------------------------------------------------------
 using EncodeTiledFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                    const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,

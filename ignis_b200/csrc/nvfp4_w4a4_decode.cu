@@ -20,8 +20,8 @@
 //  * The fused SwiGLU (a gate|up parent) pairs a tile's 128 gate rows with their up rows: per K
 //    stage two ring entries, each with its own weight tile, sharing the first one's token tile,
 //    into two accumulators; the epilogue writes BF16(silu(BF16(g alpha)) * BF16(u alpha)).
-//  * Narrow weights split K over the CTAs of a cluster, which meet in distributed shared memory and
-//    add their partial sums in rank order (bit-reproducible, no global scratch).
+//  * Narrow weights split K over the CTAs of a cluster, which push their partial sums to the CTA that finishes a token,
+//    where they are added in rank order (bit-reproducible, no global scratch).
 //  * Every mbarrier wait is bounded; one that runs out sets a bit in the library's status word
 //    (b200q_nvfp4_device_status), and the CTA falls through to the common exit and frees its
 //    tensor memory.
@@ -33,7 +33,7 @@ namespace {
 
 constexpr uint32_t kABytes = 128 * 128;   // one stage of weight codes: 128 rows x 256 values
 constexpr uint32_t kSfBytes = 4 * 512;    // one stage of scales of a 128-row tile: four K-atoms
-constexpr uint32_t kProducerTimeout = 0x100u, kMmaTimeout = 0x200u, kEpilogueTimeout = 0x400u, kQuantTimeout = 0x800u;
+constexpr uint32_t kProducerTimeout = 0x100u, kMmaTimeout = 0x200u, kEpilogueTimeout = 0x400u, kQuantTimeout = 0x800u, kReduceTimeout = 0x1000u;
 constexpr int kMaxQuantGroups = 2;
 constexpr int kMaxItems = 4;              // 16-value items per quantizer thread and stage (32 tokens)
 
@@ -83,6 +83,7 @@ struct RawItem {
   uint4 lo, hi;  // 16 BF16 activations
 };
 
+template <int ITEMS>
 __global__ void __launch_bounds__(64 + 128 * kMaxQuantGroups, 2) w4a4_decode_kernel(const __grid_constant__ A4Maps maps, const __grid_constant__ A4Params p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -91,8 +92,9 @@ __global__ void __launch_bounds__(64 + 128 * kMaxQuantGroups, 2) w4a4_decode_ker
   // a stage: weight codes | token codes | weight scale tiles | token scale tiles
   const uint32_t b_bytes = p.bn * 128u;
   const uint32_t stage_bytes = kABytes + b_bytes + 2u * kSfBytes;
-  const uint32_t bars = base + p.stages * stage_bytes;  // full[stages], empty[stages], accumulator full; then the TMEM slot
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(base_ptr + p.stages * stage_bytes + 8u * (2u * p.stages + 1u) + 8u);
+  const uint32_t bars = base + p.stages * stage_bytes;  // full[stages], empty[stages], accumulator full, sums landed; then the TMEM slot
+  const uint32_t bar_acc = bars + 8u * 2u * p.stages, bar_sums = bar_acc + 8u;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(base_ptr + (bar_sums - base) + 8u);
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int producer_warp = 4 * static_cast<int>(p.groups), mma_warp = producer_warp + 1;
   const uint32_t rank = cluster_ctarank(), kc = p.kc;
@@ -136,8 +138,11 @@ __global__ void __launch_bounds__(64 + 128 * kMaxQuantGroups, 2) w4a4_decode_ker
       mbar_init(bars + 8 * s, 128 + 1);          // 128 quantizer threads and the producer's expect_tx arrival
       mbar_init(bars + 8 * (p.stages + s), 1);   // the MMA thread's commit
     }
-    mbar_init(bars + 8 * 2 * p.stages, 1);
+    mbar_init(bar_acc, 1);
+    mbar_init(bar_sums, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    // every rank of the cluster sends its sums of the tokens that this one finishes
+    if (kc > 1u) mbar_expect_tx(bar_sums, kc * ((p.tokens - rank + kc - 1u) / kc) * halves * 512u);
   }
   if (warp == mma_warp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(p.tmem_cols) : "memory");
@@ -162,75 +167,79 @@ __global__ void __launch_bounds__(64 + 128 * kMaxQuantGroups, 2) w4a4_decode_ker
     //      group g takes the CTA's stages g, g + groups, ... ----
     griddep_launch_dependents();
     griddep_wait();   // the activations may come from the previous kernel
+    // A thread's values of its group's next kDepth stages are requested together (stage by stage, the trip to the L2
+    // came once per stage and held up the short K slices: 1.3 us each).
+    constexpr int kDepth = kMaxItems / ITEMS;
     const uint32_t items = p.tokens * 16u;
     const uint32_t group = static_cast<uint32_t>(warp) >> 2, tid = threadIdx.x & 127u;
     const uint32_t first = s0 + group;
-    uint32_t tok[kMaxItems], grp[kMaxItems];
-    const uint16_t *src[kMaxItems];
+    uint32_t tok[ITEMS], grp[ITEMS];
+    const uint16_t *src[ITEMS];
 #pragma unroll
-    for (int j = 0; j < kMaxItems; ++j) {
+    for (int j = 0; j < ITEMS; ++j) {
       const uint32_t i = tid + 128u * j;
       tok[j] = i >> 4;
       grp[j] = i & 15u;
       src[j] = p.x + static_cast<size_t>(tok[j]) * p.k + grp[j] * 16u;
     }
-    RawItem cur[kMaxItems];
+    RawItem cur[kDepth][ITEMS];
+    auto request = [&](RawItem (&to)[ITEMS], uint32_t s) {
 #pragma unroll
-    for (int j = 0; j < kMaxItems; ++j) {
-      if (tid + 128u * j < items && first < s1) {
-        cur[j].lo = ldg128_coherent(src[j] + static_cast<size_t>(first) * 256u);
-        cur[j].hi = ldg128_coherent(src[j] + static_cast<size_t>(first) * 256u + 8);
+      for (int j = 0; j < ITEMS; ++j) {
+        if (tid + 128u * j < items && s < s1) {
+          to[j].lo = ldg128_coherent(src[j] + static_cast<size_t>(s) * 256u);
+          to[j].hi = ldg128_coherent(src[j] + static_cast<size_t>(s) * 256u + 8);
+        }
       }
-    }
+    };
+#pragma unroll
+    for (int d = 0; d < kDepth; ++d) request(cur[d], first + d * p.groups);
     bool ok = true;
-    for (uint32_t s = first; s < s1 && ok; s += p.groups) {
-      const uint32_t it = (s - s0) * halves;   // the stage's (first) ring entry
-      uint2 codes[kMaxItems];
-      uint8_t scale[kMaxItems];
+    for (uint32_t sd = first; sd < s1 && ok; sd += kDepth * p.groups) {
 #pragma unroll
-      for (int j = 0; j < kMaxItems; ++j) {
-        if (tid + 128u * j < items) quantize_block16(cur[j].lo, cur[j].hi, W.d_in, codes[j], scale[j]);
-      }
-      if (s + p.groups < s1) {
+      for (int d = 0; d < kDepth; ++d) {
+        const uint32_t s = sd + d * p.groups;
+        if (s >= s1 || !ok) break;
+        const uint32_t it = (s - s0) * halves;   // the stage's (first) ring entry
+        uint2 codes[ITEMS];
+        uint8_t scale[ITEMS];
 #pragma unroll
-        for (int j = 0; j < kMaxItems; ++j) {
-          if (tid + 128u * j < items) {
-            cur[j].lo = ldg128_coherent(src[j] + static_cast<size_t>(s + p.groups) * 256u);
-            cur[j].hi = ldg128_coherent(src[j] + static_cast<size_t>(s + p.groups) * 256u + 8);
-          }
+        for (int j = 0; j < ITEMS; ++j) {
+          if (tid + 128u * j < items) quantize_block16(cur[d][j].lo, cur[d][j].hi, W.d_in, codes[j], scale[j]);
         }
-      }
-      const uint32_t slot = it % p.stages;
-      if (!mbar_wait(bars + 8 * (p.stages + slot), ((it / p.stages) & 1u) ^ 1u)) {
-        if (lane == 0) atomicOr(&g_a4_status, kQuantTimeout);
-        ok = false;
-        break;
-      }
-      const uint32_t b_tile = base + slot * stage_bytes + kABytes;
-      const uint32_t sf_tile = b_tile + b_bytes + kSfBytes;
-#pragma unroll
-      for (int j = 0; j < kMaxItems; ++j) {
-        if (tid + 128u * j < items) {
-          const uint32_t t = tok[j], g = grp[j];
-          // 128-byte swizzle: row t of the tile, 16-byte unit g / 2 exchanged by the row's low bits
-          const uint32_t at = b_tile + (t >> 3) * 1024u + (t & 7u) * 128u + (((g >> 1) ^ (t & 7u)) << 4) + (g & 1u) * 8u;
-          asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(codes[j].x), "r"(codes[j].y) : "memory");
-          // scale tile of K-atom g / 4: row t at (t % 32) * 16 + (t / 32) * 4, group g % 4 within it
-          const uint32_t sat = sf_tile + (g >> 2) * 512u + (t & 31u) * 16u + (t >> 5) * 4u + (g & 3u);
-          asm volatile("st.shared.u8 [%0], %1;" ::"r"(sat), "r"(static_cast<uint32_t>(scale[j])) : "memory");
-        }
-      }
-      // the tiles are read by the tensor core (async proxy): order these writes before it
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      mbar_arrive(bars + 8 * slot);
-      if (two) {   // the second entry reads this token tile: nothing to write, only its turn to take
-        const uint32_t it2 = it + 1u, slot2 = it2 % p.stages;
-        if (!mbar_wait(bars + 8 * (p.stages + slot2), ((it2 / p.stages) & 1u) ^ 1u)) {
+        request(cur[d], s + kDepth * p.groups);
+        const uint32_t slot = it % p.stages;
+        if (!mbar_wait(bars + 8 * (p.stages + slot), ((it / p.stages) & 1u) ^ 1u)) {
           if (lane == 0) atomicOr(&g_a4_status, kQuantTimeout);
           ok = false;
           break;
         }
-        mbar_arrive(bars + 8 * slot2);
+        const uint32_t b_tile = base + slot * stage_bytes + kABytes;
+        const uint32_t sf_tile = b_tile + b_bytes + kSfBytes;
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) {
+          if (tid + 128u * j < items) {
+            const uint32_t t = tok[j], g = grp[j];
+            // 128-byte swizzle: row t of the tile, 16-byte unit g / 2 exchanged by the row's low bits
+            const uint32_t at = b_tile + (t >> 3) * 1024u + (t & 7u) * 128u + (((g >> 1) ^ (t & 7u)) << 4) + (g & 1u) * 8u;
+            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(codes[j].x), "r"(codes[j].y) : "memory");
+            // scale tile of K-atom g / 4: row t at (t % 32) * 16 + (t / 32) * 4, group g % 4 within it
+            const uint32_t sat = sf_tile + (g >> 2) * 512u + (t & 31u) * 16u + (t >> 5) * 4u + (g & 3u);
+            asm volatile("st.shared.u8 [%0], %1;" ::"r"(sat), "r"(static_cast<uint32_t>(scale[j])) : "memory");
+          }
+        }
+        // the tiles are read by the tensor core (async proxy): order these writes before it
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        mbar_arrive(bars + 8 * slot);
+        if (two) {   // the second entry reads this token tile: nothing to write, only its turn to take
+          const uint32_t it2 = it + 1u, slot2 = it2 % p.stages;
+          if (!mbar_wait(bars + 8 * (p.stages + slot2), ((it2 / p.stages) & 1u) ^ 1u)) {
+            if (lane == 0) atomicOr(&g_a4_status, kQuantTimeout);
+            ok = false;
+            break;
+          }
+          mbar_arrive(bars + 8 * slot2);
+        }
       }
     }
   } else if (warp == producer_warp) {
@@ -289,17 +298,16 @@ __global__ void __launch_bounds__(64 + 128 * kMaxQuantGroups, 2) w4a4_decode_ker
       }
       __syncwarp();
     }
-    if (ok && elect_one()) mma_commit(bars + 8 * 2 * p.stages);
+    if (ok && elect_one()) mma_commit(bar_acc);
     __syncwarp();
   }
 
   // ---- epilogue: thread r of warps 0-3 owns accumulator lane r = weight row r of the tile ----
   const uint32_t out_elem_f32 = p.epilogue & kEpilogueF32;
-  float *part = reinterpret_cast<float *>(base_ptr);   // [half][token][128] partial sums, over the (then idle) stage ring
   bool have = false;
   uint32_t v[32], u[32];
   if (warp < 4) {
-    have = mbar_wait(bars + 8 * 2 * p.stages, 0u);
+    have = mbar_wait(bar_acc, 0u);
     if (!have && lane == 0) atomicOr(&g_a4_status, kEpilogueTimeout);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (have) {
@@ -315,25 +323,25 @@ __global__ void __launch_bounds__(64 + 128 * kMaxQuantGroups, 2) w4a4_decode_ker
     }
   }
   // token tl, row r of the CTA's tile(s), from the accumulator sums (the second only with two tiles)
-  auto store = [&](size_t at, float acc) {
-    const float val = __fmul_rn(acc, W.alpha);   // not contracted into the residual add: one value for every epilogue
-    if (out_elem_f32) {
-      float *y = static_cast<float *>(W.y);
-      y[at] = (p.epilogue & kEpilogueAdd) ? y[at] + val : val;
-    } else {
-      __nv_bfloat16 *y = static_cast<__nv_bfloat16 *>(W.y);
-      y[at] = __float2bfloat16_rn((p.epilogue & kEpilogueAdd) ? val + __bfloat162float(y[at]) : val);
-    }
+  const bool add = (p.epilogue & kEpilogueAdd) != 0u;
+  auto residual = [&](uint32_t tl, uint32_t row) {
+    const size_t at = static_cast<size_t>(tl) * W.ldy + row;
+    return out_elem_f32 ? static_cast<const float *>(W.y)[at] : __bfloat162float(static_cast<const __nv_bfloat16 *>(W.y)[at]);
   };
-  auto emit = [&](uint32_t tl, uint32_t r, float acc, float acc_b) {
+  auto store = [&](size_t at, float acc, float old) {
+    const float val = __fmul_rn(acc, W.alpha);   // not contracted into the residual add: one value for every epilogue
+    if (out_elem_f32) static_cast<float *>(W.y)[at] = add ? old + val : val;
+    else static_cast<__nv_bfloat16 *>(W.y)[at] = __float2bfloat16_rn(add ? val + old : val);
+  };
+  auto emit = [&](uint32_t tl, uint32_t r, float acc, float acc_b, float old, float old_b) {
     const size_t at = static_cast<size_t>(tl) * W.ldy + r;
     if (swiglu) {
       const float gv = __bfloat162float(__float2bfloat16_rn(__fmul_rn(acc, W.alpha)));
       const float uv = __bfloat162float(__float2bfloat16_rn(__fmul_rn(acc_b, W.alpha)));
       static_cast<__nv_bfloat16 *>(W.y)[at + row_a] = __float2bfloat16_rn(gv / (1.0f + __expf(-gv)) * uv);
     } else {
-      store(at + row_a, acc);
-      if (two) store(at + row_b, acc_b);
+      store(at + row_a, acc, old);
+      if (two) store(at + row_b, acc_b, old_b);
     }
   };
   if (kc == 1u) {
@@ -341,46 +349,57 @@ __global__ void __launch_bounds__(64 + 128 * kMaxQuantGroups, 2) w4a4_decode_ker
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
         if (static_cast<uint32_t>(j) >= p.tokens) break;
-        emit(static_cast<uint32_t>(j), threadIdx.x, __uint_as_float(v[j]), two ? __uint_as_float(u[j]) : 0.0f);
+        const uint32_t tl = static_cast<uint32_t>(j);
+        emit(tl, threadIdx.x, __uint_as_float(v[j]), two ? __uint_as_float(u[j]) : 0.0f, add ? residual(tl, row_a + threadIdx.x) : 0.0f,
+             add && two ? residual(tl, row_b + threadIdx.x) : 0.0f);
       }
     }
   } else {
-    __syncthreads();   // every role is done with the stage ring: the partial sums take its place
-    float *part_up = part + p.bn * 128u;
-    if (warp < 4) {
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        if (static_cast<uint32_t>(j) < p.bn) {
-          part[static_cast<size_t>(j) * 128u + threadIdx.x] = have ? __uint_as_float(v[j]) : 0.0f;
-          if (two) part_up[static_cast<size_t>(j) * 128u + threadIdx.x] = have ? __uint_as_float(u[j]) : 0.0f;
-        }
-      }
-    }
-    __syncwarp();
+    // Token tl is finished by rank tl % kc: once every ring of the cluster is idle, every CTA pushes its sums of it over
+    // that rank's ring, [sender][turn][half][128 rows], and the bytes count at the receiver's barrier. Nobody reads
+    // another CTA's memory, so nobody waits for a reader before it leaves. (Pulled between two meetings of the cluster, a
+    // launch took 2.8 us from the last MMA to its end; with room for the sums beside the ring, and so without this
+    // meeting, a layer at 8 tokens was no faster: 42.8 us against 42.3.)
+    const uint32_t r = threadIdx.x & 127u;
+    // the residual of a thread's next token is requested before it is needed
+    float old = 0.0f, old_b = 0.0f;
+    auto request_residual = [&](uint32_t i) {
+      if (!add || i * kc + rank >= p.tokens) return;
+      old = residual(i * kc + rank, row_a + r);
+      if (two) old_b = residual(i * kc + rank, row_b + r);
+    };
+    if (warp < producer_warp) request_residual(static_cast<uint32_t>(warp) >> 2);
     cluster_sync_all();
+    const uint32_t turns = (p.tokens + kc - 1u) / kc;
     if (warp < 4) {
-      // tokens dealt over the cluster's CTAs in turn; a thread requests the kc partial sums of its
-      // output together and adds them in rank order
-      for (uint32_t tl = rank; tl < p.tokens; tl += kc) {
-        float pg[8], pu[8];
+      uint32_t at = base + (rank * turns * halves * 128u + threadIdx.x) * 4u, to = 0;
 #pragma unroll
-        for (uint32_t q = 0; q < 8u; ++q) {
-          pg[q] = q < kc ? ld_cluster_f32(part + static_cast<size_t>(tl) * 128u + threadIdx.x, q) : 0.0f;
-          pu[q] = q < kc && two ? ld_cluster_f32(part_up + static_cast<size_t>(tl) * 128u + threadIdx.x, q) : 0.0f;
-        }
-        float sum = pg[0], sum_up = pu[0];
-#pragma unroll
-        for (uint32_t q = 1; q < 8u; ++q) {
-          if (q < kc) {
-            sum += pg[q];
-            sum_up += pu[q];
+      for (uint32_t j = 0; j < 32u; ++j) {
+        if (j >= p.tokens) break;
+        const uint32_t bar = cluster_map(bar_sums, to);
+        push_f32(cluster_map(at, to), have ? __uint_as_float(v[j]) : 0.0f, bar);
+        if (two) push_f32(cluster_map(at + 512u, to), have ? __uint_as_float(u[j]) : 0.0f, bar);
+        if (++to == kc) to = 0, at += halves * 512u;
+      }
+    }
+    if (warp < producer_warp) {
+      const float *sums = reinterpret_cast<const float *>(base_ptr) + r;
+      if (mbar_wait_pushed(bar_sums)) {
+        for (uint32_t i = static_cast<uint32_t>(warp) >> 2; i * kc + rank < p.tokens; i += p.groups) {
+          float sum = 0.0f, sum_up = 0.0f;
+          for (uint32_t q = 0; q < kc; ++q) {   // in rank order
+            const float *from = sums + (q * turns + i) * halves * 128u;
+            sum = q == 0u ? from[0] : sum + from[0];
+            if (two) sum_up = q == 0u ? from[128] : sum_up + from[128];
           }
+          emit(i * kc + rank, r, sum, sum_up, old, old_b);
+          request_residual(i + p.groups);
         }
-        emit(tl, threadIdx.x, sum, sum_up);
+      } else if (lane == 0) {
+        atomicOr(&g_a4_status, kReduceTimeout);
       }
     }
     __syncwarp();
-    cluster_sync_all();   // no CTA leaves while a peer may still read its partial sums
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -400,14 +419,17 @@ uint32_t a4_ring_depth(uint32_t ctas_per_sm, uint32_t bn, uint32_t k_stages) {
   return stages < k_stages ? stages : k_stages;
 }
 
+// The ring, barriers and the tensor-memory slot behind it, alignment slack.
 size_t a4_smem_bytes(uint32_t bn, uint32_t stages) {
-  return static_cast<size_t>(stages) * (kABytes + bn * 128u + 2u * kSfBytes) + 8u * (2u * stages + 1u) + 16u + 1024u;
+  return static_cast<size_t>(stages) * (kABytes + bn * 128u + 2u * kSfBytes) + 8u * (2u * stages + 2u) + 16u + 1024u;
 }
 
 }  // namespace
 
 int32_t w4a4_decode_prepare(ErrorSlot &slot) {
-  const cudaError_t err = cudaFuncSetAttribute(w4a4_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kA4MaxSmem));
+  cudaError_t err = cudaFuncSetAttribute(w4a4_decode_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kA4MaxSmem));
+  if (err == cudaSuccess) err = cudaFuncSetAttribute(w4a4_decode_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kA4MaxSmem));
+  if (err == cudaSuccess) err = cudaFuncSetAttribute(w4a4_decode_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kA4MaxSmem));
   if (err != cudaSuccess) return fail(slot, "nvfp4 W4A4 decode kernel attributes: %s", cudaGetErrorString(err));
   if (encode_tiled_fn() == nullptr) return fail(slot, "cuTensorMapEncodeTiled is not available from this driver");
   // How many clusters of each size the device places at one CTA per SM (clusters stay inside one
@@ -428,7 +450,7 @@ int32_t w4a4_decode_prepare(ErrorSlot &slot) {
     config.attrs = attr;
     config.numAttrs = 1;
     int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, w4a4_decode_kernel, &config) == cudaSuccess && clusters > 0) {
+    if (cudaOccupancyMaxActiveClusters(&clusters, w4a4_decode_kernel<1>, &config) == cudaSuccess && clusters > 0) {
       dev->a4_slots[kc] = clusters * kc;
     } else {
       dev->a4_slots[kc] = 0;
@@ -512,6 +534,10 @@ int32_t w4a4_decode_launch(ErrorSlot &slot, const DeviceState &dev, const A4Item
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(ctas, 1, 1);
   config.blockDim = dim3(64 + 128 * p.groups, 1, 1);
+  // the cluster's sums land over the ring: at least four stages of it where K is split, 32 tokens of two tiles at most
+  if (kc > 1u && stages * (kABytes + p.bn * 128u + 2u * kSfBytes) < (tokens + kc - 1u) / kc * kc * (two ? 2u : 1u) * 512u) {
+    return fail(slot, "nvfp4 W4A4 decode route: the ring is too short for a cluster of %u", kc);
+  }
   config.dynamicSmemBytes = a4_smem_bytes(p.bn, stages);
   config.stream = stream;
   cudaLaunchAttribute attr[2];
@@ -523,7 +549,9 @@ int32_t w4a4_decode_launch(ErrorSlot &slot, const DeviceState &dev, const A4Item
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attr;
   config.numAttrs = dev.pdl ? 2 : 1;
-  const cudaError_t err = cudaLaunchKernelEx(&config, w4a4_decode_kernel, maps, p);
+  const cudaError_t err = tokens <= 8u    ? cudaLaunchKernelEx(&config, w4a4_decode_kernel<1>, maps, p)
+                          : tokens <= 16u ? cudaLaunchKernelEx(&config, w4a4_decode_kernel<2>, maps, p)
+                                          : cudaLaunchKernelEx(&config, w4a4_decode_kernel<4>, maps, p);
   if (err != cudaSuccess) return fail(slot, "nvfp4 W4A4 decode launch: %s", cudaGetErrorString(err));
   return 0;
 }

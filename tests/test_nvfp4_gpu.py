@@ -681,6 +681,39 @@ def test_w4a4_decode_route(nv, oracle, tokens, n, k):
     assert nv.device_status() == 0
 
 
+@pytest.mark.parametrize("tokens", [4, 8, 9, 16, 17, 31, 32])
+def test_w4a4_decode_cluster_sums(nv, monkeypatch, tokens):
+    """Every cluster size of the decode route finishes the same sums: ranks with no token, one token or several, one and
+    two row tiles per CTA, stored, added and fused. Both sides add the same exactly representable products in FP32, in
+    other orders: their difference is within k 2^-24 of the sums of magnitudes, here against the largest output."""
+    n, k = 512, 4096
+    rng = np.random.default_rng(tokens)
+    w = nv.Weight.from_planes(*make_weight(rng, n, k)[:2], 448.0, 448.0)
+    x = torch.randn(tokens, k, generator=torch.Generator().manual_seed(tokens)).to(torch.bfloat16).cuda()
+    base = torch.randn(tokens, n, generator=torch.Generator().manual_seed(1)).cuda()
+    results = {}
+    try:
+        for kc, pair in [(1, 0)] + [(c, p) for c in (2, 3, 5, 8) for p in (0, 1)]:
+            monkeypatch.setenv("B200Q_A4_DECODE_KC", str(kc))
+            monkeypatch.setenv("B200Q_A4_DECODE_PAIR", str(pair))
+            nv.prepare()
+            results[kc, pair] = (nv.linear(x, w, policy=nv.ALLOW_A4, epilogue=nv.OUT_F32),
+                                 nv.linear(x, w, out=base.clone(), policy=nv.ALLOW_A4, epilogue=nv.OUT_F32 | nv.ADD),
+                                 nv.linear_swiglu(x, w, policy=nv.ALLOW_A4))
+    finally:
+        monkeypatch.undo()
+        nv.prepare()
+    assert nv.device_status() == 0
+    plain, added, fused = results.pop((1, 0))
+    assert torch.equal(added, plain + base)
+    tol = k * 2.0 ** -24 * float(plain.abs().max())
+    for y, y_added, h in results.values():
+        assert float((y - plain).abs().max()) <= tol
+        assert torch.equal(y_added, y + base)
+        # silu(BF16(g)) BF16(u): a sum on the other side of a rounding moves each factor by 2^-8 of itself
+        assert torch.all((h.float() - fused.float()).abs() <= 2.0 ** -6 * fused.float().abs() + 1e-3 * fused.float().abs().max())
+
+
 def test_config1_gate_up_full_size_under_allow_a4(nv, oracle):
     """A 27B-style layer's widest product (gate|up, 34816 x 5120, 8 tokens) under ALLOW_A4 at full size: sampled
     row tiles against the host arithmetic, and the token-order property (the same tokens in reverse
