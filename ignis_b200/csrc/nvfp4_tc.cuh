@@ -93,6 +93,10 @@ struct RingAt {
   __device__ __forceinline__ void advance(uint32_t by, uint32_t depth) {
     for (slot += by; slot >= depth; slot -= depth) phase ^= 1u;
   }
+  __device__ __forceinline__ void step(uint32_t by, uint32_t depth) {   // by at most depth
+    slot += by;
+    if (slot >= depth) slot -= depth, phase ^= 1u;
+  }
 };
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -215,6 +219,11 @@ __device__ __forceinline__ uint32_t cluster_map(uint32_t local, uint32_t rank) {
 __device__ __forceinline__ void push_f32(uint32_t remote, float v, uint32_t remote_bar) {
   asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];"
                ::"r"(remote), "r"(__float_as_uint(v)), "r"(remote_bar) : "memory");
+}
+__device__ __forceinline__ void push_f32x4(uint32_t remote, const float4 v, uint32_t remote_bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+               ::"r"(remote), "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)), "r"(__float_as_uint(v.w)), "r"(remote_bar)
+               : "memory");
 }
 // The wait for what the other CTAs of a cluster push: longer than the waits that can hold each of them up together,
 // so that no CTA leaves while a push to it is still to come.

@@ -425,6 +425,29 @@ def test_swiglu_on_the_a16_tensor_core_route(nv, oracle, tokens, inter, k):
     assert torch.equal(nv.mlp(x.cuda(), w, down, ws), nv.linear(h, down))
 
 
+@pytest.mark.parametrize("tokens,inter,k", [(9, 128, 64), (16, 256, 320), (192, 128, 576), (193, 256, 320), (224, 128, 1088), (225, 128, 64),
+                                            (450, 384, 192)])
+def test_a16_decoded_weights_in_tensor_memory(nv, oracle, tokens, inter, k):
+    """Both sizes of the pieces that decoded weights take in tensor memory: whole stages up to 192 tokens a tile, half ones
+    for two row tiles from 193 to 224 (the fused form), with K of less than four stages, of a whole number of fours and of
+    neither; the plain product of the same parent beside it, stored and added."""
+    rng = np.random.default_rng(tokens + k)
+    codes, scales, d_w = make_weight(rng, 2 * inter, k, d_w=2000.0)
+    w = nv.Weight.from_planes(codes, scales, d_w)
+    x = torch.randn(tokens, k, generator=torch.Generator().manual_seed(tokens)).to(torch.bfloat16)
+    ref = ref_product(oracle, codes, scales, 2 * inter, k, d_w, x)
+    y32 = nv.linear(x.cuda(), w, epilogue=nv.OUT_F32)
+    check_f32(y32, ref)
+    base = torch.randn(tokens, 2 * inter, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16)
+    assert torch.equal(nv.linear(x.cuda(), w, out=base.clone().cuda(), epilogue=nv.ADD).cpu(), (y32.cpu() + base.float()).to(torch.bfloat16))
+    g, u = ref[:, :inter], ref[:, inter:]
+    want = g / (1.0 + np.exp(-g)) * u
+    got = nv.linear_swiglu(x.cuda(), w).double().cpu().numpy()
+    assert nv.device_status() == 0
+    assert np.abs(got - want).max() <= 2.0 ** -7 * np.abs(want).max()
+    assert np.linalg.norm(got - want) <= 2.0 ** -8 * np.linalg.norm(want)
+
+
 def test_every_launch_plan_gives_the_same_answer_within_tolerance(nv, oracle):
     """Rows per CTA and cluster size only move where partial sums meet."""
     n, k, tokens = 1024, 2048 + 64, 8
