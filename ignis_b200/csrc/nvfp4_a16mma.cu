@@ -1,6 +1,6 @@
 // NVFP4 A16 products on the tensor cores: y[t][r] = sum_k w[r][k] x[t][k] with BF16 activations
 // kept as they are and the weights decoded exactly, for token counts where the decode kernel's
-// warp-level MMAs become the limit (more than 16 tokens) up to prefill widths. Stands where the
+// warp-level MMAs become the limit (more than 8 tokens) up to prefill widths. Stands where the
 // reference runs nvfp4_small_t_kernel above a few tokens and nvfp4_a16_mma_kernel from 64 tokens
 // (kernel/vendor/src/ops/linear/nvfp4/nvfp4_small_t.cuh:211-377, kernel/src/linear.cu:119-124);
 // the design is not theirs.

@@ -61,8 +61,9 @@ int32_t decode_route(ErrorSlot &slot, const DeviceState &dev, const b200q_nvfp4_
   const size_t out_elem = (epilogue & kEpilogueF32) ? 4u : 2u;
   uint32_t groups = 0;
   for (uint32_t i = 0; i < count; ++i) groups += w[i]->n / 32u;
-  if (dev.a16_mma != 0 && tokens > 16u && peers == 1u && wait_for == nullptr && a16mma_takes(k, x)) {
-    // beyond two token tiles the warp-level MMAs of the decode kernel are the limit: the weights
+  if (dev.a16_mma != 0 && tokens > 8u && peers == 1u && wait_for == nullptr && a16mma_takes(k, x)) {
+    // beyond one token tile the warp-level MMAs of the decode kernel are the limit (a layer at 9 and 16 tokens: 92 and 94 us
+    // there, 80 and 82 here; at 8 it takes 65): the weights
     // are decoded once per tile of up to 256 tokens and multiplied on the tensor cores
     GemvWeight gw[kMaxGroup];
     for (uint32_t i = 0; i < count; ++i) {
