@@ -276,11 +276,12 @@ int32_t b200q_nvfp4_linear_group(const b200q_nvfp4_weight *const *w, uint32_t co
 int32_t b200q_nvfp4_device_status(void *stream, uint32_t *status) {
   ErrorSlot &slot = nvfp4_error();
   if (status == nullptr) return fail(slot, "b200q_nvfp4_device_status: status is NULL");
-  uint32_t a16 = 0, a4 = 0, noalloc = 0;
+  uint32_t gemv = 0, a16 = 0, a4 = 0, noalloc = 0;
+  if (gemv_status(slot, static_cast<cudaStream_t>(stream), &gemv) != 0) return -1;
   if (a16mma_status(slot, static_cast<cudaStream_t>(stream), &a16) != 0) return -1;
   if (w4a4_decode_status(slot, static_cast<cudaStream_t>(stream), &a4) != 0) return -1;
   if (w4a4_noalloc_status(slot, static_cast<cudaStream_t>(stream), &noalloc) != 0) return -1;
-  *status = a16 | a4 | noalloc;
+  *status = gemv | a16 | a4 | noalloc;
   return 0;
 }
 

@@ -18,12 +18,14 @@
 //    memory, scaled per (token, slice) by a power of two so the largest magnitude sits in
 //    [2^13, 2^14): every BF16 value within 2^-27 of the slice's maximum converts exactly. The
 //    inverse scale is applied to the slice's fp32 partial sums.
-//  * K is split over the warps of a CTA and over the CTAs of a thread-block cluster; partial sums
-//    meet in distributed shared memory and are added in a fixed order, so results are
-//    bit-reproducible and the call needs no global scratch.
+//  * K is split over the warps of a CTA and over the CTAs of a thread-block cluster; every CTA pushes its sums to
+//    the one that finishes them (st.async, counted at its mbarrier), where they are added in a fixed order, so results
+//    are bit-reproducible and the call needs no global scratch. (Pulled between two meetings of the cluster: a layer at 8
+//    tokens 65.2 us against 62.7.)
 //  * Programmatic dependent launch: the first weight loads are issued before the grid waits for
 //    its predecessor, so in a chain of layers the weight stream does not stop between kernels.
 #include "nvfp4_internal.cuh"
+#include "nvfp4_tc.cuh"
 
 namespace b200q {
 
@@ -31,6 +33,16 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = 8;
+constexpr uint32_t kSumsTimeout = 0x2000u;
+
+__device__ uint32_t g_gemv_status = 0;   // bounded waits for the cluster's sums that ran out
+
+// Places of 32 float4 that the cluster's CTAs push to one of them: (turn, sender, gate or up).
+__host__ __device__ constexpr int gemv_part_slots(int nt, int rm, int kc, bool swiglu) {
+  const int items = (swiglu ? rm / 2 : rm) * 2 * nt;
+  return (items + kc - 1) / kc * kc * (swiglu ? 2 : 1);
+}
+
 
 // A build with -DB200Q_GEMV_TRACE (python -m ignis_b200.build --trace: a second library, never the
 // shipped one) stamps the global timer at the phase boundaries of every CTA, for the timeline of a
@@ -165,25 +177,6 @@ __device__ __forceinline__ void compute_stage(const Stage &st, const uint4 *xs_s
   }
 }
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n"
-               "barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// float4 at the same shared-memory offset in CTA `rank` of this cluster.
-__device__ __forceinline__ float4 ld_cluster_f4(const void *local_smem, uint32_t rank) {
-  const uint32_t local = static_cast<uint32_t>(__cvta_generic_to_shared(local_smem));
-  uint32_t remote;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
-  return v;
-}
-
 __device__ __forceinline__ float silu_f32(float v) { return v / (1.0f + __expf(-v)); }
 
 // Eight BF16 values (one 16-byte chunk) times a power of two, as fp16, in the order the MMA
@@ -239,15 +232,82 @@ __device__ __forceinline__ float pow2f(int e) { return __uint_as_float(static_ca
 constexpr int kNoShiftYet = 1 << 20;  // a token whose chunks so far held nothing to scale
 constexpr int kPrepRegs = 5;  // chunks a lane keeps in registers between the amax and the store
 
+// A token's scale in a chunk that is not its slice's first: the accumulators are carried from one chunk of a slice into
+// the next chunk's units, and a chunk far smaller than an earlier one of its token must not pull them up by its whole ratio
+// (the sums gathered so far would leave the range of a float): its shift stays within 64 of the lowest shift the token has
+// had, and what it then loses lies 2^-50 below the earlier sums.
+__device__ __forceinline__ int shift_cap(int low) { return low != kNoShiftYet ? min(126, low + 64) : 126; }
+
+// prepare_activations for up to four tokens, `share` warps per token: warp w prepares steps w share / 8, + share, ... of token
+// w % (8 / share), all of them in registers.
+template <int XU, bool CHUNKED>
+__device__ __forceinline__ void prepare_shared(const GemvParams &p, int cb, int nsteps, int share, uint4 *xs, float *inv_s, float *scale_s,
+                                               int *low_s, uint32_t *tops, bool first, int warp, int lane) {
+  const int tokens8 = kWarps / share;   // token slots dealt to the warps
+  const int tok = warp & (tokens8 - 1), m0 = warp / tokens8;
+  const int t = lane >> 3, i = lane & 7;
+  const bool live = static_cast<uint32_t>(tok) < p.tokens;
+  const uint4 *src = reinterpret_cast<const uint4 *>(p.x + static_cast<size_t>(live ? tok : 0) * p.k + static_cast<size_t>(cb) * 256u) + lane;
+  const int inside = (static_cast<int>(p.k / 8u) - cb * 32 - lane + 31) / 32;   // steps whose chunk for this lane lies inside K
+  const int valid = live ? min(nsteps, max(inside, 0)) : 0;
+  uint4 held[kPrepRegs];
+  uint32_t amax = 0u;
+#pragma unroll
+  for (int j = 0; j < kPrepRegs; ++j) {
+    held[j] = make_uint4(0u, 0u, 0u, 0u);
+    if (m0 + j * share < valid) held[j] = ldg128_coherent(src + (m0 + j * share) * 32);
+  }
+#pragma unroll
+  for (int j = 0; j < kPrepRegs; ++j) amax = chunk_amax_bits(held[j], amax);
+  const uint32_t mine = __reduce_max_sync(0xFFFFFFFFu, max(amax & 0xFFFFu, amax >> 16));
+  if (lane == 0) tops[warp] = mine;
+  int low = kNoShiftYet;
+  if (CHUNKED && !first && live) low = low_s[tok];
+  __syncthreads();
+  uint32_t top = 0u;
+  for (int w = tok; w < kWarps; w += tokens8) top = max(top, tops[w]);
+  const int shift = CHUNKED ? min(amax_shift(top), shift_cap(low)) : amax_shift(top);
+  const float scale = pow2f(shift);
+  if (lane == 0 && m0 == 0) {
+    if (CHUNKED) low_s[tok] = (top == 0u || top >= 0x7F80u) ? low : min(low, shift);
+    inv_s[tok] = live ? pow2f(-shift) : 0.0f;
+    scale_s[tok] = scale;
+  }
+  if (tok + tokens8 < kWarps && m0 == 0 && lane == 0) {   // token slots that no warp prepares
+    for (int z = tok + tokens8; z < kWarps; z += tokens8) {
+      inv_s[z] = 0.0f;
+      scale_s[z] = 1.0f;
+    }
+  }
+  const int word = ((i << 2) | (t ^ ((i >> 1) & 3))) ^ (tok << 2);
+#pragma unroll
+  for (int j = 0; j < kPrepRegs; ++j) {
+    const int m = m0 + j * share;
+    if (m >= nsteps) break;
+    uint4 *dst = xs + (static_cast<size_t>(m) * 8 + i) * 32;
+    dst[word] = convert_chunk<XU>(held[j], scale, i);
+    for (int z = tok + tokens8; z < kWarps; z += tokens8) dst[word ^ ((z ^ tok) << 2)] = make_uint4(0u, 0u, 0u, 0u);
+  }
+}
+
 // Rewrites steps [cb, ce) of the activations as scaled fp16 B fragments. Warp w prepares token
-// slots w, w + 8, ...; a lane owns one 16-byte chunk of every step (t: the lane quarter that will
-// read it, i: the word it multiplies). The slot's inverse scale goes to
+// slots w, w + 8, ...; with few tokens the CTA's warps share a token's steps instead (one token: all eight; the layer at
+// one token 60.1 -> 56.6 us) and exchange their maxima through `tops`. A lane owns one 16-byte chunk of every step (t: the
+// lane quarter that will read it, i: the word it multiplies). The slot's inverse scale goes to
 // inv_s, its scale to scale_s.
 template <int NT, int XU, bool CHUNKED>
 __device__ __forceinline__ void prepare_activations(const GemvParams &p, int cb, int ce, uint4 *xs, float *inv_s,
-                                                    float *scale_s, int *low_s, bool first, int warp, int lane,
+                                                    float *scale_s, int *low_s, uint32_t *tops, bool first, int warp, int lane,
                                                     int trace_launch) {
   const int nsteps = ce - cb;
+  if (NT == 1) {
+    // `share` warps per token, as many as keep every warp at work; a warp's steps must fit in its registers
+    const int share = p.tokens > 4u ? 1 : (p.tokens > 2u ? 2 : (p.tokens > 1u ? 4 : 8));
+    if (share > 1 && nsteps <= share * kPrepRegs) {
+      prepare_shared<XU, CHUNKED>(p, cb, nsteps, share, xs, inv_s, scale_s, low_s, tops, first, warp, lane);
+      return;
+    }
+  }
   // Lane l takes chunk l of a step: t = l / 8 is the lane quarter that will read it, i = l % 8 the
   // word it multiplies. (Dealing the chunks so that the fragment stores avoid their four-way bank
   // conflict scatters each quarter-warp's global load over four lines, and measured slower.)
@@ -314,14 +374,10 @@ __device__ __forceinline__ void prepare_activations(const GemvParams &p, int cb,
     for (int o = 16; o > 0; o >>= 1) amax = __vmaxu2(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
     if (tt == 0) GEMV_TRACE(8);
     const uint32_t top = max(amax & 0xFFFFu, amax >> 16);
-    // The accumulators are carried from one chunk of a slice into the next chunk's units. A chunk
-    // far smaller than an earlier one of its token must not pull them up by its whole ratio (the
-    // sums gathered so far would leave the range of a float): its shift stays within 64 of the
-    // lowest shift the token has had, and what it then loses lies 2^-50 below the earlier sums.
     int cap = 126, low = kNoShiftYet;
     if (CHUNKED && !first) {
       low = low_s[tt * 8 + warp];
-      if (low != kNoShiftYet) cap = min(126, low + 64);
+      cap = shift_cap(low);
       __syncwarp();  // every lane has read the token's lowest shift before lane 0 replaces it
     }
     int shift = min(amax_shift(top), cap);
@@ -375,9 +431,11 @@ __global__ void __launch_bounds__(kThreads, NT <= 2 ? 2 : 1) nvfp4_gemv_kernel(c
   uint4 *xs = reinterpret_cast<uint4 *>(smem_raw);
   float4 *red = reinterpret_cast<float4 *>(smem_raw + static_cast<size_t>(p.xs_steps) * 4096u * NT);
   float4 *part = red + static_cast<size_t>(kw_count - 1) * rm * 2 * NT * 32;
-  float *inv_s = reinterpret_cast<float *>(part + static_cast<size_t>(rm) * 2 * NT * 32);
+  float *inv_s = reinterpret_cast<float *>(part + gemv_part_slots(NT, rm, static_cast<int>(kc), (p.epilogue & kEpilogueSwiglu) != 0u) * 32);
   float *scale_s = inv_s + 8 * NT;
   int *low_s = reinterpret_cast<int *>(scale_s + 8 * NT);
+  uint32_t *tops = reinterpret_cast<uint32_t *>(low_s + 8 * NT);   // [warp]
+  const uint32_t bar_sums = smem_u32(tops + kWarps);
 
   // which weight of the group this CTA serves
   uint32_t wi = 0;
@@ -388,6 +446,16 @@ __global__ void __launch_bounds__(kThreads, NT <= 2 ? 2 : 1) nvfp4_gemv_kernel(c
   const GemvWeight &W = p.w[wi];
   const uint32_t row_block = (blockIdx.x - W.block_begin) / kc;
   const bool swiglu = (p.epilogue & kEpilogueSwiglu) != 0u;
+  // The CTA's sums are items (row group, half, token tile) of 512 bytes, an item finished by rank item % kc: what this CTA
+  // will be sent, said before any other CTA can send it.
+  const uint32_t items = static_cast<uint32_t>(swiglu ? rm / 2 : rm) * 2u * NT, sides = swiglu ? 2u : 1u;
+  if (threadIdx.x == 0) {
+    mbar_init(bar_sums, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    mbar_expect_tx(bar_sums, kc * ((items + kc - 1u - rank) / kc) * sides * 512u);
+  }
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   const uint32_t groups_total = W.n / 32u;
   uint32_t group;  // 32-row group of this warp
   bool active;
@@ -468,7 +536,7 @@ __global__ void __launch_bounds__(kThreads, NT <= 2 ? 2 : 1) nvfp4_gemv_kernel(c
       }
       __syncthreads();  // the previous chunk's fragments and scales are no longer read
     }
-    prepare_activations<NT, XU, CHUNKED>(p, cb, ce, xs, inv_s, scale_s, low_s, cb == c0, warp, lane, cb == c0 ? trace_launch : -1);
+    prepare_activations<NT, XU, CHUNKED>(p, cb, ce, xs, inv_s, scale_s, low_s, tops, cb == c0, warp, lane, cb == c0 ? trace_launch : -1);
     if (cb == c0) GEMV_TRACE(9);
     __syncthreads();
     if (cb == c0) GEMV_TRACE(3);
@@ -535,28 +603,43 @@ __global__ void __launch_bounds__(kThreads, NT <= 2 ? 2 : 1) nvfp4_gemv_kernel(c
           tot[a][tt][3] += v.w;
         }
     }
+  }
+
+  // ---- K reduction across the cluster, then the epilogue: an item's sums are pushed to the rank that finishes it, where
+  //      the bytes count at its barrier ([turn][sender][gate, up][lane]); nobody reads another CTA's memory, so nobody
+  //      waits for a reader before it leaves ----
+  GEMV_TRACE(5);
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // every CTA's barrier has been set up (it was, long ago)
+  const uint32_t out_groups = swiglu ? static_cast<uint32_t>(rm) / 2u : static_cast<uint32_t>(rm);
+  if (kw == 0) {
+    const uint32_t up = static_cast<uint32_t>(rgl) >= out_groups ? 1u : 0u;
+    const uint32_t f0 = (static_cast<uint32_t>(rgl) - up * out_groups) * 2u * NT;
+    uint32_t turn = f0 / kc, to = f0 % kc;
 #pragma unroll
     for (int a = 0; a < 2; ++a)
 #pragma unroll
-      for (int tt = 0; tt < NT; ++tt)
-        part[((rgl * 2 + a) * NT + tt) * 32 + lane] = make_float4(tot[a][tt][0], tot[a][tt][1], tot[a][tt][2], tot[a][tt][3]);
+      for (int tt = 0; tt < NT; ++tt) {
+        const uint32_t at = smem_u32(part) + (((turn * kc + rank) * sides + up) * 32u + static_cast<uint32_t>(lane)) * 16u;
+        push_f32x4(cluster_map(at, to), make_float4(tot[a][tt][0], tot[a][tt][1], tot[a][tt][2], tot[a][tt][3]), cluster_map(bar_sums, to));
+        if (++to == kc) to = 0u, ++turn;
+      }
   }
-
-  // ---- K reduction across the cluster, then the epilogue, the items dealt over ranks and warps ----
-  GEMV_TRACE(5);
-  cluster_sync_all();
-  GEMV_TRACE(6);
-  const int out_groups = swiglu ? rm / 2 : rm;
-  const int items = out_groups * 2 * NT;
   const float coef = W.inv_dw * 128.0f;  // the operands carried 2^-7
-  for (int f = static_cast<int>(rank) + static_cast<int>(kc) * warp; f < items; f += static_cast<int>(kc) * kWarps) {
-    const int og = f / (2 * NT), a = (f / NT) & 1, tt = f % NT;
+  bool landed = false;
+  for (uint32_t turn = static_cast<uint32_t>(warp), f = rank + kc * turn; f < items; turn += kWarps, f += kc * kWarps) {
+    if (!landed && !(landed = mbar_wait_pushed(bar_sums))) {
+      if (lane == 0) atomicOr(&g_gemv_status, kSumsTimeout);
+      break;
+    }
+    if (turn == static_cast<uint32_t>(warp)) GEMV_TRACE(6);
+    const uint32_t og = f / (2 * NT), a = (f / NT) & 1, tt = f % NT;
     float4 sum = make_float4(0.f, 0.f, 0.f, 0.f), sum_up = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (uint32_t r = 0; r < kc; ++r) {
-      const float4 v = ld_cluster_f4(&part[((og * 2 + a) * NT + tt) * 32 + lane], r);
+    for (uint32_t r = 0; r < kc; ++r) {   // in rank order
+      const float4 *from = part + (turn * kc + r) * sides * 32u + lane;
+      const float4 v = from[0];
       sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
       if (swiglu) {
-        const float4 u = ld_cluster_f4(&part[(((og + out_groups) * 2 + a) * NT + tt) * 32 + lane], r);
+        const float4 u = from[32];
         sum_up.x += u.x; sum_up.y += u.y; sum_up.z += u.z; sum_up.w += u.w;
       }
     }
@@ -590,15 +673,14 @@ __global__ void __launch_bounds__(kThreads, NT <= 2 ? 2 : 1) nvfp4_gemv_kernel(c
       }
     }
   }
-  cluster_sync_all();  // no CTA leaves while a peer may still read its partial sums
 }
 
 constexpr size_t kGemvMaxSmem = 160 * 1024;
 
-size_t gemv_smem_bytes(int nt, int rm, int xs_steps) {
+size_t gemv_smem_bytes(int nt, int rm, int kc, bool swiglu, int xs_steps) {
   const int kw_count = kWarps / rm;
   return static_cast<size_t>(xs_steps) * 4096u * nt + static_cast<size_t>(kw_count - 1) * rm * 2 * nt * 32 * 16 +
-         static_cast<size_t>(rm) * 2 * nt * 32 * 16 + static_cast<size_t>(24 * nt) * 4;
+         static_cast<size_t>(gemv_part_slots(nt, rm, kc, swiglu)) * 512u + static_cast<size_t>(24 * nt + kWarps) * 4 + 16u;
 }
 
 template <int NT, int XU, bool CHUNKED>
@@ -755,7 +837,7 @@ int32_t gemv_launch(ErrorSlot &slot, const DeviceState &dev, GemvParams &p, int 
   static uint32_t trace_counter = 0;
   p.epilogue = (p.epilogue & 0xFFFFu) | ((trace_counter++ & 127u) << 16);
 #endif
-  const size_t smem = gemv_smem_bytes(nt, plan.rm, plan.xs_steps);
+  const size_t smem = gemv_smem_bytes(nt, plan.rm, plan.kc, (p.epilogue & kEpilogueSwiglu) != 0u, plan.xs_steps);
   const bool chunked = (p.ksteps + plan.kc - 1u) / plan.kc > plan.xs_steps;
   if (smem > kGemvMaxSmem) return fail(slot, "nvfp4 decode: %zu bytes of shared memory exceed the kernel's limit", smem);
   cudaError_t err;
@@ -768,6 +850,13 @@ int32_t gemv_launch(ErrorSlot &slot, const DeviceState &dev, GemvParams &p, int 
     default: err = launch_for_slice<3>(chunked, nt, p, ctas, smem, stream, pdl); break;
   }
   if (err != cudaSuccess) return fail(slot, "nvfp4 decode launch: %s", cudaGetErrorString(err));
+  return 0;
+}
+
+int32_t gemv_status(ErrorSlot &slot, cudaStream_t stream, uint32_t *status) {
+  cudaError_t err = cudaMemcpyFromSymbolAsync(status, g_gemv_status, sizeof(uint32_t), 0, cudaMemcpyDeviceToHost, stream);
+  if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
+  if (err != cudaSuccess) return fail(slot, "b200q_nvfp4_device_status: %s", cudaGetErrorString(err));
   return 0;
 }
 

@@ -64,6 +64,8 @@ GemvPlan gemv_plan(const DeviceState &dev, uint32_t groups, uint32_t ksteps, int
 int32_t gemv_launch(ErrorSlot &slot, const DeviceState &dev, GemvParams &p, int nt, const GemvPlan &plan, uint32_t ctas,
                     cudaStream_t stream);
 
+int32_t gemv_status(ErrorSlot &slot, cudaStream_t stream, uint32_t *status);
+
 int32_t dequantize_launch(ErrorSlot &slot, const uint8_t *codes, const uint8_t *scales, uint32_t n, uint32_t k, float d_w,
                           float *out, cudaStream_t stream);
 int32_t quantize_activations_launch(ErrorSlot &slot, const uint16_t *x, uint32_t tokens, uint32_t k, float d_in,

@@ -287,9 +287,8 @@ int32_t b200q_nvfp4_linear_prequantized(const b200q_nvfp4_weight *w, uint32_t to
 int32_t b200q_nvfp4_linear_noalloc(const b200q_nvfp4_weight *w, const void *x, uint32_t tokens, void *y,
                                    uint32_t ldy, uint32_t epilogue, void *stream);
 
-/* The status word of the kernels that take no workspace - A16 calls of more than 8 tokens and
- * B200Q_NVFP4_ALLOW_A4 calls of up to 32 tokens run on the tensor cores with bounded device-side
- * waits - OR-ed with the status line of b200q_nvfp4_linear_noalloc's built-in scratch (bits 0..2 as
+/* The status word of the kernels that take no workspace - A16 calls, and B200Q_NVFP4_ALLOW_A4
+ * calls of up to 32 tokens, have bounded device-side waits - OR-ed with the status line of b200q_nvfp4_linear_noalloc's built-in scratch (bits 0..2 as
  * in b200q_nvfp4_workspace_status): copied to *status after `stream` has finished. 0 unless a wait
  * ran out, in which case that call's output is not valid. The word is per device and sticky. */
 int32_t b200q_nvfp4_device_status(void *stream, uint32_t *status);

@@ -471,6 +471,35 @@ def test_every_launch_plan_gives_the_same_answer_within_tolerance(nv, oracle):
         nv.prepare()
 
 
+@pytest.mark.parametrize("tokens", [1, 2, 3, 4, 5])
+def test_few_tokens_share_their_rewrite(nv, oracle, monkeypatch, tokens):
+    """Up to four tokens the warps of a decode CTA share a token's activations: slices that fit their registers and slices
+    that do not, one chunk and several, clusters of one and eight whose sums meet at the rank that finishes an item; the
+    sizes of x change by 2^20 from block to block, and a token of zeros is among them."""
+    n, k = 256, 8256
+    rng = np.random.default_rng(tokens)
+    codes, scales, d_w = make_weight(rng, n, k)
+    w = nv.Weight.from_planes(codes, scales, d_w)
+    x = torch.randn(tokens, k, generator=torch.Generator().manual_seed(tokens))
+    x *= 2.0 ** torch.randint(-10, 11, (tokens, (k + 255) // 256), generator=torch.Generator().manual_seed(7)).repeat_interleave(256, dim=1)[:, :k]
+    x[tokens - 1] *= 0.0 if tokens > 1 else 1.0
+    x = x.to(torch.bfloat16)
+    ref = ref_product(oracle, codes, scales, n, k, d_w, x)
+    try:
+        for rm, kc in ((1, 1), (8, 1), (2, 3), (8, 8)):
+            monkeypatch.setenv("B200Q_GEMV_RM", str(rm))
+            monkeypatch.setenv("B200Q_GEMV_KC", str(kc))
+            nv.prepare()
+            y = nv.linear(x.cuda(), w, epilogue=nv.OUT_F32)
+            for t in range(tokens):   # token by token: their sizes differ
+                check_f32(y[t: t + 1], ref[t: t + 1])
+            check_bf16(nv.linear(x.cuda(), w), ref)
+    finally:
+        monkeypatch.undo()
+        nv.prepare()
+    assert nv.device_status() == 0
+
+
 def test_long_k_takes_several_fragment_chunks(nv, oracle):
     """K = 17408 with one CTA per row block: the activation fragments are rebuilt chunk by chunk."""
     n, k, tokens = 256, 17408, 8
