@@ -48,7 +48,7 @@ struct ExpertParams {
 // tcgen05. `p` as for the warp-level kernels; frag_in / scale_in and frag_h / scale_h hold the
 // rotated rows and their inverse scales instead of fragments.
 int32_t moe_tc_prepare(ErrorSlot &slot);
-constexpr uint32_t kMoeTcItemRows = 256;
+constexpr uint32_t kMoeTcItemRows = 192;
 int32_t moe_tc_experts(ErrorSlot &slot, const DeviceState &dev, const ExpertParams &p, uint32_t rows, uint32_t items_max,
                        const uint32_t *offsets, cudaStream_t stream, const char *what);
 

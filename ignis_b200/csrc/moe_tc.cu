@@ -109,15 +109,15 @@ __global__ void __launch_bounds__(kRotateThreads) moe_tc_rotate_kernel(const __g
 }
 
 // PHASE 0: gate | up products of an item into gu. PHASE 1: down, weighted, into the rows the fold
-// kernel adds up. One CTA per (item, 16 DW output columns); no CTA waits for another.
-template <int PHASE, int DW>
-__global__ void __launch_bounds__(Shape<DW>::kThreads, DW == 16 ? 1 : 2) moe_tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
-                                                                 const __grid_constant__ ExpertParams p) {
+// kernel adds up. One CTA per (item, 128 output columns); no CTA waits for another.
+constexpr uint32_t kBoxRows = 32;   // rows of one TMA load: an item loads as many as it has rows for
+
+template <int PHASE>
+__global__ void __launch_bounds__(kThreads, 2) moe_tc_gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ ExpertParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t in = PHASE == 0 ? p.hidden : p.inter;
   const uint32_t out_plane = PHASE == 0 ? 2u * p.inter : p.hidden;
-  constexpr uint32_t kCols = Shape<DW>::kCols, kBlocks = Shape<DW>::kBlocks;
-  const uint32_t col_tiles = (out_plane + kCols - 1u) / kCols;
+  const uint32_t col_tiles = out_plane / 128u;
   const uint32_t item_index = blockIdx.x / col_tiles, col_tile = blockIdx.x % col_tiles;
   griddep_launch_dependents();
   griddep_wait();   // the item list and the rotated rows come from the kernels before
@@ -128,76 +128,43 @@ __global__ void __launch_bounds__(Shape<DW>::kThreads, DW == 16 ? 1 : 2) moe_tc_
     if (threadIdx.x == 0 && col_tile == 0) atomicOr(p.status, kStatusAbsentRecord);
     return;
   }
-  const Core c = core_setup<DW>(smem_raw);
   Job job;
   job.trellis = static_cast<const uint32_t *>(slot.record);
   job.k2 = slot.k2;
   job.tile_stride = out_plane / 16u;
   job.stage0 = 0u;
   job.stage1 = in / 64u;
-  job.blk0 = kBlocks * col_tile;
-  job.blk1 = kBlocks * col_tile + 1u;
-  job.nblk = kBlocks == 2u && job.blk1 < out_plane / 128u ? 2u : 1u;
+  job.blk = col_tile;
   job.row0 = item.first;
   job.rows = item.count;
+  job.box = kBoxRows;
+  const Core c = core_setup(smem_raw, job, kWhole);
   const uint64_t trellis_bytes = static_cast<uint64_t>(in) * out_plane * slot.k2 / 16u;
   const uint16_t *svh = reinterpret_cast<const uint16_t *>(static_cast<const uint8_t *>(slot.record) + trellis_bytes) + in;
   const float *inv_rows = reinterpret_cast<const float *>(PHASE == 0 ? p.scale_in : p.scale_h);
-  const bool decoded = core_roles<DW>(c, job, &map_a, p.status + 1);   // word 1 of the status line: waits of this kernel that ran out
-  if (c.warp < DW) {
-    // One row tile: (block, half of its columns) per warp group, all groups at work. Two row
-    // tiles: (row tile, block) per group. What the epilogue needs from global memory is asked for
-    // here, before the wait for the accumulator: the loads travel while the last MMAs retire.
-    const uint32_t tiles = job.rows > 128u ? 2u : 1u, items = tiles * job.nblk;
-    const uint32_t group = static_cast<uint32_t>(c.warp) >> 2, quad = static_cast<uint32_t>(c.warp) & 3u;
-    const uint32_t lane = static_cast<uint32_t>(c.lane);
-    const bool split = tiles == 1u;
-    const uint32_t tt = split ? 0u : group / job.nblk, cb = split ? group % kBlocks : group % job.nblk;
-    const uint32_t half = group / kBlocks;   // split jobs: which 64 columns of the block
-    const bool live = split ? cb < job.nblk : group < items;
-    const uint32_t first = tt * 128u + quad * 32u;                         // the warp's first row of the item
-    const uint32_t rows = !live || item.count <= first ? 0u : (item.count - first < 32u ? item.count - first : 32u);
-    const bool valid = lane < rows;
-    const uint32_t row = item.first + first + (valid ? lane : 0u);
-    const uint32_t col0 = (cb == 0u ? job.blk0 : job.blk1) * 128u;
-    const float inv = valid ? inv_rows[row] : 0.0f;
-    // the lane's own row (PHASE 1): which assignment (token, rank) it is and its routing weight
-    const uint32_t my_a = PHASE == 1 && valid ? p.sorted[row] : 0u;
-    const float my_weight = PHASE == 1 && valid ? p.weights[my_a] : 0.0f;
-    const uint32_t col = 4u * (lane & 15u);
-    float4 sv[2];   // svh of the columns a lane writes: 64 pass + 4 (lane % 16) .. + 3
-#pragma unroll
-    for (int ps = 0; ps < 2; ++ps) sv[ps] = live ? four_halves(svh + col0 + 64u * ps + col) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (core_accumulator<DW>(c, decoded, p.status + 1) && (split || live)) {
-      float *areas = reinterpret_cast<float *>(smem_raw + (c.base - smem_u32(smem_raw)));
-      float *mine = areas + group * kArea;
-      const float *other = areas + (group ^ kBlocks) * kArea;
-      const uint32_t taddr = c.tmem + ((quad * 32u) << 16) + tt * kCols + cb * 128u;
-      if (PHASE == 0) {
-        float *out = p.gu + static_cast<size_t>(item.first + first) * 2u * p.inter + col0 + col;
-        auto emit = [&](uint32_t ps, uint32_t r, bool there, const float4 &v) {
-          if (there) {
-            *reinterpret_cast<float4 *>(out + static_cast<size_t>(r) * 2u * p.inter + 64u * ps) =
-                make_float4(v.x * sv[ps].x, v.y * sv[ps].y, v.z * sv[ps].z, v.w * sv[ps].w);
-          }
-        };
-        if (split) half_epilogue<DW>(taddr, half, live, inv, valid, mine, other, quad, lane, rows, kWhole, emit);
-        else block_epilogue(taddr, inv, valid, mine, quad, lane, rows, kWhole, emit);
-      } else {
-        auto emit = [&](uint32_t ps, uint32_t r, bool there, const float4 &v) {   // the row's assignment and weight, handed round by shuffle
-          const uint32_t a = __shfl_sync(0xFFFFFFFFu, my_a, static_cast<int>(r));
-          const float wr = __shfl_sync(0xFFFFFFFFu, my_weight, static_cast<int>(r));
-          if (there) {
-            *reinterpret_cast<float4 *>(p.down_rows + static_cast<size_t>(a) * p.hidden + col0 + 64u * ps + col) =
-                make_float4(wr * (v.x * sv[ps].x), wr * (v.y * sv[ps].y), wr * (v.z * sv[ps].z), wr * (v.w * sv[ps].w));
-          }
-        };
-        if (split) half_epilogue<DW>(taddr, half, live, inv, valid, mine, other, quad, lane, rows, kWhole, emit);
-        else block_epilogue(taddr, inv, valid, mine, quad, lane, rows, kWhole, emit);
-      }
-    }
-  }
-  core_finish<DW>(c);
+  const bool decoded = core_roles(c, job, &map_rows, p.status + 1);   // word 1 of the status line: waits of this kernel that ran out
+  const uint32_t col = col_tile * 128u + 4u * static_cast<uint32_t>(c.lane);
+  const float4 sv = four_halves(svh + col);
+  struct Choice {
+    uint32_t a;     // PHASE 1: which assignment (token, rank) the row is, and its routing weight
+    float weight;
+  };
+  core_finish_rows(
+      c, job, kWhole, decoded, p.status + 1, [&](uint32_t r) { return inv_rows[item.first + r]; },
+      [&](uint32_t r) {
+        Choice choice = {item.first + r, 1.0f};
+        if (PHASE == 1) {
+          choice.a = p.sorted[item.first + r];
+          choice.weight = p.weights[choice.a];
+        }
+        return choice;
+      },
+      [&](uint32_t, const Choice &choice, const float4 &v) {
+        float *dst = PHASE == 0 ? p.gu + static_cast<size_t>(choice.a) * 2u * p.inter + col : p.down_rows + static_cast<size_t>(choice.a) * p.hidden + col;
+        float4 o = make_float4(v.x * sv.x, v.y * sv.y, v.z * sv.z, v.w * sv.w);
+        if (PHASE == 1) o = make_float4(choice.weight * o.x, choice.weight * o.y, choice.weight * o.z, choice.weight * o.w);
+        *reinterpret_cast<float4 *>(dst) = o;
+      });
 }
 
 // One CTA per token: the token's weighted down products (one row per choice that had an expert with a
@@ -256,26 +223,11 @@ __global__ void __launch_bounds__(256) moe_tc_fold_kernel(const __grid_constant_
 
 constexpr size_t kRotateSmemMax = 200 * 1024;
 
-template <int DW>
-cudaError_t set_gemm_attrs() {
-  cudaError_t err = cudaFuncSetAttribute(moe_tc_gemm_kernel<0, DW>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Shape<DW>::kSmemBytes));
-  if (err == cudaSuccess) err = cudaFuncSetAttribute(moe_tc_gemm_kernel<1, DW>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Shape<DW>::kSmemBytes));
-  return err;
-}
-
-template <int DW>
-cudaError_t launch_gemm(int phase, uint32_t items_max, uint32_t out_plane, cudaStream_t stream, bool pdl, const CUtensorMap &map_a, const ExpertParams &p) {
-  const uint32_t col_tiles = (out_plane + Shape<DW>::kCols - 1u) / Shape<DW>::kCols;
-  const dim3 grid(items_max * col_tiles);
-  return phase == 0 ? launch(moe_tc_gemm_kernel<0, DW>, grid, dim3(Shape<DW>::kThreads), Shape<DW>::kSmemBytes, stream, pdl, map_a, p)
-                    : launch(moe_tc_gemm_kernel<1, DW>, grid, dim3(Shape<DW>::kThreads), Shape<DW>::kSmemBytes, stream, pdl, map_a, p);
-}
-
 }  // namespace
 
 int32_t moe_tc_prepare(ErrorSlot &slot) {
-  cudaError_t err = set_gemm_attrs<16>();
-  if (err == cudaSuccess) err = set_gemm_attrs<8>();
+  cudaError_t err = cudaFuncSetAttribute(moe_tc_gemm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemBytes));
+  if (err == cudaSuccess) err = cudaFuncSetAttribute(moe_tc_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemBytes));
   if (err == cudaSuccess) err = cudaFuncSetAttribute(moe_tc_rotate_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRotateSmemMax));
   if (err == cudaSuccess) err = cudaFuncSetAttribute(moe_tc_rotate_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRotateSmemMax));
   if (err != cudaSuccess) return fail(slot, "MoE tensor-core kernel attributes: %s", cudaGetErrorString(err));
@@ -295,12 +247,13 @@ int32_t moe_tc_experts(ErrorSlot &slot, const DeviceState &dev, const ExpertPara
     cudaError_t err = phase == 0 ? launch(moe_tc_rotate_kernel<0>, dim3(rows), dim3(kRotateThreads), static_cast<size_t>(in) * 4u, stream, pdl, p, offsets)
                                  : launch(moe_tc_rotate_kernel<1>, dim3(rows), dim3(kRotateThreads), static_cast<size_t>(in) * 4u, stream, pdl, p, offsets);
     if (err != cudaSuccess) return fail(slot, "%s: rotation launch failed: %s", what, cudaGetErrorString(err));
-    CUtensorMap map_a;
-    if (!make_rows_map(&map_a, phase == 0 ? static_cast<const void *>(p.frag_in) : static_cast<const void *>(p.frag_h), rows, in)) {
+    CUtensorMap map_rows;
+    if (!make_rows_map(&map_rows, phase == 0 ? static_cast<const void *>(p.frag_in) : static_cast<const void *>(p.frag_h), rows, in, kBoxRows)) {
       return fail(slot, "%s: tensor map encoding failed", what);
     }
-    // 8 decoder warps and two CTAs per SM unless B200Q_MOE_TC_WIDE is set
-    err = dev.moe_dw == 16 ? launch_gemm<16>(phase, items_max, out_plane, stream, pdl, map_a, p) : launch_gemm<8>(phase, items_max, out_plane, stream, pdl, map_a, p);
+    const dim3 grid(items_max * (out_plane / 128u));
+    err = phase == 0 ? launch(moe_tc_gemm_kernel<0>, grid, dim3(kThreads), kSmemBytes, stream, pdl, map_rows, p)
+                     : launch(moe_tc_gemm_kernel<1>, grid, dim3(kThreads), kSmemBytes, stream, pdl, map_rows, p);
     if (err != cudaSuccess) return fail(slot, "%s: expert launch failed: %s", what, cudaGetErrorString(err));
   }
   const cudaError_t err = launch(moe_tc_fold_kernel, dim3(tokens), dim3(256), 0, stream, pdl, p, tokens);

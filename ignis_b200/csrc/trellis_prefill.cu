@@ -80,85 +80,48 @@ struct DenseParams {
   const float *inv;      // the tokens' inverse scales
   uint16_t *y;           // BF16 [tokens][ldy]
   uint32_t k2, tile_stride, in, out, tokens, ldy, epilogue;
+  uint32_t tile;         // tokens per CTA
   uint32_t ranks;        // the CTAs of a cluster share an item's K stages (1: no cluster)
 };
 
-// DW: the core's shape - 16 (256 columns a CTA, one CTA per SM) or 8 (128 columns, two per SM).
-template <int DW>
-__global__ void __launch_bounds__(Shape<DW>::kThreads, DW == 16 ? 1 : 2) trellis_tc_dense_kernel(const __grid_constant__ CUtensorMap map_a,
-                                                                                              const __grid_constant__ DenseParams p) {
-  constexpr int kDenseDw = DW;
-  constexpr uint32_t kCols = Shape<DW>::kCols, kBlocks = Shape<DW>::kBlocks;
+__global__ void __launch_bounds__(kThreads, 2) trellis_tc_dense_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ DenseParams p) {
   extern __shared__ uint8_t smem_raw[];
-  const Core c = core_setup<kDenseDw>(smem_raw);
   // Token tiles run fastest over the grid, so the CTAs at work at one time decode the same columns
   // of the plane (read from HBM once, then from the L2).
-  const uint32_t row_tiles = (p.tokens + 255u) / 256u;
-  const Split split_k = {p.ranks, p.ranks == 1u ? 0u : cluster_ctarank()};
-  const uint32_t item = blockIdx.x / p.ranks, col_tile = item / row_tiles, row_tile = item % row_tiles;
+  const uint32_t row_tiles = (p.tokens + p.tile - 1u) / p.tile;
+  const Split split = {p.ranks, p.ranks == 1u ? 0u : cluster_ctarank()};
+  const uint32_t item = blockIdx.x / p.ranks;
   Job job;
   job.trellis = p.trellis;
   job.k2 = p.k2;
   job.tile_stride = p.tile_stride;
   const uint32_t stages = p.in / 64u;
-  job.stage0 = stages * split_k.rank / p.ranks;
-  job.stage1 = stages * (split_k.rank + 1u) / p.ranks;
-  job.blk0 = kBlocks * col_tile;
-  job.blk1 = kBlocks * col_tile + 1u;
-  job.nblk = kBlocks == 2u && job.blk1 < p.out / 128u ? 2u : 1u;
-  job.row0 = row_tile * 256u;
-  job.rows = p.tokens - job.row0 < 256u ? p.tokens - job.row0 : 256u;
-  const bool decoded = core_roles<kDenseDw>(c, job, &map_a, &g_trellis_tc_status);
-  if (c.warp < kDenseDw) {
-    // Two row tiles: the (row tile, block) items go to the groups of four warps. One: a group takes
-    // half a block's columns, so that all groups are at work. A warp's lanes are the rows
-    // 32 (warp % 4) .. + 31 of the row tile. What the epilogue needs from global memory is asked
-    // for before the wait for the accumulator, while the last MMAs retire.
-    const uint32_t tiles = job.rows > 128u ? 2u : 1u, items = tiles * job.nblk;
-    const uint32_t group = static_cast<uint32_t>(c.warp) >> 2, quad = static_cast<uint32_t>(c.warp) & 3u;
-    const uint32_t lane = static_cast<uint32_t>(c.lane);
-    const bool split = tiles == 1u;
-    const uint32_t tt = split ? 0u : group / job.nblk, cb = split ? group % kBlocks : group % job.nblk;
-    const uint32_t half = group / kBlocks;   // split jobs: which 64 columns of the block
-    const bool live = split ? cb < job.nblk : group < items;
-    const uint32_t first = tt * 128u + quad * 32u;   // the warp's first row of the job
-    const uint32_t rows = !live || job.rows <= first ? 0u : (job.rows - first < 32u ? job.rows - first : 32u);
-    const bool valid = lane < rows;
-    const uint32_t token0 = job.row0 + first;
-    const uint32_t col0 = (cb == 0u ? job.blk0 : job.blk1) * 128u;
-    const float inv = valid ? p.inv[token0 + lane] : 0.0f;
-    const uint32_t col = 4u * (lane & 15u);
-    float4 sv[2];   // svh of the columns a lane writes: 64 pass + 4 (lane % 16) .. + 3
-#pragma unroll
-    for (int ps = 0; ps < 2; ++ps) sv[ps] = live ? four_halves(p.svh + col0 + 64u * ps + col) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (core_accumulator<kDenseDw>(c, decoded, &g_trellis_tc_status) && (split || live)) {
-      float *areas = reinterpret_cast<float *>(smem_raw + (c.base - smem_u32(smem_raw)));
-      uint16_t *out = p.y + static_cast<size_t>(token0) * p.ldy + col0 + col;
-      auto emit = [&](uint32_t ps, uint32_t r, bool there, const float4 &o) {
-        if (!there) return;
-        uint2 *dst = reinterpret_cast<uint2 *>(out + static_cast<size_t>(r) * p.ldy + 64u * ps);
-        float v[4] = {o.x * sv[ps].x, o.y * sv[ps].y, o.z * sv[ps].z, o.w * sv[ps].w};
+  job.stage0 = stages * split.rank / p.ranks;
+  job.stage1 = stages * (split.rank + 1u) / p.ranks;
+  job.blk = item / row_tiles;
+  job.row0 = item % row_tiles * p.tile;
+  job.rows = min(p.tokens - job.row0, p.tile);
+  job.box = p.tile;
+  const Core c = core_setup(smem_raw, job, split);
+  const bool decoded = core_roles(c, job, &map_rows, &g_trellis_tc_status);
+  const uint32_t col = job.blk * 128u + 4u * static_cast<uint32_t>(c.lane);
+  const float4 sv = four_halves(p.svh + col);
+  uint16_t *out = p.y + static_cast<size_t>(job.row0) * p.ldy + col;
+  core_finish_rows(
+      c, job, split, decoded, &g_trellis_tc_status, [&](uint32_t r) { return p.inv[job.row0 + r]; },
+      [&](uint32_t r) { return p.epilogue != kEpiStore ? *reinterpret_cast<const uint2 *>(out + static_cast<size_t>(r) * p.ldy) : make_uint2(0u, 0u); },
+      [&](uint32_t r, const uint2 &old, const float4 &o) {
+        float v[4] = {o.x * sv.x, o.y * sv.y, o.z * sv.z, o.w * sv.w};
         if (p.epilogue != kEpiStore) {
-          const uint2 old = *dst;
           const float was[4] = {bf16_bits_to_f32(old.x & 0xFFFFu), __uint_as_float(old.x & 0xFFFF0000u), bf16_bits_to_f32(old.y & 0xFFFFu),
                                 __uint_as_float(old.y & 0xFFFF0000u)};
 #pragma unroll
           for (int e = 0; e < 4; ++e) v[e] = p.epilogue == kEpiAdd ? v[e] + was[e] : was[e] / (1.0f + __expf(-was[e])) * v[e];
         }
         const __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
-        *dst = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
-      };
-      const uint32_t taddr = c.tmem + ((quad * 32u) << 16) + tt * kCols + cb * 128u;
-      float *mine = areas + group * kArea;
-      if (split) half_epilogue<kDenseDw>(taddr, half, live, inv, valid, mine, areas + (group ^ kBlocks) * kArea, quad, lane, rows, split_k, emit);
-      else block_epilogue(taddr, inv, valid, mine, quad, lane, rows, split_k, emit);
-    } else {
-      split_meetings(split_k, tiles);
-    }
-  } else {
-    split_meetings(split_k, job.rows > 128u ? 2u : 1u);
-  }
-  core_finish<kDenseDw>(c);
+        *reinterpret_cast<uint2 *>(out + static_cast<size_t>(r) * p.ldy) =
+            make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
+      });
 }
 
 uint64_t align256(uint64_t v) { return (v + 255u) & ~static_cast<uint64_t>(255u); }
@@ -174,19 +137,15 @@ uint64_t trellis_tc_workspace_bytes(uint32_t in, uint32_t weights, uint32_t toke
   return 256u + static_cast<uint64_t>(weights) * (align256(static_cast<uint64_t>(tokens) * in * 2u) + align256(static_cast<uint64_t>(tokens) * 4u));
 }
 
-// Which shape a dense product takes: the narrow one (8 decoder warps, two CTAs per SM), which
-// measured faster at 256, 1024 and 4096 tokens (a decoded tile serves 256 tokens in both, and the
-// narrow CTAs overlap each other's fill, drain and epilogue); B200Q_TRELLIS_TC_SHAPE = 16 selects
-// the wide one (DeviceState::trellis_dw).
 namespace {
-// The CTAs of a cluster that share the K stages of an item (the narrow shape).
+// The CTAs of a cluster that share the K stages of an item.
 constexpr uint32_t kMaxRanks = 8;
 
 cudaLaunchConfig_t dense_config(uint32_t items, uint32_t ranks, cudaStream_t stream, bool pdl, cudaLaunchAttribute (&attr)[2]) {
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(items * ranks);
-  config.blockDim = dim3(Shape<8>::kThreads);
-  config.dynamicSmemBytes = Shape<8>::kSmemBytes;
+  config.blockDim = dim3(kThreads);
+  config.dynamicSmemBytes = kSmemBytes;
   config.stream = stream;
   unsigned n = 0;
   if (pdl) {
@@ -232,8 +191,7 @@ uint32_t dense_ranks(const DeviceState &dev, uint32_t items, uint32_t stages, ui
 int32_t trellis_tc_prepare(ErrorSlot &slot) {
   DeviceState *dev = device_state(slot);
   if (dev == nullptr) return -1;
-  cudaError_t err = cudaFuncSetAttribute(trellis_tc_dense_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Shape<16>::kSmemBytes));
-  if (err == cudaSuccess) err = cudaFuncSetAttribute(trellis_tc_dense_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Shape<8>::kSmemBytes));
+  cudaError_t err = cudaFuncSetAttribute(trellis_tc_dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemBytes));
   if (err == cudaSuccess) {
     err = cudaFuncSetAttribute(trellis_rotate_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRotateMaxSmem));
   }
@@ -242,7 +200,7 @@ int32_t trellis_tc_prepare(ErrorSlot &slot) {
     cudaLaunchAttribute attr[2];
     const cudaLaunchConfig_t config = dense_config(1u, ranks, nullptr, false, attr);
     int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, trellis_tc_dense_kernel<8>, &config) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&clusters, trellis_tc_dense_kernel, &config) != cudaSuccess) {
       (void)cudaGetLastError();
       clusters = 0;
     }
@@ -267,8 +225,10 @@ int32_t one_product(ErrorSlot &slot, const DeviceState &dev, const ignis_trellis
   cudaError_t err = launch(trellis_rotate_rows_kernel, dim3(tokens), dim3(256), static_cast<size_t>(w->in) * 4u, stream, dev.pdl != 0, x,
                            static_cast<const uint16_t *>(w->suh), w->in, rows, inv);
   if (err != cudaSuccess) return fail(slot, "%s: rotation launch failed: %s", what, cudaGetErrorString(err));
-  CUtensorMap map_a;
-  if (!make_rows_map(&map_a, rows, tokens, w->in)) return fail(slot, "%s: tensor map encoding failed", what);
+  const uint32_t row_tiles = (tokens + kMaxRows - 1u) / kMaxRows;
+  CUtensorMap map_rows;
+  const uint32_t tile = ((tokens + row_tiles - 1u) / row_tiles + 15u) / 16u * 16u;
+  if (!make_rows_map(&map_rows, rows, tokens, w->in, tile)) return fail(slot, "%s: tensor map encoding failed", what);
   DenseParams p = {};
   p.trellis = static_cast<const uint32_t *>(w->trellis);
   p.svh = static_cast<const uint16_t *>(w->svh);
@@ -281,18 +241,12 @@ int32_t one_product(ErrorSlot &slot, const DeviceState &dev, const ignis_trellis
   p.tokens = tokens;
   p.ldy = ldy;
   p.epilogue = epilogue;
-  const uint32_t row_tiles = (tokens + 255u) / 256u;
-  if (dev.trellis_dw == 16) {
-    p.ranks = 1u;
-    err = launch(trellis_tc_dense_kernel<16>, dim3((w->out + 255u) / 256u * row_tiles), dim3(Shape<16>::kThreads), Shape<16>::kSmemBytes, stream,
-                 dev.pdl != 0, map_a, p);
-  } else {
-    const uint32_t items = w->out / 128u * row_tiles;
-    p.ranks = dense_ranks(dev, items, w->in / 64u, tokens > 128u ? 2u : 1u);
-    cudaLaunchAttribute attr[2];
-    cudaLaunchConfig_t config = dense_config(items, p.ranks, stream, dev.pdl != 0, attr);
-    err = cudaLaunchKernelEx(&config, trellis_tc_dense_kernel<8>, map_a, p);
-  }
+  p.tile = tile;
+  const uint32_t items = w->out / 128u * ((tokens + p.tile - 1u) / p.tile);
+  p.ranks = dense_ranks(dev, items, w->in / 64u, p.tile > 128u ? 2u : 1u);
+  cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t config = dense_config(items, p.ranks, stream, dev.pdl != 0, attr);
+  err = cudaLaunchKernelEx(&config, trellis_tc_dense_kernel, map_rows, p);
   if (err != cudaSuccess) return fail(slot, "%s: launch failed: %s", what, cudaGetErrorString(err));
   return 0;
 }
