@@ -84,8 +84,18 @@ Layout layout_for(const Geometry &g, uint32_t tokens_max) {
 }
 
 // ---- grouping ------------------------------------------------------------------------------
+// A CTA counts in shared memory and adds its counts to the experts' once (`in_shared`: up to kSmallExperts of them): added one
+// by one, a popular expert's rows queue at one address (13 us for 40 960 rows under Zipf routing).
+constexpr uint32_t kSmallRows = 4096, kSmallExperts = 4096;
+
 __global__ void __launch_bounds__(256) moe_count_kernel(const int32_t *ids, uint32_t rows, uint32_t experts,
                                                         uint32_t *counts, uint32_t *status) {
+  __shared__ uint32_t mine[kSmallExperts];
+  const bool in_shared = experts <= kSmallExperts;
+  if (in_shared) {
+    for (uint32_t e = threadIdx.x; e < experts; e += blockDim.x) mine[e] = 0u;
+    __syncthreads();
+  }
   griddep_launch_dependents();
   griddep_wait();
   for (uint32_t a = blockIdx.x * blockDim.x + threadIdx.x; a < rows; a += gridDim.x * blockDim.x) {
@@ -93,12 +103,18 @@ __global__ void __launch_bounds__(256) moe_count_kernel(const int32_t *ids, uint
     if (e < 0 || static_cast<uint32_t>(e) >= experts) {
       if (e != IGNIS_MOE_NO_EXPERT) atomicOr(status, kStatusBadExpert);  // -1 is "no expert for this choice": skipped, not an error
     } else {
-      atomicAdd(&counts[e], 1u);
+      atomicAdd(in_shared ? &mine[e] : &counts[e], 1u);
     }
+  }
+  if (!in_shared) return;
+  __syncthreads();
+  for (uint32_t e = threadIdx.x; e < experts; e += blockDim.x) {
+    if (mine[e] != 0u) atomicAdd(&counts[e], mine[e]);
   }
 }
 
-// One CTA: exclusive scans of the per-expert row, item and tile counts, then the item and tile lists.
+// One CTA: exclusive scans of the per-expert row, item and tile counts, then the item and tile lists (`tiles` nullptr: no tile
+// list - the tensor-core route has none, and a popular expert's tiles, written by one thread, took 15 of 24 us).
 __global__ void __launch_bounds__(1024) moe_scan_kernel(const uint32_t *counts, uint32_t experts, uint32_t item_rows,
                                                         uint32_t *offsets, uint32_t *n_items, Item *items, Tile *tiles) {
   griddep_launch_dependents();
@@ -133,7 +149,7 @@ __global__ void __launch_bounds__(1024) moe_scan_kernel(const uint32_t *counts, 
     for (uint32_t j = 0; j < c; j += item_rows) {
       items[item_at++] = Item{e, row_at + j, c - j < item_rows ? c - j : item_rows, tile_at + j / 8u};
     }
-    for (uint32_t j = 0; j < c; j += 8) tiles[tile_at++] = Tile{e, row_at + j, c - j < 8u ? c - j : 8u, 0u};
+    for (uint32_t j = 0; tiles != nullptr && j < c; j += 8) tiles[tile_at++] = Tile{e, row_at + j, c - j < 8u ? c - j : 8u, 0u};
     row_at += c;
   }
   if (threadIdx.x == 1023) {
@@ -143,23 +159,41 @@ __global__ void __launch_bounds__(1024) moe_scan_kernel(const uint32_t *counts, 
   }
 }
 
+// The rows of one expert are independent of each other, so their order inside the group does not change any output bit. A
+// CTA's rows of an expert take their places together, as they were counted.
 __global__ void __launch_bounds__(256) moe_scatter_kernel(const int32_t *ids, uint32_t rows, uint32_t experts,
                                                           const uint32_t *offsets, uint32_t *cursor, uint32_t *sorted) {
+  __shared__ uint32_t mine[kSmallExperts];   // rows of the CTA, then their first place
+  const bool in_shared = experts <= kSmallExperts;
+  if (in_shared) {
+    for (uint32_t e = threadIdx.x; e < experts; e += blockDim.x) mine[e] = 0u;
+    __syncthreads();
+  }
   griddep_launch_dependents();
   griddep_wait();
-  for (uint32_t a = blockIdx.x * blockDim.x + threadIdx.x; a < rows; a += gridDim.x * blockDim.x) {
-    const int32_t e = ids[a];
-    if (e < 0 || static_cast<uint32_t>(e) >= experts) continue;
-    // rows of one expert are independent of each other, so their order inside the group does
-    // not change any output bit
-    sorted[offsets[e] + atomicAdd(&cursor[e], 1u)] = a;
+  for (uint32_t a0 = blockIdx.x * blockDim.x; a0 < rows; a0 += gridDim.x * blockDim.x) {
+    const uint32_t a = a0 + threadIdx.x;
+    const int32_t e = a < rows ? ids[a] : -1;
+    const bool there = e >= 0 && static_cast<uint32_t>(e) < experts;
+    if (!in_shared) {
+      if (there) sorted[offsets[e] + atomicAdd(&cursor[e], 1u)] = a;
+      continue;
+    }
+    const uint32_t rank = there ? atomicAdd(&mine[e], 1u) : 0u;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < experts; i += blockDim.x) {
+      if (mine[i] != 0u) mine[i] = offsets[i] + atomicAdd(&cursor[i], mine[i]);
+    }
+    __syncthreads();
+    if (there) sorted[mine[e] + rank] = a;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < experts; i += blockDim.x) mine[i] = 0u;
+    __syncthreads();
   }
 }
 
 // Count, scan and scatter in one CTA for calls of a few rows (the decode widths): the three launches
 // above cost more than their work there. Counts and cursors live in shared memory.
-constexpr uint32_t kSmallRows = 4096, kSmallExperts = 4096;
-
 __global__ void __launch_bounds__(1024) moe_group_small_kernel(const int32_t *ids, uint32_t rows, uint32_t experts, uint32_t item_rows,
                                                                uint32_t *offsets, uint32_t *n_items, Item *items, Tile *tiles,
                                                                uint32_t *sorted, uint32_t *status) {
@@ -208,7 +242,7 @@ __global__ void __launch_bounds__(1024) moe_group_small_kernel(const int32_t *id
     for (uint32_t j = 0; j < c; j += item_rows) {
       items[item_at++] = Item{e, row_at + j, c - j < item_rows ? c - j : item_rows, tile_at + j / 8u};
     }
-    for (uint32_t j = 0; j < c; j += 8) tiles[tile_at++] = Tile{e, row_at + j, c - j < 8u ? c - j : 8u, 0u};
+    for (uint32_t j = 0; tiles != nullptr && j < c; j += 8) tiles[tile_at++] = Tile{e, row_at + j, c - j < 8u ? c - j : 8u, 0u};
     row_at += c;
   }
   if (threadIdx.x == 1023) {
@@ -627,17 +661,18 @@ int32_t run_experts(const Geometry &g, const void *x, uint32_t tokens, const int
   Item *items = reinterpret_cast<Item *>(base + l.items);
   uint32_t *status = reinterpret_cast<uint32_t *>(base + l.status);
   const bool pdl = dev->pdl != 0;
+  Tile *tiles = item_rows == kMoeTcItemRows ? nullptr : reinterpret_cast<Tile *>(base + l.tiles);
   cudaError_t err = cudaSuccess;
   if (rows <= kSmallRows && g.experts <= kSmallExperts) {
     err = launch(moe_group_small_kernel, dim3(1), dim3(1024), 0, stream, false, ids, rows, g.experts, item_rows, offsets, n_items, items,
-                 reinterpret_cast<Tile *>(base + l.tiles), sorted, status);
+                 tiles, sorted, status);
     if (err != cudaSuccess) return fail(slot, "%s: grouping launch failed: %s", what, cudaGetErrorString(err));
   } else {
   err = cudaMemsetAsync(counts, 0, l.offsets - l.counts, stream);  // counts and cursor
   if (err != cudaSuccess) return fail(slot, "%s: %s", what, cudaGetErrorString(err));
   const uint32_t grid_rows = (rows + 255u) / 256u < 1184u ? (rows + 255u) / 256u : 1184u;
   err = launch(moe_count_kernel, dim3(grid_rows), dim3(256), 0, stream, false, ids, rows, g.experts, counts, status);
-  if (err == cudaSuccess) err = launch(moe_scan_kernel, dim3(1), dim3(1024), 0, stream, pdl, static_cast<const uint32_t *>(counts), g.experts, item_rows, offsets, n_items, items, reinterpret_cast<Tile *>(base + l.tiles));
+  if (err == cudaSuccess) err = launch(moe_scan_kernel, dim3(1), dim3(1024), 0, stream, pdl, static_cast<const uint32_t *>(counts), g.experts, item_rows, offsets, n_items, items, tiles);
   if (err == cudaSuccess) err = launch(moe_scatter_kernel, dim3(grid_rows), dim3(256), 0, stream, pdl, ids, rows, g.experts, static_cast<const uint32_t *>(offsets), cursor, sorted);
   if (err != cudaSuccess) return fail(slot, "%s: grouping launch failed: %s", what, cudaGetErrorString(err));
   }
@@ -666,7 +701,7 @@ int32_t run_experts(const Geometry &g, const void *x, uint32_t tokens, const int
   // Grids are sized for the worst case the host can know (the grouping happened on the device);
   // CTAs beyond the item or tile count return at once.
   const uint32_t items_max = items_bound(g, rows, item_rows);
-  if (item_rows == kMoeTcItemRows) {   // the tensor-core route: items of up to 256 rows
+  if (item_rows == kMoeTcItemRows) {   // the tensor-core route
     return moe_tc_experts(slot, *dev, p, rows, items_max, offsets, stream, what);
   }
   const uint32_t tiles_max = items_bound(g, rows, 8u);
@@ -815,7 +850,7 @@ int32_t b200q_moe_experts_prefill(const b200q_moe_geometry *geometry, const void
   if (check_geometry(moe_error(), geometry, "ignis_moe_experts_prefill") != 0) return -1;
   const uint32_t limit = workspace != nullptr ? workspace->prefill_tokens : 0u;
   // up to 8 tokens the decode entry's item size; up to 64 tokens items of 64 rows on the warp-level
-  // MMAs; beyond, items of 256 rows on the tensor cores (B200Q_MOE_TC = 0 keeps the warp-level kernels)
+  // MMAs; beyond, items of 192 rows on the tensor cores (B200Q_MOE_TC = 0 keeps the warp-level kernels)
   const DeviceState *dev = device_state(moe_error());
   const bool tc = dev != nullptr && dev->prepared && dev->moe_tc != 0 && tokens > 64u;
   return run_experts(*geometry, x, tokens, ids, weights, slots, workspace, acc, stream, limit, tokens > 8u ? (tc ? kMoeTcItemRows : 64u) : 8u,
