@@ -2,15 +2,15 @@
 //
 // Stands where the reference's prefill entry multiplies items of up to 64 rows with warp-level MMAs
 // (kernel/src/moe_prefill.cu:252-262, kernels :405 and :421). Under skewed routing a few experts see
-// hundreds of rows; here a work item is up to 256 sorted rows of one expert, and every item is
+// hundreds of rows; here a work item is up to 192 sorted rows of one expert, and every item is
 // multiplied with its expert's record by the kernel core of trellis_tc.cuh: the rows rotated once
-// into plain fp16 rows with one scale per row, the record's trellis tiles decoded into swizzled
-// shared memory, tcgen05.mma kind::f16 with the accumulator in tensor memory, and the output
-// Hadamard in registers. Five launches behind the grouping:
+// into plain fp16 rows with one scale per row, the record's trellis tiles decoded into
+// tensor memory, tcgen05.mma kind::f16 with the accumulator beside them, and the output
+// Hadamard in the epilogue. Five launches behind the grouping:
 //
-//   moe_tc_rotate_kernel<0>   x o suh (the row's expert's gate|up record), Hadamard, fp16 rows
+//   moe_tc_rotate_x_kernel    x o suh (the row's expert's gate|up record), Hadamard, fp16 rows
 //   moe_tc_gemm_kernel<0>     rows x gate|up record -> gu fp32 [row][2 inter] (gate columns, then up)
-//   moe_tc_rotate_kernel<1>   silu(g) u o suh (the down record), Hadamard, fp16 rows
+//   moe_tc_rotate_h_kernel    silu(g) u o suh (the down record), Hadamard, fp16 rows
 //   moe_tc_gemm_kernel<1>     rows x down record, times the routing weight -> fp32 [token][rank][hidden]
 //   moe_tc_fold_kernel        a token's products as 2^-32 fixed-point integers, summed, added to the
 //                             token's int64 accumulator row (84 M atomic additions into the
@@ -25,18 +25,59 @@ namespace b200q {
 namespace {
 
 using namespace trellis_tc;
+static_assert(kMoeTcItemRows == Shape<2>::kMaxRows, "an item is what a CTA takes");
 
+// The sorted rows' activations (rotate_row, trellis_device.cuh), a CTA going from row to row: the token's `hidden` values times the
+// expert's suh, the 128-wide Hadamard per block, one power-of-two scale per row, fp16. A lane holds 32 values, so that five of
+// the seven Hadamard stages are additions of two values an instruction. (Four values a lane: 102 us for 40 960 rows of 2048 inputs
+// against 77.) THREADS: the most a launch has.
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) moe_tc_rotate_x_kernel(const __grid_constant__ ExpertParams p, const uint32_t *offsets) {
+  __shared__ float warp_max[2][32];
+  griddep_launch_dependents();
+  griddep_wait();
+  const uint32_t in = p.hidden;
+  const uint32_t rows = offsets[p.experts];   // fewer than the launch may have been sized for
+  float *const inv = reinterpret_cast<float *>(p.scale_in);
+  struct Source {
+    uint32_t a;
+    ignis_moe_slot slot;
+  };
+  auto source = [&](uint32_t row) {   // four loads that depend on one another: for the next row while this one is transformed
+    Source s = {};
+    if (row < rows) {
+      s.a = p.sorted[row];
+      s.slot = p.slots[static_cast<uint32_t>(p.ids[s.a]) * 2u];
+    }
+    return s;
+  };
+  Source here = source(blockIdx.x);
+  for (uint32_t row = blockIdx.x, turn = 0; row < rows; row += gridDim.x, turn ^= 1u) {
+    const Source next = source(row + gridDim.x);
+    const ignis_moe_slot slot = here.slot;
+    uint16_t *const to = reinterpret_cast<uint16_t *>(p.frag_in) + static_cast<size_t>(row) * in;
+    if (slot.record == nullptr || !(slot.k2 == 4 || slot.k2 == 5 || slot.k2 == 6 || slot.k2 == 8)) {
+      // an absent record: the product kernel flags it and skips the item; leave finite rows behind
+      for (uint32_t i = threadIdx.x * 4u; i < in; i += 4u * blockDim.x) *reinterpret_cast<uint2 *>(to + i) = make_uint2(0u, 0u);
+      if (threadIdx.x == 0) inv[row] = 0.0f;
+      __syncthreads();   // as a rotated row would: the turn after the next writes its maxima where the turn before wrote its own
+    } else {
+      const uint64_t trellis_bytes = static_cast<uint64_t>(in) * 2u * p.inter * slot.k2 / 16u;
+      const uint16_t *suh = reinterpret_cast<const uint16_t *>(static_cast<const uint8_t *>(slot.record) + trellis_bytes);
+      const uint16_t *x = p.x + static_cast<size_t>(here.a / p.top_k) * in;
+      rotate_row(in, to, inv + row, warp_max[turn],
+                 [&](uint32_t k, float2 (&v)[4]) { scaled_inputs(ldg128_coherent(x + k), __ldg(reinterpret_cast<const uint4 *>(suh + k)), v); });
+    }
+    here = next;
+  }
+}
+
+// silu(g) u of a sorted row's gate|up products, rotated for the down record: a CTA of two warps per row, a warp per 128-input
+// block, the row's values waiting in shared memory for its scale. Bound by the sigmoid and the division as much as by the
+// transform: 70 us for 40 960 rows of 768, where rotate_row takes 76 (a warp with a quarter of its lanes idle) and 108 from row
+// to row.
 constexpr uint32_t kRotateThreads = 64;
-
-// One CTA of two warps per sorted row: the row's `in` values times the expert's suh, the 128-wide
-// Hadamard per block (a warp per block), one power-of-two scale per row (largest magnitude in
-// [2^13, 2^14)), fp16. PHASE 0 reads the token's activations, PHASE 1 silu(g) u of the row's gate|up
-// products. The kernel is bound by instruction issue, and what every warp repeats for its row (the
-// walk to the expert's record, the row maximum, the scale) weighs as much as the transforms: hence
-// two warps a row (eight: 147 + 132 us for 40 960 rows of 2048 and 768 inputs; four: 106 + 91; two: a
-// further 1.4 % on the step), and the scale from the maximum's exponent bits.
-template <int PHASE>
-__global__ void __launch_bounds__(kRotateThreads) moe_tc_rotate_kernel(const __grid_constant__ ExpertParams p, const uint32_t *offsets) {
+__global__ void __launch_bounds__(kRotateThreads) moe_tc_rotate_h_kernel(const __grid_constant__ ExpertParams p, const uint32_t *offsets) {
   extern __shared__ __align__(16) float rot[];
   __shared__ float warp_max[kRotateThreads / 32];
   griddep_launch_dependents();
@@ -46,20 +87,18 @@ __global__ void __launch_bounds__(kRotateThreads) moe_tc_rotate_kernel(const __g
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t a = p.sorted[row];
   const uint32_t expert = static_cast<uint32_t>(p.ids[a]);
-  const ignis_moe_slot slot = p.slots[expert * 2u + PHASE];
-  const uint32_t in = PHASE == 0 ? p.hidden : p.inter;
-  uint16_t *dst = reinterpret_cast<uint16_t *>(PHASE == 0 ? p.frag_in : p.frag_h) + static_cast<size_t>(row) * in;
-  float *inv = reinterpret_cast<float *>(PHASE == 0 ? p.scale_in : p.scale_h) + row;
+  const ignis_moe_slot slot = p.slots[expert * 2u + 1u];
+  const uint32_t in = p.inter;
+  uint16_t *dst = reinterpret_cast<uint16_t *>(p.frag_h) + static_cast<size_t>(row) * in;
+  float *inv = reinterpret_cast<float *>(p.scale_h) + row;
   if (slot.record == nullptr || !(slot.k2 == 4 || slot.k2 == 5 || slot.k2 == 6 || slot.k2 == 8)) {
     // an absent record: the product kernel flags it and skips the item; leave finite rows behind
     for (uint32_t i = threadIdx.x * 4u; i < in; i += 4u * kRotateThreads) *reinterpret_cast<uint2 *>(dst + i) = make_uint2(0u, 0u);
     if (threadIdx.x == 0) *inv = 0.0f;
     return;
   }
-  const uint32_t out_plane = PHASE == 0 ? 2u * p.inter : p.hidden;
-  const uint64_t trellis_bytes = static_cast<uint64_t>(in) * out_plane * slot.k2 / 16u;
+  const uint64_t trellis_bytes = static_cast<uint64_t>(in) * p.hidden * slot.k2 / 16u;
   const uint16_t *suh = reinterpret_cast<const uint16_t *>(static_cast<const uint8_t *>(slot.record) + trellis_bytes);
-  const uint32_t token = a / p.top_k;
   const uint32_t nblk = in / 128u;
   float m = 0.0f;
   for (uint32_t bl = static_cast<uint32_t>(warp); bl < nblk; bl += kRotateThreads / 32u) {
@@ -68,20 +107,12 @@ __global__ void __launch_bounds__(kRotateThreads) moe_tc_rotate_kernel(const __g
     const __half2 s01 = *reinterpret_cast<const __half2 *>(&sb.x), s23 = *reinterpret_cast<const __half2 *>(&sb.y);
     const float sv[4] = {__low2float(s01), __high2float(s01), __low2float(s23), __high2float(s23)};
     float v[4];
-    if (PHASE == 0) {
-      const uint2 xb = ldg64_coherent(p.x + static_cast<size_t>(token) * p.hidden + k0);
-      v[0] = bf16_bits_to_f32(xb.x & 0xFFFFu) * sv[0];
-      v[1] = __uint_as_float(xb.x & 0xFFFF0000u) * sv[1];
-      v[2] = bf16_bits_to_f32(xb.y & 0xFFFFu) * sv[2];
-      v[3] = __uint_as_float(xb.y & 0xFFFF0000u) * sv[3];
-    } else {
-      const float *g = p.gu + static_cast<size_t>(row) * 2u * p.inter + k0;
-      const uint4 gb = ldg128_coherent(g), ub = ldg128_coherent(g + p.inter);
-      const float gv[4] = {__uint_as_float(gb.x), __uint_as_float(gb.y), __uint_as_float(gb.z), __uint_as_float(gb.w)};
-      const float uv[4] = {__uint_as_float(ub.x), __uint_as_float(ub.y), __uint_as_float(ub.z), __uint_as_float(ub.w)};
+    const float *g = p.gu + static_cast<size_t>(row) * 2u * p.inter + k0;
+    const uint4 gb = ldg128_coherent(g), ub = ldg128_coherent(g + p.inter);
+    const float gv[4] = {__uint_as_float(gb.x), __uint_as_float(gb.y), __uint_as_float(gb.z), __uint_as_float(gb.w)};
+    const float uv[4] = {__uint_as_float(ub.x), __uint_as_float(ub.y), __uint_as_float(ub.z), __uint_as_float(ub.w)};
 #pragma unroll
-      for (int i = 0; i < 4; ++i) v[i] = gv[i] / (1.0f + __expf(-gv[i])) * uv[i] * sv[i];
-    }
+    for (int i = 0; i < 4; ++i) v[i] = gv[i] / (1.0f + __expf(-gv[i])) * uv[i] * sv[i];
     hadamard128(v, lane);
     *reinterpret_cast<float4 *>(rot + k0) = make_float4(v[0], v[1], v[2], v[3]);
     m = fmaxf(m, fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))));
@@ -113,7 +144,7 @@ __global__ void __launch_bounds__(kRotateThreads) moe_tc_rotate_kernel(const __g
 constexpr uint32_t kBoxRows = 32;   // rows of one TMA load: an item loads as many as it has rows for
 
 template <int PHASE>
-__global__ void __launch_bounds__(kThreads, 2) moe_tc_gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ ExpertParams p) {
+__global__ void __launch_bounds__(Shape<2>::kThreads, 2) moe_tc_gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ ExpertParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t in = PHASE == 0 ? p.hidden : p.inter;
   const uint32_t out_plane = PHASE == 0 ? 2u * p.inter : p.hidden;
@@ -138,32 +169,29 @@ __global__ void __launch_bounds__(kThreads, 2) moe_tc_gemm_kernel(const __grid_c
   job.row0 = item.first;
   job.rows = item.count;
   job.box = kBoxRows;
-  const Core c = core_setup(smem_raw, job, kWhole);
+  const Core c = core_setup<2>(smem_raw, job, kWhole);
   const uint64_t trellis_bytes = static_cast<uint64_t>(in) * out_plane * slot.k2 / 16u;
   const uint16_t *svh = reinterpret_cast<const uint16_t *>(static_cast<const uint8_t *>(slot.record) + trellis_bytes) + in;
   const float *inv_rows = reinterpret_cast<const float *>(PHASE == 0 ? p.scale_in : p.scale_h);
-  const bool decoded = core_roles(c, job, &map_rows, p.status + 1);   // word 1 of the status line: waits of this kernel that ran out
-  const uint32_t col = col_tile * 128u + 4u * static_cast<uint32_t>(c.lane);
-  const float4 sv = four_halves(svh + col);
-  struct Choice {
-    uint32_t a;     // PHASE 1: which assignment (token, rank) the row is, and its routing weight
-    float weight;
+  const bool decoded = core_roles<2>(c, job, &map_rows, p.status + 1);   // word 1 of the status line: waits of this kernel that ran out
+  struct Row {
+    float *y;
+    float weight;   // PHASE 1: the routing weight
   };
-  core_finish_rows(
+  core_finish_rows<2>(
       c, job, kWhole, decoded, p.status + 1, [&](uint32_t r) { return inv_rows[item.first + r]; },
       [&](uint32_t r) {
-        Choice choice = {item.first + r, 1.0f};
-        if (PHASE == 1) {
-          choice.a = p.sorted[item.first + r];
-          choice.weight = p.weights[choice.a];
-        }
-        return choice;
+        const uint32_t row = item.first + r;
+        if (PHASE == 0) return Row{p.gu + static_cast<size_t>(row) * 2u * p.inter + col_tile * 128u, 1.0f};
+        const uint32_t a = p.sorted[row];   // which assignment (token, rank) the row is
+        return Row{p.down_rows + static_cast<size_t>(a) * p.hidden + col_tile * 128u, p.weights[a]};
       },
-      [&](uint32_t, const Choice &choice, const float4 &v) {
-        float *dst = PHASE == 0 ? p.gu + static_cast<size_t>(choice.a) * 2u * p.inter + col : p.down_rows + static_cast<size_t>(choice.a) * p.hidden + col;
+      [](const Row &, uint32_t) { return 0u; },
+      [&](const Row &row, uint32_t col, uint32_t, const float4 &v) {
+        const float4 sv = four_halves(__ldg(reinterpret_cast<const uint2 *>(svh + col_tile * 128u + col)));
         float4 o = make_float4(v.x * sv.x, v.y * sv.y, v.z * sv.z, v.w * sv.w);
-        if (PHASE == 1) o = make_float4(choice.weight * o.x, choice.weight * o.y, choice.weight * o.z, choice.weight * o.w);
-        *reinterpret_cast<float4 *>(dst) = o;
+        if (PHASE == 1) o = make_float4(row.weight * o.x, row.weight * o.y, row.weight * o.z, row.weight * o.w);
+        *reinterpret_cast<float4 *>(row.y + col) = o;
       });
 }
 
@@ -221,15 +249,14 @@ __global__ void __launch_bounds__(256) moe_tc_fold_kernel(const __grid_constant_
   if (range) atomicOr(p.status, kStatusRange);
 }
 
-constexpr size_t kRotateSmemMax = 200 * 1024;
+constexpr uint32_t kRotateMaxIn = 51200;   // inputs of a row the route takes
 
 }  // namespace
 
 int32_t moe_tc_prepare(ErrorSlot &slot) {
-  cudaError_t err = cudaFuncSetAttribute(moe_tc_gemm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemBytes));
-  if (err == cudaSuccess) err = cudaFuncSetAttribute(moe_tc_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemBytes));
-  if (err == cudaSuccess) err = cudaFuncSetAttribute(moe_tc_rotate_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRotateSmemMax));
-  if (err == cudaSuccess) err = cudaFuncSetAttribute(moe_tc_rotate_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRotateSmemMax));
+  cudaError_t err = cudaFuncSetAttribute(moe_tc_gemm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Shape<2>::kSmemBytes));
+  if (err == cudaSuccess) err = cudaFuncSetAttribute(moe_tc_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Shape<2>::kSmemBytes));
+  if (err == cudaSuccess) err = cudaFuncSetAttribute(moe_tc_rotate_h_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRotateMaxIn * 4u));
   if (err != cudaSuccess) return fail(slot, "MoE tensor-core kernel attributes: %s", cudaGetErrorString(err));
   if (encode_tiled_fn() == nullptr) return fail(slot, "cuTensorMapEncodeTiled is not available from this driver");
   return 0;
@@ -243,17 +270,19 @@ int32_t moe_tc_experts(ErrorSlot &slot, const DeviceState &dev, const ExpertPara
   for (int phase = 0; phase < 2; ++phase) {
     const uint32_t in = phase == 0 ? p.hidden : p.inter;
     const uint32_t out_plane = phase == 0 ? 2u * p.inter : p.hidden;
-    if (static_cast<size_t>(in) * 4u > kRotateSmemMax) return fail(slot, "%s: a dimension is too long for the tensor-core route", what);
-    cudaError_t err = phase == 0 ? launch(moe_tc_rotate_kernel<0>, dim3(rows), dim3(kRotateThreads), static_cast<size_t>(in) * 4u, stream, pdl, p, offsets)
-                                 : launch(moe_tc_rotate_kernel<1>, dim3(rows), dim3(kRotateThreads), static_cast<size_t>(in) * 4u, stream, pdl, p, offsets);
+    if (in > kRotateMaxIn) return fail(slot, "%s: a dimension is too long for the tensor-core route", what);
+    const uint32_t threads = 32u * rotate_warps(in), at_once = static_cast<uint32_t>(dev.sm_count) * (threads <= 256u ? 1024u / threads : 1u);
+    cudaError_t err = phase != 0 ? launch(moe_tc_rotate_h_kernel, dim3(rows), dim3(kRotateThreads), static_cast<size_t>(in) * 4u, stream, pdl, p, offsets)
+                                 : launch(threads <= 256u ? moe_tc_rotate_x_kernel<256> : moe_tc_rotate_x_kernel<1024>, dim3(rows < at_once ? rows : at_once),
+                                          dim3(threads), 0, stream, pdl, p, offsets);
     if (err != cudaSuccess) return fail(slot, "%s: rotation launch failed: %s", what, cudaGetErrorString(err));
     CUtensorMap map_rows;
     if (!make_rows_map(&map_rows, phase == 0 ? static_cast<const void *>(p.frag_in) : static_cast<const void *>(p.frag_h), rows, in, kBoxRows)) {
       return fail(slot, "%s: tensor map encoding failed", what);
     }
     const dim3 grid(items_max * (out_plane / 128u));
-    err = phase == 0 ? launch(moe_tc_gemm_kernel<0>, grid, dim3(kThreads), kSmemBytes, stream, pdl, map_rows, p)
-                     : launch(moe_tc_gemm_kernel<1>, grid, dim3(kThreads), kSmemBytes, stream, pdl, map_rows, p);
+    err = phase == 0 ? launch(moe_tc_gemm_kernel<0>, grid, dim3(Shape<2>::kThreads), Shape<2>::kSmemBytes, stream, pdl, map_rows, p)
+                     : launch(moe_tc_gemm_kernel<1>, grid, dim3(Shape<2>::kThreads), Shape<2>::kSmemBytes, stream, pdl, map_rows, p);
     if (err != cudaSuccess) return fail(slot, "%s: expert launch failed: %s", what, cudaGetErrorString(err));
   }
   const cudaError_t err = launch(moe_tc_fold_kernel, dim3(tokens), dim3(256), 0, stream, pdl, p, tokens);

@@ -81,6 +81,7 @@ int32_t prepare_device(ErrorSlot &slot, DeviceState *state) {
   fresh.w4a4_pair = env_int("B200Q_W4A4_PAIR", -1);
   fresh.sm_cap = env_int("IGNIS_TRELLIS_SM_CAP", 0);
   if (fresh.sm_cap < 0 || fresh.sm_cap > fresh.sm_count) fresh.sm_cap = 0;
+  fresh.trellis_dw = env_int("B200Q_TRELLIS_TC_SHAPE", 0);
   fresh.trellis_tc = env_int("B200Q_TRELLIS_TC", 1);
   fresh.moe_tc = env_int("B200Q_MOE_TC", 1);
   fresh.peer_barrier_polls = env_int("B200Q_PEER_BARRIER_POLLS", 1 << 22);

@@ -93,6 +93,152 @@ __device__ __forceinline__ void hadamard128(float (&v)[4], int lane) {
   for (int i = 0; i < 4; ++i) v[i] *= 0.08838834764831845f;
 }
 
+// Two floats at a time (one instruction for both).
+__device__ __forceinline__ float2 add_f32x2(float2 a, float2 b) {
+  float2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<unsigned long long &>(r)) : "l"(reinterpret_cast<unsigned long long &>(a)), "l"(reinterpret_cast<unsigned long long &>(b)));
+  return r;
+}
+__device__ __forceinline__ float2 mul_f32x2(float2 a, float2 b) {
+  float2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<unsigned long long &>(r)) : "l"(reinterpret_cast<unsigned long long &>(a)), "l"(reinterpret_cast<unsigned long long &>(b)));
+  return r;
+}
+__device__ __forceinline__ float2 fma_f32x2(float2 a, float2 b, float2 c) {
+  float2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(reinterpret_cast<unsigned long long &>(r)) : "l"(reinterpret_cast<unsigned long long &>(a)), "l"(reinterpret_cast<unsigned long long &>(b)), "l"(reinterpret_cast<unsigned long long &>(c)));
+  return r;
+}
+
+// The same transform, without its 1 / sqrt(128), of a 128-vector that four lanes hold: lane q (0..3) its units q, q + 4, ... of
+// 2 PAIRS values each. `low` and `high` are the lane masks of q's two bits. The stages run in hadamard128's order and round
+// alike; five of them lie inside a lane, two values an instruction, so that eight vectors in a warp take 192 instructions
+// where one takes 56.
+template <int UNITS, int PAIRS>
+__device__ __forceinline__ void hadamard_quad(float2 (&v)[UNITS][PAIRS], int lane, int low, int high) {
+  static_assert(UNITS * PAIRS == 16, "32 values a lane");
+  const float2 minus = make_float2(-1.0f, -1.0f);
+#pragma unroll
+  for (int u = 0; u < UNITS; ++u) {
+#pragma unroll
+    for (int p = 0; p < PAIRS; ++p) v[u][p] = make_float2(v[u][p].x + v[u][p].y, v[u][p].x - v[u][p].y);
+#pragma unroll
+    for (int h = 1; h < PAIRS; h <<= 1) {
+#pragma unroll
+      for (int p = 0; p < PAIRS; ++p) {
+        if ((p & h) == 0) {
+          const float2 a = v[u][p], b = v[u][p + h];
+          v[u][p] = add_f32x2(a, b);
+          v[u][p + h] = fma_f32x2(b, minus, a);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    const int mask = s == 0 ? low : high;
+    const float sign = (lane & mask) != 0 ? -1.0f : 1.0f;   // as in hadamard128
+    const float2 sign2 = make_float2(sign, sign);
+#pragma unroll
+    for (int u = 0; u < UNITS; ++u) {
+#pragma unroll
+      for (int p = 0; p < PAIRS; ++p) {
+        const float2 o = make_float2(__shfl_xor_sync(0xFFFFFFFFu, v[u][p].x, mask), __shfl_xor_sync(0xFFFFFFFFu, v[u][p].y, mask));
+        v[u][p] = fma_f32x2(sign2, v[u][p], o);
+      }
+    }
+  }
+#pragma unroll
+  for (int h = 1; h < UNITS; h <<= 1) {
+#pragma unroll
+    for (int u = 0; u < UNITS; ++u) {
+      if ((u & h) == 0) {
+#pragma unroll
+        for (int p = 0; p < PAIRS; ++p) {
+          const float2 a = v[u][p], b = v[u + h][p];
+          v[u][p] = add_f32x2(a, b);
+          v[u + h][p] = fma_f32x2(b, minus, a);
+        }
+      }
+    }
+  }
+}
+
+// ---- a row's rotation into fp16, for the tensor-core routes ------------------------------------------------------
+// Warp w of the CTA takes blocks 8 w .. + 7 of the row's 128-input blocks (a row has as many warps as that makes, up to 32, and
+// goes round beyond), four lanes a block, lane q its units q, q + 4, q + 8, q + 12 of eight inputs. `fetch(k, v)` gives the
+// eight products x o suh at input k. One power-of-two scale for the row brings its largest magnitude into [2^13, 2^14); the
+// inverse goes to *inv.
+constexpr float kHadamardNorm = 0.08838834764831845f;   // 1 / sqrt(128)
+__host__ __device__ constexpr uint32_t rotate_warps(uint32_t in) { return (in / 128u + 7u) / 8u < 32u ? (in / 128u + 7u) / 8u : 32u; }
+
+template <class Fetch>
+__device__ __forceinline__ void rotate_row(uint32_t in, uint16_t *dst, float *inv, float *warp_max, Fetch fetch) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t nblk = in / 128u, warps = blockDim.x / 32u, q = static_cast<uint32_t>(lane) & 3u;
+  float2 v[4][4];
+  auto transform = [&](uint32_t bl) {   // block bl of the row, zeros past its end
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (bl < nblk) {
+        fetch(bl * 128u + (4u * u + q) * 8u, v[u]);
+      } else {
+#pragma unroll
+        for (int p = 0; p < 4; ++p) v[u][p] = make_float2(0.0f, 0.0f);
+      }
+    }
+    hadamard_quad<4, 4>(v, lane, 1, 2);
+  };
+  float m = 0.0f;
+  const uint32_t first = static_cast<uint32_t>(warp) * 8u + (static_cast<uint32_t>(lane) >> 2);
+  const bool once = nblk <= 8u * warps;   // the row's values stay in registers
+  for (uint32_t bl0 = 0; bl0 < nblk; bl0 += 8u * warps) {
+    transform(bl0 + first);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int p = 0; p < 4; ++p) m = fmaxf(m, fmaxf(fabsf(v[u][p].x), fabsf(v[u][p].y)));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+  if (warps > 1u) {
+    if (lane == 0) warp_max[warp] = m;
+    __syncthreads();
+    m = warp_max[lane < static_cast<int>(warps) ? lane : 0];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+  }
+  m *= kHadamardNorm;
+  // m in [2^(e-1), 2^e) with e = (exponent field) - 126: the scale 2^(14 - e), held to what a float carries
+  int shift = 0;
+  if (m > 0.0f && m <= 3.0e38f) shift = max(-126, min(126, 140 - static_cast<int>(__float_as_uint(m) >> 23)));
+  const float scale = __uint_as_float(static_cast<uint32_t>(shift + 127) << 23);
+  if (threadIdx.x == 0) *inv = __uint_as_float(static_cast<uint32_t>(127 - shift) << 23);
+  for (uint32_t bl0 = 0; bl0 < nblk; bl0 += 8u * warps) {
+    if (!once) transform(bl0 + first);
+    if (bl0 + first >= nblk) continue;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      uint32_t packed[4];
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        const __half2 h = __floats2half2_rn(v[u][p].x * kHadamardNorm * scale, v[u][p].y * kHadamardNorm * scale);
+        packed[p] = *reinterpret_cast<const uint32_t *>(&h);
+      }
+      *reinterpret_cast<uint4 *>(dst + (bl0 + first) * 128u + (4u * u + q) * 8u) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+    }
+  }
+}
+// Eight inputs times their suh, both in 16-byte pieces: BF16 and FP16.
+__device__ __forceinline__ void scaled_inputs(const uint4 x, const uint4 suh, float2 (&v)[4]) {
+  const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, ss[4] = {suh.x, suh.y, suh.z, suh.w};
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    v[p] = mul_f32x2(make_float2(bf16_bits_to_f32(xs[p] & 0xFFFFu), __uint_as_float(xs[p] & 0xFFFF0000u)),
+                     __half22float2(*reinterpret_cast<const __half2 *>(&ss[p])));
+  }
+}
+
 }  // namespace trellis_dev
 }  // namespace b200q
 

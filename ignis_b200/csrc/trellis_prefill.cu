@@ -13,6 +13,8 @@
 #include "trellis_internal.cuh"
 #include "trellis_tc.cuh"
 
+#include <cmath>
+
 namespace b200q {
 namespace {
 
@@ -20,55 +22,18 @@ using namespace trellis_tc;
 
 __device__ uint32_t g_trellis_tc_status = 0;
 
-// ---- rotation: one CTA per token ------------------------------------------------------------------
-// x o suh, the 128-wide Hadamard per block (a warp per block, fp32), one power-of-two scale for the
-// whole token (largest magnitude in [2^13, 2^14)), fp16. The token's rotated values wait in shared
-// memory between the two passes (4 bytes per input).
-__global__ void __launch_bounds__(256) trellis_rotate_rows_kernel(const uint16_t *x, const uint16_t *suh, uint32_t in,
-                                                                  uint16_t *rows_f16, float *inv) {
-  extern __shared__ __align__(16) float rot[];
-  __shared__ float warp_max[8];
+// ---- rotation: one CTA per token (rotate_row, trellis_device.cuh) --------------------------------------------------
+// THREADS: the most a launch has (fewer leave a thread more registers for loads in flight).
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) trellis_rotate_rows_kernel(const uint16_t *x, const uint16_t *suh, uint32_t in, uint16_t *rows_f16, float *inv) {
+  __shared__ float warp_max[32];
   griddep_launch_dependents();
+  const size_t token = blockIdx.x;
   griddep_wait();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t token = blockIdx.x;
-  const uint32_t nblk = in / 128u;
-  float m = 0.0f;
-  for (uint32_t bl = static_cast<uint32_t>(warp); bl < nblk; bl += 8u) {
-    const size_t k0 = static_cast<size_t>(bl) * 128u + 4u * lane;
-    const uint2 xb = ldg64_coherent(x + static_cast<size_t>(token) * in + k0);
-    const uint2 sb = *reinterpret_cast<const uint2 *>(suh + k0);
-    const __half2 s01 = *reinterpret_cast<const __half2 *>(&sb.x), s23 = *reinterpret_cast<const __half2 *>(&sb.y);
-    float v[4];
-    v[0] = bf16_bits_to_f32(xb.x & 0xFFFFu) * __low2float(s01);
-    v[1] = __uint_as_float(xb.x & 0xFFFF0000u) * __high2float(s01);
-    v[2] = bf16_bits_to_f32(xb.y & 0xFFFFu) * __low2float(s23);
-    v[3] = __uint_as_float(xb.y & 0xFFFF0000u) * __high2float(s23);
-    hadamard128(v, lane);
-    *reinterpret_cast<float4 *>(rot + k0) = make_float4(v[0], v[1], v[2], v[3]);
-    m = fmaxf(m, fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))));
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
-  if (lane == 0) warp_max[warp] = m;
-  __syncthreads();
-  m = warp_max[0];
-#pragma unroll
-  for (int i = 1; i < 8; ++i) m = fmaxf(m, warp_max[i]);
-  // m in [2^(e-1), 2^e) with e = (exponent field) - 126: the scale 2^(14 - e), held to what a float carries
-  int shift = 0;
-  if (m > 0.0f && m <= 3.0e38f) shift = max(-126, min(126, 140 - static_cast<int>(__float_as_uint(m) >> 23)));
-  const float scale = __uint_as_float(static_cast<uint32_t>(shift + 127) << 23);
-  if (threadIdx.x == 0) inv[token] = __uint_as_float(static_cast<uint32_t>(127 - shift) << 23);
-  uint16_t *dst = rows_f16 + static_cast<size_t>(token) * in;
-  for (uint32_t i = threadIdx.x * 4u; i < in; i += 1024u) {
-    const float4 v = *reinterpret_cast<const float4 *>(rot + i);
-    const __half2 h01 = __floats2half2_rn(v.x * scale, v.y * scale), h23 = __floats2half2_rn(v.z * scale, v.w * scale);
-    uint2 packed;
-    packed.x = *reinterpret_cast<const uint32_t *>(&h01);
-    packed.y = *reinterpret_cast<const uint32_t *>(&h23);
-    *reinterpret_cast<uint2 *>(dst + i) = packed;
-  }
+  rotate_row(in, rows_f16 + token * in, inv + token, warp_max, [&](uint32_t k, float2 (&v)[4]) {
+    const uint2 lo = __ldg(reinterpret_cast<const uint2 *>(suh + k)), hi = __ldg(reinterpret_cast<const uint2 *>(suh + k + 4));   // 8-byte aligned
+    scaled_inputs(ldg128_coherent(x + token * in + k), make_uint4(lo.x, lo.y, hi.x, hi.y), v);
+  });
 }
 
 // ---- the product -----------------------------------------------------------------------------------
@@ -84,7 +49,8 @@ struct DenseParams {
   uint32_t ranks;        // the CTAs of a cluster share an item's K stages (1: no cluster)
 };
 
-__global__ void __launch_bounds__(kThreads, 2) trellis_tc_dense_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ DenseParams p) {
+template <int GROUPS>
+__global__ void __launch_bounds__(Shape<GROUPS>::kThreads, GROUPS == 2 ? 2 : 1) trellis_tc_dense_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ DenseParams p) {
   extern __shared__ uint8_t smem_raw[];
   // Token tiles run fastest over the grid, so the CTAs at work at one time decode the same columns
   // of the plane (read from HBM once, then from the L2).
@@ -101,16 +67,17 @@ __global__ void __launch_bounds__(kThreads, 2) trellis_tc_dense_kernel(const __g
   job.blk = item / row_tiles;
   job.row0 = item % row_tiles * p.tile;
   job.rows = min(p.tokens - job.row0, p.tile);
-  job.box = p.tile;
-  const Core c = core_setup(smem_raw, job, split);
-  const bool decoded = core_roles(c, job, &map_rows, &g_trellis_tc_status);
-  const uint32_t col = job.blk * 128u + 4u * static_cast<uint32_t>(c.lane);
-  const float4 sv = four_halves(p.svh + col);
-  uint16_t *out = p.y + static_cast<size_t>(job.row0) * p.ldy + col;
-  core_finish_rows(
+  job.box = p.tile > 256u ? p.tile / 2u : p.tile;
+  const Core c = core_setup<GROUPS>(smem_raw, job, split);
+  const bool decoded = core_roles<GROUPS>(c, job, &map_rows, &g_trellis_tc_status);
+  const uint16_t *svh = p.svh + job.blk * 128u;
+  uint16_t *out = p.y + static_cast<size_t>(job.row0) * p.ldy + job.blk * 128u;
+  core_finish_rows<GROUPS>(
       c, job, split, decoded, &g_trellis_tc_status, [&](uint32_t r) { return p.inv[job.row0 + r]; },
-      [&](uint32_t r) { return p.epilogue != kEpiStore ? *reinterpret_cast<const uint2 *>(out + static_cast<size_t>(r) * p.ldy) : make_uint2(0u, 0u); },
-      [&](uint32_t r, const uint2 &old, const float4 &o) {
+      [&](uint32_t r) { return out + static_cast<size_t>(r) * p.ldy; },
+      [&](const uint16_t *y, uint32_t col) { return p.epilogue != kEpiStore ? *reinterpret_cast<const uint2 *>(y + col) : make_uint2(0u, 0u); },
+      [&](uint16_t *y, uint32_t col, const uint2 &old, const float4 &o) {
+        const float4 sv = four_halves(__ldg(reinterpret_cast<const uint2 *>(svh + col)));
         float v[4] = {o.x * sv.x, o.y * sv.y, o.z * sv.z, o.w * sv.w};
         if (p.epilogue != kEpiStore) {
           const float was[4] = {bf16_bits_to_f32(old.x & 0xFFFFu), __uint_as_float(old.x & 0xFFFF0000u), bf16_bits_to_f32(old.y & 0xFFFFu),
@@ -119,14 +86,13 @@ __global__ void __launch_bounds__(kThreads, 2) trellis_tc_dense_kernel(const __g
           for (int e = 0; e < 4; ++e) v[e] = p.epilogue == kEpiAdd ? v[e] + was[e] : was[e] / (1.0f + __expf(-was[e])) * v[e];
         }
         const __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
-        *reinterpret_cast<uint2 *>(out + static_cast<size_t>(r) * p.ldy) =
-            make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
+        *reinterpret_cast<uint2 *>(y + col) = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
       });
 }
 
 uint64_t align256(uint64_t v) { return (v + 255u) & ~static_cast<uint64_t>(255u); }
 
-constexpr size_t kRotateMaxSmem = 200 * 1024;   // 4 bytes per input: in <= 51200
+constexpr uint32_t kRotateMaxIn = 51200;   // inputs of a row the route takes
 
 bool aligned_to(const void *p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
 
@@ -141,11 +107,11 @@ namespace {
 // The CTAs of a cluster that share the K stages of an item.
 constexpr uint32_t kMaxRanks = 8;
 
-cudaLaunchConfig_t dense_config(uint32_t items, uint32_t ranks, cudaStream_t stream, bool pdl, cudaLaunchAttribute (&attr)[2]) {
+cudaLaunchConfig_t dense_config(bool wide, uint32_t items, uint32_t ranks, cudaStream_t stream, bool pdl, cudaLaunchAttribute (&attr)[2]) {
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(items * ranks);
-  config.blockDim = dim3(kThreads);
-  config.dynamicSmemBytes = kSmemBytes;
+  config.blockDim = dim3(wide ? Shape<4>::kThreads : Shape<2>::kThreads);
+  config.dynamicSmemBytes = wide ? Shape<4>::kSmemBytes : Shape<2>::kSmemBytes;
   config.stream = stream;
   unsigned n = 0;
   if (pdl) {
@@ -163,26 +129,46 @@ cudaLaunchConfig_t dense_config(uint32_t items, uint32_t ranks, cudaStream_t str
   return config;
 }
 
-// How many CTAs share an item: the count for which a model of the launch gives the least time. In microseconds, from
-// measurements of four shapes at 70 to 2000 tokens: a stage takes 1.17 with two CTAs on the SM, 0.72 alone (0.95 in a cluster,
-// whose CTAs may share an SM all the same); the epilogue 3 per row tile of 128 and 0.9 more per rank (its reads from the other
-// CTAs' shared memory). The last wave is counted for what is left in it. Few items leave SMs idle and walk all of K alone
-// (17408 -> 5120 at 128 tokens: 40 items of 272 stages, 190 us; six ranks each: 63), a last wave that is nearly empty costs as
-// much as a full one (the same at 1000 tokens: 160 items, 306 us; three ranks: 250); many items need no sharing. At least eight
-// stages per rank: what a CTA spends before its first and after its last stage is as long.
-uint32_t dense_ranks(const DeviceState &dev, uint32_t items, uint32_t stages, uint32_t row_tiles128) {
-  uint32_t best = 1u;
+// The CTA's shape, the tokens per CTA and the CTAs per item: those for which a model of the launch gives the least time. In
+// microseconds, fitted to every choice for five shapes (5120 -> 1024, 6144 and 17408, 6144 and 17408 -> 5120) at 70 to 4096 tokens
+// and 3 and 5 bits; what it picks is within 1 % of the fastest measured on average, 20 % at worst (a 1024-column weight at 300
+// tokens). The two-group shape takes 0.62 a stage with two CTAs on the SM and 0.41 alone while the decoder warps bound it, 4 ns
+// a token where the rows do; the four-group shape, one CTA an SM, 0.46 and 1.4 ns a token, but nothing runs under its fill and
+// epilogue. Then the epilogue and a cluster's exchange. Few items leave SMs idle and walk all of K alone (17408 -> 5120 at 200
+// tokens: 80 items, 174 us; 40 of the other shape, three ranks each: 57). At least four stages per rank.
+struct DensePlan {
+  uint32_t tile, ranks;
+  bool wide;   // four decoder groups
+};
+DensePlan dense_plan(const DeviceState &dev, uint32_t blocks, uint32_t stages, uint32_t tokens) {
+  DensePlan best = {0u, 1u, false};
   float least = 0.0f;
-  for (uint32_t ranks = 1; ranks <= kMaxRanks && (ranks == 1u || stages / ranks >= 8u); ++ranks) {
-    const uint32_t at_once = ranks == 1u ? 2u * static_cast<uint32_t>(dev.sm_count) : static_cast<uint32_t>(dev.trellis_clusters[ranks]);
-    if (at_once == 0u) continue;
-    const uint32_t waves = items / at_once, left = items % at_once;
-    const float epilogue = static_cast<float>(row_tiles128) * (3.0f + 0.9f * static_cast<float>(ranks));
-    const float walked = static_cast<float>((stages + ranks - 1u) / ranks);
-    const bool alone = left * ranks <= static_cast<uint32_t>(dev.sm_count);
-    float t = static_cast<float>(waves) * (1.17f * walked + epilogue);
-    if (left != 0u) t += (!alone ? 1.17f : ranks == 1u ? 0.72f : 0.95f) * walked + epilogue;
-    if (ranks == 1u || t < least) least = t, best = ranks;
+  for (const bool wide : {false, true}) {
+    if (dev.trellis_dw == (wide ? 8 : 16)) continue;   // B200Q_TRELLIS_TC_SHAPE asks for the other
+    const uint32_t most = wide ? Shape<4>::kMaxRows : Shape<2>::kMaxRows, fewest = (tokens + most - 1u) / most;
+    for (uint32_t nt = fewest; nt <= fewest + 2u; ++nt) {
+      const uint32_t tile = ((tokens + nt - 1u) / nt + 15u) / 16u * 16u;
+      if (nt > fewest && tile < 48u) break;
+      const uint32_t items = blocks * ((tokens + tile - 1u) / tile);
+      const float rows = static_cast<float>(tile);
+      for (uint32_t ranks = 1; ranks <= kMaxRanks && (ranks == 1u || stages / ranks >= 4u); ++ranks) {
+        // clusters (CTAs) the device places with one CTA per SM: what the occupancy query counts
+        const uint32_t one_each = ranks == 1u ? static_cast<uint32_t>(dev.sm_count) : static_cast<uint32_t>(dev.trellis_clusters[ranks]);
+        if (one_each == 0u) continue;
+        const float walked = static_cast<float>((stages + ranks - 1u) / ranks), r = static_cast<float>(ranks);
+        float t;
+        if (wide) {
+          const float cta = walked * fmaxf(0.46f, 0.0014f * rows) + 0.45f + 0.022f * rows / r + (ranks > 1u ? 1.0f + 0.022f * rows : 0.0f);
+          t = static_cast<float>((items + one_each - 1u) / one_each) * cta;
+        } else {
+          const float pair = fmaxf(0.62f, 0.004f * rows), alone = fmaxf(0.41f, 0.0005f * rows);
+          const float rest = 0.34f + 0.012f * rows / r + (ranks > 1u ? 1.6f + 0.023f * rows : 0.0f);
+          const uint32_t left = items % (2u * one_each);
+          t = static_cast<float>(items / (2u * one_each)) * (walked * pair + rest) + (left == 0u ? 0.0f : walked * (left > one_each ? pair : alone) + rest);
+        }
+        if (best.tile == 0u || t < least) least = t, best = {tile, ranks, wide};
+      }
+    }
   }
   return best;
 }
@@ -191,16 +177,14 @@ uint32_t dense_ranks(const DeviceState &dev, uint32_t items, uint32_t stages, ui
 int32_t trellis_tc_prepare(ErrorSlot &slot) {
   DeviceState *dev = device_state(slot);
   if (dev == nullptr) return -1;
-  cudaError_t err = cudaFuncSetAttribute(trellis_tc_dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemBytes));
-  if (err == cudaSuccess) {
-    err = cudaFuncSetAttribute(trellis_rotate_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRotateMaxSmem));
-  }
+  cudaError_t err = cudaFuncSetAttribute(trellis_tc_dense_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Shape<2>::kSmemBytes));
+  if (err == cudaSuccess) err = cudaFuncSetAttribute(trellis_tc_dense_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Shape<4>::kSmemBytes));
   if (err != cudaSuccess) return fail(slot, "trellis prefill kernel attributes: %s", cudaGetErrorString(err));
   for (uint32_t ranks = 2; ranks <= kMaxRanks && !dev->counted; ++ranks) {
     cudaLaunchAttribute attr[2];
-    const cudaLaunchConfig_t config = dense_config(1u, ranks, nullptr, false, attr);
+    const cudaLaunchConfig_t config = dense_config(false, 1u, ranks, nullptr, false, attr);
     int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, trellis_tc_dense_kernel, &config) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&clusters, trellis_tc_dense_kernel<2>, &config) != cudaSuccess) {
       (void)cudaGetLastError();
       clusters = 0;
     }
@@ -212,7 +196,7 @@ int32_t trellis_tc_prepare(ErrorSlot &slot) {
 
 bool trellis_tc_takes(const DeviceState &dev, uint32_t in, uint32_t tokens, uint32_t weights, const ignis_trellis_workspace *workspace) {
   if (dev.trellis_tc == 0 || tokens <= IGNIS_TRELLIS_DECODE_MAX_TOKENS) return false;
-  if (static_cast<size_t>(in) * 4u > kRotateMaxSmem) return false;
+  if (in > kRotateMaxIn) return false;
   if (workspace == nullptr || workspace->base == nullptr || !aligned_to(workspace->base, 256)) return false;
   return workspace->bytes >= trellis_tc_workspace_bytes(in, weights, tokens);
 }
@@ -222,13 +206,13 @@ int32_t one_product(ErrorSlot &slot, const DeviceState &dev, const ignis_trellis
                     uint32_t ldy, uint32_t epilogue, uint8_t *region, cudaStream_t stream, const char *what) {
   uint16_t *rows = reinterpret_cast<uint16_t *>(region);
   float *inv = reinterpret_cast<float *>(region + align256(static_cast<uint64_t>(tokens) * w->in * 2u));
-  cudaError_t err = launch(trellis_rotate_rows_kernel, dim3(tokens), dim3(256), static_cast<size_t>(w->in) * 4u, stream, dev.pdl != 0, x,
-                           static_cast<const uint16_t *>(w->suh), w->in, rows, inv);
+  const uint32_t threads = 32u * rotate_warps(w->in);
+  cudaError_t err = launch(threads <= 256u ? trellis_rotate_rows_kernel<256> : threads <= 640u ? trellis_rotate_rows_kernel<640> : trellis_rotate_rows_kernel<1024>,
+                           dim3(tokens), dim3(threads), 0, stream, dev.pdl != 0, x, static_cast<const uint16_t *>(w->suh), w->in, rows, inv);
   if (err != cudaSuccess) return fail(slot, "%s: rotation launch failed: %s", what, cudaGetErrorString(err));
-  const uint32_t row_tiles = (tokens + kMaxRows - 1u) / kMaxRows;
+  const DensePlan plan = dense_plan(dev, w->out / 128u, w->in / 64u, tokens);
   CUtensorMap map_rows;
-  const uint32_t tile = ((tokens + row_tiles - 1u) / row_tiles + 15u) / 16u * 16u;
-  if (!make_rows_map(&map_rows, rows, tokens, w->in, tile)) return fail(slot, "%s: tensor map encoding failed", what);
+  if (!make_rows_map(&map_rows, rows, tokens, w->in, plan.tile > 256u ? plan.tile / 2u : plan.tile)) return fail(slot, "%s: tensor map encoding failed", what);
   DenseParams p = {};
   p.trellis = static_cast<const uint32_t *>(w->trellis);
   p.svh = static_cast<const uint16_t *>(w->svh);
@@ -241,12 +225,12 @@ int32_t one_product(ErrorSlot &slot, const DeviceState &dev, const ignis_trellis
   p.tokens = tokens;
   p.ldy = ldy;
   p.epilogue = epilogue;
-  p.tile = tile;
+  p.tile = plan.tile;
+  p.ranks = plan.ranks;
   const uint32_t items = w->out / 128u * ((tokens + p.tile - 1u) / p.tile);
-  p.ranks = dense_ranks(dev, items, w->in / 64u, p.tile > 128u ? 2u : 1u);
   cudaLaunchAttribute attr[2];
-  cudaLaunchConfig_t config = dense_config(items, p.ranks, stream, dev.pdl != 0, attr);
-  err = cudaLaunchKernelEx(&config, trellis_tc_dense_kernel, map_rows, p);
+  cudaLaunchConfig_t config = dense_config(plan.wide, items, p.ranks, stream, dev.pdl != 0, attr);
+  err = cudaLaunchKernelEx(&config, plan.wide ? trellis_tc_dense_kernel<4> : trellis_tc_dense_kernel<2>, map_rows, p);
   if (err != cudaSuccess) return fail(slot, "%s: launch failed: %s", what, cudaGetErrorString(err));
   return 0;
 }

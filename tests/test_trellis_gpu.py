@@ -432,6 +432,43 @@ def test_both_shapes_of_the_tensor_core_route_give_the_same_bits(tr, oracle, tok
         tr.prepare()
 
 
+@pytest.mark.parametrize("shape", ["8", "16"])
+@pytest.mark.parametrize("tokens,in_,k2", [(65, 128, 4), (80, 256, 6), (191, 640, 5), (193, 384, 8), (256, 128, 12), (257, 896, 10), (384, 256, 6), (385, 640, 8)])
+def test_edges_of_the_tensor_core_shapes(tr, oracle, monkeypatch, shape, tokens, in_, k2):
+    """Both shapes at the edges of their row tiles (one MMA and two, one tile and several), with K of two stages and more,
+    shared by a cluster where the plan does; stored, added and as a fused SwiGLU."""
+    from oracle import oracle as orc
+
+    out = 256
+    rng = np.random.default_rng(tokens)
+    words = [oracle.hash_trellis_words(700 + tokens + i, in_, out, k2) for i in (0, 1)]
+    suh, svh = [make_scales(rng, in_, 0.05) for _ in words], [make_scales(rng, out, 0.03) for _ in words]
+    w = [tr.Weight.from_numpy(words[i], suh[i], svh[i], k2, in_, out) for i in (0, 1)]
+    x = torch.randn(tokens, in_, generator=torch.Generator().manual_seed(tokens)).to(torch.bfloat16)
+    x[tokens - 1] = 0.0
+    ref, s = zip(*[orc.trellis_project_rows(oracle.trellis_decode(words[i], k2, in_, out), suh[i], svh[i], x.double().numpy()) for i in (0, 1)])
+    monkeypatch.setenv("B200Q_TRELLIS_TC_SHAPE", shape)
+    try:
+        tr.prepare()
+        ws = tr.WorkspaceBuffer(tr.workspace_bytes(in_, out, 2, tokens))
+        y = tr.linear(w[0], x.cuda(), workspace=ws)
+        check_linear(y[:-1], ref[0][:-1], s[0][:-1])   # the row of zeros has a bound of zero
+        assert torch.all(y[-1] == 0)
+        base = torch.randn(tokens, out, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16)
+        check_linear(tr.linear(w[0], x.cuda(), base.clone().cuda(), epilogue=tr.ADD, workspace=ws), ref[0] + base.double().numpy(),
+                     s[0] + np.abs(base.double().numpy()))
+        h = tr.linear_swiglu(w[0], w[1], x.cuda(), workspace=ws).double().cpu().numpy()
+        assert tr.device_status() == 0
+    finally:
+        monkeypatch.undo()
+        tr.prepare()
+    want = ref[0] / (1.0 + np.exp(-ref[0])) * ref[1]
+    # the gate is stored in BF16 between the products: 2^-8 of it reaches h with |d silu / dg| <= 1.1, and the products' own
+    # tolerance reaches it through the other factor
+    tol = 2.0 ** -7 * np.abs(want) + (2.0 ** -8 * np.abs(ref[0]) + 2.0 ** -9 * s[0]) * 1.1 * np.abs(ref[1]) + 2.0 ** -9 * s[1] * np.abs(ref[0])
+    assert np.all(np.abs(h - want) <= tol)
+
+
 def test_full_size_gate_projection(tr, oracle):
     """A 27B-style layer's gate projection, 5120 -> 17408 at 3 bits per weight, 1 and 8 tokens, every output inside the
     reference's tolerance."""
