@@ -50,6 +50,7 @@ int32_t check_geometry(ErrorSlot &slot, const Geometry *g, const char *what) {
 struct Layout {
   uint64_t status, counts, cursor, offsets, n_items, sorted, items, tiles, frag_in, scale_in, gu, frag_h, scale_h, down_rows, total;
   uint32_t rows_max, items_max, tiles_max;
+  bool down_fits;   // the tensor-core route's weighted down products have a place
 };
 
 uint64_t align256(uint64_t v) { return (v + 255u) & ~static_cast<uint64_t>(255u); }
@@ -78,7 +79,17 @@ Layout layout_for(const Geometry &g, uint32_t tokens_max) {
   l.gu = at; at = align256(at + 8ull * l.rows_max * g.inter);           // fp32 [rows][2 inter]
   l.frag_h = at; at = align256(at + 2048ull * l.tiles_max * nblk_i);    // rotated silu(g) u
   l.scale_h = at; at = align256(at + 64ull * l.tiles_max * nblk_i);
-  l.down_rows = at; at = align256(at + (tokens_max > 8u ? 4ull * l.rows_max * g.hidden : 0ull));   // wide calls only (the tensor-core route)
+  // The weighted down products of the tensor-core route, fp32 [tokens][top_k][hidden]: a region of their own in wide
+  // workspaces; in one for decode widths they take the place of the rotated x and the gate|up products, which nothing reads
+  // any more when they are written (it is large enough except for a few experts of inter < hidden / 4).
+  const uint64_t down = 4ull * l.rows_max * g.hidden;
+  if (tokens_max > 8u) {
+    l.down_rows = at; at = align256(at + down);
+    l.down_fits = true;
+  } else {
+    l.down_rows = l.frag_in;
+    l.down_fits = l.frag_in + down <= l.frag_h;
+  }
   l.total = at;
   return l;
 }
@@ -637,8 +648,7 @@ const DeviceState *prepared(ErrorSlot &slot, const char *what) {
 }
 
 int32_t run_experts(const Geometry &g, const void *x, uint32_t tokens, const int32_t *ids, const float *weights, const ignis_moe_slot *slots,
-                    const ignis_moe_workspace *workspace, int64_t *acc, void *stream_v, uint32_t limit, uint32_t item_rows,
-                    const char *what) {
+                    const ignis_moe_workspace *workspace, int64_t *acc, void *stream_v, uint32_t limit, const char *what) {
   ErrorSlot &slot = moe_error();
   if (x == nullptr || ids == nullptr || weights == nullptr || slots == nullptr || workspace == nullptr || acc == nullptr ||
       workspace->base == nullptr) {
@@ -653,6 +663,8 @@ int32_t run_experts(const Geometry &g, const void *x, uint32_t tokens, const int
   uint8_t *base = static_cast<uint8_t *>(workspace->base);
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
   const uint32_t rows = tokens * g.top_k;
+  // the tensor-core route's items, or the warp-level kernels': 8 rows at decode widths, 64 beyond
+  const uint32_t item_rows = dev->moe_tc != 0 && l.down_fits ? kMoeTcItemRows : tokens > 8u ? 64u : 8u;
   uint32_t *counts = reinterpret_cast<uint32_t *>(base + l.counts);
   uint32_t *cursor = reinterpret_cast<uint32_t *>(base + l.cursor);
   uint32_t *offsets = reinterpret_cast<uint32_t *>(base + l.offsets);
@@ -664,7 +676,7 @@ int32_t run_experts(const Geometry &g, const void *x, uint32_t tokens, const int
   Tile *tiles = item_rows == kMoeTcItemRows ? nullptr : reinterpret_cast<Tile *>(base + l.tiles);
   cudaError_t err = cudaSuccess;
   if (rows <= kSmallRows && g.experts <= kSmallExperts) {
-    err = launch(moe_group_small_kernel, dim3(1), dim3(1024), 0, stream, false, ids, rows, g.experts, item_rows, offsets, n_items, items,
+    err = launch(moe_group_small_kernel, dim3(1), dim3(1024), 0, stream, pdl, ids, rows, g.experts, item_rows, offsets, n_items, items,
                  tiles, sorted, status);
     if (err != cudaSuccess) return fail(slot, "%s: grouping launch failed: %s", what, cudaGetErrorString(err));
   } else {
@@ -841,7 +853,7 @@ int32_t b200q_moe_experts_decode(const b200q_moe_geometry *geometry, const void 
                                  const struct ignis_moe_workspace *workspace, int64_t *acc, void *stream) {
   if (check_geometry(moe_error(), geometry, "ignis_moe_experts_decode") != 0) return -1;
   const uint32_t limit = workspace != nullptr ? workspace->decode_tokens : 0u;
-  return run_experts(*geometry, x, tokens, ids, weights, slots, workspace, acc, stream, limit, 8u, "ignis_moe_experts_decode");
+  return run_experts(*geometry, x, tokens, ids, weights, slots, workspace, acc, stream, limit, "ignis_moe_experts_decode");
 }
 
 int32_t b200q_moe_experts_prefill(const b200q_moe_geometry *geometry, const void *x, uint32_t tokens, const int32_t *ids,
@@ -849,12 +861,7 @@ int32_t b200q_moe_experts_prefill(const b200q_moe_geometry *geometry, const void
                                   const struct ignis_moe_workspace *workspace, int64_t *acc, void *stream) {
   if (check_geometry(moe_error(), geometry, "ignis_moe_experts_prefill") != 0) return -1;
   const uint32_t limit = workspace != nullptr ? workspace->prefill_tokens : 0u;
-  // up to 8 tokens the decode entry's item size; up to 64 tokens items of 64 rows on the warp-level
-  // MMAs; beyond, items of 192 rows on the tensor cores (B200Q_MOE_TC = 0 keeps the warp-level kernels)
-  const DeviceState *dev = device_state(moe_error());
-  const bool tc = dev != nullptr && dev->prepared && dev->moe_tc != 0 && tokens > 64u;
-  return run_experts(*geometry, x, tokens, ids, weights, slots, workspace, acc, stream, limit, tokens > 8u ? (tc ? kMoeTcItemRows : 64u) : 8u,
-                     "ignis_moe_experts_prefill");
+  return run_experts(*geometry, x, tokens, ids, weights, slots, workspace, acc, stream, limit, "ignis_moe_experts_prefill");
 }
 
 int32_t ignis_moe_decode_cluster_size(void) { return 0; }

@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(Shape<2>::kThreads, 2) moe_tc_gemm_kernel(cons
       });
 }
 
-// One CTA per token: the token's weighted down products (one row per choice that had an expert with a
+// One CTA per token, several with few tokens: the token's weighted down products (one row per choice that had an expert with a
 // record) become 2^-32 fixed-point integers and are added to the token's accumulator row. Integer
 // sums do not depend on their order: the bits are those of adding every product on its own.
 __global__ void __launch_bounds__(256) moe_tc_fold_kernel(const __grid_constant__ ExpertParams p, uint32_t tokens) {
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(256) moe_tc_fold_kernel(const __grid_constant_
   // four columns per thread and trip (hidden is a multiple of 128), the choices' loads issued together
   const float4 *rows4 = reinterpret_cast<const float4 *>(p.down_rows + static_cast<size_t>(token) * p.top_k * p.hidden);
   const uint32_t quads = p.hidden / 4u;
-  for (uint32_t c4 = threadIdx.x; c4 < quads; c4 += 256u) {
+  for (uint32_t c4 = blockIdx.y * 256u + threadIdx.x; c4 < quads; c4 += gridDim.y * 256u) {
     long long sum[4] = {0, 0, 0, 0};
     for (uint32_t k0 = 0; k0 < top_k; k0 += 8u) {
       float4 v[8];
@@ -285,7 +285,7 @@ int32_t moe_tc_experts(ErrorSlot &slot, const DeviceState &dev, const ExpertPara
                      : launch(moe_tc_gemm_kernel<1>, grid, dim3(Shape<2>::kThreads), Shape<2>::kSmemBytes, stream, pdl, map_rows, p);
     if (err != cudaSuccess) return fail(slot, "%s: expert launch failed: %s", what, cudaGetErrorString(err));
   }
-  const cudaError_t err = launch(moe_tc_fold_kernel, dim3(tokens), dim3(256), 0, stream, pdl, p, tokens);
+  const cudaError_t err = launch(moe_tc_fold_kernel, dim3(tokens, tokens < static_cast<uint32_t>(dev.sm_count) ? (p.hidden + 1023u) / 1024u : 1u), dim3(256), 0, stream, pdl, p, tokens);
   if (err != cudaSuccess) return fail(slot, "%s: fold launch failed: %s", what, cudaGetErrorString(err));
   return 0;
 }
