@@ -2,32 +2,25 @@
 //
 // Routed experts (the reference's ignis_moe_experts_prefill / _decode, kernel/src/moe_prefill.cu:
 // 41-492 and moe_decode.cu:325-399): the (token, rank) assignments are grouped by expert on the
-// device (count, scan, scatter) and cut into work items of at most 64 rows of one expert (8 from
-// the decode entry) made of row tiles of 8. Every row is rotated once into MMA B fragments in the
-// workspace (x o suh, Hadamard, power-of-two scale per row and 128 inputs, fp16); a grouped launch
-// multiplies each item with its expert's gate|up record, one CTA per 128 output columns, warp j
-// walking tile column j: every tile is decoded once in registers and used for all the item's row
-// tiles. silu(g) u is rotated the same way and the down launch adds the weighted result to `acc`
-// in 64-bit fixed point (2^-32), so the sum does not depend on arrival order. No CTA waits for
-// another; a row's arithmetic does not depend on the item it is in, so the decode and prefill
-// entries give the same bits.
+// device (count, scan, scatter) and cut into work items of at most 192 rows of one expert, which
+// moe_tc.cu multiplies with the expert's records on the tensor cores at every size, the decode
+// entry's included. (Warp-level kernels with the decoded tiles in registers stood here for up to 64
+// tokens: 75.8 us against 66.4 at one token, 107.8 against 88 at eight, 258 against 210 at 64, 2048
+// x 768 with 512 experts, ten of them a token.) Products are added to `acc` in 64-bit fixed point
+// (2^-32), so the sum does not depend on arrival order. No CTA waits for another; a row's
+// arithmetic does not depend on the item it is in, so the decode and prefill entries give the same
+// bits.
 //
 // Nothing here traps or spins: a bad expert id, an absent record or an out-of-range contribution
 // is skipped and recorded in the workspace's status word.
 #include "../../include/ignis_moe.h"
 
 #include "moe_internal.cuh"
-#include "trellis_device.cuh"
 
 #include <mutex>
 
 namespace b200q {
 namespace {
-
-using namespace trellis_dev;
-
-constexpr int kThreads = 256;
-constexpr int kWarps = 8;
 
 using Geometry = b200q_moe_geometry;
 // The geometry the reference's own entry points (no geometry argument) work at: the reference
@@ -48,9 +41,8 @@ int32_t check_geometry(ErrorSlot &slot, const Geometry *g, const char *what) {
 
 // Workspace regions for `tokens_max` tokens.
 struct Layout {
-  uint64_t status, counts, cursor, offsets, n_items, sorted, items, tiles, frag_in, scale_in, gu, frag_h, scale_h, down_rows, total;
-  uint32_t rows_max, items_max, tiles_max;
-  bool down_fits;   // the tensor-core route's weighted down products have a place
+  uint64_t status, counts, cursor, offsets, n_items, sorted, items, x_rows, x_scale, gu, h_rows, h_scale, down_rows, total;
+  uint32_t rows_max, items_max;
 };
 
 uint64_t align256(uint64_t v) { return (v + 255u) & ~static_cast<uint64_t>(255u); }
@@ -62,34 +54,22 @@ uint32_t items_bound(const Geometry &g, uint32_t rows, uint32_t item_rows) {
 Layout layout_for(const Geometry &g, uint32_t tokens_max) {
   Layout l = {};
   l.rows_max = tokens_max * g.top_k;
-  l.items_max = items_bound(g, l.rows_max, 8u);  // the bound for 8-row items covers 64-row items too
-  l.tiles_max = items_bound(g, l.rows_max, 8u);
-  const uint64_t nblk_h = g.hidden / 128u, nblk_i = g.inter / 128u;
+  l.items_max = items_bound(g, l.rows_max, kMoeTcItemRows);
+  const uint64_t rows = l.rows_max;
   uint64_t at = 0;
   l.status = at; at += 256;
   l.counts = at; at = align256(at + 4ull * g.experts);
   l.cursor = at; at = align256(at + 4ull * g.experts);
   l.offsets = at; at = align256(at + 4ull * (g.experts + 1));
-  l.n_items = at; at += 256;  // [0] items, [1] tiles
-  l.sorted = at; at = align256(at + 4ull * l.rows_max);
+  l.n_items = at; at += 256;
+  l.sorted = at; at = align256(at + 4ull * rows);
   l.items = at; at = align256(at + 16ull * l.items_max);
-  l.tiles = at; at = align256(at + 16ull * l.tiles_max);
-  l.frag_in = at; at = align256(at + 2048ull * l.tiles_max * nblk_h);   // rotated x, fragment order
-  l.scale_in = at; at = align256(at + 64ull * l.tiles_max * nblk_h);    // (inverse scale, scale) x 8 rows
-  l.gu = at; at = align256(at + 8ull * l.rows_max * g.inter);           // fp32 [rows][2 inter]
-  l.frag_h = at; at = align256(at + 2048ull * l.tiles_max * nblk_i);    // rotated silu(g) u
-  l.scale_h = at; at = align256(at + 64ull * l.tiles_max * nblk_i);
-  // The weighted down products of the tensor-core route, fp32 [tokens][top_k][hidden]: a region of their own in wide
-  // workspaces; in one for decode widths they take the place of the rotated x and the gate|up products, which nothing reads
-  // any more when they are written (it is large enough except for a few experts of inter < hidden / 4).
-  const uint64_t down = 4ull * l.rows_max * g.hidden;
-  if (tokens_max > 8u) {
-    l.down_rows = at; at = align256(at + down);
-    l.down_fits = true;
-  } else {
-    l.down_rows = l.frag_in;
-    l.down_fits = l.frag_in + down <= l.frag_h;
-  }
+  l.x_rows = at; at = align256(at + 2ull * rows * g.hidden);      // rotated x: fp16 [rows][hidden]
+  l.x_scale = at; at = align256(at + 4ull * rows);                // inverse scale per row
+  l.gu = at; at = align256(at + 8ull * rows * g.inter);           // fp32 [rows][2 inter]
+  l.h_rows = at; at = align256(at + 2ull * rows * g.inter);       // rotated silu(g) u: fp16 [rows][inter]
+  l.h_scale = at; at = align256(at + 4ull * rows);
+  l.down_rows = at; at = align256(at + 4ull * rows * g.hidden);   // weighted down products: fp32 [tokens][top_k][hidden]
   l.total = at;
   return l;
 }
@@ -124,49 +104,42 @@ __global__ void __launch_bounds__(256) moe_count_kernel(const int32_t *ids, uint
   }
 }
 
-// One CTA: exclusive scans of the per-expert row, item and tile counts, then the item and tile lists (`tiles` nullptr: no tile
-// list - the tensor-core route has none, and a popular expert's tiles, written by one thread, took 15 of 24 us).
+// One CTA: exclusive scans of the per-expert row and item counts, then the item list.
 __global__ void __launch_bounds__(1024) moe_scan_kernel(const uint32_t *counts, uint32_t experts, uint32_t item_rows,
-                                                        uint32_t *offsets, uint32_t *n_items, Item *items, Tile *tiles) {
+                                                        uint32_t *offsets, uint32_t *n_items, Item *items) {
   griddep_launch_dependents();
   griddep_wait();
-  __shared__ uint32_t row_sum[1024], item_sum[1024], tile_sum[1024];
+  __shared__ uint32_t row_sum[1024], item_sum[1024];
   const uint32_t per = (experts + 1023u) / 1024u;  // experts per thread, consecutive
   const uint32_t e0 = threadIdx.x * per;
-  uint32_t rows = 0, its = 0, tls = 0;
+  uint32_t rows = 0, its = 0;
   for (uint32_t e = e0; e < e0 + per && e < experts; ++e) {
     rows += counts[e];
     its += (counts[e] + item_rows - 1u) / item_rows;
-    tls += (counts[e] + 7u) / 8u;
   }
   row_sum[threadIdx.x] = rows;
   item_sum[threadIdx.x] = its;
-  tile_sum[threadIdx.x] = tls;
   __syncthreads();
   for (uint32_t d = 1; d < 1024; d <<= 1) {  // Hillis-Steele inclusive scan
     const uint32_t r = threadIdx.x >= d ? row_sum[threadIdx.x - d] : 0u;
     const uint32_t i = threadIdx.x >= d ? item_sum[threadIdx.x - d] : 0u;
-    const uint32_t t = threadIdx.x >= d ? tile_sum[threadIdx.x - d] : 0u;
     __syncthreads();
     row_sum[threadIdx.x] += r;
     item_sum[threadIdx.x] += i;
-    tile_sum[threadIdx.x] += t;
     __syncthreads();
   }
-  uint32_t row_at = row_sum[threadIdx.x] - rows, item_at = item_sum[threadIdx.x] - its, tile_at = tile_sum[threadIdx.x] - tls;
+  uint32_t row_at = row_sum[threadIdx.x] - rows, item_at = item_sum[threadIdx.x] - its;
   for (uint32_t e = e0; e < e0 + per && e < experts; ++e) {
     offsets[e] = row_at;
     const uint32_t c = counts[e];
     for (uint32_t j = 0; j < c; j += item_rows) {
-      items[item_at++] = Item{e, row_at + j, c - j < item_rows ? c - j : item_rows, tile_at + j / 8u};
+      items[item_at++] = Item{e, row_at + j, c - j < item_rows ? c - j : item_rows, 0u};
     }
-    for (uint32_t j = 0; tiles != nullptr && j < c; j += 8) tiles[tile_at++] = Tile{e, row_at + j, c - j < 8u ? c - j : 8u, 0u};
     row_at += c;
   }
   if (threadIdx.x == 1023) {
     offsets[experts] = row_sum[1023];
     n_items[0] = item_sum[1023];
-    n_items[1] = tile_sum[1023];
   }
 }
 
@@ -206,12 +179,12 @@ __global__ void __launch_bounds__(256) moe_scatter_kernel(const int32_t *ids, ui
 // Count, scan and scatter in one CTA for calls of a few rows (the decode widths): the three launches
 // above cost more than their work there. Counts and cursors live in shared memory.
 __global__ void __launch_bounds__(1024) moe_group_small_kernel(const int32_t *ids, uint32_t rows, uint32_t experts, uint32_t item_rows,
-                                                               uint32_t *offsets, uint32_t *n_items, Item *items, Tile *tiles,
+                                                               uint32_t *offsets, uint32_t *n_items, Item *items,
                                                                uint32_t *sorted, uint32_t *status) {
   griddep_launch_dependents();
   griddep_wait();
   __shared__ uint32_t counts[kSmallExperts], start[kSmallExperts];
-  __shared__ uint32_t row_sum[1024], item_sum[1024], tile_sum[1024];
+  __shared__ uint32_t row_sum[1024], item_sum[1024];
   for (uint32_t e = threadIdx.x; e < experts; e += 1024) counts[e] = 0u;
   __syncthreads();
   for (uint32_t a = threadIdx.x; a < rows; a += 1024) {
@@ -225,333 +198,41 @@ __global__ void __launch_bounds__(1024) moe_group_small_kernel(const int32_t *id
   __syncthreads();
   const uint32_t per = (experts + 1023u) / 1024u;
   const uint32_t e0 = threadIdx.x * per;
-  uint32_t nrows = 0, its = 0, tls = 0;
+  uint32_t nrows = 0, its = 0;
   for (uint32_t e = e0; e < e0 + per && e < experts; ++e) {
     nrows += counts[e];
     its += (counts[e] + item_rows - 1u) / item_rows;
-    tls += (counts[e] + 7u) / 8u;
   }
   row_sum[threadIdx.x] = nrows;
   item_sum[threadIdx.x] = its;
-  tile_sum[threadIdx.x] = tls;
   __syncthreads();
   for (uint32_t d = 1; d < 1024; d <<= 1) {
     const uint32_t r = threadIdx.x >= d ? row_sum[threadIdx.x - d] : 0u;
     const uint32_t i = threadIdx.x >= d ? item_sum[threadIdx.x - d] : 0u;
-    const uint32_t t = threadIdx.x >= d ? tile_sum[threadIdx.x - d] : 0u;
     __syncthreads();
     row_sum[threadIdx.x] += r;
     item_sum[threadIdx.x] += i;
-    tile_sum[threadIdx.x] += t;
     __syncthreads();
   }
-  uint32_t row_at = row_sum[threadIdx.x] - nrows, item_at = item_sum[threadIdx.x] - its, tile_at = tile_sum[threadIdx.x] - tls;
+  uint32_t row_at = row_sum[threadIdx.x] - nrows, item_at = item_sum[threadIdx.x] - its;
   for (uint32_t e = e0; e < e0 + per && e < experts; ++e) {
     offsets[e] = row_at;
     start[e] = row_at;
     const uint32_t c = counts[e];
     for (uint32_t j = 0; j < c; j += item_rows) {
-      items[item_at++] = Item{e, row_at + j, c - j < item_rows ? c - j : item_rows, tile_at + j / 8u};
+      items[item_at++] = Item{e, row_at + j, c - j < item_rows ? c - j : item_rows, 0u};
     }
-    for (uint32_t j = 0; tiles != nullptr && j < c; j += 8) tiles[tile_at++] = Tile{e, row_at + j, c - j < 8u ? c - j : 8u, 0u};
     row_at += c;
   }
   if (threadIdx.x == 1023) {
     offsets[experts] = row_sum[1023];
     n_items[0] = item_sum[1023];
-    n_items[1] = tile_sum[1023];
   }
   __syncthreads();
   for (uint32_t a = threadIdx.x; a < rows; a += 1024) {
     const int32_t e = ids[a];
     if (e < 0 || static_cast<uint32_t>(e) >= experts) continue;
     sorted[atomicAdd(&start[e], 1u)] = a;  // rows of one expert are independent: their order changes no output bit
-  }
-}
-
-// ---- the expert kernels ----------------------------------------------------------------------
-// Rotates the rows of one tile into B fragments, once per row: PHASE 0 x o suh of the gate/up
-// record, PHASE 1 silu(g) u o suh of the down record; then the 128-wide Hadamard in fp32, a
-// power-of-two scale per (row, block) (largest value in [2^13, 2^14)) and fp16. One CTA per tile,
-// warp r = row r; a block's fragment (2 KB) is put together in shared memory and written out whole.
-template <int PHASE>
-__global__ void __launch_bounds__(kThreads) moe_rotate_kernel(const __grid_constant__ ExpertParams p) {
-  __shared__ __align__(16) uint2 frag[2][256];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  griddep_launch_dependents();
-  griddep_wait();
-  const uint32_t tile_index = blockIdx.x;
-  if (tile_index >= p.n_items[1]) return;
-  const Tile tile = p.tiles[tile_index];
-  const ignis_moe_slot slot = p.slots[tile.expert * 2u + PHASE];
-  if (slot.record == nullptr || !(slot.k2 == 4 || slot.k2 == 5 || slot.k2 == 6 || slot.k2 == 8)) return;  // flagged by the walk
-  const uint32_t in = PHASE == 0 ? p.hidden : p.inter;
-  const uint32_t out_plane = PHASE == 0 ? 2u * p.inter : p.hidden;
-  const uint64_t trellis_bytes = static_cast<uint64_t>(in) * out_plane * slot.k2 / 16u;
-  const uint16_t *suh = reinterpret_cast<const uint16_t *>(static_cast<const uint8_t *>(slot.record) + trellis_bytes);
-  const uint32_t nblk = in / 128u;
-  const bool live = static_cast<uint32_t>(warp) < tile.count;
-  const uint32_t row = tile.first + static_cast<uint32_t>(warp);
-  uint32_t token = 0;
-  if (live && PHASE == 0) token = p.sorted[row] / p.top_k;
-  uint2 *dst_frag = (PHASE == 0 ? p.frag_in : p.frag_h) + static_cast<size_t>(tile_index) * nblk * 256u;
-  float2 *dst_scale = (PHASE == 0 ? p.scale_in : p.scale_h) + static_cast<size_t>(tile_index) * nblk * 8u;
-  for (uint32_t bl = 0; bl < nblk; ++bl) {
-    float v[4] = {0.f, 0.f, 0.f, 0.f};
-    if (live) {
-      const size_t k0 = static_cast<size_t>(bl) * 128u + 4u * lane;
-      const uint2 sb = *reinterpret_cast<const uint2 *>(suh + k0);
-      const __half2 s01 = *reinterpret_cast<const __half2 *>(&sb.x), s23 = *reinterpret_cast<const __half2 *>(&sb.y);
-      if (PHASE == 0) {
-        const uint2 xb = ldg64_coherent(p.x + static_cast<size_t>(token) * p.hidden + k0);
-        v[0] = bf16_bits_to_f32(xb.x & 0xFFFFu) * __low2float(s01);
-        v[1] = __uint_as_float(xb.x & 0xFFFF0000u) * __high2float(s01);
-        v[2] = bf16_bits_to_f32(xb.y & 0xFFFFu) * __low2float(s23);
-        v[3] = __uint_as_float(xb.y & 0xFFFF0000u) * __high2float(s23);
-      } else {
-        const float *g = p.gu + static_cast<size_t>(row) * 2u * p.inter + k0;
-        const uint4 gb = ldg128_coherent(g), ub = ldg128_coherent(g + p.inter);
-        const float gv[4] = {__uint_as_float(gb.x), __uint_as_float(gb.y), __uint_as_float(gb.z), __uint_as_float(gb.w)};
-        const float uv[4] = {__uint_as_float(ub.x), __uint_as_float(ub.y), __uint_as_float(ub.z), __uint_as_float(ub.w)};
-        const float sv[4] = {__low2float(s01), __high2float(s01), __low2float(s23), __high2float(s23)};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = gv[i] / (1.0f + __expf(-gv[i])) * uv[i] * sv[i];
-      }
-    }
-    hadamard128(v, lane);
-    float m = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
-    int shift = 0;
-    if (m > 0.0f && m <= 3.0e38f) {
-      int e;
-      (void)frexpf(m, &e);
-      shift = max(-126, min(126, 14 - e));
-    }
-    const float scale = ldexpf(1.0f, shift);
-    const __half2 h01 = __floats2half2_rn(v[0] * scale, v[1] * scale);
-    const __half2 h23 = __floats2half2_rn(v[2] * scale, v[3] * scale);
-    // element e = 4 lane + i of the block: step kt = e / 16, inside it k16 = e % 16; the reader
-    // lane (g = row, t) keeps k16 in {2t, 2t+1} in .x and {2t+8, 2t+9} in .y
-    const int kt = lane >> 2, k16 = (lane & 3) * 4;
-    const int t_first = (k16 & 7) >> 1, reg = k16 >> 3;
-    uint32_t *dst = reinterpret_cast<uint32_t *>(&frag[bl & 1][kt * 32 + warp * 4]);
-    dst[t_first * 2 + reg] = *reinterpret_cast<const uint32_t *>(&h01);
-    dst[(t_first + 1) * 2 + reg] = *reinterpret_cast<const uint32_t *>(&h23);
-    if (lane == 0) dst_scale[bl * 8u + warp] = make_float2(live ? ldexpf(1.0f, -shift) : 0.0f, scale);
-    __syncthreads();  // the block's fragment is whole; the other buffer is free for the next block
-    dst_frag[static_cast<size_t>(bl) * 256u + threadIdx.x] = frag[bl & 1][threadIdx.x];
-  }
-}
-
-__device__ __forceinline__ void cp_async16(void *smem_dst, const void *src) {
-  const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// What a CTA has staged of the item: kDepth slots, each one 128-input block - the packed words of the column block's 8 x 8 tiles
-// (eight contiguous rows of 128 k2 bytes), the fragments (2 KB per live row tile) and the (inverse scale, scale) pairs.
-template <int NT>
-struct Staging {
-  static constexpr int kDepth = NT == 1 ? 4 : 3;
-  static constexpr uint32_t kFrag = 8192, kScale = kFrag + NT * 2048, kSlot = kScale + NT * 64;
-  static constexpr uint32_t kBytes = kDepth * kSlot;
-};
-
-// Warp j of the CTA walks tile column j of the item's column block down all the inputs: one tile
-// per 16 inputs, decoded once and multiplied with every live row tile of the item (up to NT tiles
-// of 8 rows). The blocks to come are copied into the staging slots by all threads (one CTA barrier
-// per block). Sums are in the units of the current block's per-row scale and carried exactly into the
-// next block's. Bound by instruction issue: words that every lane read from global memory itself were
-// three loads with addresses of a runtime stride per tile, and one block ahead of their use.
-template <int K2, int NT>
-__device__ __forceinline__ void walk_tile_column(const uint8_t *col, uint64_t row_pitch, uint32_t nblk, const uint2 *frag,
-                                                 const float2 *scales, uint32_t ntiles, int warp, int lane, uint8_t *smem, float (&tot)[NT][4]) {
-  using S = Staging<NT>;
-  constexpr uint32_t kRowChunks = 8u * K2;   // 16-byte pieces of a tile row
-  const LaneWindow win = lane_window(K2, lane);
-  auto stage = [&](uint32_t bl, uint32_t slot) {
-    uint8_t *to = smem + slot * S::kSlot;
-    const uint8_t *from = col + static_cast<uint64_t>(bl) * 8u * row_pitch;
-#pragma unroll
-    for (uint32_t c0 = 0; c0 < 8u * kRowChunks; c0 += kThreads) {
-      const uint32_t c = c0 + threadIdx.x;
-      if (8u * kRowChunks % kThreads == 0u || c < 8u * kRowChunks) {
-        cp_async16(to + c * 16u, from + static_cast<uint64_t>(c / kRowChunks) * row_pitch + c % kRowChunks * 16u);
-      }
-    }
-    for (uint32_t c = threadIdx.x; c < ntiles * 128u; c += kThreads) {
-      const uint32_t tt = c >> 7, off = c & 127u;  // 16-byte chunk `off` of tile tt's fragment
-      cp_async16(to + S::kFrag + c * 16u, frag + (static_cast<size_t>(tt) * nblk + bl) * 256u + off * 2u);
-    }
-    if (threadIdx.x < ntiles * 4u) {
-      const uint32_t tt = threadIdx.x >> 2, off = threadIdx.x & 3u;
-      cp_async16(to + S::kScale + threadIdx.x * 16u, scales + (static_cast<size_t>(tt) * nblk + bl) * 8u + off * 2u);
-    }
-  };
-#pragma unroll
-  for (uint32_t d = 0; d + 1u < S::kDepth; ++d) {
-    if (d < nblk) stage(d, d);
-    cp_async_commit();
-  }
-  const int t2 = (lane & 3) * 2;
-  // the lane's words of the warp's tile column in a slot: tile row kt is 128 K2 bytes further
-  const uint8_t *w0 = smem + warp * 16 * K2 + 4u * win.w0, *w1 = smem + warp * 16 * K2 + 4u * win.w1, *w2 = smem + warp * 16 * K2 + 4u * win.w2;
-  float carry[NT][2];   // the previous block's inverse scales (nothing to carry at block 0)
-#pragma unroll
-  for (int tt = 0; tt < NT; ++tt) carry[tt][0] = carry[tt][1] = 0.0f;
-  uint32_t slot = 0, fill = S::kDepth - 1u;
-  for (uint32_t bl = 0; bl < nblk; ++bl) {
-    cp_async_wait<S::kDepth - 2>();
-    __syncthreads();  // this block's copies are visible; nobody still reads the slot refilled next
-    if (bl + S::kDepth - 1u < nblk) stage(bl + S::kDepth - 1u, fill);
-    cp_async_commit();
-    const uint32_t at = slot * S::kSlot;
-    const uint2 *fb = reinterpret_cast<const uint2 *>(smem + at + S::kFrag) + lane;
-    const float2 *cur = reinterpret_cast<const float2 *>(smem + at + S::kScale) + t2;
-    uint32_t w[3];   // the next tile's words, read while the current one is decoded
-    w[0] = *reinterpret_cast<const uint32_t *>(w0 + at);
-    w[1] = *reinterpret_cast<const uint32_t *>(w1 + at);
-    w[2] = *reinterpret_cast<const uint32_t *>(w2 + at);
-    // into this block's units: the sums so far are in the previous block's (inverse scale of the
-    // previous block times scale of this one, an exact power of two)
-#pragma unroll
-    for (int tt = 0; tt < NT; ++tt) {
-      if (static_cast<uint32_t>(tt) < ntiles) {  // uniform over the CTA
-        const float4 c = *reinterpret_cast<const float4 *>(cur + tt * 8);
-        const float f0 = carry[tt][0] * c.y, f1 = carry[tt][1] * c.w;
-        carry[tt][0] = c.x;
-        carry[tt][1] = c.z;
-        tot[tt][0] *= f0;
-        tot[tt][1] *= f1;
-        tot[tt][2] *= f0;
-        tot[tt][3] *= f1;
-      }
-    }
-#pragma unroll
-    for (int kt = 0; kt < 8; ++kt) {
-      const uint32_t a0 = w[0], a1 = w[1], a2 = w[2];
-      if (kt < 7) {
-        w[0] = *reinterpret_cast<const uint32_t *>(w0 + at + (kt + 1) * 128 * K2);
-        w[1] = *reinterpret_cast<const uint32_t *>(w1 + at + (kt + 1) * 128 * K2);
-        w[2] = *reinterpret_cast<const uint32_t *>(w2 + at + (kt + 1) * 128 * K2);
-      }
-      uint32_t a[4];
-      decode8<K2>(a0, a1, a2, win.off, a);
-#pragma unroll
-      for (int tt = 0; tt < NT; ++tt) {
-        if (static_cast<uint32_t>(tt) < ntiles) {
-          const uint2 b = fb[tt * 256 + kt * 32];
-          mma_f16_f32(tot[tt], a[0], a[2], a[1], a[3], b.x, b.y);
-        }
-      }
-    }
-    slot = slot + 1u == S::kDepth ? 0u : slot + 1u;
-    fill = fill + 1u == S::kDepth ? 0u : fill + 1u;
-  }
-  // back to the rows' own units
-#pragma unroll
-  for (int tt = 0; tt < NT; ++tt) {
-    tot[tt][0] *= carry[tt][0];
-    tot[tt][1] *= carry[tt][1];
-    tot[tt][2] *= carry[tt][0];
-    tot[tt][3] *= carry[tt][1];
-  }
-}
-
-// PHASE 0: gate | up products of an item into gu. PHASE 1: down, weighted, into acc.
-// One CTA per (item, block of 128 output columns); no CTA waits for another.
-template <int PHASE, int NT>
-__global__ void __launch_bounds__(kThreads, NT <= 2 ? 3 : 2) moe_experts_kernel(const __grid_constant__ ExpertParams p) {
-  // the staging slots, taken over after the walk by the partial sums [tile column 8][row tile NT][lane 32]
-  extern __shared__ __align__(128) uint8_t staging[];
-  float4 *part = reinterpret_cast<float4 *>(staging);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t in = PHASE == 0 ? p.hidden : p.inter;
-  const uint32_t out_plane = PHASE == 0 ? 2u * p.inter : p.hidden;   // columns of the stored plane
-  const uint32_t col_blocks = out_plane / 128u;
-  const uint32_t item_index = blockIdx.x / col_blocks;
-  const uint32_t col_block = blockIdx.x % col_blocks;
-
-  griddep_launch_dependents();
-  griddep_wait();  // the item list and the fragments come from the kernels before
-
-  if (item_index >= p.n_items[0]) return;
-  const Item item = p.items[item_index];
-  const ignis_moe_slot slot = p.slots[item.expert * 2u + PHASE];
-  const uint32_t k2 = slot.k2;
-  if (slot.record == nullptr || !(k2 == 4 || k2 == 5 || k2 == 6 || k2 == 8)) {
-    if (threadIdx.x == 0 && col_block == 0) atomicOr(p.status, kStatusAbsentRecord);
-    return;
-  }
-  const uint32_t *trellis = static_cast<const uint32_t *>(slot.record);
-  const uint64_t trellis_bytes = static_cast<uint64_t>(in) * out_plane * k2 / 16u;
-  const uint16_t *svh = reinterpret_cast<const uint16_t *>(static_cast<const uint8_t *>(slot.record) + trellis_bytes) + in;
-  const uint32_t nblk = in / 128u;
-  const uint32_t ntiles = (item.count + 7u) / 8u;
-  const uint2 *frag = (PHASE == 0 ? p.frag_in : p.frag_h) + static_cast<size_t>(item.tile_first) * nblk * 256u;
-  const float2 *scales = (PHASE == 0 ? p.scale_in : p.scale_h) + static_cast<size_t>(item.tile_first) * nblk * 8u;
-
-  float tot[NT][4];
-#pragma unroll
-  for (int tt = 0; tt < NT; ++tt)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) tot[tt][e] = 0.0f;
-  {
-    const uint8_t *col = reinterpret_cast<const uint8_t *>(trellis) + static_cast<uint64_t>(col_block) * 128u * k2;
-    const uint64_t pitch = static_cast<uint64_t>(out_plane) * k2;   // bytes from a tile row to the next
-    switch (k2) {
-      case 4: walk_tile_column<4, NT>(col, pitch, nblk, frag, scales, ntiles, warp, lane, staging, tot); break;
-      case 5: walk_tile_column<5, NT>(col, pitch, nblk, frag, scales, ntiles, warp, lane, staging, tot); break;
-      case 6: walk_tile_column<6, NT>(col, pitch, nblk, frag, scales, ntiles, warp, lane, staging, tot); break;
-      default: walk_tile_column<8, NT>(col, pitch, nblk, frag, scales, ntiles, warp, lane, staging, tot); break;
-    }
-  }
-  __syncthreads();  // every warp is done with the staging buffers: the partial sums take their place
-#pragma unroll
-  for (int tt = 0; tt < NT; ++tt) part[(warp * NT + tt) * 32 + lane] = make_float4(tot[tt][0], tot[tt][1], tot[tt][2], tot[tt][3]);
-  __syncthreads();
-
-  // ---- finish: rows dealt to the warps; lane = 4 output columns of the block ----
-  for (uint32_t r = static_cast<uint32_t>(warp); r < item.count; r += kWarps) {
-    const uint32_t tt = r >> 3, rs = r & 7u;
-    const int tq = static_cast<int>(rs >> 1), te = static_cast<int>(rs & 1u);
-    float v[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int c = 4 * lane + i, j = c >> 4, cc = c & 15;
-      v[i] = *(reinterpret_cast<const float *>(&part[(j * NT + tt) * 32 + (cc & 7) * 4 + tq]) + te + 2 * (cc >> 3));
-    }
-    hadamard128(v, lane);
-    const uint2 sv = *reinterpret_cast<const uint2 *>(svh + static_cast<size_t>(col_block) * 128u + 4u * lane);
-    const __half2 s01 = *reinterpret_cast<const __half2 *>(&sv.x), s23 = *reinterpret_cast<const __half2 *>(&sv.y);
-    v[0] *= __low2float(s01);
-    v[1] *= __high2float(s01);
-    v[2] *= __low2float(s23);
-    v[3] *= __high2float(s23);
-    const uint32_t row = item.first + r;
-    if (PHASE == 0) {
-      *reinterpret_cast<float4 *>(p.gu + static_cast<size_t>(row) * 2u * p.inter + col_block * 128u + 4u * lane) =
-          make_float4(v[0], v[1], v[2], v[3]);
-    } else {
-      const uint32_t a = p.sorted[row];
-      const uint32_t token = a / p.top_k;
-      const float wr = p.weights[a];
-      long long *dst = p.acc + static_cast<size_t>(token) * p.hidden + col_block * 128u + 4u * lane;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float c = wr * v[i];
-        if (!(fabsf(c) < 2147483648.0f)) {  // also catches NaN
-          atomicOr(p.status, kStatusRange);
-        } else {
-          atomicAdd(reinterpret_cast<unsigned long long *>(dst + i),
-                    static_cast<unsigned long long>(__double2ll_rn(static_cast<double>(c) * 4294967296.0)));
-        }
-      }
-    }
   }
 }
 
@@ -663,8 +344,6 @@ int32_t run_experts(const Geometry &g, const void *x, uint32_t tokens, const int
   uint8_t *base = static_cast<uint8_t *>(workspace->base);
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
   const uint32_t rows = tokens * g.top_k;
-  // the tensor-core route's items, or the warp-level kernels': 8 rows at decode widths, 64 beyond
-  const uint32_t item_rows = dev->moe_tc != 0 && l.down_fits ? kMoeTcItemRows : tokens > 8u ? 64u : 8u;
   uint32_t *counts = reinterpret_cast<uint32_t *>(base + l.counts);
   uint32_t *cursor = reinterpret_cast<uint32_t *>(base + l.cursor);
   uint32_t *offsets = reinterpret_cast<uint32_t *>(base + l.offsets);
@@ -673,18 +352,17 @@ int32_t run_experts(const Geometry &g, const void *x, uint32_t tokens, const int
   Item *items = reinterpret_cast<Item *>(base + l.items);
   uint32_t *status = reinterpret_cast<uint32_t *>(base + l.status);
   const bool pdl = dev->pdl != 0;
-  Tile *tiles = item_rows == kMoeTcItemRows ? nullptr : reinterpret_cast<Tile *>(base + l.tiles);
   cudaError_t err = cudaSuccess;
   if (rows <= kSmallRows && g.experts <= kSmallExperts) {
-    err = launch(moe_group_small_kernel, dim3(1), dim3(1024), 0, stream, pdl, ids, rows, g.experts, item_rows, offsets, n_items, items,
-                 tiles, sorted, status);
+    err = launch(moe_group_small_kernel, dim3(1), dim3(1024), 0, stream, pdl, ids, rows, g.experts, kMoeTcItemRows, offsets, n_items, items,
+                 sorted, status);
     if (err != cudaSuccess) return fail(slot, "%s: grouping launch failed: %s", what, cudaGetErrorString(err));
   } else {
   err = cudaMemsetAsync(counts, 0, l.offsets - l.counts, stream);  // counts and cursor
   if (err != cudaSuccess) return fail(slot, "%s: %s", what, cudaGetErrorString(err));
   const uint32_t grid_rows = (rows + 255u) / 256u < 1184u ? (rows + 255u) / 256u : 1184u;
   err = launch(moe_count_kernel, dim3(grid_rows), dim3(256), 0, stream, false, ids, rows, g.experts, counts, status);
-  if (err == cudaSuccess) err = launch(moe_scan_kernel, dim3(1), dim3(1024), 0, stream, pdl, static_cast<const uint32_t *>(counts), g.experts, item_rows, offsets, n_items, items, tiles);
+  if (err == cudaSuccess) err = launch(moe_scan_kernel, dim3(1), dim3(1024), 0, stream, pdl, static_cast<const uint32_t *>(counts), g.experts, kMoeTcItemRows, offsets, n_items, items);
   if (err == cudaSuccess) err = launch(moe_scatter_kernel, dim3(grid_rows), dim3(256), 0, stream, pdl, ids, rows, g.experts, static_cast<const uint32_t *>(offsets), cursor, sorted);
   if (err != cudaSuccess) return fail(slot, "%s: grouping launch failed: %s", what, cudaGetErrorString(err));
   }
@@ -693,16 +371,15 @@ int32_t run_experts(const Geometry &g, const void *x, uint32_t tokens, const int
   p.ids = ids;
   p.slots = slots;
   p.items = items;
-  p.tiles = reinterpret_cast<const Tile *>(base + l.tiles);
   p.n_items = n_items;
   p.sorted = sorted;
   p.x = static_cast<const uint16_t *>(x);
   p.weights = weights;
-  p.frag_in = reinterpret_cast<uint2 *>(base + l.frag_in);
-  p.scale_in = reinterpret_cast<float2 *>(base + l.scale_in);
+  p.x_rows = reinterpret_cast<uint16_t *>(base + l.x_rows);
+  p.x_scale = reinterpret_cast<float *>(base + l.x_scale);
   p.gu = reinterpret_cast<float *>(base + l.gu);
-  p.frag_h = reinterpret_cast<uint2 *>(base + l.frag_h);
-  p.scale_h = reinterpret_cast<float2 *>(base + l.scale_h);
+  p.h_rows = reinterpret_cast<uint16_t *>(base + l.h_rows);
+  p.h_scale = reinterpret_cast<float *>(base + l.h_scale);
   p.down_rows = reinterpret_cast<float *>(base + l.down_rows);
   p.acc = reinterpret_cast<long long *>(acc);
   p.status = status;
@@ -710,39 +387,15 @@ int32_t run_experts(const Geometry &g, const void *x, uint32_t tokens, const int
   p.inter = g.inter;
   p.top_k = g.top_k;
   p.experts = g.experts;
-  // Grids are sized for the worst case the host can know (the grouping happened on the device);
-  // CTAs beyond the item or tile count return at once.
-  const uint32_t items_max = items_bound(g, rows, item_rows);
-  if (item_rows == kMoeTcItemRows) {   // the tensor-core route
-    return moe_tc_experts(slot, *dev, p, rows, items_max, offsets, stream, what);
-  }
-  const uint32_t tiles_max = items_bound(g, rows, 8u);
-  const bool wide = item_rows > 8u;
-  for (int phase = 0; phase < 2; ++phase) {
-    const uint32_t col_blocks = (phase == 0 ? 2u * g.inter : g.hidden) / 128u;
-    err = phase == 0 ? launch(moe_rotate_kernel<0>, dim3(tiles_max), dim3(kThreads), 0, stream, pdl, p)
-                     : launch(moe_rotate_kernel<1>, dim3(tiles_max), dim3(kThreads), 0, stream, pdl, p);
-    if (err != cudaSuccess) return fail(slot, "%s: rotation launch failed: %s", what, cudaGetErrorString(err));
-    const dim3 grid(items_max * col_blocks);
-    if (phase == 0) {
-      err = wide ? launch(moe_experts_kernel<0, 8>, grid, dim3(kThreads), Staging<8>::kBytes, stream, pdl, p)
-                 : launch(moe_experts_kernel<0, 1>, grid, dim3(kThreads), Staging<1>::kBytes, stream, pdl, p);
-    } else {
-      err = wide ? launch(moe_experts_kernel<1, 8>, grid, dim3(kThreads), Staging<8>::kBytes, stream, pdl, p)
-                 : launch(moe_experts_kernel<1, 1>, grid, dim3(kThreads), Staging<1>::kBytes, stream, pdl, p);
-    }
-    if (err != cudaSuccess) return fail(slot, "%s: expert launch failed: %s", what, cudaGetErrorString(err));
-  }
-  return 0;
+  // The grid is sized for the worst case the host can know (the grouping happened on the device);
+  // CTAs beyond the item count return at once.
+  return moe_tc_experts(slot, *dev, p, rows, items_bound(g, rows, kMoeTcItemRows), offsets, stream, what);
 }
 
 }  // namespace
 
 int32_t prepare_moe_kernels(ErrorSlot &slot) {
   if (moe_rows_prepare(slot) != 0) return -1;
-  cudaError_t err = cudaFuncSetAttribute(moe_experts_kernel<0, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Staging<8>::kBytes));
-  if (err == cudaSuccess) err = cudaFuncSetAttribute(moe_experts_kernel<1, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Staging<8>::kBytes));
-  if (err != cudaSuccess) return fail(slot, "expert kernel attributes: %s", cudaGetErrorString(err));
   if (moe_tc_prepare(slot) != 0) return -1;
   return moe_fp8_tc_prepare(slot);
 }

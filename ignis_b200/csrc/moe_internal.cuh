@@ -1,4 +1,4 @@
-// Types shared by the MoE expert kernels (moe.cu) and their tensor-core form (moe_tc.cu).
+// Types shared by the MoE entry points and grouping (moe.cu) and the kernels behind them.
 #ifndef B200Q_MOE_INTERNAL_CUH
 #define B200Q_MOE_INTERNAL_CUH
 
@@ -11,14 +11,8 @@ namespace b200q {
 constexpr uint32_t kStatusBadExpert = 1u, kStatusAbsentRecord = 2u, kStatusRange = 4u;
 constexpr uint32_t kStatusTcWait = 8u;   // a bounded wait of the tensor-core expert kernels ran out
 
-// A work item: up to `item_rows` sorted rows of one expert (64 from the prefill entry, 8 from the
-// decode entry), i.e. up to 8 row tiles of 8.
+// A work item: up to kMoeTcItemRows sorted rows of one expert.
 struct Item {
-  uint32_t expert, first, count, tile_first;
-};
-// A row tile: 8 consecutive sorted rows of one expert (the MMA's N), the unit the activations are
-// rotated in.
-struct Tile {
   uint32_t expert, first, count, pad;
 };
 
@@ -26,27 +20,24 @@ struct ExpertParams {
   const int32_t *ids;        // expert of every assignment: [tokens][top_k]
   const ignis_moe_slot *slots;
   const Item *items;
-  const Tile *tiles;
-  const uint32_t *n_items;  // [0] items, [1] tiles
+  const uint32_t *n_items;  // items
   const uint32_t *sorted;   // row -> assignment index (token * top_k + rank)
   const uint16_t *x;        // BF16 [tokens][hidden]
   const float *weights;     // routing weights [tokens][top_k]
-  uint2 *frag_in;           // rotated x: [tile][hidden / 128][step 8][lane 32]
-  float2 *scale_in;         // (inverse scale, scale): [tile][hidden / 128][row 8]
+  uint16_t *x_rows;         // rotated x: fp16 [rows][hidden]
+  float *x_scale;           // inverse scale per row
   float *gu;                // fp32 [rows][2 inter]: gate | up products
-  uint2 *frag_h;            // rotated silu(g) u: [tile][inter / 128][step 8][lane 32]
-  float2 *scale_h;
-  float *down_rows;         // fp32 [tokens][top_k][hidden]: the weighted down products of the tensor-core route, before they are added
+  uint16_t *h_rows;         // rotated silu(g) u: fp16 [rows][inter]
+  float *h_scale;
+  float *down_rows;         // fp32 [tokens][top_k][hidden]: the weighted down products, before they are added
   long long *acc;           // int64 [tokens][hidden]
   uint32_t *status;
   uint32_t hidden, inter, top_k, experts;
 };
 
 
-// The routed experts of a wide call on the tensor cores (moe_tc.cu): rows rotated once into fp16
-// rows with one scale per row, items of up to 256 rows multiplied with their expert's records by
-// tcgen05. `p` as for the warp-level kernels; frag_in / scale_in and frag_h / scale_h hold the
-// rotated rows and their inverse scales instead of fragments.
+// The routed experts on the tensor cores (moe_tc.cu): rows rotated once into fp16 rows with one
+// scale per row, items multiplied with their expert's records by tcgen05.
 int32_t moe_tc_prepare(ErrorSlot &slot);
 constexpr uint32_t kMoeTcItemRows = 192;
 int32_t moe_tc_experts(ErrorSlot &slot, const DeviceState &dev, const ExpertParams &p, uint32_t rows, uint32_t items_max,

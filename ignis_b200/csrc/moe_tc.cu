@@ -1,7 +1,8 @@
-// The routed experts of wide calls on the tensor cores.
+// The routed experts on the tensor cores.
 //
 // Stands where the reference's prefill entry multiplies items of up to 64 rows with warp-level MMAs
-// (kernel/src/moe_prefill.cu:252-262, kernels :405 and :421). Under skewed routing a few experts see
+// (kernel/src/moe_prefill.cu:252-262, kernels :405 and :421) and its decode entry walks the records
+// with vector dot products (moe_decode.cu:325-399). Under skewed routing a few experts see
 // hundreds of rows; here a work item is up to 192 sorted rows of one expert, and every item is
 // multiplied with its expert's record by the kernel core of trellis_tc.cuh: the rows rotated once
 // into plain fp16 rows with one scale per row, the record's trellis tiles decoded into
@@ -38,7 +39,7 @@ __global__ void __launch_bounds__(THREADS) moe_tc_rotate_x_kernel(const __grid_c
   griddep_wait();
   const uint32_t in = p.hidden;
   const uint32_t rows = offsets[p.experts];   // fewer than the launch may have been sized for
-  float *const inv = reinterpret_cast<float *>(p.scale_in);
+  float *const inv = p.x_scale;
   struct Source {
     uint32_t a;
     ignis_moe_slot slot;
@@ -55,7 +56,7 @@ __global__ void __launch_bounds__(THREADS) moe_tc_rotate_x_kernel(const __grid_c
   for (uint32_t row = blockIdx.x, turn = 0; row < rows; row += gridDim.x, turn ^= 1u) {
     const Source next = source(row + gridDim.x);
     const ignis_moe_slot slot = here.slot;
-    uint16_t *const to = reinterpret_cast<uint16_t *>(p.frag_in) + static_cast<size_t>(row) * in;
+    uint16_t *const to = p.x_rows + static_cast<size_t>(row) * in;
     if (slot.record == nullptr || !(slot.k2 == 4 || slot.k2 == 5 || slot.k2 == 6 || slot.k2 == 8)) {
       // an absent record: the product kernel flags it and skips the item; leave finite rows behind
       for (uint32_t i = threadIdx.x * 4u; i < in; i += 4u * blockDim.x) *reinterpret_cast<uint2 *>(to + i) = make_uint2(0u, 0u);
@@ -89,8 +90,8 @@ __global__ void __launch_bounds__(kRotateThreads) moe_tc_rotate_h_kernel(const _
   const uint32_t expert = static_cast<uint32_t>(p.ids[a]);
   const ignis_moe_slot slot = p.slots[expert * 2u + 1u];
   const uint32_t in = p.inter;
-  uint16_t *dst = reinterpret_cast<uint16_t *>(p.frag_h) + static_cast<size_t>(row) * in;
-  float *inv = reinterpret_cast<float *>(p.scale_h) + row;
+  uint16_t *dst = p.h_rows + static_cast<size_t>(row) * in;
+  float *inv = p.h_scale + row;
   if (slot.record == nullptr || !(slot.k2 == 4 || slot.k2 == 5 || slot.k2 == 6 || slot.k2 == 8)) {
     // an absent record: the product kernel flags it and skips the item; leave finite rows behind
     for (uint32_t i = threadIdx.x * 4u; i < in; i += 4u * kRotateThreads) *reinterpret_cast<uint2 *>(dst + i) = make_uint2(0u, 0u);
@@ -172,7 +173,7 @@ __global__ void __launch_bounds__(Shape<2>::kThreads, 2) moe_tc_gemm_kernel(cons
   const Core c = core_setup<2>(smem_raw, job, kWhole);
   const uint64_t trellis_bytes = static_cast<uint64_t>(in) * out_plane * slot.k2 / 16u;
   const uint16_t *svh = reinterpret_cast<const uint16_t *>(static_cast<const uint8_t *>(slot.record) + trellis_bytes) + in;
-  const float *inv_rows = reinterpret_cast<const float *>(PHASE == 0 ? p.scale_in : p.scale_h);
+  const float *inv_rows = PHASE == 0 ? p.x_scale : p.h_scale;
   const bool decoded = core_roles<2>(c, job, &map_rows, p.status + 1);   // word 1 of the status line: waits of this kernel that ran out
   struct Row {
     float *y;
@@ -277,7 +278,7 @@ int32_t moe_tc_experts(ErrorSlot &slot, const DeviceState &dev, const ExpertPara
                                           dim3(threads), 0, stream, pdl, p, offsets);
     if (err != cudaSuccess) return fail(slot, "%s: rotation launch failed: %s", what, cudaGetErrorString(err));
     CUtensorMap map_rows;
-    if (!make_rows_map(&map_rows, phase == 0 ? static_cast<const void *>(p.frag_in) : static_cast<const void *>(p.frag_h), rows, in, kBoxRows)) {
+    if (!make_rows_map(&map_rows, phase == 0 ? p.x_rows : p.h_rows, rows, in, kBoxRows)) {
       return fail(slot, "%s: tensor map encoding failed", what);
     }
     const dim3 grid(items_max * (out_plane / 128u));

@@ -25,8 +25,8 @@
  * large for the accumulator does not trap the kernel as the reference's does (ignis_moe.h:76-81,
  * :166-170): the contribution is skipped and a bit is set in the workspace's status word, which
  * ignis_moe_workspace_status reads back. Both routes (decode, prefill) run the same grouped
- * kernels: assignments are grouped by expert on the device, work items of at most 8 rows each
- * decode their expert's tiles once; `decode_route` is accepted and ignored.
+ * kernels: assignments are grouped by expert on the device, work items of at most 192 rows
+ * each decode their expert's tiles once; `decode_route` is accepted and ignored.
  */
 #ifndef IGNIS_MOE_H
 #define IGNIS_MOE_H
