@@ -6,8 +6,11 @@
 //
 //  * The weights are the MMA's A operand: a CTA owns 128 weight rows (M) and up to 128 tokens (N, as few as the
 //    call has, in steps of 16) and walks a slice of K in stages of 256 values; the CTAs of a cluster
-//    split K, so that narrow weights fill the device too, and add their sums through distributed
-//    shared memory in rank order.
+//    split K, so that narrow weights fill the device too. Each pushes its sums (st.async) to the CTA
+//    that finishes the token, which adds them in rank order: nothing waits for a remote read's round
+//    trip, and no CTA waits for the others' ends. Four tokens of a row go in one store: a layer at 33 / 77 / 128
+//    tokens takes 56.1 / 67.7 / 79.3 us, 58.1 / 71.0 / 83.8 where the finishing CTA reads its peers' sums, and
+//    58.9 / 73.4 / 86.9 with one token a store.
 //  * Warp 8 brings a stage's weight codes and token codes by TMA (128-byte swizzle) and their scale tiles by
 //    bulk copies; the weights' first stages are requested before the wait for the kernel that quantizes.
 //  * Warp 9 owns tensor memory, copies a stage's scale tiles there and issues its MMAs, in the pipe's order, from
@@ -75,9 +78,9 @@ __global__ void __launch_bounds__(kNarrowThreads, 2) w4a4_narrow_kernel(const __
   // a stage: weight codes [TILES] | token codes | weight scales [TILES] | token scales
   const uint32_t sf_off = TILES * kABytes + x_bytes;
   const uint32_t stage_bytes = sf_off + (TILES + 1) * kSfBytes, stage_pitch = (stage_bytes + 1023u) & ~1023u;
-  const uint32_t bars = base + p.stages * stage_pitch;   // full[stages], empty[stages], accumulator full; then the TMEM slot
-  const uint32_t bar_empty = bars + 8u * p.stages, bar_acc = bar_empty + 8u * p.stages;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(base_ptr + (bar_acc - base) + 8u);
+  const uint32_t bars = base + p.stages * stage_pitch;   // full[stages], empty[stages], accumulator full, sums here; then the TMEM slot
+  const uint32_t bar_empty = bars + 8u * p.stages, bar_acc = bar_empty + 8u * p.stages, bar_sums = bar_acc + 8u;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(base_ptr + (bar_acc - base) + 16u);
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank(), kc = p.kc;
 
@@ -108,6 +111,11 @@ __global__ void __launch_bounds__(kNarrowThreads, 2) w4a4_narrow_kernel(const __
       mbar_init(bar_empty + 8 * s, 1);
     }
     mbar_init(bar_acc, 1);
+    mbar_init(bar_sums, 1);
+    if (kc > 1u) {   // quads of tokens are dealt over the ranks; every rank pushes its sums of this one's
+      const uint32_t quads = (live + 3u) / 4u;
+      mbar_expect_tx(bar_sums, (quads + kc - 1u - rank) / kc * kc * TILES * 2048u);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kEpiWarps + 1) {
@@ -216,8 +224,10 @@ __global__ void __launch_bounds__(kNarrowThreads, 2) w4a4_narrow_kernel(const __
   const uint32_t r = quad * 32u + static_cast<uint32_t>(lane), row = row_a + r;
   const uint32_t lane_base = tmem + ((quad * 32u) << 16);
   const bool quantize = TILES == 2 && (p.epilogue & kEpilogueQuant) != 0u;
-  float *part = reinterpret_cast<float *>(base_ptr);   // [tile][token][128] partial sums, over the (by then idle) ring
-  __nv_bfloat16 *h_tile = reinterpret_cast<__nv_bfloat16 *>(base_ptr + (kc > 1u ? TILES * p.tile * 512u : 0u));   // quantized form: [token][row 128]
+  // Over the (by then idle) ring: partial sums of this rank's tokens, [source rank][turn][tile][row 128][token 4]; behind
+  // them h of the quantized form, [token][row 128].
+  const uint32_t turns = (p.tile / 4u + kc - 1u) / kc;
+  __nv_bfloat16 *h_tile = reinterpret_cast<__nv_bfloat16 *>(base_ptr + (kc > 1u ? kc * turns * TILES * 2048u : 0u));
   constexpr uint32_t kHPitch = 136;   // values: 16-byte rows, a quarter-warp's 16-byte reads on different banks
   bool have = false;
   if (warp < kEpiWarps) {
@@ -226,7 +236,22 @@ __global__ void __launch_bounds__(kNarrowThreads, 2) w4a4_narrow_kernel(const __
     if (!have && lane == 0) atomicOr(p.status, kEpilogueTimeout);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   }
-  auto emit = [&](uint32_t tl, float va, float vb) {   // token tl of the tile
+  // What the residual add finds in the output, as the stored type's bits: `n` tokens from `first` on (past the last one: the
+  // last), requested together before any of them is needed. One at a time, each with its own branches, they are round trips
+  // one after another.
+  const bool add = TILES == 1 && (p.epilogue & kEpilogueAdd) != 0u, f32 = (p.epilogue & kEpilogueF32) != 0u;
+  auto request = [&](auto &bits, uint32_t first) {
+    if (!add) return;
+    constexpr uint32_t n = sizeof(bits) / 4u;
+    if (f32) {
+#pragma unroll
+      for (uint32_t j = 0; j < n; ++j) bits[j] = static_cast<const uint32_t *>(W.y)[static_cast<size_t>(tok0 + min(first + j, live - 1u)) * W.ldy + row];
+    } else {
+#pragma unroll
+      for (uint32_t j = 0; j < n; ++j) bits[j] = static_cast<const uint16_t *>(W.y)[static_cast<size_t>(tok0 + min(first + j, live - 1u)) * W.ldy + row];
+    }
+  };
+  auto emit = [&](uint32_t tl, float va, float vb, uint32_t bits) {   // token tl of the tile
     if (quantize) {
       h_tile[tl * kHPitch + r] = swiglu_bf16(va, vb, W.alpha);
       return;
@@ -237,76 +262,92 @@ __global__ void __launch_bounds__(kNarrowThreads, 2) w4a4_narrow_kernel(const __
       return;
     }
     const float val = __fmul_rn(va, W.alpha);   // not contracted into the residual add: one value for every epilogue
-    if (p.epilogue & kEpilogueF32) {
-      float *y = static_cast<float *>(W.y);
-      y[at] = (p.epilogue & kEpilogueAdd) ? y[at] + val : val;
+    const float old = __uint_as_float(f32 ? bits : bits << 16);
+    if (f32) {
+      static_cast<float *>(W.y)[at] = add ? old + val : val;
     } else {
-      __nv_bfloat16 *y = static_cast<__nv_bfloat16 *>(W.y);
-      y[at] = __float2bfloat16_rn((p.epilogue & kEpilogueAdd) ? val + __bfloat162float(y[at]) : val);
+      static_cast<__nv_bfloat16 *>(W.y)[at] = __float2bfloat16_rn(add ? val + old : val);
     }
   };
   if (kc == 1u) {
     if (warp < kEpiWarps && have) {
       for (uint32_t c = group * 16u; c < live; c += 32u) {
         uint32_t v[16], u[16];
+        uint32_t old[16] = {};
         tmem_ld16(lane_base + c, v);
         if (TILES == 2) tmem_ld16(lane_base + p.acc_stride + c, u);
+        request(old, c);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-          if (c + j < live) emit(c + j, __uint_as_float(v[j]), TILES == 2 ? __uint_as_float(u[j]) : 0.0f);
+          if (c + j < live) emit(c + j, __uint_as_float(v[j]), TILES == 2 ? __uint_as_float(u[j]) : 0.0f, old[j]);
         }
       }
     }
   } else {
-    __syncthreads();   // every role is done with the ring: the partial sums take its place
-    float *part_b = part + static_cast<size_t>(p.tile) * 128u;
+    uint32_t old[4] = {};   // a quad's, requested before its sums are here
+    if (warp < kEpiWarps) request(old, 4u * (group * kc + rank));
+    __syncwarp();
+    cluster_sync_all();   // every role of every rank is done with its ring
     if (warp < kEpiWarps) {
-      for (uint32_t c = group * 16u; c < mma_n; c += 32u) {
+      for (uint32_t c = group * 16u; c < live; c += 32u) {
         uint32_t v[16], u[16];
         if (have) {
           tmem_ld16(lane_base + c, v);
           if (TILES == 2) tmem_ld16(lane_base + p.acc_stride + c, u);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         }
+        uint32_t to = (c >> 2) % kc, turn = (c >> 2) / kc;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          part[static_cast<size_t>(c + j) * 128u + r] = have ? __uint_as_float(v[j]) : 0.0f;
-          if (TILES == 2) part_b[static_cast<size_t>(c + j) * 128u + r] = have ? __uint_as_float(u[j]) : 0.0f;
+        for (uint32_t j = 0; j < 16u; j += 4u) {
+          if (c + j >= live) break;
+          const uint32_t at = base + ((rank * turns + turn) * TILES * 128u + r) * 16u, bar = cluster_map(bar_sums, to);
+          auto sums4 = [&](const uint32_t (&w)[16]) {
+            return have ? make_float4(__uint_as_float(w[j]), __uint_as_float(w[j + 1u]), __uint_as_float(w[j + 2u]), __uint_as_float(w[j + 3u]))
+                        : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          };
+          push_f32x4(cluster_map(at, to), sums4(v), bar);
+          if (TILES == 2) push_f32x4(cluster_map(at + 2048u, to), sums4(u), bar);
+          if (++to == kc) to = 0u, ++turn;
         }
+      }
+      // the rank's quads, every other one to a group of warps; partial sums added in rank order
+      const float4 *sums = reinterpret_cast<const float4 *>(base_ptr) + r;
+      if (mbar_wait_pushed(bar_sums)) {
+        for (uint32_t turn = group; 4u * (turn * kc + rank) < live; turn += 2u) {
+          if (turn != group) request(old, 4u * (turn * kc + rank));
+          const float4 *from = sums + turn * TILES * 128u;
+          float4 sum_a = from[0], sum_b = TILES == 2 ? from[128] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          for (uint32_t q = 1; q < kc; ++q) {
+            from += turns * TILES * 128u;
+            const float4 more = from[0];
+            sum_a.x += more.x, sum_a.y += more.y, sum_a.z += more.z, sum_a.w += more.w;
+            if (TILES == 2) {
+              const float4 more_b = from[128];
+              sum_b.x += more_b.x, sum_b.y += more_b.y, sum_b.z += more_b.z, sum_b.w += more_b.w;
+            }
+          }
+          const uint32_t tl = 4u * (turn * kc + rank);
+          emit(tl, sum_a.x, sum_b.x, old[0]);
+          if (tl + 1u < live) emit(tl + 1u, sum_a.y, sum_b.y, old[1]);
+          if (tl + 2u < live) emit(tl + 2u, sum_a.z, sum_b.z, old[2]);
+          if (tl + 3u < live) emit(tl + 3u, sum_a.w, sum_b.w, old[3]);
+        }
+      } else if (lane == 0) {
+        atomicOr(p.status, kEpilogueTimeout);
       }
     }
     __syncwarp();
-    cluster_sync_all();
-    if (warp < kEpiWarps) {
-      // tokens dealt over the cluster's CTAs and their groups of warps; partial sums added in rank order
-      for (uint32_t tl = 2u * rank + group; tl < live; tl += 2u * kc) {
-        float pa[8], pb[8];
-#pragma unroll
-        for (uint32_t q = 0; q < 8u; ++q) {   // requested together
-          pa[q] = q < kc ? ld_cluster_f32(part + static_cast<size_t>(tl) * 128u + r, q) : 0.0f;
-          pb[q] = TILES == 2 && q < kc ? ld_cluster_f32(part_b + static_cast<size_t>(tl) * 128u + r, q) : 0.0f;
-        }
-        float sum_a = pa[0], sum_b = pb[0];
-#pragma unroll
-        for (uint32_t q = 1; q < 8u; ++q) {
-          if (q < kc) sum_a += pa[q], sum_b += pb[q];
-        }
-        emit(tl, sum_a, sum_b);
-      }
-    }
-    __syncwarp();
-    cluster_sync_all();   // no CTA leaves while a peer may still read its partial sums
   }
   if (quantize) {
     // This CTA's tokens of h, in blocks of 16 along the next product's K (this tile's 128 rows are 8 blocks), quantized as
     // the standalone quantizer would from the BF16 values. Columns past the call's tokens are never read as outputs.
     __syncthreads();
     const uint32_t inter = W.n / 2u;
-    const uint32_t mine = kc == 1u ? live : (live + 2u * kc - 1u) / (2u * kc) * 2u;   // an upper bound of this CTA's tokens
+    const uint32_t mine = kc == 1u ? live : turns * 4u;   // an upper bound of this CTA's tokens
     for (uint32_t i = threadIdx.x; i < mine * 8u; i += kNarrowThreads) {
       const uint32_t j = i >> 3, b = i & 7u;
-      const uint32_t tl = kc == 1u ? j : (j >> 1) * 2u * kc + 2u * rank + (j & 1u);
+      const uint32_t tl = kc == 1u ? j : ((j >> 2) * kc + rank) * 4u + (j & 3u);
       if (tl >= live) continue;
       const uint4 *src = reinterpret_cast<const uint4 *>(h_tile + tl * kHPitch + b * 16u);
       uint2 codes;
@@ -354,7 +395,7 @@ NarrowPlan narrow_plan(const DeviceState &dev, uint32_t row_tiles, uint32_t k_st
 
 // Bytes behind the ring's start that the epilogue needs.
 size_t narrow_epilogue_bytes(const NarrowPlan &pl, bool quant) {
-  return (pl.kc > 1u ? static_cast<size_t>(pl.tiles) * pl.tile * 512u : 0u) + (quant ? static_cast<size_t>(pl.tile) * 272u : 0u);
+  return (pl.kc > 1u ? static_cast<size_t>(pl.kc) * ((pl.tile / 4u + pl.kc - 1u) / pl.kc) * pl.tiles * 2048u : 0u) + (quant ? static_cast<size_t>(pl.tile) * 272u : 0u);
 }
 
 }  // namespace

@@ -915,6 +915,31 @@ def test_w4a4_mlp_quantizes_as_its_parts_do(nv, w4a4_kernel, tokens, k, inter, n
     assert ws.status() == 0 and parts.status() == 0
 
 
+@pytest.mark.parametrize("tokens", [33, 36, 49, 66, 95, 127])   # quads of tokens dealt over the ranks: a last one of 1 to 4, ranks with one more than others
+@pytest.mark.parametrize("n,k", [(128, 1024), (128, 1536), (128, 2816), (384, 4352)])   # clusters of 1 to 4 CTAs and of 8, unequal slices
+def test_w4a4_narrow_cluster_sums(nv, oracle, monkeypatch, tokens, n, k):
+    """The sums that the CTAs of a cluster push to each other: STORE, and ADD in FP32 and BF16 onto values that are there."""
+    monkeypatch.setenv("B200Q_W4A4_PAIR", "0")
+    nv.prepare()
+    rng = np.random.default_rng(tokens + n + k)
+    codes, scales, d_w = make_weight(rng, n, k)
+    w = nv.Weight.from_planes(codes, scales, d_w, 448.0)
+    gen = torch.Generator().manual_seed(k + tokens)
+    x = torch.randn(tokens, k, generator=gen).to(torch.bfloat16)
+    ref = w4a4_reference(oracle, codes, scales, n, k, d_w, 448.0, x)
+    ws = nv.Workspace(nv.workspace_bytes(n, k, nv.ALLOW_A4, tokens))
+    plain = nv.linear(x.cuda(), w, policy=nv.ALLOW_A4, epilogue=nv.OUT_F32, workspace=ws)
+    check_f32(plain, ref)
+    base = torch.randn(tokens, n, generator=gen)
+    y = base.to(torch.bfloat16).cuda()
+    want = (plain + y.float()).to(torch.bfloat16)   # the same product, one FP32 addition, rounded once
+    nv.linear(x.cuda(), w, y, policy=nv.ALLOW_A4, epilogue=nv.ADD, workspace=ws)
+    assert torch.equal(y, want)
+    assert ws.status() == 0
+    monkeypatch.undo()
+    nv.prepare()
+
+
 def test_w4a4_kernels_agree_where_both_walk_k_in_one_piece(nv, oracle, monkeypatch):
     """The narrow kernel without a K split and the pair GEMM add a product's K in the same order: the same BF16 outputs, bit for bit."""
     tokens, n, k = 300, 640, 1024
