@@ -499,21 +499,19 @@ struct QuantTarget {
   float d_in = 1.0f;
 };
 
-// Which kernel a product takes: the cheaper by a model of each, in SM cycles. The pair kernel: waves of
-// 256 x 256 tiles on half as many pairs as SMs, 820 cycles a stage of 256 and 3000 a tile, never faster than
-// the weights come from HBM; `w4a4_narrow_cycles` beside its kernel. Both forced, the products of a 27B-style layer with
-// their quantizer, in us, narrow / pair:
-//   tokens     q|k|v         o            gate|up       down
-//      33    9.9 / 14.0    8.3 / 15.2   19.5 / 36.7   13.5 / 31.2
-//     128   15.1 / 15.7   12.1 / 18.8   26.2 / 39.6   17.5 / 36.1
-//     200   13.1 / 16.9   13.7 / 19.4   42.9 / 39.8   24.2 / 36.5
-//     300   22.3 / 18.6   14.0 / 20.9   61.2 / 61.4   26.5 / 36.8
-//     384   24.1 / 18.8   14.6 / 21.3   63.2 / 62.0   27.5 / 38.4
-//     512   25.0 / 19.1   25.8 / 21.6   82.2 / 62.4   48.8 / 39.8
-// Up to 128 tokens the models take the narrow kernel for all four, beyond them the pair kernel. That is the faster one up to 128
-// and from 512; between them it is for gate|up and, from 300, q|k|v, but not for o and down (up to 1.5 times the
-// narrow kernel's time): the narrow model charges every CTA the share of the L2 that an SM has when all of them pull, also
-// where a launch has 80 CTAs.
+// Which kernel a product takes: the cheaper by a model of each, in SM cycles, fitted to products whose weights come from HBM.
+// The pair kernel: waves of 256 x 256 tiles on half as many pairs as SMs, 820 cycles a stage of 256 and 3000 a tile (a gate|up
+// parent, whose epilogue multiplies, rounds and quantizes: 8600, and 47 500 a launch), never faster than the weights
+// come from HBM; `w4a4_narrow_cycles` beside its kernel. The narrow kernel has to be ahead by 15 %: where the models are that
+// close, products on different kernels in a row cost more (200 tokens: gate|up on the pair kernel and down on the narrow one
+// 89 us, both on the narrow one 71, both on the pair kernel 85).
+// Both forced, an MLP with its residual, in us, narrow / pair, the rule's choice last:
+//   tokens   5120 x 17408          4096 x 14336          2048 x 6144
+//     128    44.8 /  84.6 n        38.5 /  76.0 n        26.4 / 39.7 n
+//     200    70.9 /  84.8 n        61.2 /  77.4 n        28.2 / 39.5 n
+//     384    93.6 / 113.0 n        84.5 / 104.4 n        39.4 / 53.3 n
+//     640   158.6 / 144.8 p       124.6 / 120.9 p        48.9 / 53.8 n
+//    1024   244.3 / 197.8 p       182.9 / 142.7 p        65.3 / 68.3 n
 bool narrow_is_cheaper(const DeviceState &dev, const A4Item *items, uint32_t count, uint32_t k, uint32_t tokens, bool swiglu) {
   if (dev.w4a4_pair >= 0) return dev.w4a4_pair == 0;
   uint32_t row_tiles = 0, n_tiles = 0;
@@ -522,9 +520,9 @@ bool narrow_is_cheaper(const DeviceState &dev, const A4Item *items, uint32_t cou
     n_tiles += (items[i].n + 255u) / 256u;
   }
   const double tiles = static_cast<double>(n_tiles) * ((tokens + 255u) / 256u);
-  const double walk = ceil(tiles / (dev.sm_count / 2)) * ((k / 256u) * 820.0 + 3000.0);
+  const double walk = ceil(tiles / (dev.sm_count / 2)) * ((k / 256u) * 820.0 + (swiglu ? 8600.0 : 3000.0)) + (swiglu ? 47500.0 : 0.0);
   const double stream = row_tiles * (swiglu ? 144.0 : 72.0) * k / 3150.0;
-  return w4a4_narrow_cycles(dev, row_tiles, k, tokens, swiglu) < 5000.0 + (walk > stream ? walk : stream);
+  return w4a4_narrow_cycles(dev, row_tiles, k, tokens, swiglu) * 1.15 < 8500.0 + (walk > stream ? walk : stream);
 }
 
 int32_t quantize_rows(ErrorSlot &slot, const DeviceState &dev, const uint16_t *x, uint32_t tokens, uint32_t k, float d_in, uint8_t *codes,

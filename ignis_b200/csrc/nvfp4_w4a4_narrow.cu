@@ -411,7 +411,10 @@ double w4a4_narrow_cycles(const DeviceState &dev, uint32_t row_tiles, uint32_t k
   const uint32_t k_stages = k / 256u;
   const NarrowPlan pl = narrow_plan(dev, row_tiles, k_stages, tokens, swiglu);
   const double ctas = static_cast<double>(row_tiles) * ((tokens + pl.tile - 1u) / pl.tile) * pl.kc;
-  const double stage = narrow_pitch(pl) / 42.0;   // what an SM brings from the L2 in a cycle
+  // What an SM brings from the L2 in a cycle: 42 bytes when all of them pull, up to 64 when fewer do (5120 x 17408 at 160 and 320
+  // tokens, 80 and 120 CTAs: 27.3 and 29.7 us). The waves of a gate|up parent beyond the first: 28 (20 us each at 34816 x 5120).
+  const double share = 42.0 * dev.sm_count / (ctas < dev.sm_count ? ctas : dev.sm_count);
+  const double stage = narrow_pitch(pl) / (swiglu && ctas > dev.sm_count ? 28.0 : share < 64.0 ? share : 64.0);
   const double walk = ceil(ctas / dev.sm_count) * (ceil(static_cast<double>(k_stages) / pl.kc) * (stage > 350.0 ? stage : 350.0) + 4000.0 + (pl.kc > 1u ? 2000.0 : 0.0));
   const double stream = row_tiles * pl.tiles * 72.0 * k / 3150.0;   // the weights at the rate of HBM, per cycle of 1.9 GHz
   return 4000.0 + (walk > stream ? walk : stream);
