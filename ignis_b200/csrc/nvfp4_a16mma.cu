@@ -129,14 +129,28 @@ __device__ __forceinline__ void mma_f16_ts(uint32_t d, uint32_t a, uint64_t b, u
 }
 
 // `coef`: the weight's inverse divisor times what the A tiles leave out.
-__device__ __forceinline__ void a16_store(const A16Weight &W, uint32_t epilogue, size_t at, float acc, float coef) {
+// `bits`: what the residual add found there, as the stored type's bits.
+__device__ __forceinline__ void a16_store(const A16Weight &W, uint32_t epilogue, size_t at, float acc, float coef, uint32_t bits) {
   const float val = __fmul_rn(acc, coef);  // not contracted into the residual add: one value for every epilogue
+  const float old = __uint_as_float((epilogue & kEpilogueF32) ? bits : bits << 16);
   if (epilogue & kEpilogueF32) {
-    float *y = static_cast<float *>(W.y);
-    y[at] = (epilogue & kEpilogueAdd) ? y[at] + val : val;
+    static_cast<float *>(W.y)[at] = (epilogue & kEpilogueAdd) ? old + val : val;
   } else {
-    __nv_bfloat16 *y = static_cast<__nv_bfloat16 *>(W.y);
-    y[at] = __float2bfloat16_rn((epilogue & kEpilogueAdd) ? val + __bfloat162float(y[at]) : val);
+    static_cast<__nv_bfloat16 *>(W.y)[at] = __float2bfloat16_rn((epilogue & kEpilogueAdd) ? val + old : val);
+  }
+}
+// The residuals of several of a tile's `live` tokens, `step` apart (past the last one: the last), requested together before any
+// of them is needed. One at a time, each behind its own branches, they are round trips one after another.
+template <int N>
+__device__ __forceinline__ void a16_residuals(uint32_t (&bits)[N], const A16Weight &W, uint32_t epilogue, size_t row, uint32_t tok0, uint32_t first,
+                                              uint32_t step, uint32_t live) {
+  if (!(epilogue & kEpilogueAdd)) return;
+  if (epilogue & kEpilogueF32) {
+#pragma unroll
+    for (uint32_t j = 0; j < N; ++j) bits[j] = static_cast<const uint32_t *>(W.y)[static_cast<size_t>(tok0 + min(first + j * step, live - 1u)) * W.ldy + row];
+  } else {
+#pragma unroll
+    for (uint32_t j = 0; j < N; ++j) bits[j] = static_cast<const uint16_t *>(W.y)[static_cast<size_t>(tok0 + min(first + j * step, live - 1u)) * W.ldy + row];
   }
 }
 __device__ __forceinline__ void a16_store_swiglu(const A16Weight &W, size_t at, float acc_g, float acc_u, float coef) {
@@ -363,25 +377,33 @@ __global__ void __launch_bounds__(kA16Threads, 1) nvfp4_a16_mma_kernel(const __g
     if (!have && lane == 0) atomicOr(&g_a16_status, kEpilogueTimeout);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   }
-  auto store = [&](uint32_t token, float va, float vb) {
-    const size_t at = static_cast<size_t>(token) * W.ldy;
-    if (swiglu) {
-      a16_store_swiglu(W, at + row_a, va, vb, coef);
-    } else {
-      a16_store(W, p.epilogue, at + row_a, va, coef);
-      if (TILES == 2) a16_store(W, p.epilogue, at + row_b, vb, coef);
-    }
-  };
   if (kc == 1u) {
     if (warp < kDecoders && have) {
       for (uint32_t c = group * 16u; c < p.bn && tok0 + c < p.tokens; c += kGroups * 16u) {
-        uint32_t v[16], u[16];
+        uint32_t v[16], u[16], old[16] = {};
         tmem_ld16(lane_base + c, v);
         if (TILES == 2) tmem_ld16(lane_base + p.acc_stride + c, u);
+        a16_residuals(old, W, p.epilogue, row_a, tok0, c, 1u, live);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (swiglu) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            if (tok0 + c + j < p.tokens) {
+              a16_store_swiglu(W, static_cast<size_t>(tok0 + c + j) * W.ldy + row_a, __uint_as_float(v[j]), TILES == 2 ? __uint_as_float(u[j]) : 0.0f, coef);
+            }
+          }
+          continue;
+        }
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-          if (tok0 + c + j < p.tokens) store(tok0 + c + j, __uint_as_float(v[j]), TILES == 2 ? __uint_as_float(u[j]) : 0.0f);
+          if (tok0 + c + j < p.tokens) a16_store(W, p.epilogue, static_cast<size_t>(tok0 + c + j) * W.ldy + row_a, __uint_as_float(v[j]), coef, old[j]);
+        }
+        if (TILES == 2) {
+          a16_residuals(old, W, p.epilogue, row_b, tok0, c, 1u, live);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            if (tok0 + c + j < p.tokens) a16_store(W, p.epilogue, static_cast<size_t>(tok0 + c + j) * W.ldy + row_b, __uint_as_float(u[j]), coef, old[j]);
+          }
         }
       }
     }
@@ -389,6 +411,14 @@ __global__ void __launch_bounds__(kA16Threads, 1) nvfp4_a16_mma_kernel(const __g
     // Token tl of the tile is finished by rank tl % kc: once every ring of the cluster is idle, every CTA pushes its sums of
     // it over that rank's rings, [sender][turn][tile][128 rows], and the bytes count at the receiver's barrier. Nobody reads
     // another CTA's memory, so nobody waits for a reader before it leaves.
+    constexpr uint32_t kAtOnce = 4;   // tokens of a group whose residuals are requested together, the first before the sums are here
+    uint32_t old_a[kAtOnce] = {}, old_b[kAtOnce] = {};
+    auto residuals = [&](uint32_t i) {
+      a16_residuals(old_a, W, p.epilogue, row_a, tok0, i * kc + rank, kGroups * kc, live);
+      if (TILES == 2 && !swiglu) a16_residuals(old_b, W, p.epilogue, row_b, tok0, i * kc + rank, kGroups * kc, live);
+    };
+    if (warp < kDecoders) residuals(group);
+    __syncwarp();
     cluster_sync_all();
     const uint32_t turns = (live + kc - 1u) / kc;
     if (warp < kDecoders) {
@@ -412,14 +442,26 @@ __global__ void __launch_bounds__(kA16Threads, 1) nvfp4_a16_mma_kernel(const __g
       }
       if (mbar_wait_pushed(bar_sums)) {
         const float *sums = reinterpret_cast<const float *>(base_ptr) + r;
-        for (uint32_t i = group; i * kc + rank < live; i += kGroups) {
-          float sum_a = 0.0f, sum_b = 0.0f;
-          for (uint32_t q = 0; q < kc; ++q) {   // in rank order
-            const float *from = sums + (q * turns + i) * TILES * 128u;
-            sum_a = q == 0u ? from[0] : sum_a + from[0];
-            if (TILES == 2) sum_b = q == 0u ? from[128] : sum_b + from[128];
+        for (uint32_t first = group; first * kc + rank < live; first += kAtOnce * kGroups) {
+          if (first != group) residuals(first);
+#pragma unroll
+          for (uint32_t b = 0; b < kAtOnce; ++b) {
+            const uint32_t i = first + b * kGroups;
+            if (i * kc + rank >= live) break;
+            float sum_a = 0.0f, sum_b = 0.0f;
+            for (uint32_t q = 0; q < kc; ++q) {   // in rank order
+              const float *from = sums + (q * turns + i) * TILES * 128u;
+              sum_a = q == 0u ? from[0] : sum_a + from[0];
+              if (TILES == 2) sum_b = q == 0u ? from[128] : sum_b + from[128];
+            }
+            const size_t at = static_cast<size_t>(tok0 + i * kc + rank) * W.ldy;
+            if (swiglu) {
+              a16_store_swiglu(W, at + row_a, sum_a, sum_b, coef);
+            } else {
+              a16_store(W, p.epilogue, at + row_a, sum_a, coef, old_a[b]);
+              if (TILES == 2) a16_store(W, p.epilogue, at + row_b, sum_b, coef, old_b[b]);
+            }
           }
-          store(tok0 + i * kc + rank, sum_a, sum_b);
         }
       } else if (lane == 0) {
         atomicOr(&g_a16_status, kReduceTimeout);

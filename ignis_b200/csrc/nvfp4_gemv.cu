@@ -625,14 +625,30 @@ __global__ void __launch_bounds__(kThreads, NT <= 2 ? 2 : 1) nvfp4_gemv_kernel(c
       }
   }
   const float coef = W.inv_dw * 128.0f;  // the operands carried 2^-7
+  const bool add = (p.epilogue & kEpilogueAdd) != 0u, f32 = (p.epilogue & kEpilogueF32) != 0u;
   bool landed = false;
   for (uint32_t turn = static_cast<uint32_t>(warp), f = rank + kc * turn; f < items; turn += kWarps, f += kc * kWarps) {
+    const uint32_t og = f / (2 * NT), a = (f / NT) & 1, tt = f % NT;
+    const uint32_t og_group = swiglu ? row_block * out_groups + og : row_block * rm + og;
+    const uint32_t og_limit = swiglu ? groups_total / 2u : groups_total;
+    const uint32_t out_row = (og_group >> 2) * 128u + (og_group & 3u) * 8u + g + 64u * a;  // q = 2a, 2a + 1
+    const uint32_t tok0 = tt * 8 + 2 * t;
+    // what a residual add finds, as the stored type's bits: the four values together, and ahead of the wait for the sums (a
+    // token past the last: the last)
+    uint32_t old[4] = {};
+    auto request = [&](const void *y) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const size_t at = static_cast<size_t>(min(tok0 + (e & 1), p.tokens - 1u)) * W.ldy + out_row + (e >> 1) * 32u;
+        old[e] = f32 ? static_cast<const uint32_t *>(y)[at] : static_cast<const uint16_t *>(y)[at];
+      }
+    };
+    if (add && og_group < og_limit) request(W.y[0]);
     if (!landed && !(landed = mbar_wait_pushed(bar_sums))) {
       if (lane == 0) atomicOr(&g_gemv_status, kSumsTimeout);
       break;
     }
     if (turn == static_cast<uint32_t>(warp)) GEMV_TRACE(6);
-    const uint32_t og = f / (2 * NT), a = (f / NT) & 1, tt = f % NT;
     float4 sum = make_float4(0.f, 0.f, 0.f, 0.f), sum_up = make_float4(0.f, 0.f, 0.f, 0.f);
     for (uint32_t r = 0; r < kc; ++r) {   // in rank order
       const float4 *from = part + (turn * kc + r) * sides * 32u + lane;
@@ -643,32 +659,25 @@ __global__ void __launch_bounds__(kThreads, NT <= 2 ? 2 : 1) nvfp4_gemv_kernel(c
         sum_up.x += u.x; sum_up.y += u.y; sum_up.z += u.z; sum_up.w += u.w;
       }
     }
-    const uint32_t og_group = swiglu ? row_block * out_groups + og : row_block * rm + og;
-    const uint32_t og_limit = swiglu ? groups_total / 2u : groups_total;
     if (og_group >= og_limit) continue;
-    const uint32_t out_row = (og_group >> 2) * 128u + (og_group & 3u) * 8u + g + 64u * a;  // q = 2a, 2a + 1
-    const uint32_t tok0 = tt * 8 + 2 * t;
     float v[4] = {sum.x * coef, sum.y * coef, sum.z * coef, sum.w * coef};
     if (swiglu) {
       const float u[4] = {sum_up.x * coef, sum_up.y * coef, sum_up.z * coef, sum_up.w * coef};
 #pragma unroll
       for (int e = 0; e < 4; ++e) v[e] = silu_f32(v[e]) * u[e];
     }
+    // one buffer, or the same value into every rank's buffer (peer stores over NVLink)
+    for (uint32_t pp = 0; pp < W.peers; ++pp) {
+      if (add && pp != 0u) request(W.y[pp]);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const uint32_t tok = tok0 + (e & 1);
-      const uint32_t row = out_row + (e >> 1) * 32u;
-      if (tok >= p.tokens) continue;
-      const size_t at = static_cast<size_t>(tok) * W.ldy + row;
-      // one buffer, or the same value into every rank's buffer (peer stores over NVLink)
-      for (uint32_t pp = 0; pp < W.peers; ++pp) {
-        if (p.epilogue & kEpilogueF32) {
-          float *y = static_cast<float *>(W.y[pp]);
-          y[at] = (p.epilogue & kEpilogueAdd) ? y[at] + v[e] : v[e];
+      for (int e = 0; e < 4; ++e) {
+        const uint32_t tok = tok0 + (e & 1);
+        if (tok >= p.tokens) continue;
+        const size_t at = static_cast<size_t>(tok) * W.ldy + out_row + (e >> 1) * 32u;
+        if (f32) {
+          static_cast<float *>(W.y[pp])[at] = add ? __uint_as_float(old[e]) + v[e] : v[e];
         } else {
-          __nv_bfloat16 *y = static_cast<__nv_bfloat16 *>(W.y[pp]);
-          const float r = (p.epilogue & kEpilogueAdd) ? v[e] + __bfloat162float(y[at]) : v[e];
-          y[at] = __float2bfloat16_rn(r);
+          static_cast<__nv_bfloat16 *>(W.y[pp])[at] = __float2bfloat16_rn(add ? v[e] + __uint_as_float(old[e] << 16) : v[e]);
         }
       }
     }
