@@ -24,6 +24,7 @@
 
 #include "nvfp4_internal.cuh"
 #include "nvfp4_tc.cuh"
+#include "w4a4_pair_control.h"
 
 #include <cmath>
 #include <mutex>
@@ -244,10 +245,9 @@ __device__ __forceinline__ void w4a4_epilogue_tile(const W4A4Params &p, const W4
 // its commits arrive at both CTAs' barriers (two plain commits, one per CTA). The scale tiles
 // travel as TMA tiles too (a bulk copy cannot report to the peer's barrier): the scale planes as
 // [tile][128] words.
-constexpr int kPairStages = 5;
 constexpr uint32_t kPairBBytes = 128 * kBKBytes;                                   // this CTA's half of the weight rows
 constexpr uint32_t kPairStageBytes = kABytes + kPairBBytes + kSfaBytes + 2 * 2048;  // + token scales + both halves' weight scales
-constexpr uint32_t kPairSmemBytes = kPairStages * kPairStageBytes + 256 + 1024;
+constexpr uint32_t kPairSmemBytes = kPairStages * kPairStageBytes + kPairControlBytes + 1024;
 constexpr uint32_t kPairSfCols = 48;  // per stage: 16 columns of token scales, 32 of weight scales
 // The shared::cluster address of this CTA's `addr` in the cluster's CTA `rank`.
 __device__ __forceinline__ uint32_t in_cta(uint32_t addr, uint32_t rank) {
@@ -290,11 +290,10 @@ __global__ void __launch_bounds__(256, 1) w4a4_gemm_pair_kernel(const __grid_con
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;   // the same offset in both CTAs: they run the same kernel
   uint8_t *base_ptr = smem_raw + (base - raw);
-  // barriers: full[5], empty[5], accumulator full, accumulator empty; then the tensor-memory slot
-  const uint32_t bars = base + kStages * kPairStageBytes;
-  const uint32_t bar_acc_full = bars + 8 * 2 * kStages, bar_acc_empty = bar_acc_full + 8;
-  const uint32_t bar_sf_ready = bar_acc_empty + 8;   // [5], the first CTA's: a stage's scales are in both CTAs' tensor memory
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(base_ptr + kStages * kPairStageBytes + 128);
+  const uint32_t control = base + kStages * kPairStageBytes;   // barriers and the tensor-memory slot (PairControl)
+  const uint32_t bars = control + kPairFull, bars_empty = control + kPairEmpty;
+  const uint32_t bar_acc_full = control + kPairAccFull, bar_acc_empty = control + kPairAccEmpty, bar_sf_ready = control + kPairSfReady;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(base_ptr + kStages * kPairStageBytes + kPairTmemSlot);
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();        // 0: the pair's first CTA, which issues the MMAs
   const uint32_t k_iters = p.k / 256u, k_atoms = p.k / 64u;
@@ -306,7 +305,7 @@ __global__ void __launch_bounds__(256, 1) w4a4_gemm_pair_kernel(const __grid_con
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(bars + 8 * s, 1);               // the first CTA's: its producer's expect_tx arrival (the bytes of both CTAs)
-      mbar_init(bars + 8 * (kStages + s), 1);   // one commit
+      mbar_init(bars_empty + 8 * s, 1);         // one commit
     }
     mbar_init(bar_acc_full, 1);
     mbar_init(bar_acc_empty, 8);                // the first CTA's: one arrival per epilogue warp of the pair
@@ -340,7 +339,7 @@ __global__ void __launch_bounds__(256, 1) w4a4_gemm_pair_kernel(const __grid_con
       const int32_t row = static_cast<int32_t>(rank == 0u ? row_a : row_b);
       const uint32_t sfa0 = m_tile * k_atoms, sfb0 = row_a / 128u * k_atoms, sfb1 = row_b / 128u * k_atoms;
       for (uint32_t it = 0; it < k_iters; ++it, at.advance(1u, kStages)) {
-        if (!mbar_wait(bars + 8 * (kStages + at.slot), at.phase ^ 1u)) {
+        if (!mbar_wait(bars_empty + 8 * at.slot, at.phase ^ 1u)) {
           if (lane == 0) atomicOr(p.status, kStatusProducerTimeout);
           ok = false;
           break;
@@ -361,7 +360,7 @@ __global__ void __launch_bounds__(256, 1) w4a4_gemm_pair_kernel(const __grid_con
     // ---- MMA issuer of the pair: M 256 (128 per CTA), N 256, K 64 ----
     if (rank == 0u) {
       const uint32_t idesc = (1u << 7) | (1u << 10) | ((kBN >> 3) << 17) | ((256u >> 4) << 24);
-      const uint32_t own_empty = in_cta(bars + 8 * kStages, 0u), peer_empty = in_cta(bars + 8 * kStages, 1u);
+      const uint32_t own_empty = in_cta(bars_empty, 0u), peer_empty = in_cta(bars_empty, 1u);
       const uint32_t own_acc = in_cta(bar_acc_full, 0u), peer_acc = in_cta(bar_acc_full, 1u);
       const uint64_t desc0 = smem_desc(base, 1024u, 2u);
       RingAt at;

@@ -135,3 +135,37 @@ def test_moe_geometry_is_an_argument_and_the_verbatim_entries_keep_a_default():
     finally:
         assert lib.b200q_moe_set_geometry(2560, 640, 512, 10) == 0
     assert C.sizeof(_lib.MoeGeometry) == 16
+
+
+def test_pair_kernel_barriers_and_tensor_memory_slot_lie_apart(tmp_path):
+    """The words behind the W4A4 pair kernel's ring (csrc/w4a4_pair_control.h), as the kernel addresses them: eight-byte barriers
+    on eight-byte boundaries and a four-byte slot, no two of them on one byte and all of them in the bytes that the launch asks for."""
+    import shutil
+    import subprocess
+
+    compiler = shutil.which("g++")
+    if compiler is None:
+        pytest.skip("no host compiler")
+    src = tmp_path / "spans.cpp"
+    src.write_text("""
+#include <cstdio>
+#include "w4a4_pair_control.h"
+using namespace b200q;
+int main() {
+  const struct { const char *name; uint32_t at, bytes; } spans[] = {
+      {"full", kPairFull, 8u * kPairStages},   {"empty", kPairEmpty, 8u * kPairStages},       {"acc_full", kPairAccFull, 8u},
+      {"acc_empty", kPairAccEmpty, 8u},        {"sf_ready", kPairSfReady, 8u * kPairStages},  {"tmem_slot", kPairTmemSlot, 4u}};
+  for (const auto &s : spans) std::printf("%s %u %u\\n", s.name, s.at, s.bytes);
+  std::printf("end %u 0\\n", kPairControlBytes);
+}
+""")
+    exe = str(tmp_path / "spans")
+    subprocess.run([compiler, "-std=c++17", "-Wall", "-Werror", f"-I{os.path.join(ROOT, 'ignis_b200', 'csrc')}", str(src), "-o", exe], check=True)
+    spans = [(name, int(at), int(n)) for name, at, n in (line.split() for line in subprocess.check_output([exe], text=True).splitlines())]
+    end = dict((name, at) for name, at, _ in spans)["end"]
+    used = {}
+    for name, at, n in spans[:-1]:
+        assert at % (4 if name == "tmem_slot" else 8) == 0 and at + n <= end, name
+        for byte in range(at, at + n):
+            assert byte not in used, f"{name} and {used[byte]} share byte {byte}"
+            used[byte] = name
