@@ -40,6 +40,7 @@ struct ExpertParams {
 // scale per row, items multiplied with their expert's records by tcgen05.
 int32_t moe_tc_prepare(ErrorSlot &slot);
 constexpr uint32_t kMoeTcItemRows = 192;
+constexpr uint32_t kMoeNarrowTokens = 64;   // calls of up to this many tokens may share an accumulator with others at work
 int32_t moe_tc_experts(ErrorSlot &slot, const DeviceState &dev, const ExpertParams &p, uint32_t rows, uint32_t items_max,
                        const uint32_t *offsets, cudaStream_t stream, const char *what);
 

@@ -198,7 +198,9 @@ __global__ void __launch_bounds__(Shape<2>::kThreads, 2) moe_tc_gemm_kernel(cons
 
 // One CTA per token, several with few tokens: the token's weighted down products (one row per choice that had an expert with a
 // record) become 2^-32 fixed-point integers and are added to the token's accumulator row. Integer
-// sums do not depend on their order: the bits are those of adding every product on its own.
+// sums do not depend on their order: the bits are those of adding every product on its own. SHARED: by atomic additions, so that
+// calls on several streams may add into one accumulator; wide calls read and write the row, whose calls must be ordered.
+template <bool SHARED>
 __global__ void __launch_bounds__(256) moe_tc_fold_kernel(const __grid_constant__ ExpertParams p, uint32_t tokens) {
   griddep_launch_dependents();
   griddep_wait();
@@ -245,7 +247,10 @@ __global__ void __launch_bounds__(256) moe_tc_fold_kernel(const __grid_constant_
     }
     long long *dst = p.acc + static_cast<size_t>(token) * p.hidden + 4u * c4;   // the caller's buffer: 8-byte alignment is all it promises
 #pragma unroll
-    for (int i = 0; i < 4; ++i) dst[i] += sum[i];
+    for (int i = 0; i < 4; ++i) {
+      if (SHARED) atomicAdd(reinterpret_cast<unsigned long long *>(dst + i), static_cast<unsigned long long>(sum[i]));
+      else dst[i] += sum[i];
+    }
   }
   if (range) atomicOr(p.status, kStatusRange);
 }
@@ -286,7 +291,7 @@ int32_t moe_tc_experts(ErrorSlot &slot, const DeviceState &dev, const ExpertPara
                      : launch(moe_tc_gemm_kernel<1>, grid, dim3(Shape<2>::kThreads), Shape<2>::kSmemBytes, stream, pdl, map_rows, p);
     if (err != cudaSuccess) return fail(slot, "%s: expert launch failed: %s", what, cudaGetErrorString(err));
   }
-  const cudaError_t err = launch(moe_tc_fold_kernel, dim3(tokens, tokens < static_cast<uint32_t>(dev.sm_count) ? (p.hidden + 1023u) / 1024u : 1u), dim3(256), 0, stream, pdl, p, tokens);
+  const cudaError_t err = launch(tokens <= kMoeNarrowTokens ? moe_tc_fold_kernel<true> : moe_tc_fold_kernel<false>, dim3(tokens, tokens < static_cast<uint32_t>(dev.sm_count) ? (p.hidden + 1023u) / 1024u : 1u), dim3(256), 0, stream, pdl, p, tokens);
   if (err != cudaSuccess) return fail(slot, "%s: fold launch failed: %s", what, cudaGetErrorString(err));
   return 0;
 }

@@ -235,6 +235,31 @@ def test_two_geometries_side_by_side(mo, oracle):
         check_tokens(first[: x.shape[0]], routed_reference(oracle, rec, x, ids, w, g.hidden))
 
 
+@pytest.mark.parametrize("tokens", [1, 8, 64])
+def test_narrow_calls_on_two_streams_add_into_one_accumulator(mo, oracle, tokens):
+    """Calls of up to 64 tokens add atomically: two streams with workspaces of their own and one accumulator leave exactly the sum
+    of all their calls, whatever their order."""
+    hidden, inter, experts, top_k, calls = 512, 128, 8, 2, 40
+    mo.set_geometry(hidden, inter, experts, top_k)
+    rng = np.random.default_rng(tokens)
+    rec = Records(mo, oracle, rng, hidden, inter, experts)
+    x = (torch.randn(tokens, hidden, generator=torch.Generator().manual_seed(tokens)) * 0.5).to(torch.bfloat16).cuda()
+    ids, w = (torch.from_numpy(v).cuda() for v in make_routing(rng, tokens, experts, top_k))
+    spaces = [mo.Workspace(min(8, tokens), tokens) for _ in range(2)]
+    one = mo.experts_prefill(x, ids, w, rec.table, spaces[0]).clone()
+    spaces[0].acc.zero_()
+    spaces[1].acc = spaces[0].acc
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    for _ in range(calls):
+        for stream, ws in zip(streams, spaces):
+            with torch.cuda.stream(stream):
+                mo.experts_prefill(x, ids, w, rec.table, ws)
+    torch.cuda.synchronize()
+    assert all(ws.status() == 0 for ws in spaces)
+    assert torch.equal(spaces[0].acc, 2 * calls * one)
+
+
 def test_absent_records_and_bad_ids_are_skipped_and_reported(mo, oracle):
     mo.set_geometry(256, 128, 8, 2)
     rng = np.random.default_rng(5)
