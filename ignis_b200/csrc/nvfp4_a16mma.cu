@@ -485,6 +485,10 @@ struct A16Plan {
 };
 
 size_t a16_ring_bytes(const A16Plan &pl) { return static_cast<size_t>(pl.x_stages) * pl.bn * 128u + static_cast<size_t>(pl.raws) * pl.tiles * kRawTileBytes; }
+// What the CTAs of a cluster push to one of them lies over the rings: the tile's tokens in whole turns of the cluster, whose
+// ranks finish one each.
+constexpr size_t a16_sums_bytes(uint32_t tiles, uint32_t tokens, uint32_t kc) { return static_cast<size_t>(tiles) * ((tokens + kc - 1u) / kc * kc) * 512u; }
+static_assert(a16_sums_bytes(1u, 16u, 3u) == 18u * 512u && a16_sums_bytes(2u, 16u, 8u) == 32u * 512u, "whole turns");
 size_t a16_smem_bytes(const A16Plan &pl) { return a16_ring_bytes(pl) + 16u * (pl.a_slots + pl.x_stages + pl.raws) + 48u + 1024u; }
 
 // Columns of tensor memory: the accumulators, then as many pieces of decoded weights as fit, up to four stages; half ones
@@ -537,7 +541,8 @@ A16Plan a16_plan(const DeviceState &dev, uint32_t row_tiles, uint32_t k_stages, 
       if (!a16_rings(pl)) continue;
       const uint32_t token_tiles = (tokens + pl.bn - 1u) / pl.bn, blocks = tiles == 2u && !swiglu ? row_tiles / 2u : row_tiles;
       for (uint32_t kc = 1; kc <= 8u; ++kc) {
-        if (kc > 1u && (k_stages / kc < 8u || static_cast<size_t>(tiles) * pl.bn * 512u > a16_ring_bytes(pl))) break;
+        if (kc > 1u && k_stages / kc < 8u) break;
+        if (kc > 1u && a16_sums_bytes(tiles, pl.bn, kc) > a16_ring_bytes(pl)) continue;
         const double ctas = static_cast<double>(blocks) * token_tiles * kc, sms = dev.sm_count;
         const double waves = ceil(ctas / (kc <= 2u ? sms : sms * (kc <= 4u ? 0.89 : 0.87)));   // wide clusters leave some SMs out
         const double decode = tiles * 380.0, mma = tiles * 2.46 * pl.bn, load = (pl.bn * 128.0 + tiles * 4608.0) / 61.0;

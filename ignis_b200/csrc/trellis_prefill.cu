@@ -104,9 +104,6 @@ uint64_t trellis_tc_workspace_bytes(uint32_t in, uint32_t weights, uint32_t toke
 }
 
 namespace {
-// The CTAs of a cluster that share the K stages of an item.
-constexpr uint32_t kMaxRanks = 8;
-
 cudaLaunchConfig_t dense_config(bool wide, uint32_t items, uint32_t ranks, cudaStream_t stream, bool pdl, cudaLaunchAttribute (&attr)[2]) {
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(items * ranks);

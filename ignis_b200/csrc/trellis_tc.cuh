@@ -39,6 +39,7 @@ using namespace trellis_dev;
 
 constexpr uint32_t kStageCols = 32;                // tensor-memory columns of a decoded stage: 128 lanes x 64 fp16
 constexpr uint32_t kMaxStages = 8;
+constexpr uint32_t kMaxRanks = 8;                  // the CTAs of a cluster that share the K stages of an item
 
 // Two shapes of the CTA, by its groups of four decoder warps (which run the epilogue too). Two groups: up to 192 rows, half of
 // an SM, so that one CTA's setup, fill and epilogue run under the other's decoding. Four: up to 384 rows, so that a decoded
@@ -52,7 +53,7 @@ struct Shape {
   static constexpr uint32_t kRingBytes = (GROUPS == 2 ? 110 : 212) * 1024;
   static constexpr uint32_t kWordBytes = (GROUPS == 2 ? 36 : 48) * 1024;  // of them for packed words, at most
   static constexpr uint32_t kSmemBytes = kRingBytes + 8u * (2u * (2u * kMaxStages + 4u) + 2u) + 16u + 1024u;   // + barriers, the tensor-memory slot, alignment slack
-  static_assert(kMaxRows * 512u <= kRingBytes, "the epilogue's sums fit into the rings");
+  static_assert((kMaxRows + kMaxRanks - 1u) * 512u <= kRingBytes, "the epilogue's sums fit into the rings, in whole turns of a cluster");
 };
 constexpr uint32_t kStatusProducer = 1u, kStatusMma = 2u, kStatusEpilogue = 4u, kStatusDecoder = 8u;
 
