@@ -27,12 +27,14 @@ using Geometry = b200q_moe_geometry;
 // compiles it in; here it starts at the reference's and b200q_moe_set_geometry replaces it.
 Geometry g_default = {IGNIS_MOE_HIDDEN, IGNIS_MOE_INTERMEDIATE, IGNIS_MOE_EXPERTS, IGNIS_MOE_TOP_K};
 
+constexpr uint32_t kMaxExperts = 4096;
+
 int32_t check_geometry(ErrorSlot &slot, const Geometry *g, const char *what) {
   if (g == nullptr) return fail(slot, "%s: geometry is NULL", what);
   if (g->hidden == 0 || (g->hidden % 128u) != 0 || g->inter == 0 || (g->inter % 128u) != 0) {
     return fail(slot, "%s: hidden and inter must be positive multiples of 128", what);
   }
-  if (g->experts == 0 || g->experts > 4096u || g->top_k == 0 || g->top_k > 32u || g->top_k > g->experts) {
+  if (g->experts == 0 || g->experts > kMaxExperts || g->top_k == 0 || g->top_k > 32u || g->top_k > g->experts) {
     return fail(slot, "%s: experts must lie in 1..4096 and top_k in 1..min(32, experts)", what);
   }
   if (g->hidden / 128u > 8u * 40u || g->inter / 128u > 8u * 40u) return fail(slot, "%s: dimension too long", what);
@@ -75,18 +77,15 @@ Layout layout_for(const Geometry &g, uint32_t tokens_max) {
 }
 
 // ---- grouping ------------------------------------------------------------------------------
-// A CTA counts in shared memory and adds its counts to the experts' once (`in_shared`: up to kSmallExperts of them): added one
-// by one, a popular expert's rows queue at one address (13 us for 40 960 rows under Zipf routing).
-constexpr uint32_t kSmallRows = 4096, kSmallExperts = 4096;
+// A CTA counts in shared memory and adds its counts to the experts' once: added one by one, a popular expert's rows queue at
+// one address (13 us for 40 960 rows under Zipf routing).
+constexpr uint32_t kSmallRows = 4096;
 
 __global__ void __launch_bounds__(256) moe_count_kernel(const int32_t *ids, uint32_t rows, uint32_t experts,
                                                         uint32_t *counts, uint32_t *status) {
-  __shared__ uint32_t mine[kSmallExperts];
-  const bool in_shared = experts <= kSmallExperts;
-  if (in_shared) {
-    for (uint32_t e = threadIdx.x; e < experts; e += blockDim.x) mine[e] = 0u;
-    __syncthreads();
-  }
+  __shared__ uint32_t mine[kMaxExperts];
+  for (uint32_t e = threadIdx.x; e < experts; e += blockDim.x) mine[e] = 0u;
+  __syncthreads();
   griddep_launch_dependents();
   griddep_wait();
   for (uint32_t a = blockIdx.x * blockDim.x + threadIdx.x; a < rows; a += gridDim.x * blockDim.x) {
@@ -94,10 +93,9 @@ __global__ void __launch_bounds__(256) moe_count_kernel(const int32_t *ids, uint
     if (e < 0 || static_cast<uint32_t>(e) >= experts) {
       if (e != IGNIS_MOE_NO_EXPERT) atomicOr(status, kStatusBadExpert);  // -1 is "no expert for this choice": skipped, not an error
     } else {
-      atomicAdd(in_shared ? &mine[e] : &counts[e], 1u);
+      atomicAdd(&mine[e], 1u);
     }
   }
-  if (!in_shared) return;
   __syncthreads();
   for (uint32_t e = threadIdx.x; e < experts; e += blockDim.x) {
     if (mine[e] != 0u) atomicAdd(&counts[e], mine[e]);
@@ -147,22 +145,15 @@ __global__ void __launch_bounds__(1024) moe_scan_kernel(const uint32_t *counts, 
 // CTA's rows of an expert take their places together, as they were counted.
 __global__ void __launch_bounds__(256) moe_scatter_kernel(const int32_t *ids, uint32_t rows, uint32_t experts,
                                                           const uint32_t *offsets, uint32_t *cursor, uint32_t *sorted) {
-  __shared__ uint32_t mine[kSmallExperts];   // rows of the CTA, then their first place
-  const bool in_shared = experts <= kSmallExperts;
-  if (in_shared) {
-    for (uint32_t e = threadIdx.x; e < experts; e += blockDim.x) mine[e] = 0u;
-    __syncthreads();
-  }
+  __shared__ uint32_t mine[kMaxExperts];   // rows of the CTA, then their first place
+  for (uint32_t e = threadIdx.x; e < experts; e += blockDim.x) mine[e] = 0u;
+  __syncthreads();
   griddep_launch_dependents();
   griddep_wait();
   for (uint32_t a0 = blockIdx.x * blockDim.x; a0 < rows; a0 += gridDim.x * blockDim.x) {
     const uint32_t a = a0 + threadIdx.x;
     const int32_t e = a < rows ? ids[a] : -1;
     const bool there = e >= 0 && static_cast<uint32_t>(e) < experts;
-    if (!in_shared) {
-      if (there) sorted[offsets[e] + atomicAdd(&cursor[e], 1u)] = a;
-      continue;
-    }
     const uint32_t rank = there ? atomicAdd(&mine[e], 1u) : 0u;
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < experts; i += blockDim.x) {
@@ -183,7 +174,7 @@ __global__ void __launch_bounds__(1024) moe_group_small_kernel(const int32_t *id
                                                                uint32_t *sorted, uint32_t *status) {
   griddep_launch_dependents();
   griddep_wait();
-  __shared__ uint32_t counts[kSmallExperts], start[kSmallExperts];
+  __shared__ uint32_t counts[kMaxExperts], start[kMaxExperts];
   __shared__ uint32_t row_sum[1024], item_sum[1024];
   for (uint32_t e = threadIdx.x; e < experts; e += 1024) counts[e] = 0u;
   __syncthreads();
@@ -353,7 +344,7 @@ int32_t run_experts(const Geometry &g, const void *x, uint32_t tokens, const int
   uint32_t *status = reinterpret_cast<uint32_t *>(base + l.status);
   const bool pdl = dev->pdl != 0;
   cudaError_t err = cudaSuccess;
-  if (rows <= kSmallRows && g.experts <= kSmallExperts) {
+  if (rows <= kSmallRows) {
     err = launch(moe_group_small_kernel, dim3(1), dim3(1024), 0, stream, pdl, ids, rows, g.experts, kMoeTcItemRows, offsets, n_items, items,
                  sorted, status);
     if (err != cudaSuccess) return fail(slot, "%s: grouping launch failed: %s", what, cudaGetErrorString(err));
