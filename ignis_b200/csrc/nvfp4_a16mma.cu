@@ -120,13 +120,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&r)[16]
                  "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
                : "memory");
 }
-// kind::f16 with A in tensor memory: row r in lane r, two values of K a column.
-__device__ __forceinline__ void mma_f16_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{ .reg .pred p; setp.ne.u32 p, %4, 0;\n"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p; }"
-               ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
-               : "memory");
-}
 
 // `coef`: the weight's inverse divisor times what the A tiles leave out.
 // `bits`: what the residual add found there, as the stored type's bits.

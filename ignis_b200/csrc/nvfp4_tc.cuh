@@ -209,6 +209,14 @@ __device__ __forceinline__ float ld_cluster_f32(const float *local_smem, uint32_
   return v;
 }
 
+// kind::f16 with A in tensor memory: row r in lane r, two values of K a column.
+__device__ __forceinline__ void mma_f16_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{ .reg .pred p; setp.ne.u32 p, %4, 0;\n"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p; }"
+               ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
+               : "memory");
+}
+
 // The address of this CTA's shared-memory address `local` in CTA `rank` of the cluster, and a store there that
 // counts its bytes at an mbarrier of the same CTA.
 __device__ __forceinline__ uint32_t cluster_map(uint32_t local, uint32_t rank) {

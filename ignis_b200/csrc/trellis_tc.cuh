@@ -156,13 +156,6 @@ __device__ __forceinline__ void tmem_st_16x128b_x4(uint32_t addr, const uint32_t
                ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                : "memory");
 }
-// kind::f16 with A in tensor memory: row r in lane r, two values of K a column.
-__device__ __forceinline__ void mma_f16_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{ .reg .pred p; setp.ne.u32 p, %4, 0;\n"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p; }"
-               ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
-               : "memory");
-}
 
 // The decoder warps' loop: group g (warp / 4) takes the job's stages g, g + GROUPS, ...; warp w of it the tile columns 2 w and
 // 2 w + 1 of the block, whose values are lanes 32 w .. + 31 of the MMA's A operand.
