@@ -402,14 +402,16 @@ def test_tensor_core_route_at_every_bit_width_and_on_column_views(tr, oracle, k2
     assert torch.equal(yv, y[:, 128:640])
 
 
-@pytest.mark.parametrize("tokens", [100, 333])   # one row tile (a warp group per half block) and ragged row-tile pairs
-def test_both_shapes_of_the_tensor_core_route_give_the_same_bits(tr, oracle, tokens):
-    """The wide-token route in its default shape (eight decoder warps, 128 columns a CTA, two CTAs per
-    SM) and in the other (sixteen, 256 columns, one per SM): every output element is the same sum in
-    the same order, so the outputs are equal bit for bit; the first is held to the oracle."""
+@pytest.mark.parametrize("tokens", [100, 333])   # one row tile and several, their last one ragged
+@pytest.mark.parametrize("in_", [448, 768])      # too short for a split of K, and split by the plan
+def test_both_shapes_of_the_tensor_core_route(tr, oracle, monkeypatch, tokens, in_):
+    """The wide-token route forced to each of its shapes: two groups of decoder warps, up to 192 rows a CTA and two CTAs per SM; four
+    groups, up to 384 rows, one per SM. Both are held to the oracle. Where K is not split, every output is the same sum in the same
+    order whatever the shape, and the bits are equal; ranks that share K add up partial sums, and the shapes may have different
+    numbers of them."""
     from oracle import oracle as orc
 
-    in_, out, k2 = 768, 640, 6
+    out, k2 = 640, 6
     rng = np.random.default_rng(tokens)
     words = oracle.hash_trellis_words(5200 + tokens, in_, out, k2)
     suh, svh = make_scales(rng, in_, 0.05), make_scales(rng, out, 0.03)
@@ -418,18 +420,20 @@ def test_both_shapes_of_the_tensor_core_route_give_the_same_bits(tr, oracle, tok
     x = torch.randn(tokens, in_, generator=torch.Generator().manual_seed(tokens)).to(torch.bfloat16)
     ref, s = orc.trellis_project_rows(inner, suh, svh, x.double().numpy())
     ws = tr.WorkspaceBuffer(tr.workspace_bytes(in_, out, 1, tokens))
-    y = tr.linear(w, x.cuda(), workspace=ws)
-    got = y.float().cpu().numpy().astype(np.float64)
-    assert (np.abs(got - ref) <= 2.0 ** -8 * np.abs(ref) + 2.0 ** -9 * s).all()
-    os.environ["B200Q_TRELLIS_TC_SHAPE"] = "16"
+    outputs = []
     try:
-        tr.prepare()
-        y16 = tr.linear(w, x.cuda(), workspace=ws)
-        assert tr.device_status() == 0
-        assert torch.equal(y16, y)
+        for shape in ("8", "16"):
+            monkeypatch.setenv("B200Q_TRELLIS_TC_SHAPE", shape)
+            tr.prepare()
+            outputs.append(tr.linear(w, x.cuda(), workspace=ws))
+            assert tr.device_status() == 0
     finally:
-        os.environ.pop("B200Q_TRELLIS_TC_SHAPE", None)
+        monkeypatch.undo()
         tr.prepare()
+    for y in outputs:
+        check_linear(y, ref, s)
+    if in_ // 64 < 8:
+        assert torch.equal(*outputs)
 
 
 @pytest.mark.parametrize("shape", ["8", "16"])
