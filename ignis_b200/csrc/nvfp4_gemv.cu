@@ -1,5 +1,7 @@
 // NVFP4 decode route: y[t][r] = sum_k w[r][k] x[t][k] for 1..32 tokens, the weights streamed from
-// HBM exactly once for all tokens. One kernel per call, no workspace.
+// HBM exactly once for all tokens. One kernel per call, no workspace. Calls of more than one token tile (8)
+// come here from the gather entry, and where B200Q_A16_MMA is 0 or the shape is not the tensor-core kernel's
+// (decode_route, nvfp4_api.cu).
 //
 // Stands where the reference runs nvfp4_gemv_kernel (T = 1) and nvfp4_small_t_kernel (T = 2..32)
 // (kernel/vendor/src/ops/linear/nvfp4/nvfp4_gemv.cuh:199, nvfp4_small_t.cuh:211-377) under the A16

@@ -1,5 +1,5 @@
-// NVFP4 W4A4 products of calls with few tokens - from 33, up to 128 in a 27B-style layer: the rule and what both kernels
-// measured stand at narrow_is_cheaper, nvfp4_w4a4.cu - over activations already quantized in the operand
+// NVFP4 W4A4 products of calls with few tokens - from 33 to some hundreds, by the weights' sizes: the rule and what both
+// kernels measured stand at narrow_is_cheaper, nvfp4_w4a4.cu - over activations already quantized in the operand
 // layout (nvfp4_w4a4.cu's quantizer): out[t][r] = bf16(alpha * sum_k E2M1(a) E4M3(sa) E2M1(w) E4M3(sw)).
 // The pair GEMM's 256 x 256 tiles leave most of the device idle there - 20 tiles for a 5120-row weight
 // on 74 CTA pairs, each walking all of K - while the weights still bound the call: 48 to 100 MB of them.
