@@ -500,8 +500,8 @@ struct QuantTarget {
 
 // Which kernel a product takes: the cheaper by a model of each, in SM cycles, fitted to products whose weights come from HBM.
 // The pair kernel: waves of 256 x 256 tiles on half as many pairs as SMs, 820 cycles a stage of 256 and 3000 a tile (a gate|up
-// parent, whose epilogue multiplies, rounds and quantizes: 8600, and 47 500 a launch), never faster than the weights
-// come from HBM; `w4a4_narrow_cycles` beside its kernel. The narrow kernel has to be ahead by 15 %: where the models are that
+// parent, whose epilogue multiplies, rounds and quantizes: 8600, and 47 500 a launch, a fit whose cause has not been taken
+// apart), never faster than the weights come from HBM; `w4a4_narrow_cycles` beside its kernel. The narrow kernel has to be ahead by 15 %: where the models are that
 // close, products on different kernels in a row cost more (200 tokens: gate|up on the pair kernel and down on the narrow one
 // 89 us, both on the narrow one 71, both on the pair kernel 85).
 // Both forced, an MLP with its residual, in us, narrow / pair, the rule's choice last:
