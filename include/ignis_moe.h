@@ -134,6 +134,8 @@ int32_t ignis_moe_plan_bytes(uint32_t decode_tokens, uint32_t prefill_tokens, st
  * ops ADD into it). Decode: 1..workspace->decode_tokens tokens; prefill: 1..prefill_tokens.
  * Calls of up to 64 tokens add atomically: several of them, each with a workspace of its own, may add into one `acc` from
  * several streams at once. A call of more tokens reads and writes `acc`: order it against every other call on the same rows.
+ * At every size the rotated inputs of a product are FP16 under one power of two per row, the sums FP32: a value 2^28 or more below
+ * its row's largest keeps fewer than eleven bits, and what it loses, 2^-38 of the largest, lies below the resolution of the sum.
  * reference: ignis_moe.h:185-192 */
 int32_t ignis_moe_experts_decode(const void *x, uint32_t tokens, const int32_t *ids, const float *weights,
                                  const struct ignis_moe_slot *slots, const struct ignis_moe_workspace *workspace,

@@ -168,19 +168,17 @@ def test_config4_geometry_under_zipf_routing(mo, oracle, k2s):
     acc = mo.experts_prefill(x.cuda(), torch.from_numpy(ids).cuda(), torch.from_numpy(w).cuda(), rec.table, ws)
     assert ws.status() == 0
     got = acc[torch.tensor(sample).cuda()].cpu().numpy().astype(np.float64) * 2.0 ** -32
-    # the expert products' other shape (sixteen decoder warps, 256 columns, one CTA per SM): a row's
-    # arithmetic does not depend on the shape, so the accumulators hold the same integers
-    kept = acc.clone()
-    os.environ["B200Q_MOE_TC_WIDE"] = "1"
-    try:
-        mo.prepare()
-        ws.acc.zero_()
-        wide = mo.experts_prefill(x.cuda(), torch.from_numpy(ids).cuda(), torch.from_numpy(w).cuda(), rec.table, ws)
-        assert ws.status() == 0
-        assert torch.equal(wide, kept)
-    finally:
-        os.environ.pop("B200Q_MOE_TC_WIDE", None)
-        mo.prepare()
+    # the same tokens in calls of 150: the hottest expert's rows lie in one item there and in several of 192 here, and a row's
+    # arithmetic does not depend on the item it is in, so the accumulators hold the same integers
+    parts = mo.Workspace(8, 150)
+    for t0 in range(0, tokens, 150):
+        part = slice(t0, min(t0 + 150, tokens))
+        n = part.stop - t0
+        parts.acc.zero_()
+        mo.experts_prefill(x[part].cuda(), torch.from_numpy(ids[part]).cuda(), torch.from_numpy(w[part]).cuda(), rec.table, parts)
+        assert np.bincount(ids[part].reshape(-1), minlength=experts)[hottest] <= 192
+        assert torch.equal(parts.acc[:n], acc[part])
+    assert parts.status() == 0
 
     def one(t):
         x64 = x[t].double().numpy()
@@ -195,18 +193,61 @@ def test_config4_geometry_under_zipf_routing(mo, oracle, k2s):
         l2 = np.linalg.norm(got[i] - ref[i]) / np.linalg.norm(ref[i])
         linf = np.abs(got[i] - ref[i]).max() / np.abs(ref[i]).max()
         assert l2 <= 2e-3 and linf <= 1e-2, (t, l2, linf)
-    # the decode entry on eight of the sampled tokens: other kernels (warp-level MMAs, a scale per
-    # 128 inputs), the same fp64 reference and bars
-    eight = torch.tensor(sample[:8])
-    ws8 = mo.Workspace(8, 8)
-    dec = mo.experts_decode(x[eight].cuda(), torch.from_numpy(ids)[eight].cuda(), torch.from_numpy(w)[eight].cuda(), rec.table, ws8)
-    assert ws8.status() == 0
-    check_tokens(dec[:8], ref[:8])
-    # 40 tokens take the warp-level prefill kernels (items of 64 rows): the decode entry's bits
-    few = torch.tensor(sample[:40])
-    ws40 = mo.Workspace(8, 40)
-    pre = mo.experts_prefill(x[few].cuda(), torch.from_numpy(ids)[few].cuda(), torch.from_numpy(w)[few].cuda(), rec.table, ws40)
-    assert torch.equal(pre[:8], dec[:8])
+    # the decode entry on eight of the sampled tokens and a prefill call of 40: grouped by one CTA instead of three launches, the
+    # sums added atomically; the same integers
+    for n, entry in ((8, mo.experts_decode), (40, mo.experts_prefill)):
+        few = torch.tensor(sample[:n])
+        space = mo.Workspace(8, n)
+        narrow = entry(x[few].cuda(), torch.from_numpy(ids)[few].cuda(), torch.from_numpy(w)[few].cuda(), rec.table, space)
+        assert space.status() == 0
+        assert torch.equal(narrow[:n], acc[few.cuda()])
+        check_tokens(narrow[:n], ref[:n])
+
+
+@pytest.mark.parametrize("rows", [191, 192, 193, 385, 4096, 4097])
+def test_items_end_at_192_rows_of_an_expert(mo, oracle, rows):
+    """Every token on one expert: an item short of a row, a full one, one more row, two and one row; grouped by one CTA
+    up to 4096 rows and by three launches beyond. The rows at the items' edges are held to the fp64 reference, all of them to the
+    integers that calls of at most 64 tokens give."""
+    hidden, inter = 256, 128
+    mo.set_geometry(hidden, inter, 3, 1)
+    rng = np.random.default_rng(rows)
+    rec = Records(mo, oracle, rng, hidden, inter, 3)
+    x = (torch.randn(rows, hidden, generator=torch.Generator().manual_seed(rows)) * 0.5).to(torch.bfloat16)
+    ids, w = np.full((rows, 1), 1, np.int32), rng.uniform(0.2, 1.2, (rows, 1)).astype(np.float32)
+    d_x, d_ids, d_w = x.cuda(), torch.from_numpy(ids).cuda(), torch.from_numpy(w).cuda()
+    ws, narrow = mo.Workspace(8, rows), mo.Workspace(8, 64)
+    acc = mo.experts_prefill(d_x, d_ids, d_w, rec.table, ws)
+    for t0 in range(0, rows, 64):
+        n = min(64, rows - t0)
+        narrow.acc.zero_()
+        mo.experts_prefill(d_x[t0:t0 + n], d_ids[t0:t0 + n], d_w[t0:t0 + n], rec.table, narrow)
+        assert torch.equal(narrow.acc[:n], acc[t0:t0 + n])
+    assert ws.status() == 0 and narrow.status() == 0
+    edges = sorted({t for e in range(0, rows + 192, 192) for t in (e - 1, e, e + 1) if 0 <= t < rows} | {rows - 1})
+    check_tokens(acc[torch.tensor(edges).cuda()], routed_reference(oracle, rec, x[edges], ids[edges], w[edges], hidden))
+
+
+@pytest.mark.parametrize("tokens", [3, 40, 150])
+def test_rows_whose_blocks_lie_far_apart(mo, oracle, tokens):
+    """A row has one power of two for all of its inputs, and FP16 then keeps fewer than eleven bits of a value that lies 2^28 below
+    the row's largest. Blocks of 128 inputs up to 2^40 apart, the large one in turn first, in the middle and last: what is lost
+    is at most 2^-38 of the largest input a value, below what the FP32 sums resolve (2^-24 of a sum that holds the largest), so the bars
+    are those of ordinary rows."""
+    hidden, inter, experts, top_k = 640, 256, 8, 2
+    mo.set_geometry(hidden, inter, experts, top_k)
+    rng = np.random.default_rng(tokens)
+    rec = Records(mo, oracle, rng, hidden, inter, experts)
+    x = torch.randn(tokens, hidden, generator=torch.Generator().manual_seed(tokens)) * 0.5
+    for t in range(tokens):
+        for block in range(hidden // 128):
+            x[t, 128 * block:128 * (block + 1)] *= 2.0 ** (-10 * ((block + t) % 5))
+    x = x.to(torch.bfloat16)
+    ids, w = make_routing(rng, tokens, experts, top_k)
+    ws = mo.Workspace(min(8, tokens), tokens)
+    acc = mo.experts_prefill(x.cuda(), torch.from_numpy(ids).cuda(), torch.from_numpy(w).cuda(), rec.table, ws)
+    assert ws.status() == 0
+    check_tokens(acc[:tokens], routed_reference(oracle, rec, x, ids, w, hidden))
 
 
 def test_two_geometries_side_by_side(mo, oracle):
@@ -274,7 +315,7 @@ def test_absent_records_and_bad_ids_are_skipped_and_reported(mo, oracle):
     check_tokens(acc[:3], ref)
 
 
-@pytest.mark.parametrize("tokens", [6, 40, 150])   # one warp per row; warp-level MMAs; tcgen05 with the fold
+@pytest.mark.parametrize("tokens", [6, 40, 150])   # sums added atomically, by several CTAs a token; read and written
 def test_contributions_beyond_the_fixed_point_range_are_skipped_and_reported(mo, oracle, tokens):
     """A weighted contribution of 2^31 or more in magnitude does not fit the 2^-32 fixed-point
     accumulator: it is left out and bit 2 of the status word says so (the reference's rule,
