@@ -403,7 +403,7 @@ def test_tensor_core_route_at_every_bit_width_and_on_column_views(tr, oracle, k2
 
 
 @pytest.mark.parametrize("tokens", [100, 333])   # one row tile and several, their last one ragged
-@pytest.mark.parametrize("in_", [448, 768])      # too short for a split of K, and split by the plan
+@pytest.mark.parametrize("in_", [384, 768])      # too short for a split of K, and split by the plan
 def test_both_shapes_of_the_tensor_core_route(tr, oracle, monkeypatch, tokens, in_):
     """The wide-token route forced to each of its shapes: two groups of decoder warps, up to 192 rows a CTA and two CTAs per SM; four
     groups, up to 384 rows, one per SM. Both are held to the oracle. Where K is not split, every output is the same sum in the same
