@@ -39,6 +39,7 @@ struct DeviceState {
   int sm_count = 0;
   int gemv_slots[9] = {};        // CTAs of the NVFP4 decode kernel
   int a4_slots[9] = {};          // CTAs of the W4A4 decode kernel, one per SM
+  int a16_slots[9] = {};         // CTAs of the A16 tensor-core kernel
   int trellis_clusters[9] = {};  // clusters of the dense trellis tensor-core kernel
   int pdl = 1;           // programmatic dependent launch between the kernels of a call chain
   int gemv_rb = 0;       // B200Q_GEMV_RM: 32-row groups per CTA of the NVFP4 decode kernel (0: auto)

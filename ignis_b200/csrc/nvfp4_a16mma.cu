@@ -537,7 +537,11 @@ A16Plan a16_plan(const DeviceState &dev, uint32_t row_tiles, uint32_t k_stages, 
         if (kc > 1u && k_stages / kc < 8u) break;
         if (kc > 1u && a16_sums_bytes(tiles, pl.bn, kc) > a16_ring_bytes(pl)) continue;
         const double ctas = static_cast<double>(blocks) * token_tiles * kc, sms = dev.sm_count;
-        const double waves = ceil(ctas / (kc <= 2u ? sms : sms * (kc <= 4u ? 0.89 : 0.87)));   // wide clusters leave some SMs out
+        // Clusters are placed inside one GPC, and how many CTAs that leaves room for differs from size to size and from device
+        // to device (135, 132, 130, 132, 105 and 120 of 148 for 3 to 8 on one). With 0.87 of the SMs for the wide ones 16 clusters of 8 were
+        // planned as one wave and ran as two: 4096 x 14336 at 9 tokens 36.9 us, 22.6 here (cold), 2048 x 6144 at 16 20.5 and 14.6,
+        // 1024 x 5120 at 150 22.5 and 16.3.
+        const double waves = ceil(ctas / (dev.a16_slots[kc] > 0 ? dev.a16_slots[kc] : sms * 0.7));
         const double decode = tiles * 380.0, mma = tiles * 2.46 * pl.bn, load = (pl.bn * 128.0 + tiles * 4608.0) / 61.0;
         double stage = 400.0;
         for (const double limit : {decode, mma, load}) stage = stage > limit ? stage : limit;
@@ -563,6 +567,27 @@ int32_t a16mma_prepare(ErrorSlot &slot) {
   if (err == cudaSuccess) err = cudaFuncSetAttribute(nvfp4_a16_mma_kernel<2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
   if (err != cudaSuccess) return fail(slot, "nvfp4 A16 tensor-core kernel attributes: %s", cudaGetErrorString(err));
   if (encode_tiled_fn() == nullptr) return fail(slot, "cuTensorMapEncodeTiled is not available from this driver");
+  DeviceState *dev = device_state(slot);
+  if (dev == nullptr) return -1;
+  for (int kc = 1; kc <= 8 && !dev->counted; ++kc) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(static_cast<unsigned>(kc) * 1024u, 1, 1);
+    config.blockDim = dim3(kA16Threads, 1, 1);
+    config.dynamicSmemBytes = kA16MaxSmem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(kc);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    config.attrs = attr;
+    config.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, nvfp4_a16_mma_kernel<1, 2>, &config) != cudaSuccess) {
+      (void)cudaGetLastError();
+      clusters = 0;
+    }
+    dev->a16_slots[kc] = clusters * kc;
+  }
   return 0;
 }
 
